@@ -49,7 +49,7 @@ __device__ __forceinline__ bool hyb_pass(const LeanCols& lc, const uint32_t (&v)
     bool ok = true;
     #pragma unroll
     for (int c = 0; c < NCOL; ++c) {
-        const uint32_t key = v[c] ^ (((uint32_t)((int32_t)v[c] >> 31) & lc.fm[c]) ^ lc.xm[c]);
+        const uint32_t key = v[c] ^ ((uint32_t)((int32_t)v[c] >> 31) & lc.fm[c]);
         ok &= (key - lc.lo[c]) <= lc.span[c];
     }
     return ok;

@@ -233,9 +233,10 @@ struct LabelCountArgs {
 // label pass with attributes (rj_lean_kernels.cu).
 struct LeanCols {
     int ncol;
+    int nint;                    // uint / int columns come first, then the floats
     const uint2* col[4];         // filter columns, read as value pairs (8-byte aligned)
-    uint32_t lo[4], span[4];     // the predicates of column c hold iff key - lo <= span
-    uint32_t fm[4], xm[4];       // order key = v ^ ((sign(v) & fm) ^ xm)
+    uint32_t lo[4], span[4];     // the predicates of column c hold iff key - lo <= span (mod 2^32)
+    uint32_t fm[4];              // key = v ^ (sign(v) & fm): the value (uint, int), or 2^31-1 for floats
     int aggr;                    // 1: sum the aggregate
     int aggr_ci;                 // the aggregate is filter column aggr_ci, or -1
     const uint2* aggr_col;       // else this column
@@ -291,28 +292,53 @@ struct SplatLeanArgs {
     uint64_t zrow0;
     float4 qbox;
 };
-// Lean point pass over a tiered canvas (rj_tier_lean.cu): one or several
-// canvas tiles, the label form (histogram per polygon) or the canvas form
-// (block and mixed-pixel sums), interval-form filters (LeanCols).
+// Lean point pass of the label form (rj_label_core.cuh): one or several canvas
+// tiles held as 16 x 16-pixel blocks (TierArgs: code, plabel), interval-form
+// filters (LeanCols), count or sum into per-polygon histograms.
+constexpr uint32_t kCellMagic = 0x4B400000u;   // bits of 1.5 * 2^23
+// One axis of a canvas's tiles: all tiles share the scale and the resolution.
+struct TileAxis {
+    const float4* xf;            // [split] (s, t, h, tile extent)
+    int split, res;              // tiles, pixels of a tile
+    float s, H;                  // scale, 256 * half resolution
+    float lb, inv_td;            // canvas edge, 1 / tile extent (for the tile guess)
+};
+struct LabelPointArgs {
+    const float4* xy;            // location column as point pairs, 16-byte aligned
+    uint64_t n;
+    TileAxis ax, ay;
+    TierArgs tr;
+    // cells: index of a coordinate = bits(fma(v, ca, cc)) - kCellMagic; codes
+    // [cny + 1][cnx + 1], the last row and column "none"
+    float cax, ccx, cay, ccy;
+    int cnx, cny;
+    const uint16_t* cells;
+    int cell_words;              // 32-bit words of the map
+    int P;
+    unsigned long long* out_count;
+    const float4* zones;         // zone map (bounds of every 1024 rows; zrow0 = table row of xy[0]) or null
+    uint64_t zrow0;
+    float4 qbox;
+};
+int label_shapes();
+size_t label_points_smem(int shape, int cell_words, int P, bool agg);
+bool launch_label_points(int shape, const LabelPointArgs& a, const LeanCols& lc, int sms, cudaStream_t st);
+void launch_label_cells(const LabelPointArgs& a, float ox, float oy, float errx, float erry, uint16_t* cells, int sms,
+                        cudaStream_t st);
+// Lean point pass over a tiered canvas in its canvas form (rj_tier_lean.cu):
+// one or several canvas tiles, block and mixed-pixel sums, interval-form
+// filters (LeanCols).
 struct TierLeanArgs {
     const float4* xy;            // location column as point pairs, 16-byte aligned
     uint64_t n;
-    const float4* colxf;         // [splitx] (s, t, h, tile extent) per tile column
-    const float4* rowxf;         // [splity]
-    int splitx, splity;
-    int resx, resy;              // tile resolution
-    float lbx, lby;              // canvas lower-left, for the tile guess
-    float inv_tdx, inv_tdy;      // 1 / tile extent, for the tile guess
+    TileAxis ax, ay;
     TierArgs tr;
-    int P;
-    unsigned long long* out_count;
-    const float4* zones;         // zone map or null (as LabelCountArgs)
+    const float4* zones;         // zone map or null (as LabelPointArgs)
     uint64_t zrow0;
     float4 qbox;
 };
 int tier_lean_shapes();
-size_t tier_lean_smem(bool label, int P, bool agg);
-bool launch_tier_lean(int shape, bool label, const TierLeanArgs& a, const LeanCols& lc, int sms, cudaStream_t st);
+bool launch_tier_lean(int shape, const TierLeanArgs& a, const LeanCols& lc, int sms, cudaStream_t st);
 int splat_lean_shapes();
 // shared memory of a shape for a canvas (1 for the global-atomic shapes), 0
 // when the canvas does not fit

@@ -9,9 +9,8 @@
 // per-warp-group histogram copies, fully coalesced loads (each lane two
 // consecutive points: x, y as one float4, each 4-byte column as one uint2).
 // The predicates are the interval form the host compiles them to: per column
-// the query holds exactly when order_key(value) - lo <= span (unsigned); the
-// order key of a float, int or uint column is value ^ ((sign & fm) ^ xm),
-// branch-free.  Sums are the runtime's exact int64 fixed-point values,
+// the query holds exactly when key(value) - lo <= span (modulo 2^32); the key
+// of a float, int or uint column is value ^ (sign & fm), branch-free.  Sums are the runtime's exact int64 fixed-point values,
 // accumulated in shared memory as two 32-bit words (low word with carry into
 // the high word: the pair is the sum modulo 2^64, order-independent) so that
 // every shared atomic stays a native 32-bit one; non-finite values go to the
@@ -25,7 +24,7 @@ __device__ __forceinline__ bool lean_pass(const LeanCols& lc, const uint32_t (&v
     bool ok = true;
     #pragma unroll
     for (int c = 0; c < NCOL; ++c) {
-        const uint32_t key = v[c] ^ (((uint32_t)((int32_t)v[c] >> 31) & lc.fm[c]) ^ lc.xm[c]);
+        const uint32_t key = v[c] ^ ((uint32_t)((int32_t)v[c] >> 31) & lc.fm[c]);
         ok &= (key - lc.lo[c]) <= lc.span[c];
     }
     return ok;

@@ -740,7 +740,9 @@ int poly_pass(rj_ctx* ctx, int mode, PolyPassArgs& a, const TierArgs* tier = nul
 // then the label form (disjoint coverage) or the canvas form.  Results equal
 // the flat canvas's; polygon-side work follows the perimeters.
 int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, const TierArgs& tr,
-                   bool label, size_t nblk, size_t spx, ExecState& es, bool* done);   // below
+                   size_t nblk, size_t spx, ExecState& es, bool* done);   // below
+int label_points_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, const TierArgs& tr,
+                      ExecState& es, bool* done);                         // below
 
 int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const DevFilter& f, ExecState& es,
                      PolyPassArgs& a, const CanvasXf& cx, uint64_t ckey, bool bounds) {
@@ -796,7 +798,7 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
     es.ph->mark(2);
     if (label) {
         bool lean = false;
-        if ((rc = tier_lean_pass(ctx, f, rp, cx, tr, true, nblk, spx, es, &lean))) return rc;
+        if ((rc = label_points_pass(ctx, f, rp, cx, tr, es, &lean))) return rc;
         if (!lean && (rc = point_pass(ctx, f, es.out_count, es.out_sum, [&](const PointArgs& pa) {
                           launch_tier_label_points(pa, cx, tr, ctx->sms, ctx->stream);
                       })))
@@ -817,7 +819,7 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
         RJ_CUDA(cudaMemsetAsync(tr.psum, 0, spx * 8, ctx->stream));
     }
     bool lean = false;
-    if ((rc = tier_lean_pass(ctx, f, rp, cx, tr, false, nblk, spx, es, &lean))) return rc;
+    if ((rc = tier_lean_pass(ctx, f, rp, cx, tr, nblk, spx, es, &lean))) return rc;
     if (!lean && (rc = point_pass(ctx, f, es.out_count, es.out_sum, [&](const PointArgs& pa) {
                       launch_tier_splat_points(pa, cx, tr, ctx->sms, ctx->stream);
                   })))
@@ -887,19 +889,25 @@ inline int tune_bucket(double v) { return (int)std::floor(std::log2(std::max(v, 
 // predicates on value pairs); false when a column is not 8-byte aligned.
 bool lean_cols_of(const PointArgs& pa, unsigned long long* out_sum, LeanCols& lc) {
     lc = LeanCols{};
-    lc.ncol = pa.f.ncol;
-    for (int c = 0; c < lc.ncol; ++c) {
-        if (((uintptr_t)pa.f.col[c] & 7) != 0) return false;
-        lc.col[c] = reinterpret_cast<const uint2*>(pa.f.col[c]);
-        lc.lo[c] = pa.f.lo[c];
-        lc.span[c] = pa.f.span[c];
-        const int t = pa.f.ctyp[c];
-        lc.fm[c] = (t == RJ_FLOAT) ? 0x7FFFFFFFu : 0u;
-        lc.xm[c] = (t == RJ_FLOAT || t == RJ_INT) ? 0x80000000u : 0u;
-    }
     lc.aggr = pa.f.aggr ? 1 : 0;
+    lc.aggr_ci = -1;
+    // uint and int columns first, then the floats
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int i = 0; i < pa.f.ncol; ++i) {
+            const int t = pa.f.ctyp[i];
+            if ((t == RJ_FLOAT) != (pass == 1)) continue;
+            if (((uintptr_t)pa.f.col[i] & 7) != 0 || lc.ncol >= 4) return false;
+            const int c = lc.ncol++;
+            lc.col[c] = reinterpret_cast<const uint2*>(pa.f.col[i]);
+            // the order keys of int and float values less 2^31 (modulo 2^32)
+            lc.lo[c] = t == RJ_UINT ? pa.f.lo[i] : pa.f.lo[i] ^ 0x80000000u;
+            lc.span[c] = pa.f.span[i];
+            lc.fm[c] = t == RJ_FLOAT ? 0x7FFFFFFFu : 0u;
+            if (lc.aggr && pa.f.aggr_ci == i) lc.aggr_ci = c;
+        }
+        if (pass == 0) lc.nint = lc.ncol;
+    }
     if (lc.aggr) {
-        lc.aggr_ci = pa.f.aggr_ci;
         if (lc.aggr_ci < 0) {
             if (((uintptr_t)pa.f.aggr_col & 7) != 0) return false;
             lc.aggr_col = reinterpret_cast<const uint2*>(pa.f.aggr_col);
@@ -1298,15 +1306,168 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
     return RJ_OK;
 }
 
-// Lean point pass over the tiered canvas (rj_tier_lean.cu): a resident
-// table, interval-form filters on at most four columns, count or sum; label
-// form into the per-polygon outputs, canvas form into the block and slot
-// sums.  Shapes forced with rj_set_tuning (RJ_TUNE_COUNT_SHAPE), else
-// autotuned per query class; tuning runs of the canvas form write into its
-// sums, which are cleared again after them.  *done = false: the pass does
+// The tiles of one canvas axis; false when their scales differ (the extents,
+// computed in double, are equal up to rounding, so their fp32 scales almost
+// always are).
+bool tile_axis(const std::vector<float4>& xf, const float4* dxf, int res, float lb, TileAxis& x) {
+    for (const float4& t : xf)
+        if (t.x != xf[0].x || t.z != xf[0].z) return false;
+    x = TileAxis{dxf, (int)xf.size(), res, xf[0].x, xf[0].z * (float)kSub, lb, (float)(1.0 / (double)xf[0].w)};
+    return true;
+}
+
+// Lean point pass of the label form (rj_label_core.cuh) over a canvas held as
+// 16 x 16-pixel blocks: a resident table, interval-form filters on at most
+// four columns, count or sum.  Builds the cell codes and runs the pass.  The
+// shape and the cell side are the ones forced with rj_set_tuning, else
+// autotuned per query class.  *done = false: the pass does not apply (the
+// caller takes the generic pass).
+int label_points_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, const TierArgs& tr,
+                      ExecState& es, bool* done) {
+    *done = false;
+    ctx->last_count_shape = ctx->last_count_bshift = -1;
+    if (ctx->streamed || f.general || f.ncol > label_lean_max_cols()) return RJ_OK;
+    PointArgs pa = make_point_args(ctx, f, es.out_count, es.out_sum);
+    if (((uintptr_t)pa.xy & 15) != 0) return RJ_OK;
+    LeanCols lc{};
+    if (!lean_cols_of(pa, es.out_sum, lc)) return RJ_OK;
+    const bool agg = lc.aggr != 0;
+    LabelPointArgs a{};
+    a.xy = reinterpret_cast<const float4*>(pa.xy);
+    a.n = pa.n;
+    if (!tile_axis(rp.colxf, cx.colxf, rp.resx, cx.lbx, a.ax) || !tile_axis(rp.rowxf, cx.rowxf, rp.resy, cx.lby, a.ay))
+        return RJ_OK;
+    a.tr = tr;
+    a.P = ctx->ps->P;
+    a.out_count = es.out_count;
+    a.zones = pa.zones;
+    a.zrow0 = pa.row0;
+    a.qbox = pa.qbox;
+    // A cell grid of one axis: cells of `side` pixels covering [lo, hi] and
+    // two pixels beyond; index = round(v * ca + o) with an integer offset o.
+    struct Axis {
+        float ca, cc;
+        double o;
+        int n;
+        bool ok;
+    };
+    auto axis = [](double lo, double hi, double pixel, double side) {
+        Axis x{};
+        x.ca = (float)(1.0 / (side * pixel));
+        x.o = std::ceil(-0.5 - (lo - 2.0 * pixel) * (double)x.ca);
+        x.n = (int)std::floor((hi + 2.0 * pixel) * (double)x.ca + x.o + 0.5) + 1;
+        x.cc = (float)(12582912.0 + x.o);   // an integer below 2^24: exact
+        x.ok = std::fabs(x.o) + x.n < (double)(1 << 21);
+        return x;
+    };
+    const double* bb = ctx->ps->bbox;
+    const double px = (bb[2] - bb[0]) / ((double)rp.resx * rp.splitx), py = (bb[3] - bb[1]) / ((double)rp.resy * rp.splity);
+    auto grid = [&](LabelPointArgs& g, double side, double* ox, double* oy) {
+        const Axis x = axis(bb[0], bb[2], px, side), y = axis(bb[1], bb[3], py, side);
+        g.cax = x.ca; g.ccx = x.cc; g.cnx = x.n;
+        g.cay = y.ca; g.ccy = y.cc; g.cny = y.n;
+        *ox = x.o;
+        *oy = y.o;
+        g.cell_words = (int)(((long long)(x.n + 1) * (y.n + 1) + 1) / 2);
+        return x.ok && y.ok && (long long)(x.n + 1) * (y.n + 1) <= 100 * 1024;
+    };
+    // fp32 error in pixels of the exact window coordinate (each of its four
+    // operations rounds once; s and t are rounded too) and of the cell edges'
+    // (three roundings more), plus the snap's half step; beyond half a pixel
+    // no cell is taken as uniform
+    auto err_of = [](const std::vector<float4>& xf, double lo, double hi) {
+        double e = 0;
+        for (const float4& t : xf)
+            e = std::max(e, (double)t.z * (6.0 * std::fabs((double)t.x) * std::max(std::fabs(lo), std::fabs(hi)) + 16.0));
+        e = e * std::ldexp(1.0, -23) + 1.0 / 256.0;
+        return e < 0.5 ? e : 1e30;
+    };
+    const double ex = err_of(rp.colxf, bb[0], bb[2]), ey = err_of(rp.rowxf, bb[1], bb[3]);
+    // Cell sides: about 64k or 16k cells (128 KB or 32 KB of codes), at least
+    // 4 pixels.  Small scans take the coarse map, whose load they feel.
+    const bool small = a.n < kTuneMinPoints;
+    const double npx = (double)rp.resx * rp.splitx * rp.resy * rp.splity;
+    std::vector<std::pair<double, int>> sides;   // (pixels, reported shift)
+    if (ctx->count_bshift >= 4 && ctx->count_bshift <= 8) sides.push_back({(double)(1 << ctx->count_bshift), ctx->count_bshift});
+    else
+        for (double cells : {62500.0, 15625.0}) {
+            const double side = std::max(4.0, std::sqrt(npx / cells));
+            sides.push_back({side, (int)std::lround(std::log2(side))});
+        }
+    std::vector<std::pair<int, int>> cands;   // (shape, side)
+    for (size_t k = 0; k < sides.size(); ++k)
+        for (int sh = 0; sh < label_shapes(); ++sh) {
+            if (ctx->count_shape >= 0 && ctx->count_shape != sh) continue;
+            LabelPointArgs g = a;
+            double ox, oy;
+            if (!grid(g, sides[k].first, &ox, &oy)) continue;
+            if (label_points_smem(sh, g.cell_words, a.P, agg) <= 224 * 1024) cands.push_back({sh, (int)k});
+        }
+    if (cands.empty()) return RJ_OK;
+    char key[200];
+    std::snprintf(key, sizeof key, "label:%d:%d:%d:%d:%d:%d:%d:%d:%d", lc.ncol, lc.aggr, lc.aggr_ci >= 0,
+                  rp.splitx * rp.splity > 1, tune_bucket((double)a.P), tune_bucket(npx), tune_bucket((double)a.n),
+                  ctx->count_shape, ctx->count_bshift);
+    int tuned_i = -1;
+    const bool have = tuned_get(ctx, key, &tuned_i);
+    const bool known = cands.size() == 1 || have || small || ctx->capturing;
+    std::pair<int, int> pick = cands.back();
+    if (have) pick = cands[std::min<size_t>((size_t)tuned_i, cands.size() - 1)];
+    else if (cands.size() > 1)
+        for (const auto& c : cands)
+            if (c.first == 1) pick = c;   // small scans: 1024 threads, two pairs, the coarsest cells
+    int rc;
+    std::vector<LabelPointArgs> args(sides.size(), a);
+    for (size_t k = 0; k < sides.size(); ++k) {
+        if (known && (int)k != pick.second) continue;
+        double ox, oy;
+        if (!grid(args[k], sides[k].first, &ox, &oy)) continue;
+        uint16_t* cells;
+        if ((rc = scratch_t(ctx, k == 0 ? "label_cells0" : "label_cells1", (size_t)args[k].cell_words * 2, &cells))) return rc;
+        launch_label_cells(args[k], (float)ox, (float)oy, (float)ex, (float)ey, cells, ctx->sms, ctx->stream);
+        args[k].cells = cells;
+    }
+    es.ph->mark(2);   // the cell codes belong to the polygon side
+    if (!known) {
+        unsigned long long *tout, *tsum;
+        double* tnf;
+        if ((rc = scratch_t(ctx, "tune_count", (size_t)a.P, &tout))) return rc;
+        if ((rc = scratch_t(ctx, "tune_sum", (size_t)a.P, &tsum))) return rc;
+        if ((rc = scratch_t(ctx, "tune_nonfinite", (size_t)a.P, &tnf))) return rc;
+        LeanCols tl = lc;
+        tl.out_sum = tsum;
+        tl.nonfinite = tnf;
+        const int pi = tune_pick(ctx, key, cands.size(), [&](size_t i) {
+            LabelPointArgs b = args[(size_t)cands[i].second];
+            b.out_count = tout;
+            LabelPointArgs w = b;
+            w.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 16);   // first launch of a shape loads it
+            if (!launch_label_points(cands[i].first, w, tl, ctx->sms, ctx->stream)) return false;
+            b.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 28);
+            return launch_label_points(cands[i].first, b, tl, ctx->sms, ctx->stream);
+        });
+        RJ_CUDA(cudaGetLastError());
+        if (pi < 0) return RJ_OK;
+        pick = cands[(size_t)pi];
+    }
+    ctx->passes = 1;
+    ctx->copy_ms = 0;
+    if (!launch_label_points(pick.first, args[(size_t)pick.second], lc, ctx->sms, ctx->stream)) return RJ_OK;
+    RJ_CUDA(cudaGetLastError());
+    ctx->last_count_shape = pick.first;
+    ctx->last_count_bshift = sides[(size_t)pick.second].second;
+    *done = true;
+    return RJ_OK;
+}
+
+// Lean point pass over the tiered canvas in its canvas form (rj_tier_lean.cu):
+// a resident table, interval-form filters on at most four columns, count or
+// sum into the block and slot sums.  Shapes forced with rj_set_tuning
+// (RJ_TUNE_COUNT_SHAPE), else autotuned per query class; tuning runs write
+// into the sums, which are cleared again after them.  *done = false: the pass does
 // not apply (the caller takes the generic pass).
 int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, const TierArgs& tr,
-                   bool label, size_t nblk, size_t spx, ExecState& es, bool* done) {
+                   size_t nblk, size_t spx, ExecState& es, bool* done) {
     *done = false;
     ctx->last_count_shape = ctx->last_count_bshift = -1;
     if (ctx->streamed || f.general || f.ncol > label_lean_max_cols()) return RJ_OK;
@@ -1317,60 +1478,34 @@ int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const 
     TierLeanArgs a{};
     a.xy = reinterpret_cast<const float4*>(pa.xy);
     a.n = pa.n;
-    a.colxf = cx.colxf;
-    a.rowxf = cx.rowxf;
-    a.splitx = rp.splitx;
-    a.splity = rp.splity;
-    a.resx = rp.resx;
-    a.resy = rp.resy;
-    a.lbx = cx.lbx;
-    a.lby = cx.lby;
-    a.inv_tdx = (float)(1.0 / (double)cx.tdx);
-    a.inv_tdy = (float)(1.0 / (double)cx.tdy);
+    if (!tile_axis(rp.colxf, cx.colxf, rp.resx, cx.lbx, a.ax) || !tile_axis(rp.rowxf, cx.rowxf, rp.resy, cx.lby, a.ay))
+        return RJ_OK;
     a.tr = tr;
-    a.P = ctx->ps->P;
-    a.out_count = es.out_count;
     a.zones = pa.zones;
     a.zrow0 = pa.row0;
     a.qbox = pa.qbox;
-    const bool agg = lc.aggr != 0;
     std::vector<int> cands;
     for (int sh = 0; sh < tier_lean_shapes(); ++sh)
         if (ctx->count_shape < 0 || ctx->count_shape == sh) cands.push_back(sh);
-    if (cands.empty() || tier_lean_smem(label, a.P, agg) > 200 * 1024) return RJ_OK;
+    if (cands.empty()) return RJ_OK;
     char key[200];
-    std::snprintf(key, sizeof key, "tier:%d:%d:%d:%d:%d:%d:%d:%d:%d", label ? 1 : 0, lc.ncol, lc.aggr,
-                  lc.aggr_ci >= 0, rp.splitx * rp.splity, tune_bucket((double)a.P), tune_bucket((double)nblk),
-                  tune_bucket((double)a.n), ctx->count_shape);
+    std::snprintf(key, sizeof key, "tier:%d:%d:%d:%d:%d:%d:%d", lc.ncol, lc.aggr, lc.aggr_ci >= 0,
+                  rp.splitx * rp.splity, tune_bucket((double)nblk), tune_bucket((double)a.n), ctx->count_shape);
     int tuned_i = -1;
     const bool have = tuned_get(ctx, key, &tuned_i);
     const bool small = a.n < kTuneMinPoints;
-    int rc;
-    unsigned long long *tout = nullptr, *tsum = nullptr;
-    double* tnf = nullptr;
-    if (!have && !small && label) {
-        if ((rc = scratch_t(ctx, "tune_count", (size_t)a.P, &tout))) return rc;
-        if ((rc = scratch_t(ctx, "tune_sum", (size_t)a.P, &tsum))) return rc;
-        if ((rc = scratch_t(ctx, "tune_nonfinite", (size_t)a.P, &tnf))) return rc;
-    }
     bool timed_any = false;
     const int pi = small && !have ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i) {
         timed_any = true;
         TierLeanArgs b = a;
-        LeanCols tl = lc;
-        if (label) {
-            b.out_count = tout;
-            tl.out_sum = tsum;
-            tl.nonfinite = tnf;
-        }
-        TierLeanArgs w = b;
+        TierLeanArgs w = a;
         w.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 16);   // first launch of a shape loads it
-        if (!launch_tier_lean(cands[i], label, w, tl, ctx->sms, ctx->stream)) return false;
+        if (!launch_tier_lean(cands[i], w, lc, ctx->sms, ctx->stream)) return false;
         b.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 27);
-        return launch_tier_lean(cands[i], label, b, tl, ctx->sms, ctx->stream);
+        return launch_tier_lean(cands[i], b, lc, ctx->sms, ctx->stream);
     });
     RJ_CUDA(cudaGetLastError());
-    if (timed_any && !label) {
+    if (timed_any) {
         RJ_CUDA(cudaMemsetAsync(tr.bcnt, 0, nblk * 4, ctx->stream));
         RJ_CUDA(cudaMemsetAsync(tr.pcnt, 0, spx * 4, ctx->stream));
         if (tr.bsum) RJ_CUDA(cudaMemsetAsync(tr.bsum, 0, nblk * 8, ctx->stream));
@@ -1379,7 +1514,7 @@ int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const 
     if (pi < 0) return RJ_OK;
     ctx->passes = 1;
     ctx->copy_ms = 0;
-    if (!launch_tier_lean(cands[(size_t)pi], label, a, lc, ctx->sms, ctx->stream)) return RJ_OK;
+    if (!launch_tier_lean(cands[(size_t)pi], a, lc, ctx->sms, ctx->stream)) return RJ_OK;
     RJ_CUDA(cudaGetLastError());
     ctx->last_count_shape = cands[(size_t)pi];
     *done = true;
