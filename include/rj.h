@@ -94,9 +94,10 @@ typedef struct {
 #define RJ_FLAG_NO_CACHE           0x40u /* rebuild every polygon-side structure
                                            (grid, labels, masks) for this call,
                                            as each reference execute() does */
-#define RJ_FLAG_FLAT_CANVAS        0x80u /* raster: one entry per pixel even for
-                                           large canvases (no 16 x 16 block
-                                           tiers; same results)              */
+#define RJ_FLAG_FLAT_CANVAS        0x80u /* raster: point canvases and label maps
+                                           of several tiles keep one entry per
+                                           pixel even when large (no 16 x 16
+                                           block tiers; same results)        */
 #define RJ_FLAG_COUNT_EDGE_TESTS   0x200u /* index/hybrid: count the exact edge tests
                                            into rj_timings.edge_tests (one atomic
                                            per tested point)                  */
@@ -282,14 +283,14 @@ RJ_API int rj_column_absmax(const rj_ctx *ctx, int32_t attrib_id, double *out);
  *   RJ_TUNE_POINT_SHAPE      generic point pass: -1 = default per join,
  *                            0 = 4 points x 256 threads, 2 = bulk-copy
  *                            pipeline, 3 = 4 points x 512 threads
- *   RJ_TUNE_COUNT_SHAPE      lean raster label pass (one canvas tile, label
- *                            map, a resident table): -1 = autotuned (each
+ *   RJ_TUNE_COUNT_SHAPE      lean raster label pass (polygons that do not
+ *                            overlap, a resident table): -1 = autotuned (each
  *                            shape is timed once per context and query
  *                            class on the table itself, the fastest is
  *                            kept), else a shape index
  *                            0..rj_get_tuning(RJ_TUNE_COUNT_SHAPES)-1
- *   RJ_TUNE_COUNT_BLOCK_SHIFT block-code map of that pass: -1 = autotuned,
- *                            else log2 of the block side (4..8)
+ *   RJ_TUNE_COUNT_BLOCK_SHIFT code map of that pass: -1 = autotuned, else
+ *                            log2 of the block or cell side in pixels (4..8)
  *   RJ_TUNE_HYBRID_EXACT_SCALE classified grid of the hybrid join's exact
  *                            tests: the query grid refined 1, 2 or 4 times
  *   RJ_TUNE_COUNT_SHAPES     (read only) number of plain count-pass shapes

@@ -245,7 +245,7 @@ void plan_query(rj_ctx* ctx, QPlan& p, bool no_fuse, bool fuse_all) {
         p.mode = (label_ok && known != 1) ? BQ_LABEL : BQ_SPLAT;
         p.check_overlap = p.mode == BQ_LABEL && known != 0;
         if (!fuse_all && (p.mode == BQ_LABEL || p.mode == BQ_SPLAT) && p.T == 1 && !p.f.general &&
-            p.f.ncol <= label_lean_max_cols() && p.r1 - p.r0 >= kLeanQueryRows)
+            p.f.ncol <= kLeanMaxCols && p.r1 - p.r0 >= kLeanQueryRows)
             p.fused = false;   // rj_execute's lean pass (same results)
     }
 }
@@ -514,7 +514,7 @@ int run_fused(Engine& e, std::vector<QPlan>& plans, uint32_t flags, BatchOut& bo
                     RJ_CUDA(cudaMemsetAsync(p->tr.plabel, 0xFF, std::max<size_t>(spx, 1) * 2, st));
                     if (!query_poly_pass(e, *p, MODE_TIER_LABEL, ps, nullptr, nullptr, tcnt + 3 * i + 1, &p->tr))
                         return fail(ctx, RJ_E_INVALID, "too many (tile, polygon) items");
-                    if (p->check_overlap) launch_tier_nonempty(p->tr.plabel, spx, tcnt + 3 * i + 2, ctx->sms, st);
+                    if (p->check_overlap) launch_tier_nonempty(p->tr, p->nblk, tcnt + 3 * i + 2, ctx->sms, st);
                 } else {
                     RJ_CUDA(cudaMemsetAsync(p->tr.bcnt, 0, p->nblk * 4, st));
                     RJ_CUDA(cudaMemsetAsync(p->tr.pcnt, 0, std::max<size_t>(spx, 1) * 4, st));

@@ -9,7 +9,7 @@
 // shared memory (the label map in L2 only for blocks whose pixels differ).
 // A labelled pixel is inside exactly one polygon and away from every
 // outline: the point goes to that polygon's histogram (plain shared-memory
-// atomics, count and two-word fixed-point sum as in rj_lean_kernels.cu).  A
+// atomics, count and two-word fixed-point sum).  A
 // pixel marked border (within the fp32 error radius of an outline, isBorder
 // hybrid.glsl:174-185) sends the point to the exact test through the
 // classified grid: such points are appended to a block-wide queue with one
@@ -289,6 +289,37 @@ __global__ void __launch_bounds__(BLOCK) k_hybrid_lean(HybLeanArgs a, LeanCols l
 template <int BLOCK, int NV, int NCOL, bool AGG, bool COMPACT>
 __global__ void __launch_bounds__(BLOCK, 2) k_hybrid_lean_r2(HybLeanArgs a, LeanCols lc) {
     hybrid_lean_body<BLOCK, NV, NCOL, AGG, COMPACT>(a, lc);
+}
+
+// Block codes from a label map: one warp per block.
+__global__ void k_block_codes(const uint16_t* __restrict__ label, int resx, int resy, int bs, int nbx, int nby,
+                              uint16_t* __restrict__ codes) {
+    const int lane = threadIdx.x & 31;
+    const int B = 1 << bs;
+    const int nb = nbx * nby;
+    for (int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); b < nb;
+         b += (int)((gridDim.x * blockDim.x) >> 5)) {
+        const int bx = b % nbx, by = b / nbx;
+        const int x0 = bx << bs, y0 = by << bs;
+        const int w = min(x0 + B, resx) - x0, h = min(y0 + B, resy) - y0;
+        const uint16_t first = __ldg(label + (size_t)y0 * resx + x0);
+        bool same = true;
+        for (int i = lane; i < w * h; i += 32) {
+            const int yy = y0 + i / w, xx = x0 + i % w;
+            same &= (__ldg(label + (size_t)yy * resx + xx) == first);
+        }
+        same = __all_sync(0xffffffffu, same);
+        if (lane == 0) codes[b] = same ? first : kCodeMixed;
+    }
+}
+
+void launch_block_codes(const uint16_t* label, int resx, int resy, int bs, int nbx, int nby, uint16_t* codes,
+                        int sms, cudaStream_t st) {
+    const long long warps = (long long)nbx * nby;
+    long long blocks = (warps * 32 + 255) / 256;
+    blocks = std::max(1LL, std::min(blocks, (long long)sms * 16));
+    k_block_codes<<<(unsigned)blocks, 256, 0, st>>>(label, resx, resy, bs, nbx, nby, codes);
+    ++g_kernel_launches;
 }
 
 // 16-bit cell labels of the classified grid for the lean pass (mode 1).

@@ -149,6 +149,26 @@ __device__ __forceinline__ void label_add(uint32_t* hist, uint32_t P, const Lean
     }
 }
 
+// The block's histogram copies into the outputs.
+template <int BLOCK, bool AGG>
+__device__ __forceinline__ void label_flush(const LabelPointArgs& a, const LeanCols& lc, const uint32_t* s_hist) {
+    constexpr int HW = AGG ? 3 : 1;
+    for (int b = threadIdx.x; b < a.P; b += BLOCK) {
+        uint32_t cnt = 0;
+        unsigned long long sum = 0;
+        #pragma unroll 1
+        for (int w = 0; w < lc.copies; ++w) {
+            const uint32_t* h = s_hist + w * HW * a.P;
+            cnt += h[b];
+            if (AGG) sum += ((unsigned long long)h[2 * a.P + b] << 32) + h[a.P + b];
+        }
+        if (cnt) {
+            atomicAdd(a.out_count + b, (unsigned long long)cnt);
+            if (AGG) atomicAdd(lc.out_sum + b, sum);
+        }
+    }
+}
+
 // ---- the pass -------------------------------------------------------------------
 template <int BLOCK, int NV, int MINB, int NI, int NF, bool AGG>
 __global__ void __launch_bounds__(BLOCK, MINB) k_label_points(LabelPointArgs a, LeanCols lc) {
@@ -161,8 +181,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_label_points(LabelPointArgs a, 
     float* tx = reinterpret_cast<float*>(s_words);
     float* ty = tx + kLeanMaxSplit;
     float2* s_q = reinterpret_cast<float2*>(ty + kLeanMaxSplit);      // queued locations, QC per warp
-    float* s_qv = reinterpret_cast<float*>(s_q + (BLOCK / 32) * QC);  // AGG: their values
-    uint32_t* s_code = reinterpret_cast<uint32_t*>(s_qv + (AGG ? (BLOCK / 32) * QC : 0));
+    uint32_t* s_qv = reinterpret_cast<uint32_t*>(s_q + (BLOCK / 32) * QC);   // AGG: their values (raw)
+    uint32_t* s_code = s_qv + (AGG ? (BLOCK / 32) * QC : 0);
     uint32_t* s_hist = s_code + a.cell_words;                         // lc.copies x HW x P
     tl_stage_tiles<BLOCK>(a.ax, a.ay, tx, ty);
     {
@@ -176,7 +196,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_label_points(LabelPointArgs a, 
     const uint32_t P = (uint32_t)a.P;
     uint32_t* hist = s_hist + (warp & (lc.copies - 1)) * HW * a.P;
     float2* q = s_q + warp * QC;
-    float* qv = s_qv + warp * QC;
+    uint32_t* qv = s_qv + warp * QC;
     int qn = 0;                                                       // queued points (warp-uniform)
 
     auto cell_code = [&](float x, float y) -> uint32_t {
@@ -212,7 +232,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_label_points(LabelPointArgs a, 
         const int i = first + lane;
         if (i < qn) {
             const float2 p = q[i];
-            const float v = AGG ? qv[i] : 0.f;
+            const float v = AGG ? agg_value(lc.aggr_typ, qv[i]) : 0.f;
             uint32_t l = kCodeMixed;
             if (NCOL > 0) {
                 l = cell_code(p.x, p.y);
@@ -249,13 +269,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_label_points(LabelPointArgs a, 
             for (int c = 0; c < NCOL; ++c) cv[c][k] = live ? __ldcs(lc.col[c] + i) : make_uint2(0u, 0u);
             if (AGG) av[k] = (live && lc.aggr_ci < 0) ? __ldcs(lc.aggr_col + i) : make_uint2(0u, 0u);
         }
-        auto value = [&](int j) -> float {
-            if (!AGG) return 0.f;
+        auto value = [&](int j) -> uint32_t {
             uint32_t raw = (j & 1) ? av[j >> 1].y : av[j >> 1].x;
             #pragma unroll
             for (int c = 0; c < NCOL; ++c)
                 if (c == lc.aggr_ci) raw = (j & 1) ? cv[c][j >> 1].y : cv[c][j >> 1].x;
-            return agg_value(lc.aggr_typ, raw);
+            return raw;
         };
         #pragma unroll
         for (int g = 0; g < NV; g += G) {
@@ -272,7 +291,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_label_points(LabelPointArgs a, 
                 } else {
                     const uint32_t l =
                         cell_code((j & 1) ? p[j >> 1].z : p[j >> 1].x, (j & 1) ? p[j >> 1].w : p[j >> 1].y);
-                    if (l < P) label_add<AGG>(hist, P, lc, l, value(j));
+                    if (l < P) label_add<AGG>(hist, P, lc, l, AGG ? agg_value(lc.aggr_typ, value(j)) : 0.f);
                     push |= l == kCodeMixed ? 1u << j : 0u;
                 }
             }
@@ -325,20 +344,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_label_points(LabelPointArgs a, 
         }
     }
     __syncthreads();
-    for (int b = threadIdx.x; b < a.P; b += BLOCK) {
-        uint32_t cnt = 0;
-        unsigned long long sum = 0;
-        #pragma unroll 1
-        for (int w = 0; w < lc.copies; ++w) {
-            const uint32_t* h = s_hist + w * HW * a.P;
-            cnt += h[b];
-            if (AGG) sum += ((unsigned long long)h[2 * a.P + b] << 32) + h[a.P + b];
-        }
-        if (cnt) {
-            atomicAdd(a.out_count + b, (unsigned long long)cnt);
-            if (AGG) atomicAdd(lc.out_sum + b, sum);
-        }
-    }
+    label_flush<BLOCK, AGG>(a, lc, s_hist);
 }
 
 // Shapes: threads, point pairs in flight per thread, blocks per SM the
@@ -350,6 +356,10 @@ constexpr LabelShape kLabelShapes[] = {{1024, 4, 1}, {1024, 2, 1}, {512, 2, 3}};
 constexpr int kNumLabelShapes = (int)(sizeof(kLabelShapes) / sizeof(kLabelShapes[0]));
 
 using LabelKernel = void (*)(LabelPointArgs, LeanCols);
+// launches a label kernel on as many blocks as are resident (fewer for short
+// scans); false when it cannot run, nothing launched
+bool launch_label_kernel(LabelKernel k, int block, int nv, size_t smem, const LabelPointArgs& a, const LeanCols& lc,
+                         int sms, cudaStream_t st);
 LabelKernel label_points_count(int shape, int ni, int nf);   // rj_label_count.cu
 LabelKernel label_points_sum(int shape, int ni, int nf);     // rj_label_sum.cu
 

@@ -100,26 +100,30 @@ bool launch_label_points(int shape, const LabelPointArgs& a, const LeanCols& lc_
     const int ni = lc_in.nint, nf = lc_in.ncol - lc_in.nint;
     LabelKernel k = agg ? label_points_sum(shape, ni, nf) : label_points_count(shape, ni, nf);
     if (!k) return false;
+    LeanCols lc = lc_in;
+    lc.copies = label_copies(shape, a.P, agg);
+    return launch_label_kernel(k, kLabelShapes[shape].block, kLabelShapes[shape].nv,
+                               label_points_smem(shape, a.cell_words, a.P, agg), a, lc, sms, st);
+}
+
+bool launch_label_kernel(LabelKernel k, int block, int nv, size_t smem, const LabelPointArgs& a, const LeanCols& lc,
+                         int sms, cudaStream_t st) {
     if (g_label_optin < 0) {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&g_label_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     }
-    LeanCols lc = lc_in;
-    lc.copies = label_copies(shape, a.P, agg);
-    const size_t smem = label_points_smem(shape, a.cell_words, a.P, agg);
     if (smem > (size_t)g_label_optin) return false;
     if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    const int block = kLabelShapes[shape].block;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block, smem) != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
         return false;
     }
-    const uint64_t per_iter = (uint64_t)block * kLabelShapes[shape].nv;
+    const uint64_t per_iter = (uint64_t)block * nv;
     const uint64_t need = ((a.n >> 1) + per_iter - 1) / per_iter;
     const uint64_t blocks = std::min<uint64_t>((uint64_t)sms * per_sm, std::max<uint64_t>(need, 1));
     // shared counts are 32-bit: a block must see fewer than 2^31 points (a

@@ -20,7 +20,7 @@ struct TierArgs {
     int bw, bh;                  // blocks per tile row / per tile column
     uint32_t* full;              // [nblk] polygon covering the whole block, kTierEmpty, kTierMulti
     uint32_t* mixed;             // [nblk] 1: per-pixel block
-    const int* slot;             // [nblk] exclusive scan of mixed
+    const int* slot;             // [nblk] exclusive scan of mixed, or null: slot = block
     uint32_t* code;              // [nblk] lookup code (full polygon / empty / multi / mixed | slot)
     uint16_t* plabel;            // [nslots * 256] pixel labels of mixed blocks
     uint32_t* bcnt;              // [nblk] point counts of the blocks neither mixed nor empty (canvas form)
@@ -72,7 +72,7 @@ struct PolyPassArgs {
 size_t tier_smem_bytes();
 void launch_tier_pass(int mode, const PolyPassArgs& a, const TierArgs& tr, int sms, cudaStream_t st);
 void launch_tier_codes(const TierArgs& tr, size_t nblk, unsigned long long* multi, int sms, cudaStream_t st);
-void launch_tier_nonempty(const uint16_t* plabel, size_t n, unsigned long long* count, int sms, cudaStream_t st);
+void launch_tier_nonempty(const TierArgs& tr, size_t nblk, unsigned long long* count, int sms, cudaStream_t st);
 
 struct GridArgs {
     const float2* verts;
@@ -210,27 +210,9 @@ void launch_outline_mask(const float2* verts, const int* pindex, int P, const in
 void launch_dilate_mask(const uint32_t* in, uint32_t* out, int resx, int resy, int words, int radius,
                         int sms, cudaStream_t st);
 
-// Lean raster count over one canvas tile with a polygon label map
-// (rj_count_kernels.cu): no filter, count only.
-struct LabelCountArgs {
-    const float4* xy;            // location column as point pairs, 16-byte aligned
-    uint64_t n;                  // points
-    float4 col0, row0;           // the tile transform (s, t, h) per axis
-    int resx, resy;
-    const uint16_t* label;       // [resy][resx] polygon label, kEmptyLabel outside every polygon
-    const uint16_t* codes;       // [nby][nbx] block codes (label shared by the block, or mixed)
-    int bs;                      // log2 of the block side
-    int nbx;                     // blocks per canvas row
-    int code_words;              // 32-bit words of the code map (its u16 count rounded up)
-    int P;
-    unsigned long long* out_count;
-    // zone map (bounds of every 1024 rows; zrow0 = table row of xy[0]) or null
-    const float4* zones;
-    uint64_t zrow0;
-    float4 qbox;
-};
-// Filters (interval form, <= 4 columns) and the summed aggregate of the lean
-// label pass with attributes (rj_lean_kernels.cu).
+// Filters (interval form, at most kLeanMaxCols columns) and the summed
+// aggregate of the lean point passes.
+constexpr int kLeanMaxCols = 4;
 struct LeanCols {
     int ncol;
     int nint;                    // uint / int columns come first, then the floats
@@ -275,10 +257,6 @@ void launch_cell_labels(const uint32_t* code, int ncells, uint16_t* label, int s
 int hybrid_lean_shapes();
 size_t hybrid_lean_smem(int shape, int code_words, int P, bool agg);
 bool launch_hybrid_lean(int shape, const HybLeanArgs& a, const LeanCols& lc, int sms, cudaStream_t st);
-int label_lean_shapes();
-int label_lean_max_cols();
-size_t label_lean_smem(int shape, int code_words, int P, bool agg);
-bool launch_label_lean(int shape, const LabelCountArgs& a, const LeanCols& lc, int sms, cudaStream_t st);
 // Lean point pass onto a point canvas (rj_splat_kernels.cu): one canvas tile,
 // interval-form filters on at most four columns (LeanCols), count and sum.
 struct SplatLeanArgs {
@@ -288,7 +266,7 @@ struct SplatLeanArgs {
     int resx, resy;
     uint32_t* canvas_c;          // [resy][resx] counts
     unsigned long long* canvas_s; // [resy][resx] int64 fixed-point sums, or null
-    const float4* zones;         // zone map or null (as LabelCountArgs)
+    const float4* zones;         // zone map or null (as LabelPointArgs)
     uint64_t zrow0;
     float4 qbox;
 };
@@ -313,6 +291,8 @@ struct LabelPointArgs {
     float cax, ccx, cay, ccy;
     int cnx, cny;
     const uint16_t* cells;
+    int bs;                      // the one-tile pass without filters: cells are blocks of 2^bs x 2^bs
+                                 // pixels, cnx x cny of them, and one entry off the canvas
     int cell_words;              // 32-bit words of the map
     int P;
     unsigned long long* out_count;
@@ -320,6 +300,10 @@ struct LabelPointArgs {
     uint64_t zrow0;
     float4 qbox;
 };
+int label_tile_shapes();
+size_t label_tile_smem(int shape, int cell_words, int P, bool agg);
+bool launch_label_tile(int shape, const LabelPointArgs& a, const LeanCols& lc, int sms, cudaStream_t st);
+void launch_label_blocks(const TierArgs& tr, int bs, int nbx, int nby, int P, uint16_t* codes, int sms, cudaStream_t st);
 int label_shapes();
 size_t label_points_smem(int shape, int cell_words, int P, bool agg);
 bool launch_label_points(int shape, const LabelPointArgs& a, const LeanCols& lc, int sms, cudaStream_t st);
@@ -344,9 +328,6 @@ int splat_lean_shapes();
 // when the canvas does not fit
 size_t splat_lean_smem(int shape, size_t npix, bool agg);
 bool launch_splat_lean(int shape, const SplatLeanArgs& a, const LeanCols& lc, int sms, cudaStream_t st);
-int label_count_shapes();
-size_t label_count_smem(int shape, int code_words, int P);
-bool launch_label_count(int shape, const LabelCountArgs& a, int sms, cudaStream_t st);
 
 // point side
 // smem_hist: histogram capacity decision done by the launcher.

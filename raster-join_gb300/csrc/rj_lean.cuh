@@ -1,5 +1,5 @@
-// rj_lean.cuh -- building blocks of the lean label passes (rj_count_kernels.cu,
-// rj_lean_kernels.cu): the block-code marker and the pixel arithmetic.
+// rj_lean.cuh -- building blocks of the lean point passes: the mixed-code
+// marker and the pixel arithmetic.
 #pragma once
 #include "rj_launch.h"
 
@@ -23,27 +23,9 @@ constexpr uint16_t kCodeMixed = 0xFFFDu;
 // (Packed fp32x2 arithmetic was tried for the two coordinates: each packed
 // operation alone rounds like the scalar one, but chains of them did not
 // reproduce the scalar results on GB300, so the arithmetic stays scalar.)
-struct TileXf2 {
-    float sx, tx, Hx;            // per axis: scale, offset, 256 * half resolution
-    float sy, ty, Hy;
-};
-
-__device__ __forceinline__ TileXf2 tile_xf2(const LabelCountArgs& a) {
-    return TileXf2{a.col0.x, a.col0.y, __fmul_rn(a.col0.z, (float)kSub),
-                   a.row0.x, a.row0.y, __fmul_rn(a.row0.z, (float)kSub)};
-}
-
 __device__ __forceinline__ int snapped_pixel(float v, float s, float t, float H) {
     const float w = __fadd_rn(__fmul_rn(H, __fadd_rn(__fmul_rn(s, v), t)), H);   // window coordinate * 256
     return __float2int_rn(fmaxf(w, -kWinClamp * (float)kSub)) >> kSubpixelBits;
-}
-
-// Returns whether the pixel lies in the canvas.
-__device__ __forceinline__ bool count_pixel(const LabelCountArgs& a, const TileXf2& xf, float x, float y, int& px,
-                                            int& py) {
-    px = snapped_pixel(x, xf.sx, xf.tx, xf.Hx);
-    py = snapped_pixel(y, xf.sy, xf.ty, xf.Hy);
-    return (unsigned)px < (unsigned)a.resx && (unsigned)py < (unsigned)a.resy;
 }
 
 }  // namespace rj

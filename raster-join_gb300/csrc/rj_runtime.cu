@@ -708,41 +708,66 @@ struct ExecState {
     int passes = 1;
 };
 
-int poly_pass(rj_ctx* ctx, int mode, PolyPassArgs& a, const TierArgs* tier = nullptr) {
+// reuse: the bands of the pass just before (same polygons, tiles and band
+// layout) still stand; only the work counter is new.
+int poly_pass(rj_ctx* ctx, int mode, PolyPassArgs& a, const TierArgs* tier = nullptr, bool reuse = false) {
     unsigned int* ctr;
     int rc;
     const int TP = a.T * a.P;
     int4* info_a;
     int2* info_b;
     int *nbands, *band_start, *tmp;
-    if ((rc = scratch_t(ctx, "work_ctr", 1, &ctr))) return rc;
+    if ((rc = scratch_t(ctx, "work_ctr", 2, &ctr))) return rc;
     if ((rc = scratch_t(ctx, "pp_info_a", TP, &info_a))) return rc;
     if ((rc = scratch_t(ctx, "pp_info_b", TP, &info_b))) return rc;
     if ((rc = scratch_t(ctx, "pp_nbands", TP, &nbands))) return rc;
     if ((rc = scratch_t(ctx, "pp_band_start", (size_t)TP + 1, &band_start))) return rc;
     if ((rc = scratch_t(ctx, "pp_tmp", (size_t)scan_tmp_ints(TP), &tmp))) return rc;
-    RJ_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), ctx->stream));
-    a.work_ctr = ctr;
+    if (!reuse) RJ_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned), ctx->stream));
+    a.work_ctr = ctr + (reuse ? 1 : 0);
     a.info_a = info_a;
     a.info_b = info_b;
     a.nbands = nbands;
     a.band_start = band_start;
-    launch_poly_info(mode, a, ctx->sms, ctx->stream);
-    if (!launch_exclusive_scan(nbands, band_start, TP, tmp, ctx->stream))
-        return fail(ctx, RJ_E_INVALID, "too many (tile, polygon) items");
+    if (!reuse) {
+        launch_poly_info(mode, a, ctx->sms, ctx->stream);
+        if (!launch_exclusive_scan(nbands, band_start, TP, tmp, ctx->stream))
+            return fail(ctx, RJ_E_INVALID, "too many (tile, polygon) items");
+    }
     if (tier) launch_tier_pass(mode, a, *tier, ctx->sms, ctx->stream);
     else launch_poly_pass(mode, a, ctx->sms, ctx->stream);
     RJ_CUDA(cudaGetLastError());
     return RJ_OK;
 }
 
+// The lean label pass of a query (rj_label_core.cuh), planned on the host: its
+// arguments less the canvas, and the candidate shapes and cell sides.
+struct LabelPlan {
+    LabelPointArgs a{};
+    LeanCols lc{};
+    bool tile = false;                              // one tile, no filters: exact pixels (rj_label_tile.cu)
+    bool agg = false, small = false, have = false;
+    int tuned = -1;                                 // the candidate kept for `key` (have)
+    char key[200];
+    double errx = 0, erry = 0;                      // fp32 error of a pixel coordinate, in pixels
+    struct Side {
+        LabelPointArgs a;                           // a with the cell grid
+        double ox, oy;                              // integer offsets of the cell index
+        int shift;                                  // log2 of the cell side in pixels (reported)
+    };
+    std::vector<Side> sides;
+    std::vector<std::pair<int, int>> cands;         // (shape, side)
+};
+
 // Tiered canvas of a large raster canvas: classification of 16 x 16 blocks,
 // then the label form (disjoint coverage) or the canvas form.  Results equal
 // the flat canvas's; polygon-side work follows the perimeters.
 int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, const TierArgs& tr,
                    size_t nblk, size_t spx, ExecState& es, bool* done);   // below
-int label_points_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, const TierArgs& tr,
-                      ExecState& es, bool* done);                         // below
+struct LabelPlan;
+bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, ExecState& es,
+                       LabelPlan& lp);                                    // below
+int run_label_points(rj_ctx* ctx, LabelPlan& lp, const TierArgs& tr, ExecState& es, bool* done);   // below
 
 int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const DevFilter& f, ExecState& es,
                      PolyPassArgs& a, const CanvasXf& cx, uint64_t ckey, bool bounds) {
@@ -787,7 +812,7 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
         a.covered = cnt + 1;
         if ((rc = poly_pass(ctx, MODE_TIER_LABEL, a, &tr))) return rc;
         if (ctx->ps->overlap_on(ckey) == -1) {
-            launch_tier_nonempty(tr.plabel, (size_t)nslots * 256, cnt + 2, ctx->sms, ctx->stream);
+            launch_tier_nonempty(tr, nblk, cnt + 2, ctx->sms, ctx->stream);
             unsigned long long hc[3] = {0, 0, 0};
             RJ_CUDA(cudaMemcpyAsync(hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, ctx->stream));
             RJ_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -798,7 +823,8 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
     es.ph->mark(2);
     if (label) {
         bool lean = false;
-        if ((rc = label_points_pass(ctx, f, rp, cx, tr, es, &lean))) return rc;
+        LabelPlan lp;
+        if (plan_label_points(ctx, f, rp, cx, es, lp) && (rc = run_label_points(ctx, lp, tr, es, &lean))) return rc;
         if (!lean && (rc = point_pass(ctx, f, es.out_count, es.out_sum, [&](const PointArgs& pa) {
                           launch_tier_label_points(pa, cx, tr, ctx->sms, ctx->stream);
                       })))
@@ -882,7 +908,7 @@ int label_map(rj_ctx* ctx, PolyPassArgs& a, const char* key, size_t npix, const 
 // the polygon count, canvas size and table size in octave buckets.  Scans
 // below kTuneMinPoints take the default shape without timing anything.
 constexpr uint64_t kTuneMinPoints = 1ull << 22;
-constexpr int kCountDefaultShape = 5;     // 1024 threads, 4 pairs, block codes, per-warp histograms
+constexpr int kMaxShapes = 11;   // shape indices rj_set_tuning takes (a pass without that shape runs its generic form)
 inline int tune_bucket(double v) { return (int)std::floor(std::log2(std::max(v, 1.0))); }
 
 // Filters and aggregate of a query in the lean passes' form (interval
@@ -968,158 +994,6 @@ int tune_pick(rj_ctx* ctx, const std::string& key, size_t ncand, Timed&& timed) 
     return besti;
 }
 
-// Lean label pass (rj_count_kernels.cu for a plain count, rj_lean_kernels.cu
-// with interval-form filters on up to four columns and / or a summed
-// aggregate): one canvas tile, a resident table.  Builds the block-code
-// map(s) of the label map and runs the pass; the shape and block size are the
-// ones forced with rj_set_tuning, else autotuned: on the first query of its
-// class (form, polygons, canvas, table size) on this context every candidate
-// is timed once on the table itself, into scratch outputs, and the fastest is
-// kept.  *done = false: the pass does not apply (the caller takes the generic
-// label pass).
-int label_count_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const uint16_t* label, ExecState& es,
-                     bool* done) {
-    *done = false;
-    ctx->last_count_shape = ctx->last_count_bshift = -1;
-    if (rp.splitx != 1 || rp.splity != 1 || ctx->streamed) return RJ_OK;
-    if (f.general || f.ncol > label_lean_max_cols()) return RJ_OK;
-    const bool plain = f.ncol == 0 && !f.aggr;
-    PointArgs pa = make_point_args(ctx, f, es.out_count, es.out_sum);
-    if (((uintptr_t)pa.xy & 15) != 0) return RJ_OK;
-    LeanCols lc{};
-    if (!plain && !lean_cols_of(pa, es.out_sum, lc)) return RJ_OK;
-    const int P = ctx->ps->P;
-    LabelCountArgs a{};
-    a.xy = reinterpret_cast<const float4*>(pa.xy);
-    a.n = pa.n;
-    a.col0 = rp.colxf[0];
-    a.row0 = rp.rowxf[0];
-    a.resx = rp.resx;
-    a.resy = rp.resy;
-    a.label = label;
-    a.P = P;
-    a.out_count = es.out_count;
-    a.zones = pa.zones;
-    a.zrow0 = pa.row0;
-    a.qbox = pa.qbox;
-    auto code_words = [&](int bs) {
-        const long long nbx = ((long long)rp.resx + (1 << bs) - 1) >> bs, nby = ((long long)rp.resy + (1 << bs) - 1) >> bs;
-        return (nbx * nby + 1) / 2;
-    };
-    // candidate block sizes: the smallest whose code map leaves room in
-    // shared memory for the histograms, and the next one
-    int bs0 = 4;
-    while (bs0 < 8 && code_words(bs0) * 4 + (long long)P * 12 > 160 * 1024) ++bs0;
-    std::vector<int> bss;
-    if (ctx->count_bshift >= 4 && ctx->count_bshift <= 8) bss.push_back(ctx->count_bshift);
-    else {
-        bss.push_back(bs0);
-        if (bs0 < 8) bss.push_back(bs0 + 1);
-    }
-    const int nshapes = plain ? label_count_shapes() : label_lean_shapes();
-    auto smem_of = [&](int sh, int bs) {
-        return plain ? label_count_smem(sh, (int)code_words(bs), P)
-                     : label_lean_smem(sh, (int)code_words(bs), P, lc.aggr != 0);
-    };
-    std::vector<std::pair<int, int>> cands;   // (shape, bs)
-    for (int bs : bss)
-        for (int sh = 0; sh < nshapes; ++sh)
-            if (ctx->count_shape < 0 || ctx->count_shape == sh)
-                if (smem_of(sh, bs) > 0 && smem_of(sh, bs) <= 200 * 1024) cands.push_back({sh, bs});
-    if (cands.empty()) return RJ_OK;
-    int rc;
-    char tkey[200];
-    std::snprintf(tkey, sizeof tkey, "lean:%d:%d:%d:%d:%d:%d:%d:%d:%d", plain ? 0 : 1, lc.ncol, lc.aggr, lc.aggr_ci >= 0,
-                  tune_bucket((double)P), tune_bucket((double)rp.resx * rp.resy), tune_bucket((double)a.n),
-                  ctx->count_shape, ctx->count_bshift);
-    int tuned_i = -1;
-    const bool have = tuned_get(ctx, tkey, &tuned_i);
-    // small scans are not worth timing candidates for: the default shape
-    const bool small = a.n < kTuneMinPoints;
-    const bool known = cands.size() == 1 || have || small || ctx->capturing;
-    std::pair<int, int> pick = cands[0];
-    if (cands.size() > 1 && have)
-        pick = cands[std::min<size_t>((size_t)tuned_i, cands.size() - 1)];
-    else if (small)
-        for (const auto& c : cands)
-            if (c.first == (plain ? kCountDefaultShape : 0) && c.second == bss.back()) pick = c;
-    // code maps: the chosen block size only, or every candidate's for the tuner
-    std::map<int, uint16_t*> codes;
-    for (int bs : bss) {
-        if (known && bs != pick.second) continue;
-        const int nbx = (rp.resx + (1 << bs) - 1) >> bs, nby = (rp.resy + (1 << bs) - 1) >> bs;
-        uint16_t* c;
-        char key[32];
-        std::snprintf(key, sizeof key, "label_codes%d", bs);
-        if ((rc = scratch_t(ctx, key, (size_t)code_words(bs) * 2, &c))) return rc;
-        launch_block_codes(label, rp.resx, rp.resy, bs, nbx, nby, c, ctx->sms, ctx->stream);
-        codes[bs] = c;
-    }
-    es.ph->mark(2);   // the code maps belong to the polygon side
-    auto args_for = [&](int bs) {
-        LabelCountArgs b = a;
-        b.bs = bs;
-        b.nbx = (rp.resx + (1 << bs) - 1) >> bs;
-        b.codes = codes[bs];
-        b.code_words = (int)code_words(bs);
-        return b;
-    };
-    auto launch = [&](int sh, const LabelCountArgs& b, const LeanCols& l) {
-        return plain ? launch_label_count(sh, b, ctx->sms, ctx->stream)
-                     : launch_label_lean(sh, b, l, ctx->sms, ctx->stream);
-    };
-    if (!known) {
-        // time each candidate once on (a prefix of) the table, into scratch outputs
-        unsigned long long *tout, *tsum;
-        double* tnf;
-        if ((rc = scratch_t(ctx, "tune_count", (size_t)P, &tout))) return rc;
-        if ((rc = scratch_t(ctx, "tune_sum", (size_t)P, &tsum))) return rc;
-        if ((rc = scratch_t(ctx, "tune_nonfinite", (size_t)P, &tnf))) return rc;
-        LeanCols tl = lc;
-        tl.out_sum = tsum;
-        tl.nonfinite = tnf;
-        const uint64_t tn = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 28);
-        cudaEvent_t e0, e1;
-        RJ_CUDA(cudaEventCreate(&e0));
-        RJ_CUDA(cudaEventCreate(&e1));
-        float best = 1e30f;
-        int besti = -1;
-        for (size_t i = 0; i < cands.size(); ++i) {
-            LabelCountArgs b = args_for(cands[i].second);
-            b.out_count = tout;
-            // first launch of a shape loads it: a tiny warm-up launch
-            LabelCountArgs w = b;
-            w.n = std::min<uint64_t>(b.n & ~1ULL, 1ULL << 16);
-            if (!launch(cands[i].first, w, tl)) continue;
-            b.n = tn;
-            RJ_CUDA(cudaEventRecord(e0, ctx->stream));
-            launch(cands[i].first, b, tl);
-            RJ_CUDA(cudaEventRecord(e1, ctx->stream));
-            RJ_CUDA(cudaEventSynchronize(e1));
-            float ms = 0.f;
-            RJ_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            if (ms < best) {
-                best = ms;
-                besti = (int)i;
-            }
-        }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        RJ_CUDA(cudaGetLastError());
-        if (besti < 0) return RJ_OK;
-        tuned_put(ctx, tkey, besti);
-        pick = cands[(size_t)besti];
-    }
-    ctx->passes = 1;
-    ctx->copy_ms = 0;
-    if (!launch(pick.first, args_for(pick.second), lc)) return RJ_OK;
-    RJ_CUDA(cudaGetLastError());
-    ctx->last_count_shape = pick.first;
-    ctx->last_count_bshift = pick.second;
-    *done = true;
-    return RJ_OK;
-}
-
 // Lean point pass of the hybrid join over its label map (rj_hybrid_lean.cu):
 // a resident table, interval-form filters on at most four columns, count or
 // sum.  Shapes and block sizes as for the lean raster pass (forced with
@@ -1131,7 +1005,7 @@ int hybrid_lean_pass(rj_ctx* ctx, const DevFilter& f, int mode, const HybXf& h, 
                      const ExactIndex& ix, ExecState& es, bool* done) {
     *done = false;
     ctx->last_count_shape = ctx->last_count_bshift = -1;
-    if (ctx->streamed || f.general || f.ncol > label_lean_max_cols()) return RJ_OK;
+    if (ctx->streamed || f.general || f.ncol > kLeanMaxCols) return RJ_OK;
     PointArgs pa = make_point_args(ctx, f, es.out_count, es.out_sum);
     if (((uintptr_t)pa.xy & 15) != 0) return RJ_OK;
     LeanCols lc;
@@ -1249,7 +1123,7 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
     *done = false;
     ctx->last_count_shape = ctx->last_count_bshift = -1;
     if (rp.splitx != 1 || rp.splity != 1 || ctx->streamed) return RJ_OK;
-    if (f.general || f.ncol > label_lean_max_cols()) return RJ_OK;
+    if (f.general || f.ncol > kLeanMaxCols) return RJ_OK;
     PointArgs pa = make_point_args(ctx, f, es.out_count, es.out_sum);
     if (((uintptr_t)pa.xy & 15) != 0) return RJ_OK;
     LeanCols lc{};
@@ -1316,61 +1190,31 @@ bool tile_axis(const std::vector<float4>& xf, const float4* dxf, int res, float 
     return true;
 }
 
-// Lean point pass of the label form (rj_label_core.cuh) over a canvas held as
-// 16 x 16-pixel blocks: a resident table, interval-form filters on at most
-// four columns, count or sum.  Builds the cell codes and runs the pass.  The
-// shape and the cell side are the ones forced with rj_set_tuning, else
-// autotuned per query class.  *done = false: the pass does not apply (the
-// caller takes the generic pass).
-int label_points_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, const TierArgs& tr,
-                      ExecState& es, bool* done) {
-    *done = false;
+// Plans the lean point pass of the label form (rj_label_core.cuh) over a
+// canvas held as 16 x 16-pixel blocks: a resident table, interval-form filters
+// on at most four columns, count or sum, per-polygon histograms that fit
+// shared memory.  The shape and the cell side are the ones forced with
+// rj_set_tuning, else autotuned per query class.  False: the pass does not
+// apply (the caller takes the generic pass).
+bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, ExecState& es,
+                       LabelPlan& lp) {
     ctx->last_count_shape = ctx->last_count_bshift = -1;
-    if (ctx->streamed || f.general || f.ncol > label_lean_max_cols()) return RJ_OK;
+    if (ctx->streamed || f.general || f.ncol > kLeanMaxCols) return false;
     PointArgs pa = make_point_args(ctx, f, es.out_count, es.out_sum);
-    if (((uintptr_t)pa.xy & 15) != 0) return RJ_OK;
-    LeanCols lc{};
-    if (!lean_cols_of(pa, es.out_sum, lc)) return RJ_OK;
-    const bool agg = lc.aggr != 0;
-    LabelPointArgs a{};
+    if (((uintptr_t)pa.xy & 15) != 0) return false;
+    if (!lean_cols_of(pa, es.out_sum, lp.lc)) return false;
+    lp.agg = lp.lc.aggr != 0;
+    LabelPointArgs& a = lp.a;
     a.xy = reinterpret_cast<const float4*>(pa.xy);
     a.n = pa.n;
     if (!tile_axis(rp.colxf, cx.colxf, rp.resx, cx.lbx, a.ax) || !tile_axis(rp.rowxf, cx.rowxf, rp.resy, cx.lby, a.ay))
-        return RJ_OK;
-    a.tr = tr;
+        return false;
     a.P = ctx->ps->P;
     a.out_count = es.out_count;
     a.zones = pa.zones;
     a.zrow0 = pa.row0;
     a.qbox = pa.qbox;
-    // A cell grid of one axis: cells of `side` pixels covering [lo, hi] and
-    // two pixels beyond; index = round(v * ca + o) with an integer offset o.
-    struct Axis {
-        float ca, cc;
-        double o;
-        int n;
-        bool ok;
-    };
-    auto axis = [](double lo, double hi, double pixel, double side) {
-        Axis x{};
-        x.ca = (float)(1.0 / (side * pixel));
-        x.o = std::ceil(-0.5 - (lo - 2.0 * pixel) * (double)x.ca);
-        x.n = (int)std::floor((hi + 2.0 * pixel) * (double)x.ca + x.o + 0.5) + 1;
-        x.cc = (float)(12582912.0 + x.o);   // an integer below 2^24: exact
-        x.ok = std::fabs(x.o) + x.n < (double)(1 << 21);
-        return x;
-    };
     const double* bb = ctx->ps->bbox;
-    const double px = (bb[2] - bb[0]) / ((double)rp.resx * rp.splitx), py = (bb[3] - bb[1]) / ((double)rp.resy * rp.splity);
-    auto grid = [&](LabelPointArgs& g, double side, double* ox, double* oy) {
-        const Axis x = axis(bb[0], bb[2], px, side), y = axis(bb[1], bb[3], py, side);
-        g.cax = x.ca; g.ccx = x.cc; g.cnx = x.n;
-        g.cay = y.ca; g.ccy = y.cc; g.cny = y.n;
-        *ox = x.o;
-        *oy = y.o;
-        g.cell_words = (int)(((long long)(x.n + 1) * (y.n + 1) + 1) / 2);
-        return x.ok && y.ok && (long long)(x.n + 1) * (y.n + 1) <= 100 * 1024;
-    };
     // fp32 error in pixels of the exact window coordinate (each of its four
     // operations rounds once; s and t are rounded too) and of the cell edges'
     // (three roundings more), plus the snap's half step; beyond half a pixel
@@ -1382,69 +1226,122 @@ int label_points_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, con
         e = e * std::ldexp(1.0, -23) + 1.0 / 256.0;
         return e < 0.5 ? e : 1e30;
     };
-    const double ex = err_of(rp.colxf, bb[0], bb[2]), ey = err_of(rp.rowxf, bb[1], bb[3]);
+    lp.errx = err_of(rp.colxf, bb[0], bb[2]);
+    lp.erry = err_of(rp.rowxf, bb[1], bb[3]);
     // Cell sides: about 64k or 16k cells (128 KB or 32 KB of codes), at least
     // 4 pixels.  Small scans take the coarse map, whose load they feel.
-    const bool small = a.n < kTuneMinPoints;
+    const double px = (bb[2] - bb[0]) / ((double)rp.resx * rp.splitx), py = (bb[3] - bb[1]) / ((double)rp.resy * rp.splity);
     const double npx = (double)rp.resx * rp.splitx * rp.resy * rp.splity;
-    std::vector<std::pair<double, int>> sides;   // (pixels, reported shift)
-    if (ctx->count_bshift >= 4 && ctx->count_bshift <= 8) sides.push_back({(double)(1 << ctx->count_bshift), ctx->count_bshift});
-    else
+    // cells of one axis: `side` pixels each, covering [lo, hi] and two pixels
+    // beyond; index = round(v * ca + o) with an integer offset o
+    auto axis = [](double lo, double hi, double pixel, double side, float* ca, float* cc, int* n, double* o) {
+        *ca = (float)(1.0 / (side * pixel));
+        *o = std::ceil(-0.5 - (lo - 2.0 * pixel) * (double)*ca);
+        const double m = std::floor((hi + 2.0 * pixel) * (double)*ca + *o + 0.5) + 1.0;
+        *cc = (float)(12582912.0 + *o);   // an integer below 2^24: exact
+        *n = (int)std::min(m, 1e6);
+        return std::fabs(*o) + m < (double)(1 << 21);
+    };
+    auto add_side = [&](double side, int shift) {
+        LabelPlan::Side d{a, 0, 0, shift};
+        if (!axis(bb[0], bb[2], px, side, &d.a.cax, &d.a.ccx, &d.a.cnx, &d.ox) ||
+            !axis(bb[1], bb[3], py, side, &d.a.cay, &d.a.ccy, &d.a.cny, &d.oy))
+            return;
+        const long long cells = (long long)(d.a.cnx + 1) * (d.a.cny + 1);
+        if (cells > 100 * 1024) return;
+        d.a.cell_words = (int)((cells + 1) / 2);
+        lp.sides.push_back(d);
+    };
+    // One tile without filters: blocks of 2^bs pixels, the smallest whose codes
+    // take at most 128 KB and the next.
+    lp.tile = rp.splitx * rp.splity == 1 && lp.lc.ncol == 0;
+    auto add_blocks = [&](int bs) {
+        LabelPlan::Side d{a, 0, 0, bs};
+        d.a.bs = bs;
+        d.a.cnx = (rp.resx + (1 << bs) - 1) >> bs;
+        d.a.cny = (rp.resy + (1 << bs) - 1) >> bs;
+        d.a.cell_words = d.a.cnx * d.a.cny / 2 + 1;   // and one entry for points off the canvas
+        if (d.a.cell_words > 32 * 1024) return false;
+        lp.sides.push_back(d);
+        return true;
+    };
+    const bool forced = ctx->count_bshift >= 4 && ctx->count_bshift <= 8;
+    if (lp.tile && forced) {
+        add_blocks(ctx->count_bshift);
+    } else if (lp.tile) {
+        int bs = 4;
+        while (!add_blocks(bs)) ++bs;
+        add_blocks(bs + 1);
+    } else if (forced) {
+        add_side((double)(1 << ctx->count_bshift), ctx->count_bshift);
+    } else {
         for (double cells : {62500.0, 15625.0}) {
             const double side = std::max(4.0, std::sqrt(npx / cells));
-            sides.push_back({side, (int)std::lround(std::log2(side))});
+            add_side(side, (int)std::lround(std::log2(side)));
+            if (side == 4.0) break;
         }
-    std::vector<std::pair<int, int>> cands;   // (shape, side)
-    for (size_t k = 0; k < sides.size(); ++k)
-        for (int sh = 0; sh < label_shapes(); ++sh) {
-            if (ctx->count_shape >= 0 && ctx->count_shape != sh) continue;
-            LabelPointArgs g = a;
-            double ox, oy;
-            if (!grid(g, sides[k].first, &ox, &oy)) continue;
-            if (label_points_smem(sh, g.cell_words, a.P, agg) <= 224 * 1024) cands.push_back({sh, (int)k});
-        }
-    if (cands.empty()) return RJ_OK;
-    char key[200];
-    std::snprintf(key, sizeof key, "label:%d:%d:%d:%d:%d:%d:%d:%d:%d", lc.ncol, lc.aggr, lc.aggr_ci >= 0,
+    }
+    auto smem = [&](int sh, const LabelPointArgs& g) {
+        return lp.tile ? label_tile_smem(sh, g.cell_words, a.P, lp.agg) : label_points_smem(sh, g.cell_words, a.P, lp.agg);
+    };
+    for (size_t k = 0; k < lp.sides.size(); ++k)
+        for (int sh = 0; sh < (lp.tile ? label_tile_shapes() : label_shapes()); ++sh)
+            if ((ctx->count_shape < 0 || ctx->count_shape == sh) && smem(sh, lp.sides[k].a) <= 224 * 1024)
+                lp.cands.push_back({sh, (int)k});
+    if (lp.cands.empty()) return false;
+    lp.small = a.n < kTuneMinPoints;
+    std::snprintf(lp.key, sizeof lp.key, "label:%d:%d:%d:%d:%d:%d:%d:%d:%d", lp.lc.ncol, lp.lc.aggr, lp.lc.aggr_ci >= 0,
                   rp.splitx * rp.splity > 1, tune_bucket((double)a.P), tune_bucket(npx), tune_bucket((double)a.n),
                   ctx->count_shape, ctx->count_bshift);
-    int tuned_i = -1;
-    const bool have = tuned_get(ctx, key, &tuned_i);
-    const bool known = cands.size() == 1 || have || small || ctx->capturing;
+    lp.have = tuned_get(ctx, lp.key, &lp.tuned);
+    return true;
+}
+
+// Builds the cell codes from the canvas's block codes and runs the planned
+// pass.  *done = false: it could not be launched (the caller takes the generic
+// pass).
+int run_label_points(rj_ctx* ctx, LabelPlan& lp, const TierArgs& tr, ExecState& es, bool* done) {
+    *done = false;
+    const auto& cands = lp.cands;
+    const bool known = cands.size() == 1 || lp.have || lp.small || ctx->capturing;
     std::pair<int, int> pick = cands.back();
-    if (have) pick = cands[std::min<size_t>((size_t)tuned_i, cands.size() - 1)];
+    if (lp.have) pick = cands[std::min<size_t>((size_t)lp.tuned, cands.size() - 1)];
     else if (cands.size() > 1)
         for (const auto& c : cands)
             if (c.first == 1) pick = c;   // small scans: 1024 threads, two pairs, the coarsest cells
     int rc;
-    std::vector<LabelPointArgs> args(sides.size(), a);
-    for (size_t k = 0; k < sides.size(); ++k) {
+    for (size_t k = 0; k < lp.sides.size(); ++k) {
         if (known && (int)k != pick.second) continue;
-        double ox, oy;
-        if (!grid(args[k], sides[k].first, &ox, &oy)) continue;
+        LabelPlan::Side& d = lp.sides[k];
+        d.a.tr = tr;
         uint16_t* cells;
-        if ((rc = scratch_t(ctx, k == 0 ? "label_cells0" : "label_cells1", (size_t)args[k].cell_words * 2, &cells))) return rc;
-        launch_label_cells(args[k], (float)ox, (float)oy, (float)ex, (float)ey, cells, ctx->sms, ctx->stream);
-        args[k].cells = cells;
+        if ((rc = scratch_t(ctx, k == 0 ? "label_cells0" : "label_cells1", (size_t)d.a.cell_words * 2, &cells))) return rc;
+        if (lp.tile) launch_label_blocks(tr, d.a.bs, d.a.cnx, d.a.cny, d.a.P, cells, ctx->sms, ctx->stream);
+        else launch_label_cells(d.a, (float)d.ox, (float)d.oy, (float)lp.errx, (float)lp.erry, cells, ctx->sms, ctx->stream);
+        d.a.cells = cells;
     }
     es.ph->mark(2);   // the cell codes belong to the polygon side
+    auto launch = [&](int shape, const LabelPointArgs& b, const LeanCols& lc) {
+        return lp.tile ? launch_label_tile(shape, b, lc, ctx->sms, ctx->stream)
+                       : launch_label_points(shape, b, lc, ctx->sms, ctx->stream);
+    };
     if (!known) {
         unsigned long long *tout, *tsum;
         double* tnf;
-        if ((rc = scratch_t(ctx, "tune_count", (size_t)a.P, &tout))) return rc;
-        if ((rc = scratch_t(ctx, "tune_sum", (size_t)a.P, &tsum))) return rc;
-        if ((rc = scratch_t(ctx, "tune_nonfinite", (size_t)a.P, &tnf))) return rc;
-        LeanCols tl = lc;
+        if ((rc = scratch_t(ctx, "tune_count", (size_t)lp.a.P, &tout))) return rc;
+        if ((rc = scratch_t(ctx, "tune_sum", (size_t)lp.a.P, &tsum))) return rc;
+        if ((rc = scratch_t(ctx, "tune_nonfinite", (size_t)lp.a.P, &tnf))) return rc;
+        LeanCols tl = lp.lc;
         tl.out_sum = tsum;
         tl.nonfinite = tnf;
-        const int pi = tune_pick(ctx, key, cands.size(), [&](size_t i) {
-            LabelPointArgs b = args[(size_t)cands[i].second];
+        const int pi = tune_pick(ctx, lp.key, cands.size(), [&](size_t i) {
+            LabelPointArgs b = lp.sides[(size_t)cands[i].second].a;
+            const uint64_t n = b.n;
             b.out_count = tout;
-            LabelPointArgs w = b;
-            w.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 16);   // first launch of a shape loads it
-            if (!launch_label_points(cands[i].first, w, tl, ctx->sms, ctx->stream)) return false;
-            b.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 28);
-            return launch_label_points(cands[i].first, b, tl, ctx->sms, ctx->stream);
+            b.n = std::min<uint64_t>(n & ~1ULL, 1ULL << 16);   // first launch of a shape loads it
+            if (!launch(cands[i].first, b, tl)) return false;
+            b.n = std::min<uint64_t>(n & ~1ULL, 1ULL << 28);
+            return launch(cands[i].first, b, tl);
         });
         RJ_CUDA(cudaGetLastError());
         if (pi < 0) return RJ_OK;
@@ -1452,12 +1349,60 @@ int label_points_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, con
     }
     ctx->passes = 1;
     ctx->copy_ms = 0;
-    if (!launch_label_points(pick.first, args[(size_t)pick.second], lc, ctx->sms, ctx->stream)) return RJ_OK;
+    const LabelPlan::Side& d = lp.sides[(size_t)pick.second];
+    if (!launch(pick.first, d.a, lp.lc)) return RJ_OK;
     RJ_CUDA(cudaGetLastError());
     ctx->last_count_shape = pick.first;
-    ctx->last_count_bshift = sides[(size_t)pick.second].second;
+    ctx->last_count_bshift = d.shift;
     *done = true;
     return RJ_OK;
+}
+
+// Label form of a one-tile canvas, for the lean pass: block codes, and the
+// pixel labels of the mixed blocks alone, each at its own place (slot = block:
+// no scan, no readback, no map to clear).  *overlap = true: some pixel centre
+// lies in two polygons (the caller takes the canvas path); else *done tells
+// whether the point pass ran.
+int label_blocks(rj_ctx* ctx, const DevFilter& f, const CanvasXf& cx, PolyPassArgs& a, uint64_t ckey, LabelPlan& lp,
+                 ExecState& es, bool* overlap) {
+    int rc;
+    *overlap = false;
+    TierArgs tr{};
+    tr.bw = (a.resx + 15) / 16;
+    tr.bh = (a.resy + 15) / 16;
+    const size_t nblk = (size_t)tr.bw * tr.bh;
+    unsigned long long* cnt;   // multi blocks, covered pixel writes, labelled pixels
+    if ((rc = scratch_t(ctx, "tier_full", nblk, &tr.full))) return rc;
+    if ((rc = scratch_t(ctx, "tier_mixed", nblk, &tr.mixed))) return rc;
+    if ((rc = scratch_t(ctx, "tier_code", nblk, &tr.code))) return rc;
+    if ((rc = scratch_t(ctx, "tier_plabel", nblk * 256, &tr.plabel))) return rc;
+    if ((rc = scratch_t(ctx, "tier_cnt", 3, &cnt))) return rc;
+    RJ_CUDA(cudaMemsetAsync(tr.full, 0xFF, nblk * 4, ctx->stream));
+    RJ_CUDA(cudaMemsetAsync(tr.mixed, 0, nblk * 4, ctx->stream));
+    RJ_CUDA(cudaMemsetAsync(cnt, 0, 3 * 8, ctx->stream));
+    if ((rc = poly_pass(ctx, MODE_TIER_CLASSIFY, a, &tr))) return rc;
+    launch_tier_codes(tr, nblk, cnt, ctx->sms, ctx->stream);
+    a.covered = cnt + 1;
+    if ((rc = poly_pass(ctx, MODE_TIER_LABEL, a, &tr, true))) return rc;
+    if (ctx->ps->overlap_on(ckey) == -1) {
+        if ((rc = readback_guard(ctx, "the first label map of a polygon set on a canvas"))) return rc;
+        launch_tier_nonempty(tr, nblk, cnt + 2, ctx->sms, ctx->stream);
+        unsigned long long hc[3] = {0, 0, 0};
+        RJ_CUDA(cudaMemcpyAsync(hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, ctx->stream));
+        RJ_CUDA(cudaStreamSynchronize(ctx->stream));
+        ctx->ps->overlap[ckey] = (hc[0] != 0 || hc[1] != hc[2]) ? 1 : 0;
+    }
+    if (ctx->ps->overlap_on(ckey) == 1) {
+        *overlap = true;
+        return RJ_OK;
+    }
+    bool lean = false;
+    if ((rc = run_label_points(ctx, lp, tr, es, &lean))) return rc;
+    if (!lean)
+        rc = point_pass(ctx, f, es.out_count, es.out_sum, [&](const PointArgs& pa) {
+            launch_tier_label_points(pa, cx, tr, ctx->sms, ctx->stream);
+        });
+    return rc;
 }
 
 // Lean point pass over the tiered canvas in its canvas form (rj_tier_lean.cu):
@@ -1470,7 +1415,7 @@ int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const 
                    size_t nblk, size_t spx, ExecState& es, bool* done) {
     *done = false;
     ctx->last_count_shape = ctx->last_count_bshift = -1;
-    if (ctx->streamed || f.general || f.ncol > label_lean_max_cols()) return RJ_OK;
+    if (ctx->streamed || f.general || f.ncol > kLeanMaxCols) return RJ_OK;
     PointArgs pa = make_point_args(ctx, f, es.out_count, es.out_sum);
     if (((uintptr_t)pa.xy & 15) != 0) return RJ_OK;
     LeanCols lc{};
@@ -1567,25 +1512,29 @@ int exec_raster(rj_ctx* ctx, const rj_query* q, ExecState& es, bool bounds) {
     bool use_label = !bounds && !(q->flags & RJ_FLAG_FORCE_CANVAS) && ctx->ps->overlap_on(ckey) != 1 &&
                      ctx->ps->P <= kMaxLabelPolys;
     if (use_label) {
-        uint16_t* label;
-        int overlap = 0;
-        if ((rc = label_map(ctx, a, "label", npix, nullptr, 0, ckey, &label, &overlap))) return rc;
-        es.ph->mark(2);
-        if (!overlap) {
-            bool lean = false;
-            if ((rc = label_count_pass(ctx, f, rp, label, es, &lean))) return rc;
-            if (!lean && (rc = point_pass(ctx, f, es.out_count, es.out_sum, [&](const PointArgs& pa) {
-                              launch_raster_label(pa, cx, label, ctx->sms, ctx->stream);
-                          })))
+        bool overlap = false;
+        LabelPlan lp;
+        if (T == 1 && plan_label_points(ctx, f, rp, cx, es, lp)) {
+            if ((rc = label_blocks(ctx, f, cx, a, ckey, lp, es, &overlap))) return rc;
+        } else {
+            uint16_t* label;
+            int ov = 0;
+            if ((rc = label_map(ctx, a, "label", npix, nullptr, 0, ckey, &label, &ov))) return rc;
+            overlap = ov != 0;
+            es.ph->mark(2);
+            if (!overlap && (rc = point_pass(ctx, f, es.out_count, es.out_sum, [&](const PointArgs& pa) {
+                                 launch_raster_label(pa, cx, label, ctx->sms, ctx->stream);
+                             })))
                 return rc;
+        }
+        if (!overlap) {
             RJ_CUDA(cudaGetLastError());
             es.ph->mark(3);
             es.ph->mark(4);
             return RJ_OK;
         }
-    } else {
-        es.ph->mark(2);
     }
+    es.ph->mark(2);
     // canvas path: point pass (additive splat) then polygon pass
     uint32_t* canvas_c;
     long long* canvas_s = nullptr;
@@ -2626,8 +2575,8 @@ int rj_set_tuning(rj_ctx* ctx, int32_t knob, int32_t value) {
             ctx->point_shape = value;
             return RJ_OK;
         case RJ_TUNE_COUNT_SHAPE:
-            if (value < -1 || value >= label_count_shapes())
-                return fail(ctx, RJ_E_INVALID, "count shape %d: -1..%d", value, label_count_shapes() - 1);
+            if (value < -1 || value >= kMaxShapes)
+                return fail(ctx, RJ_E_INVALID, "count shape %d: -1..%d", value, kMaxShapes - 1);
             ctx->count_shape = value;
             return RJ_OK;
         case RJ_TUNE_COUNT_BLOCK_SHIFT:
@@ -2657,8 +2606,8 @@ int rj_get_tuning(const rj_ctx* ctx, int32_t knob, int32_t* value) {
         case RJ_TUNE_COUNT_SHAPE: *value = ctx->last_count_shape; return RJ_OK;
         case RJ_TUNE_COUNT_BLOCK_SHIFT: *value = ctx->last_count_bshift; return RJ_OK;
         case RJ_TUNE_HYBRID_EXACT_SCALE: *value = ctx->hybrid_exact_scale; return RJ_OK;
-        case RJ_TUNE_COUNT_SHAPES: *value = label_count_shapes(); return RJ_OK;
-        case RJ_TUNE_LEAN_SHAPES: *value = label_lean_shapes(); return RJ_OK;
+        case RJ_TUNE_COUNT_SHAPES: *value = label_tile_shapes(); return RJ_OK;
+        case RJ_TUNE_LEAN_SHAPES: *value = label_shapes(); return RJ_OK;
         case RJ_TUNE_SPLAT_SHAPES: *value = splat_lean_shapes(); return RJ_OK;
         case RJ_TUNE_HYBRID_SHAPES: *value = hybrid_lean_shapes(); return RJ_OK;
         case RJ_TUNE_WAIT_LIMIT: *value = (int32_t)std::min<uint64_t>(ctx->wait_ns / 1000ull, 0x7FFFFFFFull); return RJ_OK;

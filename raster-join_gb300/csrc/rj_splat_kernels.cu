@@ -63,8 +63,7 @@ __global__ void __launch_bounds__(BLOCK) k_splat_lean(SplatLeanArgs a, LeanCols 
         __syncthreads();
         s_can = s_words + ((threadIdx.x >> 5) & (lc.copies - 1)) * HW * npix;
     }
-    const TileXf2 xf{a.col0.x, a.col0.y, __fmul_rn(a.col0.z, (float)kSub),
-                     a.row0.x, a.row0.y, __fmul_rn(a.row0.z, (float)kSub)};
+    const float Hx = __fmul_rn(a.col0.z, (float)kSub), Hy = __fmul_rn(a.row0.z, (float)kSub);
     const uint2* aggr2 = lc.aggr_col;
 
     const uint64_t npairs = a.n >> 1;
@@ -104,8 +103,8 @@ __global__ void __launch_bounds__(BLOCK) k_splat_lean(SplatLeanArgs a, LeanCols 
             for (int c = 0; c < NCOL; ++c) v[c] = hi ? cv[c][k].y : cv[c][k].x;
             const float x = hi ? p[k].z : p[k].x;
             const float y = hi ? p[k].w : p[k].y;
-            const int px = snapped_pixel(x, xf.sx, xf.tx, xf.Hx);
-            const int py = snapped_pixel(y, xf.sy, xf.ty, xf.Hy);
+            const int px = snapped_pixel(x, a.col0.x, a.col0.y, Hx);
+            const int py = snapped_pixel(y, a.row0.x, a.row0.y, Hy);
             if ((unsigned)px < (unsigned)a.resx && (unsigned)py < (unsigned)a.resy && splat_pass<NCOL>(lc, v)) {
                 float val = 0.f;
                 if (AGG) {
@@ -126,8 +125,8 @@ __global__ void __launch_bounds__(BLOCK) k_splat_lean(SplatLeanArgs a, LeanCols 
         uint32_t v[NCOL > 0 ? NCOL : 1];
         #pragma unroll
         for (int c = 0; c < NCOL; ++c) v[c] = __ldg(reinterpret_cast<const uint32_t*>(lc.col[c]) + i);
-        const int px = snapped_pixel(q.x, xf.sx, xf.tx, xf.Hx);
-        const int py = snapped_pixel(q.y, xf.sy, xf.ty, xf.Hy);
+        const int px = snapped_pixel(q.x, a.col0.x, a.col0.y, Hx);
+        const int py = snapped_pixel(q.y, a.row0.x, a.row0.y, Hy);
         if ((unsigned)px < (unsigned)a.resx && (unsigned)py < (unsigned)a.resy && splat_pass<NCOL>(lc, v)) {
             float fv = 0.f;
             if (AGG) {

@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
                 const uint32_t m8 = (S.M[k * 8 + (pr >> 1)] >> ((pr & 1) * 16 + ph)) & 0xFFu;
                 if (!m8) continue;
                 const size_t b = blk0 + bc_lo + S.list[k];
-                const size_t q = (size_t)__ldg(tr.slot + b) * 256 + (size_t)pr * 16 + ph;
+                const size_t q = (tr.slot ? (size_t)__ldg(tr.slot + b) : b) * 256 + (size_t)pr * 16 + ph;
                 if (MODE == MODE_TIER_LABEL) {
                     uint16_t* dst = tr.plabel + q;
                     if (m8 == 0xFFu) {
@@ -432,28 +432,48 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
 
 // code[b]: kTierMixed | slot for mixed blocks, else the full polygon (or
 // empty / multi); counts the multi blocks (two polygons cover them whole).
+// Without slots (slot = block) it also clears the pixel labels of the mixed
+// blocks, a warp writing one block's 512 bytes at a time.
 __global__ void k_tier_codes(TierArgs tr, size_t nblk, unsigned long long* multi) {
     unsigned long long c = 0;
-    for (size_t b = blockIdx.x * (size_t)blockDim.x + threadIdx.x; b < nblk; b += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t f = tr.full[b];
-        uint32_t code;
-        if (tr.mixed[b]) code = kTierMixed | (uint32_t)tr.slot[b];
-        else code = f;
-        c += (f == kTierMulti);
-        tr.code[b] = code;
+    const int lane = threadIdx.x & 31;
+    const uint4 none = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (size_t b0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) - lane; b0 < nblk;
+         b0 += (size_t)gridDim.x * blockDim.x) {
+        const size_t b = b0 + lane;
+        bool mixed = false;
+        if (b < nblk) {
+            const uint32_t f = tr.full[b];
+            mixed = tr.mixed[b] != 0u;
+            tr.code[b] = mixed ? kTierMixed | (tr.slot ? (uint32_t)tr.slot[b] : (uint32_t)b) : f;
+            c += (f == kTierMulti);
+        }
+        if (tr.slot) continue;
+        for (unsigned m = __ballot_sync(0xffffffffu, mixed); m; m &= m - 1u)
+            reinterpret_cast<uint4*>(tr.plabel + (b0 + __ffs(m) - 1) * 256)[lane] = none;
     }
     c = warp_sum_u64(c);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(multi, c);
+    if (lane == 0 && c) atomicAdd(multi, c);
 }
 
 // labelled pixels of the mixed blocks (overlap check: equals the pixel writes
-// when no two polygons share a pixel centre)
-__global__ void k_tier_nonempty(const uint16_t* __restrict__ plabel, size_t n, unsigned long long* count) {
+// when no two polygons share a pixel centre), a warp per 32 blocks
+__global__ void k_tier_nonempty(TierArgs tr, size_t nblk, unsigned long long* count) {
     unsigned long long c = 0;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        c += plabel[i] != kEmptyLabel;
+    const int lane = threadIdx.x & 31;
+    for (size_t b0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) - lane; b0 < nblk;
+         b0 += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t code = b0 + lane < nblk ? __ldg(tr.code + b0 + lane) : kTierEmpty;
+        for (unsigned m = __ballot_sync(0xffffffffu, code >= kTierMixed && code < kTierMulti); m; m &= m - 1u) {
+            const uint32_t slot = __shfl_sync(0xffffffffu, code, __ffs(m) - 1) & ~kTierMixed;
+            const uint4 v = reinterpret_cast<const uint4*>(tr.plabel + (size_t)slot * 256)[lane];
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) c += ((w[i] & 0xFFFFu) != kEmptyLabel) + ((w[i] >> 16) != kEmptyLabel);
+        }
+    }
     c = warp_sum_u64(c);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
+    if (lane == 0 && c) atomicAdd(count, c);
 }
 
 }  // namespace
@@ -482,9 +502,9 @@ void launch_tier_codes(const TierArgs& tr, size_t nblk, unsigned long long* mult
     ++g_kernel_launches;
 }
 
-void launch_tier_nonempty(const uint16_t* plabel, size_t n, unsigned long long* count, int sms, cudaStream_t st) {
-    const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)sms * 16);
-    k_tier_nonempty<<<std::max(blocks, 1), 256, 0, st>>>(plabel, n, count);
+void launch_tier_nonempty(const TierArgs& tr, size_t nblk, unsigned long long* count, int sms, cudaStream_t st) {
+    const int blocks = (int)std::min<size_t>((nblk + 255) / 256, (size_t)sms * 16);
+    k_tier_nonempty<<<std::max(blocks, 1), 256, 0, st>>>(tr, nblk, count);
     ++g_kernel_launches;
 }
 
