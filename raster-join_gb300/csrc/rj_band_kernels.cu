@@ -1,0 +1,514 @@
+// rj_band_kernels.cu -- the polygon passes that read a point canvas: the sum
+// over every polygon's covered pixels (polygon.frag:12-27) and the error-bound
+// outline pass (line-bound.frag:243-286).
+//
+// A polygon's covered pixels of a row are spans between its crossings with the
+// row's centre line, so with the canvas rows replaced by their prefix sums
+// (k_row_prefix) a span costs two reads whatever its length: the pass follows
+// the polygons' perimeters, not their areas.
+//
+// k_poly_bands: one warp per (tile, polygon, band of 16 rows).
+//   * the band's edges are staged in shared memory;
+//   * the (edge, row) crossings of the whole band are spread over the lanes
+//     (one exact division each) and kept in lists, one per row;
+//   * spans: the sorted crossings c0 <= c1 <= ... of a row bound the spans
+//     [c0, c1), [c2, c3), ...; a crossing's contribution to the sum is its
+//     prefix with the sign of its rank's parity, which the lane finds by
+//     comparing with the row's others -- no sorting, no order between lanes;
+//   * outline: the (edge, row) pairs are spread the same way; a lane takes the
+//     few pixels of its pair (a wide pair is taken by the whole warp), reads
+//     their counts together and clips the edge only against pixels that hold
+//     points; whether a pixel centre lies inside is the parity of the row's
+//     crossings right of it.
+#include <climits>
+
+#include "rj_bands.cuh"
+#include "rj_launch.h"
+
+namespace rj {
+
+namespace {
+
+// ---------------------------------------------------------------------------
+// Rows of the canvas -> inclusive prefix sums: counts in place (or into 64
+// bits, for tables of 2^32 rows and more), fixed-point sums in place (modulo
+// 2^64).  One block per row, four pixels per thread and step.
+constexpr int kPrefixThreads = 256;
+
+template <class T>
+__device__ __forceinline__ T block_scan(T v, T* s_warp, T& total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T x = v;
+    #pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    T base = 0;
+    total = 0;
+    #pragma unroll
+    for (int w = 0; w < kPrefixThreads / 32; ++w) {
+        const T s = s_warp[w];
+        base += w < warp ? s : T(0);
+        total += s;
+    }
+    __syncthreads();
+    return base + x;   // inclusive
+}
+
+template <class IN, class OUT>
+__device__ __forceinline__ void prefix_row(const IN* in, OUT* out, int n, OUT* s_warp) {
+    OUT carry = 0;
+    for (int x0 = 0; x0 < n; x0 += kPrefixThreads * 4) {
+        const int x = x0 + (int)threadIdx.x * 4;
+        OUT v[4];
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = x + i < n ? (OUT)in[x + i] : OUT(0);
+        #pragma unroll
+        for (int i = 1; i < 4; ++i) v[i] += v[i - 1];
+        OUT total;
+        const OUT before = carry + block_scan<OUT>(v[3], s_warp, total) - v[3];
+        #pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (x + i < n) out[x + i] = before + v[i];
+        carry += total;
+    }
+}
+
+__global__ void __launch_bounds__(kPrefixThreads) k_row_prefix(uint32_t* c, unsigned long long* wide, unsigned long long* s,
+                                                               int resx, int rows) {
+    __shared__ unsigned long long s_warp[kPrefixThreads / 32];
+    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+        const size_t at = (size_t)r * resx;
+        if (wide) prefix_row(c + at, wide + at, resx, s_warp);
+        else prefix_row(c + at, c + at, resx, reinterpret_cast<uint32_t*>(s_warp));
+        if (s) prefix_row(s + at, s + at, resx, s_warp);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Cohen-Sutherland clip of an edge against one pixel and the area fraction on
+// one side, computeFraction line-bound.frag:51-211, in fp32 window units.
+__device__ __forceinline__ int cs_outcode(float x, float y, float xmin, float ymin, float xmax, float ymax) {
+    int code = 0;
+    if (x < xmin) code |= 1;
+    else if (x > xmax) code |= 2;
+    if (y < ymin) code |= 4;
+    else if (y > ymax) code |= 8;
+    return code;
+}
+
+__device__ __forceinline__ float tri_area(float ax, float ay, float bx, float by, float cx, float cy) {
+    // abs(0.5 * length(cross(b - a, c - a))) with z = 0
+    float ix = __fsub_rn(bx, ax), iy = __fsub_rn(by, ay);
+    float jx = __fsub_rn(cx, ax), jy = __fsub_rn(cy, ay);
+    float cz = __fsub_rn(__fmul_rn(ix, jy), __fmul_rn(iy, jx));
+    return fabsf(__fmul_rn(0.5f, cz));
+}
+
+__device__ bool compute_fraction(float x0, float y0, float x1, float y1,
+                                 float xmin, float ymin, float xmax, float ymax, float& frac) {
+    int oc0 = cs_outcode(x0, y0, xmin, ymin, xmax, ymax);
+    int oc1 = cs_outcode(x1, y1, xmin, ymin, xmax, ymax);
+    bool accept = false;
+    frac = 0.0f;
+    for (int it = 0; it < 16; ++it) {   // the reference loops until accept/reject
+        if ((oc0 | oc1) == 0) { accept = true; break; }
+        if ((oc0 & oc1) != 0) break;
+        float x = 0.0f, y = 0.0f;
+        int out = (oc0 != 0) ? oc0 : oc1;
+        if (out & 8) {
+            x = __fadd_rn(x0, __fdiv_rn(__fmul_rn(__fsub_rn(x1, x0), __fsub_rn(ymax, y0)), __fsub_rn(y1, y0)));
+            y = ymax;
+        } else if (out & 4) {
+            x = __fadd_rn(x0, __fdiv_rn(__fmul_rn(__fsub_rn(x1, x0), __fsub_rn(ymin, y0)), __fsub_rn(y1, y0)));
+            y = ymin;
+        } else if (out & 2) {
+            y = __fadd_rn(y0, __fdiv_rn(__fmul_rn(__fsub_rn(y1, y0), __fsub_rn(xmax, x0)), __fsub_rn(x1, x0)));
+            x = xmax;
+        } else if (out & 1) {
+            y = __fadd_rn(y0, __fdiv_rn(__fmul_rn(__fsub_rn(y1, y0), __fsub_rn(xmin, x0)), __fsub_rn(x1, x0)));
+            x = xmin;
+        }
+        if (out == oc0) { x0 = x; y0 = y; oc0 = cs_outcode(x0, y0, xmin, ymin, xmax, ymax); }
+        else            { x1 = x; y1 = y; oc1 = cs_outcode(x1, y1, xmin, ymin, xmax, ymax); }
+    }
+    if (!accept) return false;
+    if (x0 > x1) { float t = x0; x0 = x1; x1 = t; t = y0; y0 = y1; y1 = t; }
+    float v1x = 0, v1y = 0, v2x = 0, v2y = 0, v3x = 0, v3y = 0, v4x = 0, v4y = 0;
+    bool tri = false, compute = true;
+    if (x0 == xmin) {
+        if (x1 == xmax) {                      // horizontal cut
+            v1x = xmin; v1y = ymin; v2x = xmax; v2y = ymin; v3x = x1; v3y = y1; v4x = x0; v4y = y0;
+        } else if (y1 == ymax) {
+            v1x = xmin; v1y = ymax; v2x = x0; v2y = y0; v3x = x1; v3y = y1; tri = true;
+        } else if (y1 == ymin) {
+            v1x = xmin; v1y = ymin; v2x = x0; v2y = y0; v3x = x1; v3y = y1; tri = true;
+        } else {
+            compute = false;
+        }
+    } else if (x1 == xmax) {
+        if (y0 == ymax) {
+            v1x = xmax; v1y = ymax; v2x = x0; v2y = y0; v3x = x1; v3y = y1; tri = true;
+        } else if (y0 == ymin) {
+            v1x = xmax; v1y = ymin; v2x = x1; v2y = y1; v3x = x0; v3y = y0; tri = true;
+        } else {
+            compute = false;
+        }
+    } else if (y0 == ymin && y1 == ymax) {     // vertical cut
+        v1x = xmin; v1y = ymin; v2x = xmin; v2y = ymax; v3x = x1; v3y = y1; v4x = x0; v4y = y0;
+    } else if (y1 == ymin && y0 == ymax) {     // vertical cut
+        v1x = xmin; v1y = ymin; v2x = xmin; v2y = ymax; v3x = x0; v3y = y0; v4x = x1; v4y = y1;
+    } else {
+        compute = false;
+    }
+    frac = 0.5f;
+    if (compute) {
+        float area = tri_area(v1x, v1y, v2x, v2y, v3x, v3y);
+        if (!tri) area = __fadd_rn(area, tri_area(v1x, v1y, v3x, v3y, v4x, v4y));
+        frac = __fdiv_rn(area, __fmul_rn(__fsub_rn(ymax, ymin), __fsub_rn(xmax, xmin)));
+    }
+    return true;
+}
+
+// ---------------------------------------------------------------------------
+constexpr int kBW = 8;             // warps per block
+constexpr int kBEdges = 128;       // staged edges per warp
+constexpr int kBCross = 512;       // crossings held per warp (rows of the band taken in groups that fit)
+
+struct BandWarp {
+    int4 edge[kBEdges];
+    int eidx[kBEdges];
+    uint32_t cross[kBCross];       // crossing column, clamped to the polygon's columns, | row << 16
+    int start[kBand + 1];          // first crossing of each row
+    int cur[kBand];                // crossings of each row
+};
+static_assert(sizeof(BandWarp) % 16 == 0, "BandWarp keeps 16-byte alignment");
+
+template <bool SPANS, bool OUTLINE, class C>
+__global__ void __launch_bounds__(kBW * 32, OUTLINE ? 2 : 3) k_poly_bands(PolyPassArgs a, const C* __restrict__ prefix) {
+    __shared__ BandWarp s_band[kBW];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned FULL = 0xffffffffu;
+    const int TP = a.T * a.P;
+    const int total = a.band_start[TP];
+    BandWarp& S = s_band[warp];
+
+    for (;;) {
+        int item = 0;
+        if (lane == 0) item = (int)atomicAdd(a.work_ctr, 1u);
+        item = __shfl_sync(FULL, item, 0);
+        if (item >= total) break;
+        const int tp = warp_find_owner(a.band_start, TP, item, lane);
+        const int t = tp / a.P, p = tp - t * a.P;
+        const int band = item - a.band_start[tp];
+        const int4 ia = a.info_a[tp];
+        const int2 ib = a.info_b[tp];
+        const int i_lo = ia.x, i_hi = ia.y, j_lo = ib.x, j_hi = ib.y;
+        const int jb = ia.z + band * kBand;
+        const int je = min(jb + kBand - 1, ia.w);
+        const int v0 = __ldg(a.pindex + p);
+        const int n = __ldg(a.pindex + p + 1) - v0;
+        const int2* pv = a.wv + (size_t)t * a.V + v0;
+        const float2* pf = OUTLINE ? a.wf + (size_t)t * a.V + v0 : nullptr;
+        const size_t row0 = ((size_t)t * a.resy + jb) * a.resx;   // first pixel of the band's first row
+
+        // edges within a pixel of the band's rows
+        const int64_t band_lo = (int64_t)jb * kSub - kSub;
+        const int64_t band_hi = (int64_t)(je + 1) * kSub + kSub;
+        int nb = 0;
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const int k = k0 + lane;
+            bool take = false;
+            int4 e = make_int4(0, 0, 0, 0);
+            if (k < n) {
+                const int2 A = pv[k];
+                const int2 B = pv[(k + 1 == n) ? 0 : k + 1];
+                take = (max(A.y, B.y) >= band_lo) && (min(A.y, B.y) <= band_hi);
+                e = make_int4(A.x, A.y, B.x, B.y);
+            }
+            const unsigned m = __ballot_sync(FULL, take);
+            const int pos = nb + __popc(m & ((1u << lane) - 1u));
+            if (take && pos < kBEdges) {
+                S.edge[pos] = e;
+                if (OUTLINE) S.eidx[pos] = k;
+            }
+            nb += __popc(m);
+        }
+        const bool overflow = nb > kBEdges;
+        const int ne = overflow ? n : nb;
+        auto edge_at = [&](int e) -> int4 {
+            if (!overflow) return S.edge[e];
+            const int2 A = pv[e];
+            const int2 B = pv[(e + 1 == n) ? 0 : e + 1];
+            return make_int4(A.x, A.y, B.x, B.y);
+        };
+        // crossings per row (rows whose centre the polygon can cross)
+        const int cl = max(j_lo, jb) - jb, ch = min(j_hi, je) - jb;
+        if (lane <= kBand) S.start[lane] = 0;
+        __syncwarp();
+        for (int e = lane; e < ne; e += 32) {
+            const int4 q = edge_at(e);
+            int r0, r1;
+            edge_rows(q.y, q.w, jb, r0, r1);
+            r0 = max(r0, cl);
+            r1 = min(r1, ch);
+            if (r0 <= r1) {
+                atomicAdd(&S.start[r0], 1);
+                atomicAdd(&S.start[r1 + 1], -1);
+            }
+        }
+        __syncwarp();
+        {
+            // differences -> counts -> first crossing of each row
+            int c = lane < kBand ? S.start[lane] : 0;
+            #pragma unroll
+            for (int o = 1; o < kBand; o <<= 1) {
+                const int v = __shfl_up_sync(FULL, c, o);
+                if (lane >= o) c += v;
+            }
+            int x = lane < kBand ? c : 0;
+            #pragma unroll
+            for (int o = 1; o < kBand; o <<= 1) {
+                const int v = __shfl_up_sync(FULL, x, o);
+                if (lane >= o) x += v;
+            }
+            __syncwarp();
+            if (lane < kBand) S.start[lane + 1] = x;
+            if (lane == 0) S.start[0] = 0;
+        }
+        __syncwarp();
+
+        unsigned long long acc_c = 0, acc_s = 0;
+        long long b_fn = 0, b_fp = 0, b_fn1 = 0, b_fp1 = 0;
+        const int nrows = je - jb + 1;
+        // inside test over every edge (a row with more crossings than are held)
+        auto inside_slow = [&](int i, int r) {
+            const int32_t cy = (jb + r) * kSub + kSub / 2;
+            bool in = false;
+            for (int k = 0; k < n; ++k) {
+                const int2 A = pv[k];
+                const int2 B = pv[(k + 1 == n) ? 0 : k + 1];
+                if (cross_row(A.y, B.y, cy)) in ^= (i < cross_L(A.x, A.y, B.x, B.y, cy));
+            }
+            return in;
+        };
+        auto prefix_at = [&](int r, int x) -> C {   // sum of the row's pixels [0, x)
+            return x > 0 ? __ldg(prefix + row0 + (size_t)r * a.resx + x - 1) : C(0);
+        };
+
+        for (int ra = 0; ra < nrows;) {
+            int rb = ra + 1;
+            while (rb < nrows && S.start[rb + 1] - S.start[ra] <= kBCross) ++rb;
+            const int base = S.start[ra], m = S.start[rb] - base;
+            const bool slow = m > kBCross;   // then one row
+            if (lane < kBand) S.cur[lane] = 0;
+            __syncwarp();
+            if (m > 0 && !slow) {
+                for_edge_rows(ne, jb, lane, edge_at, [&](const int4& q, int r) {
+                    const int32_t cy = (jb + r) * kSub + kSub / 2;
+                    if (r < max(ra, cl) || r >= rb || r > ch || !cross_row(q.y, q.w, cy)) return;
+                    const int L = max(min(max(cross_L(q.x, q.y, q.z, q.w, cy), i_lo), i_hi + 1), 0);
+                    S.cross[S.start[r] - base + atomicAdd(&S.cur[r], 1)] = (uint32_t)L | ((uint32_t)r << 16);
+                });
+            }
+            __syncwarp();
+            if (SPANS && m > 0 && i_lo <= i_hi) {
+                if (!slow) {
+                    for (int x = lane; x < m; x += 32) {
+                        const uint32_t mine = S.cross[x];
+                        const int r = (int)(mine >> 16), L = (int)(mine & 0xFFFFu);
+                        const int f = S.start[r] - base, e = f + S.cur[r];
+                        bool odd = false;
+                        for (int k = f; k < e; ++k) {
+                            const uint32_t o = S.cross[k];
+                            odd ^= o < mine || (o == mine && k < x);
+                        }
+                        const unsigned long long c = prefix_at(r, L);
+                        acc_c += odd ? c : 0ull - c;
+                        if (a.canvas_s && L > 0) {
+                            const unsigned long long s =
+                                (unsigned long long)__ldg(a.canvas_s + row0 + (size_t)r * a.resx + L - 1);
+                            acc_s += odd ? s : 0ull - s;
+                        }
+                    }
+                } else {
+                    for (int i = i_lo + lane; i <= i_hi; i += 32)
+                        if (inside_slow(i, ra)) {
+                            acc_c += (unsigned long long)(C)(prefix_at(ra, i + 1) - prefix_at(ra, i));
+                            if (a.canvas_s) {
+                                const long long* s = a.canvas_s + row0 + (size_t)ra * a.resx + i;
+                                acc_s += (unsigned long long)__ldg(s) - (i > 0 ? (unsigned long long)__ldg(s - 1) : 0ull);
+                            }
+                        }
+                }
+            }
+            if (OUTLINE) {
+                // counts of pixels i .. i + 3 of row r (those up to last)
+                auto counts = [&](int i, int last, int r, uint32_t (&v)[4]) {
+                    if (a.tier_code) {
+                        const int j = jb + r;
+                        const size_t b0 = (size_t)t * a.tier_bw * a.tier_bh + (size_t)(j >> 4) * a.tier_bw;
+                        uint32_t code[4];
+                        #pragma unroll
+                        for (int u = 0; u < 4; ++u) code[u] = i + u <= last ? __ldg(a.tier_code + b0 + ((i + u) >> 4)) : 0u;
+                        #pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            v[u] = 0u;
+                            if (i + u > last) continue;
+                            if (!(code[u] & kTierMixed) || code[u] >= kTierMulti)
+                                atomicOr(a.err, 4);   // never: such blocks are made mixed
+                            else
+                                v[u] = __ldg(a.tier_pcnt + (size_t)(code[u] & ~kTierMixed) * 256 + (j & 15) * 16 + ((i + u) & 15));
+                        }
+                    } else {
+                        C w[5];
+                        #pragma unroll
+                        for (int u = 0; u < 5; ++u) w[u] = i + u - 1 <= last ? prefix_at(r, i + u) : C(0);
+                        #pragma unroll
+                        for (int u = 0; u < 4; ++u) v[u] = i + u <= last ? (uint32_t)(w[u + 1] - w[u]) : 0u;
+                    }
+                };
+                auto visit = [&](const float2& P0, const float2& P1, int i, int r, uint32_t val) {
+                    const int j = jb + r;
+                    if (a.line_filter) {
+                        // varying interpolation along the line (projection of
+                        // the pixel centre), kept within 0.5 px: line-bound.frag:221
+                        const float cxp = (float)i + 0.5f, cyp = (float)j + 0.5f;
+                        const float dx = __fsub_rn(P1.x, P0.x), dy = __fsub_rn(P1.y, P0.y);
+                        const float l2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+                        if (!(l2 > 0.0f)) return;
+                        const float tt = __fdiv_rn(__fadd_rn(__fmul_rn(__fsub_rn(cxp, P0.x), dx),
+                                                             __fmul_rn(__fsub_rn(cyp, P0.y), dy)), l2);
+                        const float qx = __fadd_rn(P0.x, __fmul_rn(tt, dx));
+                        const float qy = __fadd_rn(P0.y, __fmul_rn(tt, dy));
+                        if (fabsf(__fsub_rn(qx, cxp)) >= 0.5f || fabsf(__fsub_rn(qy, cyp)) >= 0.5f) return;
+                    }
+                    float frac;
+                    if (!compute_fraction(P0.x, P0.y, P1.x, P1.y, (float)i, (float)j, (float)(i + 1), (float)(j + 1), frac))
+                        return;
+                    // inside test of the pixel centre: the coverage rule (an odd
+                    // number of the row's crossings right of i)
+                    bool inside = false;
+                    if (r >= cl && r <= ch) {
+                        if (slow) inside = inside_slow(i, r);
+                        else
+                            for (int k = S.start[r] - base, e = k + S.cur[r]; k < e; ++k)
+                                inside ^= (int)(S.cross[k] & 0xFFFFu) > i;
+                    }
+                    if (frac > 0.5f) frac = __fsub_rn(1.0f, frac);
+                    const int add = (int)ceilf(__fmul_rn(frac, (float)val));
+                    if (inside) { b_fp += add; b_fp1 += val; }
+                    else        { b_fn += add; b_fn1 += val; }
+                };
+                // (edge, row) pairs whose rectangles can touch: rows j with
+                // j <= the edge's top and j + 1 >= its bottom
+                spread_rows(
+                    ne, lane, 0,
+                    [&](int e, int& k, int& r0, int& cnt) {
+                        k = overflow ? e : S.eidx[e];
+                        const float2 P0 = pf[k], P1 = pf[(k + 1 == n) ? 0 : k + 1];
+                        const float lo = fminf(P0.y, P1.y) - (float)(jb + 1), hi = fmaxf(P0.y, P1.y) - (float)jb;
+                        r0 = max(lo > -32.0f ? (lo < 32.0f ? (int)ceilf(lo) : 32) : -32, ra);
+                        cnt = max(min(hi < 32.0f ? (hi > -32.0f ? (int)floorf(hi) : -32) : 32, rb - 1) - r0 + 1, 0);
+                    },
+                    [](int k, int lo) { return __shfl_sync(0xffffffffu, k, lo); },
+                    [&](bool live, int k, int r) {
+                        int i0 = 0, i1 = -1;
+                        float2 P0 = make_float2(0.f, 0.f), P1 = P0;
+                        if (live) {
+                            P0 = pf[k];
+                            P1 = pf[(k + 1 == n) ? 0 : k + 1];
+                            const float ylo = (float)(jb + r), yhi = (float)(jb + r + 1);
+                            // x range of the edge inside the row, widened by more
+                            // than the fp32 error of the clip's own arithmetic
+                            float xa, xb;
+                            if (P0.y == P1.y) {
+                                xa = fminf(P0.x, P1.x);
+                                xb = fmaxf(P0.x, P1.x);
+                            } else {
+                                const float ta = fminf(fmaxf((ylo - P0.y) / (P1.y - P0.y), 0.0f), 1.0f);
+                                const float tb = fminf(fmaxf((yhi - P0.y) / (P1.y - P0.y), 0.0f), 1.0f);
+                                const float x_a = P0.x + (P1.x - P0.x) * ta, x_b = P0.x + (P1.x - P0.x) * tb;
+                                xa = fminf(x_a, x_b);
+                                xb = fmaxf(x_a, x_b);
+                            }
+                            const float slack = 0.05f + 2e-6f * (fabsf(P0.x) + fabsf(P1.x));
+                            i0 = max(xa - slack > 0.0f ? (int)floorf(xa - slack) : 0, 0);
+                            i1 = xb + slack < (float)a.resx ? (int)floorf(xb + slack) : a.resx - 1;
+                        }
+                        // wide pairs: the whole warp, four pixels a lane
+                        for (unsigned wide = __ballot_sync(FULL, i1 - i0 >= 16); wide; wide &= wide - 1u) {
+                            const int src = __ffs(wide) - 1;
+                            const int wk = __shfl_sync(FULL, k, src), wr = __shfl_sync(FULL, r, src);
+                            const int w0 = __shfl_sync(FULL, i0, src), w1 = __shfl_sync(FULL, i1, src);
+                            const float2 Q0 = pf[wk], Q1 = pf[(wk + 1 == n) ? 0 : wk + 1];
+                            for (int i = w0 + lane * 4; i <= w1; i += 128) {
+                                uint32_t v[4];
+                                counts(i, w1, wr, v);
+                                #pragma unroll 1
+                                for (int u = 0; u < 4; ++u)
+                                    if (v[u]) visit(Q0, Q1, i + u, wr, v[u]);
+                            }
+                        }
+                        if (i1 - i0 < 16)
+                            for (int i = i0; i <= i1; i += 4) {
+                                uint32_t v[4];
+                                counts(i, i1, r, v);
+                                #pragma unroll 1
+                                for (int u = 0; u < 4; ++u)
+                                    if (v[u]) visit(P0, P1, i + u, r, v[u]);
+                            }
+                    });
+            }
+            __syncwarp();
+            ra = rb;
+        }
+        if (SPANS) {
+            acc_c = warp_sum_u64(acc_c);
+            if (lane == 0 && acc_c) atomicAdd(a.out_count + p, acc_c);
+            if (a.canvas_s) {
+                acc_s = warp_sum_u64(acc_s);
+                if (lane == 0 && acc_s) atomicAdd(a.out_sum + p, acc_s);
+            }
+        }
+        if (OUTLINE) {
+            b_fn = (long long)warp_sum_u64((unsigned long long)b_fn);
+            b_fp = (long long)warp_sum_u64((unsigned long long)b_fp);
+            b_fn1 = (long long)warp_sum_u64((unsigned long long)b_fn1);
+            b_fp1 = (long long)warp_sum_u64((unsigned long long)b_fp1);
+            if (lane == 0) {
+                if (b_fn) atomicAdd((unsigned long long*)(a.out_bounds + p), (unsigned long long)b_fn);
+                if (b_fp) atomicAdd((unsigned long long*)(a.out_bounds + a.P + p), (unsigned long long)b_fp);
+                if (b_fn1) atomicAdd((unsigned long long*)(a.out_bounds + 2 * a.P + p), (unsigned long long)b_fn1);
+                if (b_fp1) atomicAdd((unsigned long long*)(a.out_bounds + 3 * a.P + p), (unsigned long long)b_fp1);
+            }
+        }
+    }
+}
+
+}  // namespace
+
+void launch_row_prefix(uint32_t* counts, unsigned long long* wide, long long* sums, int resx, size_t rows, int sms,
+                       cudaStream_t st) {
+    const int blocks = (int)std::max<size_t>(1, std::min<size_t>(rows, (size_t)sms * 8));
+    k_row_prefix<<<blocks, kPrefixThreads, 0, st>>>(counts, wide, reinterpret_cast<unsigned long long*>(sums), resx, (int)rows);
+    ++g_kernel_launches;
+}
+
+void launch_poly_bands(bool spans, bool outline, const PolyPassArgs& a, int sms, cudaStream_t st) {
+    auto go = [&](auto kernel, auto prefix) {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBW * 32, 0);
+        kernel<<<sms * std::max(per_sm, 1), kBW * 32, 0, st>>>(a, prefix);
+    };
+    const bool w = a.canvas_w != nullptr;
+    if (spans && outline) w ? go(k_poly_bands<true, true, unsigned long long>, a.canvas_w) : go(k_poly_bands<true, true, uint32_t>, a.canvas_c);
+    else if (spans) w ? go(k_poly_bands<true, false, unsigned long long>, a.canvas_w) : go(k_poly_bands<true, false, uint32_t>, a.canvas_c);
+    else go(k_poly_bands<false, true, uint32_t>, a.canvas_c);
+    ++g_kernel_launches;
+}
+
+}  // namespace rj

@@ -247,6 +247,7 @@ void plan_query(rj_ctx* ctx, QPlan& p, bool no_fuse, bool fuse_all) {
         if (!fuse_all && (p.mode == BQ_LABEL || p.mode == BQ_SPLAT) && p.T == 1 && !p.f.general &&
             p.f.ncol <= kLeanMaxCols && p.r1 - p.r0 >= kLeanQueryRows)
             p.fused = false;   // rj_execute's lean pass (same results)
+        if ((p.r1 - p.r0) >> 32) p.fused = false;   // the canvas rows' prefix sums are 32-bit here
     }
 }
 
@@ -306,7 +307,11 @@ bool query_poly_pass(Engine& e, const QPlan& p, int mode, PolyScratch& s, unsign
     launch_poly_info(mode, a, ctx->sms, e.st);
     if (!launch_exclusive_scan(s.nbands, s.band_start, a.T * a.P, s.tmp, e.st)) return false;
     if (tier) launch_tier_pass(mode, a, *tier, ctx->sms, e.st);
-    else launch_poly_pass(mode, a, ctx->sms, e.st);
+    else if (mode == MODE_LABEL) launch_poly_label(a, ctx->sms, e.st);
+    else {
+        launch_row_prefix(p.cc, nullptr, p.cs, a.resx, (size_t)a.T * a.resy, ctx->sms, e.st);
+        launch_poly_bands(true, false, a, ctx->sms, e.st);
+    }
     return true;
 }
 

@@ -42,12 +42,13 @@ struct PolyPassArgs {
     const int* pindex;           // [P+1]
     int P, V, T;
     int resx, resy;
-    const uint32_t* canvas_c;    // [T][resy][resx] point counts
-    const long long* canvas_s;   // [T][resy][resx] fixed-point sums or null
+    // point canvas [T][resy][resx] as prefix sums along every row
+    // (launch_row_prefix): counts (canvas_w: in 64 bits), fixed-point sums or null
+    const uint32_t* canvas_c;
+    const unsigned long long* canvas_w;
+    const long long* canvas_s;
     uint16_t* label;             // [T][resy][resx] polygon label (MODE_LABEL)
     unsigned long long* covered; // MODE_LABEL: pixels covered, summed over polygons
-    const uint32_t* border;      // dilated hybrid border mask (skip) or null
-    int border_words;
     unsigned long long* out_count;
     unsigned long long* out_sum; // fixed-point sums (int64 two's complement)
     long long* out_bounds;       // [4P]
@@ -58,9 +59,8 @@ struct PolyPassArgs {
     int2* info_b;                // j_lo, j_hi (rows whose centre can be crossed)
     int* nbands;                 // bands of kBand rows
     const int* band_start;       // exclusive scan of nbands, [T*P + 1]
-    // MODE_BOUNDS over a tiered canvas (with TierArgs::outline): per-pixel
-    // counts from the mixed blocks' slots, no per-pixel reduction (the tier
-    // reduction gives the counts); a lookup outside a mixed block sets err
+    // the outline pass over a tiered canvas (with TierArgs::outline): per-pixel
+    // counts from the mixed blocks' slots; a lookup outside a mixed block sets err
     int outline_rows;            // tier classification for error bounds: bands over
                                  // every row an edge touches (k_poly_info)
     const uint32_t* tier_code;   // [T][bh][bw] or null (flat canvas)
@@ -199,7 +199,13 @@ void launch_col_absmax(const uint32_t* col, int typ, uint64_t n, unsigned* out_b
 void launch_transform_vertices(const float2* verts, int V, const float4* colxf, const float4* rowxf,
                                int splitx, int T, int2* wv, float2* wf, int sms, cudaStream_t st);
 void launch_poly_info(int mode, const PolyPassArgs& a, int sms, cudaStream_t st);
-void launch_poly_pass(int mode, const PolyPassArgs& a, int sms, cudaStream_t st);
+void launch_poly_label(const PolyPassArgs& a, int sms, cudaStream_t st);
+// canvas rows -> inclusive prefix sums, in place (wide: the counts' into 64 bits)
+void launch_row_prefix(uint32_t* counts, unsigned long long* wide, long long* sums, int resx, size_t rows, int sms,
+                       cudaStream_t st);
+// sums over the covered pixels of prefix-summed canvases (spans) and / or the
+// error-bound outline pass
+void launch_poly_bands(bool spans, bool outline, const PolyPassArgs& a, int sms, cudaStream_t st);
 void launch_grid_count(const GridArgs& g, int sms, cudaStream_t st);
 void launch_grid_fill(const GridArgs& g, int sms, cudaStream_t st);
 void launch_grid_sort(const int* cell_start, int* entries, int ncells, int sms, cudaStream_t st);

@@ -190,14 +190,6 @@ extern "C" RJ_API int rj_raster_count_noalloc(const float* d_xy, uint64_t npoint
     cx.tdy = (float)dy;
     cx.col0 = col;
     cx.row0 = row;
-    PointArgs pa{};
-    pa.xy = (const float2*)d_xy;
-    pa.n = npoints;
-    pa.P = 0;
-    pa.err = derr;
-    launch_raster_splat(pa, cx, canvas, nullptr, nd.sms, st);
-
-    // polygon pass: sum the canvas over each polygon's covered pixels
     PolyPassArgs a{};
     a.wv = wv;
     a.pindex = d_pindex;
@@ -215,7 +207,26 @@ extern "C" RJ_API int rj_raster_count_noalloc(const float* d_xy, uint64_t npoint
     a.band_start = (int*)(base + kOffBandStart);
     launch_poly_info(MODE_REDUCE, a, nd.sms, st);
     launch_exclusive_scan(a.nbands, (int*)(base + kOffBandStart), npolys, (int*)(base + kOffScan), st);
-    launch_poly_pass(MODE_REDUCE, a, nd.sms, st);
+    // points into the canvas, then the sums over each polygon's covered pixels;
+    // 2^31 points at a time (the canvas rows become 32-bit prefix sums)
+    uint64_t done = 0;
+    do {
+        const uint64_t rows = npoints - done < (1ull << 31) ? npoints - done : 1ull << 31;
+        if (done && (cudaMemsetAsync(canvas, 0, npix * sizeof(uint32_t), st) != cudaSuccess ||
+                     cudaMemsetAsync(ctr, 0, sizeof(unsigned), st) != cudaSuccess)) {
+            cudaGetLastError();
+            return na_fail(err, errlen, RJ_E_CUDA, "cudaMemsetAsync failed");
+        }
+        PointArgs pa{};
+        pa.xy = (const float2*)d_xy + done;
+        pa.n = rows;
+        pa.P = 0;
+        pa.err = derr;
+        launch_raster_splat(pa, cx, canvas, nullptr, nd.sms, st);
+        launch_row_prefix(canvas, nullptr, nullptr, resx, (size_t)resy, nd.sms, st);
+        launch_poly_bands(true, false, a, nd.sms, st);
+        done += rows;
+    } while (done < npoints);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return na_fail(err, errlen, RJ_E_CUDA, cudaGetErrorString(e));
     return RJ_OK;

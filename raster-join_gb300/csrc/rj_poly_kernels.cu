@@ -2,19 +2,17 @@
 //
 //  * k_transform_vertices : world -> per-tile window coordinates (float and
 //    1/256-pixel fixed point), the vertex stage of polygon.vert:9-13.
-//  * k_poly_pass<MODE>    : edge-function coverage of pixel centres, one warp
-//    per (tile, polygon), rows processed in bands whose edges are staged in
-//    shared memory.  MODE_REDUCE sums canvas counts/sums of covered pixels
-//    into the polygon (polygon.frag:12-27), MODE_LABEL writes a polygon label
-//    per covered pixel, MODE_BOUNDS additionally runs the error-bound outline
-//    pass (line-bound.frag:243-286).
+//  * k_poly_info          : per (tile, polygon) the pixels and rows it can reach.
+//  * k_poly_label         : a flat map of polygon labels by edge-function
+//    coverage of pixel centres (the passes over point canvases are in
+//    rj_band_kernels.cu).
 //  * grid index build     : index-size.glsl + create-index.glsl as a CSR grid.
 //  * hybrid border mask   : outline pass of HybridJoin::drawOutline
 //    (HybridJoin.cpp:197-268) as a conservative supercover + dilation.
 #include <climits>
 #include <cstdio>
 
-#include "rj_device.cuh"
+#include "rj_bands.cuh"
 #include "rj_launch.h"
 
 namespace rj {
@@ -42,98 +40,12 @@ __global__ void k_transform_vertices(const float2* __restrict__ verts, int V,
 }
 
 // ---------------------------------------------------------------------------
-// Cohen-Sutherland clip of an edge against one pixel and the area fraction on
-// one side, computeFraction line-bound.frag:51-211, in fp32 window units.
-__device__ __forceinline__ int cs_outcode(float x, float y, float xmin, float ymin, float xmax, float ymax) {
-    int code = 0;
-    if (x < xmin) code |= 1;
-    else if (x > xmax) code |= 2;
-    if (y < ymin) code |= 4;
-    else if (y > ymax) code |= 8;
-    return code;
-}
-
-__device__ __forceinline__ float tri_area(float ax, float ay, float bx, float by, float cx, float cy) {
-    // abs(0.5 * length(cross(b - a, c - a))) with z = 0
-    float ix = __fsub_rn(bx, ax), iy = __fsub_rn(by, ay);
-    float jx = __fsub_rn(cx, ax), jy = __fsub_rn(cy, ay);
-    float cz = __fsub_rn(__fmul_rn(ix, jy), __fmul_rn(iy, jx));
-    return fabsf(__fmul_rn(0.5f, cz));
-}
-
-__device__ bool compute_fraction(float x0, float y0, float x1, float y1,
-                                 float xmin, float ymin, float xmax, float ymax, float& frac) {
-    int oc0 = cs_outcode(x0, y0, xmin, ymin, xmax, ymax);
-    int oc1 = cs_outcode(x1, y1, xmin, ymin, xmax, ymax);
-    bool accept = false;
-    frac = 0.0f;
-    for (int it = 0; it < 16; ++it) {   // the reference loops until accept/reject
-        if ((oc0 | oc1) == 0) { accept = true; break; }
-        if ((oc0 & oc1) != 0) break;
-        float x = 0.0f, y = 0.0f;
-        int out = (oc0 != 0) ? oc0 : oc1;
-        if (out & 8) {
-            x = __fadd_rn(x0, __fdiv_rn(__fmul_rn(__fsub_rn(x1, x0), __fsub_rn(ymax, y0)), __fsub_rn(y1, y0)));
-            y = ymax;
-        } else if (out & 4) {
-            x = __fadd_rn(x0, __fdiv_rn(__fmul_rn(__fsub_rn(x1, x0), __fsub_rn(ymin, y0)), __fsub_rn(y1, y0)));
-            y = ymin;
-        } else if (out & 2) {
-            y = __fadd_rn(y0, __fdiv_rn(__fmul_rn(__fsub_rn(y1, y0), __fsub_rn(xmax, x0)), __fsub_rn(x1, x0)));
-            x = xmax;
-        } else if (out & 1) {
-            y = __fadd_rn(y0, __fdiv_rn(__fmul_rn(__fsub_rn(y1, y0), __fsub_rn(xmin, x0)), __fsub_rn(x1, x0)));
-            x = xmin;
-        }
-        if (out == oc0) { x0 = x; y0 = y; oc0 = cs_outcode(x0, y0, xmin, ymin, xmax, ymax); }
-        else            { x1 = x; y1 = y; oc1 = cs_outcode(x1, y1, xmin, ymin, xmax, ymax); }
-    }
-    if (!accept) return false;
-    if (x0 > x1) { float t = x0; x0 = x1; x1 = t; t = y0; y0 = y1; y1 = t; }
-    float v1x = 0, v1y = 0, v2x = 0, v2y = 0, v3x = 0, v3y = 0, v4x = 0, v4y = 0;
-    bool tri = false, compute = true;
-    if (x0 == xmin) {
-        if (x1 == xmax) {                      // horizontal cut
-            v1x = xmin; v1y = ymin; v2x = xmax; v2y = ymin; v3x = x1; v3y = y1; v4x = x0; v4y = y0;
-        } else if (y1 == ymax) {
-            v1x = xmin; v1y = ymax; v2x = x0; v2y = y0; v3x = x1; v3y = y1; tri = true;
-        } else if (y1 == ymin) {
-            v1x = xmin; v1y = ymin; v2x = x0; v2y = y0; v3x = x1; v3y = y1; tri = true;
-        } else {
-            compute = false;
-        }
-    } else if (x1 == xmax) {
-        if (y0 == ymax) {
-            v1x = xmax; v1y = ymax; v2x = x0; v2y = y0; v3x = x1; v3y = y1; tri = true;
-        } else if (y0 == ymin) {
-            v1x = xmax; v1y = ymin; v2x = x1; v2y = y1; v3x = x0; v3y = y0; tri = true;
-        } else {
-            compute = false;
-        }
-    } else if (y0 == ymin && y1 == ymax) {     // vertical cut
-        v1x = xmin; v1y = ymin; v2x = xmin; v2y = ymax; v3x = x1; v3y = y1; v4x = x0; v4y = y0;
-    } else if (y1 == ymin && y0 == ymax) {     // vertical cut
-        v1x = xmin; v1y = ymin; v2x = xmin; v2y = ymax; v3x = x0; v3y = y0; v4x = x1; v4y = y1;
-    } else {
-        compute = false;
-    }
-    frac = 0.5f;
-    if (compute) {
-        float area = tri_area(v1x, v1y, v2x, v2y, v3x, v3y);
-        if (!tri) area = __fadd_rn(area, tri_area(v1x, v1y, v3x, v3y, v4x, v4y));
-        frac = __fdiv_rn(area, __fmul_rn(__fsub_rn(ymax, ymin), __fsub_rn(xmax, xmin)));
-    }
-    return true;
-}
-
-// ---------------------------------------------------------------------------
 constexpr int kPolyWarps = 8;
-constexpr int kBand = 16;          // pixel rows per work item
 constexpr int kBandCap = 256;      // staged edges per warp
 constexpr int kCrossCap = 512;     // crossings per row per warp (sorted into spans)
-// dynamic shared memory of k_poly_pass: per warp the staged edges, their
-// indices and one row's crossings
-constexpr size_t kPolySmem = (size_t)kPolyWarps * (kBandCap * (sizeof(int4) + sizeof(int)) + kCrossCap * sizeof(int));
+// dynamic shared memory of k_poly_label: per warp the staged edges and one
+// row's crossings
+constexpr size_t kPolySmem = (size_t)kPolyWarps * (kBandCap * sizeof(int4) + kCrossCap * sizeof(int));
 
 // Ascending sort of buf[0, m) by one warp (bitonic network in shared memory,
 // m padded to a power of two with INT_MAX).
@@ -216,22 +128,19 @@ __global__ void k_poly_info(PolyPassArgs a) {
     }
 }
 
-// One warp per (tile, polygon, band of kBand rows): the band's edges are
-// staged in shared memory, each row's centre-line crossings are computed
-// exactly, and every pixel of the row is inside iff an odd number of
+// Flat label map.  One warp per (tile, polygon, band of kBand rows): the band's
+// edges are staged in shared memory, each row's centre-line crossings are
+// computed exactly, and every pixel of the row is inside iff an odd number of
 // crossings lies to its right.
-template <int MODE>
 __global__ void __launch_bounds__(kPolyWarps * 32)
-k_poly_pass(PolyPassArgs a) {
+k_poly_label(PolyPassArgs a) {
     extern __shared__ int4 s_poly[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned FULL = 0xffffffffu;
     const int TP = a.T * a.P;
     const int total = a.band_start[TP];
     int4* my_edge = s_poly + (size_t)warp * kBandCap;
-    int* my_eidx = reinterpret_cast<int*>(s_poly + (size_t)kPolyWarps * kBandCap) + (size_t)warp * kBandCap;
-    int* my_cross = reinterpret_cast<int*>(s_poly + (size_t)kPolyWarps * kBandCap) + (size_t)kPolyWarps * kBandCap +
-                    (size_t)warp * kCrossCap;
+    int* my_cross = reinterpret_cast<int*>(s_poly + (size_t)kPolyWarps * kBandCap) + (size_t)warp * kCrossCap;
 
     for (;;) {
         int item = 0;
@@ -249,12 +158,8 @@ k_poly_pass(PolyPassArgs a) {
         const int v0 = __ldg(a.pindex + p);
         const int n = __ldg(a.pindex + p + 1) - v0;
         const int2* pv = a.wv + (size_t)t * a.V + v0;
-        const float2* pf = a.wf ? a.wf + (size_t)t * a.V + v0 : nullptr;
         const size_t tile_off = (size_t)t * a.resx * a.resy;
-
-        unsigned long long acc_c = 0;
-        long long acc_s = 0;
-        long long b_fn = 0, b_fp = 0, b_fn1 = 0, b_fp1 = 0;
+        unsigned long long covered = 0;
 
         // fixed-point y window of the band (one pixel of margin each side)
         const int64_t band_lo = (int64_t)jb * kSub - kSub;
@@ -273,13 +178,13 @@ k_poly_pass(PolyPassArgs a) {
             }
             unsigned m = __ballot_sync(FULL, take);
             int pos = nb + __popc(m & ((1u << lane) - 1u));
-            if (take && pos < kBandCap) { my_edge[pos] = e; my_eidx[pos] = k; }
+            if (take && pos < kBandCap) my_edge[pos] = e;
             nb += __popc(m);
         }
         const bool overflow = nb > kBandCap;
         __syncwarp();
 
-        for (int j = jb; j <= je; ++j) {
+        for (int j = max(jb, j_lo); j <= min(je, j_hi); ++j) {
             const int32_t cy = j * kSub + kSub / 2;
             // crossings of this row's centre line: from the staged edges, or
             // from all edges of the polygon when the band held too many
@@ -305,177 +210,38 @@ k_poly_pass(PolyPassArgs a) {
                 if (c && pos < kCrossCap) my_cross[pos] = L;
                 m += __popc(bm);
             }
-            const bool cover_slow = m > kCrossCap;
             __syncwarp();
-            const bool centre_row = (j >= j_lo && j <= j_hi);
-            if (centre_row && m > 0) {
-                // pixel i is covered when an odd number of crossings lie at or
-                // left of it: with the crossings sorted, [c0, c1), [c2, c3), ...
-                auto visit = [&](int i) {
-                    if (MODE == MODE_BOUNDS && a.tier_code) return;   // counts: the tier reduction
-                    const size_t pix = tile_off + (size_t)j * a.resx + i;
-                    if (a.border) {
-                        uint32_t w = __ldg(a.border + ((size_t)j * a.border_words + (i >> 5)));
-                        if ((w >> (i & 31)) & 1u) return;
-                    }
-                    if (MODE == MODE_LABEL) {
-                        a.label[pix] = (uint16_t)p;   // overlaps detected by counting, see k_label_finish
-                        ++acc_c;
-                    } else {
-                        acc_c += __ldg(a.canvas_c + pix);
-                        if (a.canvas_s) acc_s += __ldg(a.canvas_s + pix);
-                    }
-                };
-                if (!cover_slow) {
-                    warp_sort_ints(my_cross, m, lane);   // the outline's inside test searches them too
-                    if (!(MODE == MODE_BOUNDS && a.tier_code))
-                    for (int s2 = 0; s2 + 1 < m; s2 += 2) {
-                        const int L = max(my_cross[s2], i_lo), R = min(my_cross[s2 + 1], i_hi + 1);
-                        for (int i = L + lane; i < R; i += 32) visit(i);
-                    }
-                } else {
-                    for (int i = i_lo + lane; i <= i_hi; i += 32) {
-                        bool inside = false;
-                        for (int k = 0; k < n; ++k) {
-                            int2 A = pv[k];
-                            int2 B = pv[(k + 1 == n) ? 0 : k + 1];
-                            if (cross_row(A.y, B.y, cy)) inside ^= (i < cross_L(A.x, A.y, B.x, B.y, cy));
-                        }
-                        if (inside) visit(i);
+            // pixel i is covered when an odd number of crossings lie at or
+            // left of it: with the crossings sorted, [c0, c1), [c2, c3), ...
+            // (overlaps are detected by counting, see k_label_finish)
+            uint16_t* row = a.label + tile_off + (size_t)j * a.resx;
+            if (m <= kCrossCap) {
+                warp_sort_ints(my_cross, m, lane);
+                for (int s2 = 0; s2 + 1 < m; s2 += 2) {
+                    const int L = max(my_cross[s2], i_lo), R = min(my_cross[s2 + 1], i_hi + 1);
+                    for (int i = L + lane; i < R; i += 32) {
+                        row[i] = (uint16_t)p;
+                        ++covered;
                     }
                 }
-            }
-            if (MODE == MODE_BOUNDS) {
-                // Outline pass: every edge of the polygon touching this pixel
-                // row, every pixel of the row the edge clips.  The (edge,
-                // pixel) pairs of 32 edges at a time are spread over the
-                // lanes, so a long edge does not leave the others idle.
-                const float ylo = (float)j, yhi = (float)(j + 1);
-                for (int e0 = 0; e0 < ne; e0 += 32) {
-                    const int e = e0 + lane;
-                    int k = 0, ia0 = 0, cnt = 0;
-                    if (e < ne) {
-                        k = overflow ? e : my_eidx[e];
-                        const float2 P0 = pf[k];
-                        const float2 P1 = pf[(k + 1 == n) ? 0 : k + 1];
-                        const float eylo = fminf(P0.y, P1.y), eyhi = fmaxf(P0.y, P1.y);
-                        if (!(eyhi < ylo - 0.01f || eylo > yhi + 0.01f)) {
-                            // x range of the edge inside the slab (conservative, +-1 px)
-                            float xa, xb;
-                            if (P0.y == P1.y) {
-                                xa = fminf(P0.x, P1.x); xb = fmaxf(P0.x, P1.x);
-                            } else {
-                                float ta = (ylo - P0.y) / (P1.y - P0.y);
-                                float tb = (yhi - P0.y) / (P1.y - P0.y);
-                                ta = fminf(fmaxf(ta, 0.0f), 1.0f);
-                                tb = fminf(fmaxf(tb, 0.0f), 1.0f);
-                                float x_a = P0.x + (P1.x - P0.x) * ta;
-                                float x_b = P0.x + (P1.x - P0.x) * tb;
-                                xa = fminf(x_a, x_b); xb = fmaxf(x_a, x_b);
-                            }
-                            ia0 = max((int)floorf(xa) - 1, 0);
-                            const int ib0 = min((int)floorf(xb) + 1, a.resx - 1);
-                            cnt = max(ib0 - ia0 + 1, 0);
-                        }
+            } else {
+                for (int i = i_lo + lane; i <= i_hi; i += 32) {
+                    bool inside = false;
+                    for (int k = 0; k < n; ++k) {
+                        int2 A = pv[k];
+                        int2 B = pv[(k + 1 == n) ? 0 : k + 1];
+                        if (cross_row(A.y, B.y, cy)) inside ^= (i < cross_L(A.x, A.y, B.x, B.y, cy));
                     }
-                    int incl = cnt;
-                    #pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int v = __shfl_up_sync(FULL, incl, o);
-                        if (lane >= o) incl += v;
-                    }
-                    const int npairs = __shfl_sync(FULL, incl, 31);
-                    for (int base = 0; base < npairs; base += 32) {
-                        const int idx = base + lane;
-                        int lo = 0, hi = 31;   // the lane whose edge holds pair idx
-                        #pragma unroll
-                        for (int st = 0; st < 5; ++st) {
-                            const int mid = (lo + hi) >> 1;
-                            if (__shfl_sync(FULL, incl, mid) > idx) hi = mid; else lo = mid + 1;
-                        }
-                        const int ke = __shfl_sync(FULL, k, lo);
-                        const int i = __shfl_sync(FULL, ia0, lo) + idx -
-                                      (__shfl_sync(FULL, incl, lo) - __shfl_sync(FULL, cnt, lo));
-                        if (idx >= npairs) continue;
-                        const float2 P0 = pf[ke];
-                        const float2 P1 = pf[(ke + 1 == n) ? 0 : ke + 1];
-                        uint32_t val;
-                        if (a.tier_code) {
-                            // the pixel's count in its mixed block's slot
-                            const size_t b = (size_t)t * a.tier_bw * a.tier_bh + (size_t)(j >> 4) * a.tier_bw + (i >> 4);
-                            const uint32_t code = __ldg(a.tier_code + b);
-                            if (!(code & kTierMixed) || code >= kTierMulti) {
-                                atomicOr(a.err, 4);   // never: such blocks are made mixed
-                                continue;
-                            }
-                            val = __ldg(a.tier_pcnt + (size_t)(code & ~kTierMixed) * 256 + (size_t)(j & 15) * 16 + (i & 15));
-                        } else {
-                            val = __ldg(a.canvas_c + tile_off + (size_t)j * a.resx + i);
-                        }
-                        if (val == 0) continue;
-                        if (a.line_filter) {
-                            // varying interpolation along the line (projection of
-                            // the pixel centre), kept within 0.5 px: line-bound.frag:221
-                            float cxp = (float)i + 0.5f, cyp = (float)j + 0.5f;
-                            float dx = __fsub_rn(P1.x, P0.x), dy = __fsub_rn(P1.y, P0.y);
-                            float l2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-                            if (!(l2 > 0.0f)) continue;
-                            float tt = __fdiv_rn(__fadd_rn(__fmul_rn(__fsub_rn(cxp, P0.x), dx),
-                                                          __fmul_rn(__fsub_rn(cyp, P0.y), dy)), l2);
-                            float qx = __fadd_rn(P0.x, __fmul_rn(tt, dx));
-                            float qy = __fadd_rn(P0.y, __fmul_rn(tt, dy));
-                            if (fabsf(__fsub_rn(qx, cxp)) >= 0.5f || fabsf(__fsub_rn(qy, cyp)) >= 0.5f) continue;
-                        }
-                        float frac;
-                        if (!compute_fraction(P0.x, P0.y, P1.x, P1.y, (float)i, ylo, (float)(i + 1), yhi, frac)) continue;
-                        // inside test of the pixel centre: the same coverage rule
-                        // (an odd number of the row's crossings right of i; the
-                        // crossings are sorted, so a binary search counts them)
-                        bool inside = false;
-                        if (!cover_slow && centre_row) {
-                            int clo = 0, chi = m;   // first crossing right of i
-                            while (clo < chi) {
-                                const int mid = (clo + chi) >> 1;
-                                if (my_cross[mid] <= i) clo = mid + 1; else chi = mid;
-                            }
-                            inside = ((m - clo) & 1) != 0;
-                        } else if (centre_row) {
-                            for (int kk = 0; kk < n; ++kk) {
-                                int2 A = pv[kk];
-                                int2 B = pv[(kk + 1 == n) ? 0 : kk + 1];
-                                if (cross_row(A.y, B.y, cy)) inside ^= (i < cross_L(A.x, A.y, B.x, B.y, cy));
-                            }
-                        }
-                        if (frac > 0.5f) frac = __fsub_rn(1.0f, frac);
-                        int toAdd = (int)ceilf(__fmul_rn(frac, (float)val));
-                        if (inside) { b_fp += toAdd; b_fp1 += val; }
-                        else        { b_fn += toAdd; b_fn1 += val; }
+                    if (inside) {
+                        row[i] = (uint16_t)p;
+                        ++covered;
                     }
                 }
             }
             __syncwarp();
         }
-        if (MODE == MODE_LABEL) {
-            acc_c = warp_sum_u64(acc_c);
-            if (lane == 0 && acc_c) atomicAdd(a.covered, acc_c);
-        } else {
-            acc_c = warp_sum_u64(acc_c);
-            if (a.canvas_s) acc_s = (long long)warp_sum_u64((unsigned long long)acc_s);
-            if (lane == 0 && acc_c) atomicAdd(a.out_count + p, acc_c);
-            if (lane == 0 && a.canvas_s && acc_s != 0) atomicAdd(a.out_sum + p, (unsigned long long)acc_s);
-        }
-        if (MODE == MODE_BOUNDS) {
-            b_fn = (long long)warp_sum_u64((unsigned long long)b_fn);
-            b_fp = (long long)warp_sum_u64((unsigned long long)b_fp);
-            b_fn1 = (long long)warp_sum_u64((unsigned long long)b_fn1);
-            b_fp1 = (long long)warp_sum_u64((unsigned long long)b_fp1);
-            if (lane == 0) {
-                if (b_fn) atomicAdd((unsigned long long*)(a.out_bounds + p), (unsigned long long)b_fn);
-                if (b_fp) atomicAdd((unsigned long long*)(a.out_bounds + a.P + p), (unsigned long long)b_fp);
-                if (b_fn1) atomicAdd((unsigned long long*)(a.out_bounds + 2 * a.P + p), (unsigned long long)b_fn1);
-                if (b_fp1) atomicAdd((unsigned long long*)(a.out_bounds + 3 * a.P + p), (unsigned long long)b_fp1);
-            }
-        }
+        covered = warp_sum_u64(covered);
+        if (lane == 0 && covered) atomicAdd(a.covered, covered);
     }
 }
 
@@ -962,26 +728,12 @@ void launch_poly_info(int mode, const PolyPassArgs& a, int sms, cudaStream_t st)
     else k_poly_info<MODE_REDUCE><<<blocks, 256, 0, st>>>(a);
 }
 
-template <int MODE>
-static void launch_poly_pass_t(const PolyPassArgs& a, int sms, cudaStream_t st) {
-    static bool attr_set = false;   // per template instance
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_poly_pass<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPolySmem);
-        attr_set = true;
-    }
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_poly_pass<MODE>, kPolyWarps * 32, kPolySmem);
-    const int blocks = sms * std::max(per_sm, 1);
-    k_poly_pass<MODE><<<blocks, kPolyWarps * 32, kPolySmem, st>>>(a);
-}
-
-void launch_poly_pass(int mode, const PolyPassArgs& a, int sms, cudaStream_t st) {
+void launch_poly_label(const PolyPassArgs& a, int sms, cudaStream_t st) {
     ++g_kernel_launches;
-    switch (mode) {
-        case MODE_REDUCE: launch_poly_pass_t<MODE_REDUCE>(a, sms, st); break;
-        case MODE_LABEL: launch_poly_pass_t<MODE_LABEL>(a, sms, st); break;
-        default: launch_poly_pass_t<MODE_BOUNDS>(a, sms, st); break;
-    }
+    cudaFuncSetAttribute(k_poly_label, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPolySmem);
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_poly_label, kPolyWarps * 32, kPolySmem);
+    k_poly_label<<<sms * std::max(per_sm, 1), kPolyWarps * 32, kPolySmem, st>>>(a);
 }
 
 void launch_grid_count(const GridArgs& g, int sms, cudaStream_t st) {

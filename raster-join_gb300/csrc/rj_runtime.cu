@@ -735,7 +735,8 @@ int poly_pass(rj_ctx* ctx, int mode, PolyPassArgs& a, const TierArgs* tier = nul
             return fail(ctx, RJ_E_INVALID, "too many (tile, polygon) items");
     }
     if (tier) launch_tier_pass(mode, a, *tier, ctx->sms, ctx->stream);
-    else launch_poly_pass(mode, a, ctx->sms, ctx->stream);
+    else if (mode == MODE_LABEL) launch_poly_label(a, ctx->sms, ctx->stream);
+    else launch_poly_bands(!a.tier_code, mode == MODE_BOUNDS, a, ctx->sms, ctx->stream);
     RJ_CUDA(cudaGetLastError());
     return RJ_OK;
 }
@@ -869,6 +870,22 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
     }
     es.ph->mark(4);
     return RJ_OK;
+}
+
+// Polygon pass over a point canvas (MODE_REDUCE, MODE_BOUNDS): its rows become
+// prefix sums in place.  A row's total can pass 2^32 only on tables that
+// large, whose counts are summed in 64 bits.
+int canvas_pass(rj_ctx* ctx, int mode, PolyPassArgs& a, uint32_t* canvas_c, long long* canvas_s) {
+    const size_t rows = (size_t)a.T * a.resy;
+    unsigned long long* wide = nullptr;
+    int rc;
+    if (ctx->npts >> 32 && (rc = scratch_t(ctx, "canvas_w", rows * a.resx, &wide))) return rc;
+    launch_row_prefix(canvas_c, wide, canvas_s, a.resx, rows, ctx->sms, ctx->stream);
+    a.canvas_c = canvas_c;
+    a.canvas_w = wide;
+    a.canvas_s = canvas_s;
+    a.label = nullptr;
+    return poly_pass(ctx, mode, a);
 }
 
 // Polygon label map of a canvas (MODE_LABEL).  Returns 1 in *overlap when
@@ -1552,10 +1569,7 @@ int exec_raster(rj_ctx* ctx, const rj_query* q, ExecState& es, bool bounds) {
         return rc;
     RJ_CUDA(cudaGetLastError());
     es.ph->mark(3);
-    a.canvas_c = canvas_c;
-    a.canvas_s = canvas_s;
-    a.label = nullptr;
-    if ((rc = poly_pass(ctx, bounds ? MODE_BOUNDS : MODE_REDUCE, a))) return rc;
+    if ((rc = canvas_pass(ctx, bounds ? MODE_BOUNDS : MODE_REDUCE, a, canvas_c, canvas_s))) return rc;
     es.ph->mark(4);
     return RJ_OK;
 }
@@ -1743,13 +1757,9 @@ int exec_hybrid(rj_ctx* ctx, const rj_query* q, ExecState& es) {
         return rc;
     RJ_CUDA(cudaGetLastError());
     es.ph->mark(3);
-    // polygon-inside pass over non-border pixels (polygon-inside.frag:30-57)
-    a.label = nullptr;
-    a.canvas_c = canvas_c;
-    a.canvas_s = canvas_s;
-    a.border = mask;
-    a.border_words = words;
-    if ((rc = poly_pass(ctx, MODE_REDUCE, a))) return rc;
+    // polygon-inside pass (polygon-inside.frag:30-57); the points of border
+    // pixels are not on the canvas
+    if ((rc = canvas_pass(ctx, MODE_REDUCE, a, canvas_c, canvas_s))) return rc;
     es.ph->mark(4);
     return RJ_OK;
 }

@@ -35,7 +35,7 @@
 //     block's first-pixel coverage and a 16-bit prefix XOR;
 //   * the listed blocks' pixel slots are then read or written by the whole
 //     warp, eight pixels a lane with vector loads and stores.
-#include "rj_device.cuh"
+#include "rj_bands.cuh"
 #include "rj_launch.h"
 #include "rj_point_map.cuh"
 
@@ -44,7 +44,7 @@ namespace rj {
 namespace {
 
 constexpr int kTW = 8;            // warps per block
-constexpr int kTBand = 16;        // rows per work item (one block row)
+constexpr int kTBand = kBand;     // rows per work item: one block row
 constexpr int kTEdgeCap = 256;    // staged edges per warp
 constexpr int kTBW = 16;          // block-bitmap words per row: 512 block columns = 8192 pixels
 constexpr int kTList = 64;        // blocks whose pixels one round visits
@@ -73,56 +73,6 @@ __device__ __forceinline__ uint32_t prefix_xor(uint32_t x) {
     x ^= x << 8;
     x ^= x << 16;
     return x;
-}
-
-// Rows [r0, r1] of the band (relative to jb) whose centre line the edge
-// with fixed-point ends y = ay, by crosses: ylo < cy <= yhi, cy = j * 256 + 128.
-__device__ __forceinline__ void edge_rows(int32_t ay, int32_t by, int jb, int& r0, int& r1) {
-    const int64_t ylo = min(ay, by), yhi = max(ay, by);
-    const int64_t a0 = ((ylo - kSub / 2) >> kSubpixelBits) + 1 - jb;
-    const int64_t a1 = ((yhi - kSub / 2) >> kSubpixelBits) - jb;
-    r0 = (int)(a0 < 0 ? 0 : a0);
-    r1 = (int)(a1 > kTBand - 1 ? kTBand - 1 : a1);
-}
-
-// f(q, r) for every (edge, band row) pair whose row centre line the edge's
-// y range spans, spread over the lanes: an edge crossing 16 rows gives 16
-// lanes work instead of one lane 16 exact divisions.  Every lane calls this
-// (warp-uniform loops); edge(e) returns staged edge e < ne.
-template <class E, class F>
-__device__ __forceinline__ void for_edge_rows(int ne, int jb, int lane, E&& edge, F&& f) {
-    const unsigned FULL = 0xffffffffu;
-    for (int e0 = 0; e0 < ne; e0 += 32) {
-        const int e = e0 + lane;
-        int4 q = make_int4(0, 0, 0, 0);
-        int r0 = 0, cnt = 0;
-        if (e < ne) {
-            q = edge(e);
-            int r1;
-            edge_rows(q.y, q.w, jb, r0, r1);
-            cnt = max(r1 - r0 + 1, 0);
-        }
-        int incl = cnt;
-        #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(FULL, incl, 31);
-        for (int base = 0; base < total; base += 32) {
-            const int idx = base + lane;
-            int lo = 0, hi = 31;   // the first lane whose inclusive count exceeds idx
-            #pragma unroll
-            for (int s = 0; s < 5; ++s) {
-                const int mid = (lo + hi) >> 1;
-                if (__shfl_sync(FULL, incl, mid) > idx) hi = mid; else lo = mid + 1;
-            }
-            const int4 qe = make_int4(__shfl_sync(FULL, q.x, lo), __shfl_sync(FULL, q.y, lo),
-                                      __shfl_sync(FULL, q.z, lo), __shfl_sync(FULL, q.w, lo));
-            const int first = __shfl_sync(FULL, r0, lo) + idx - (__shfl_sync(FULL, incl, lo) - __shfl_sync(FULL, cnt, lo));
-            if (idx < total) f(qe, first);
-        }
-    }
 }
 
 template <int MODE>
