@@ -78,7 +78,7 @@ struct Engine {
                                  // allocated on first use, mid-serving)
     int id = 0;                  // names the lanes' scratch apart from other engines'
     cudaStream_t lane_st[kLanes]{};
-    int* lane_err = nullptr;     // device: one error word per lane
+    bool lane_ready = false;     // lane streams and event made
     cudaEvent_t lane_ev = nullptr;
     void* lane_pin = nullptr;    // pinned staging of the lanes' outputs
     size_t lane_pin_bytes = 0;
@@ -110,8 +110,7 @@ void engine_free(Engine& e) {
         }
         s = nullptr;
     }
-    if (e.lane_err) cudaFree(e.lane_err);
-    e.lane_err = nullptr;
+    e.lane_ready = false;
     if (e.lane_ev) cudaEventDestroy(e.lane_ev);
     e.lane_ev = nullptr;
     if (e.lane_pin) cudaFreeHost(e.lane_pin);
@@ -818,14 +817,11 @@ struct LaneRun {
 int lanes_enqueue(Engine& e, LaneRun& lr, int& launches) {
     rj_ctx* ctx = e.ctx;
     if (lr.q.empty()) return RJ_OK;
-    if (!e.lane_err) {
+    if (!e.lane_ready) {
         for (auto& s : e.lane_st)
             if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return fail(ctx, RJ_E_CUDA, "lane stream");
         if (cudaEventCreateWithFlags(&e.lane_ev, cudaEventDisableTiming) != cudaSuccess) return fail(ctx, RJ_E_CUDA, "lane event");
-        if (cudaMalloc(&e.lane_err, kLanes * sizeof(int)) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(ctx, RJ_E_OOM, "lane error words");
-        }
+        e.lane_ready = true;
     }
     const size_t nq = lr.q.size();
     lr.off.assign(nq, 0);
@@ -835,8 +831,7 @@ int lanes_enqueue(Engine& e, LaneRun& lr, int& launches) {
     for (size_t i = 0; i < nq; ++i) {
         lr.off[i] = bytes;
         lr.bounds[i] = lr.q[i]->q->function_type == RJ_RASTER_JOIN_BOUNDS;
-        const size_t P = (size_t)lr.q[i]->ps->P;
-        bytes += al256(P * 24 + (lr.bounds[i] ? P * 32 : 0) + 8);
+        bytes += al256(QueryOut((size_t)lr.q[i]->ps->P, lr.bounds[i]).read);
     }
     if (e.lane_pin_bytes < bytes) {
         if (e.lane_pin) cudaFreeHost(e.lane_pin);
@@ -862,32 +857,21 @@ int lanes_enqueue(Engine& e, LaneRun& lr, int& launches) {
         // serving slot, a submit) interleave with a long batch
         std::lock_guard<std::recursive_mutex> lock(ctx->mu);
         cudaStream_t saved_st = ctx->stream;
-        int* saved_err = ctx->d_err;
         PolySet* saved_ps = ctx->ps;
         const std::string saved_ns = ctx->scratch_ns;
         QPlan& p = *lr.q[i];
         auto it = lane_of.find(p.ps);
         const int l = it != lane_of.end() ? it->second : (lane_of[p.ps] = (next++) % e.nlanes);
         ctx->stream = e.lane_st[l];
-        ctx->d_err = e.lane_err + l;
         ctx->scratch_ns = "#e" + std::to_string(e.id) + "." + std::to_string(l);
         ctx->ps = p.ps;
-        unsigned long long *oc = nullptr, *os = nullptr;
-        double* onf = nullptr;
-        long long* ob = nullptr;
-        int rc = enqueue_query_untimed(ctx, p.q, &oc, &os, &onf, &ob);
+        char* out = nullptr;
+        int rc = enqueue_query_untimed(ctx, p.q, &out);
         launches += g_kernel_launches;
         if (!rc) {
             lr.shift[i] = ctx->sum_shift;
-            const size_t P = (size_t)p.ps->P;
-            char* b = h + lr.off[i];
-            cudaStream_t st = ctx->stream;
-            if (cudaMemcpyAsync(b, oc, P * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                cudaMemcpyAsync(b + P * 8, os, P * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                cudaMemcpyAsync(b + P * 16, onf, P * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                (lr.bounds[i] && cudaMemcpyAsync(b + P * 24, ob, P * 32, cudaMemcpyDeviceToHost, st) != cudaSuccess) ||
-                cudaMemcpyAsync(b + P * (lr.bounds[i] ? 56 : 24), ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost,
-                                st) != cudaSuccess) {
+            if (cudaMemcpyAsync(h + lr.off[i], out, QueryOut((size_t)p.ps->P, lr.bounds[i]).read, cudaMemcpyDeviceToHost,
+                                ctx->stream) != cudaSuccess) {
                 cudaGetLastError();
                 rc = fail(ctx, RJ_E_CUDA, "query %d: copying its outputs back", p.idx);
             }
@@ -897,7 +881,6 @@ int lanes_enqueue(Engine& e, LaneRun& lr, int& launches) {
             p.status = rc;
         }
         ctx->stream = saved_st;
-        ctx->d_err = saved_err;
         ctx->ps = saved_ps;
         ctx->scratch_ns = saved_ns;
     }
@@ -936,17 +919,12 @@ int lanes_finish(Engine& e, LaneRun& lr) {
     for (size_t i = 0; i < lr.q.size(); ++i) {
         QPlan& p = *lr.q[i];
         if (p.status != RJ_OK) continue;
-        const size_t P = (size_t)p.ps->P;
         const char* b = h + lr.off[i];
-        int derr = 0;
-        std::memcpy(&derr, b + P * (lr.bounds[i] ? 56 : 24), sizeof derr);
-        if (derr) {
+        if (const int derr = *(const int*)(b + QueryOut((size_t)p.ps->P, lr.bounds[i]).err)) {
             p.status = fail(e.ctx, RJ_E_TIMEOUT, "query %d: a bounded device wait ran out (status 0x%x)", p.idx, derr);
             continue;
         }
-        decode_result((int)P, (const unsigned long long*)b, (const unsigned long long*)(b + P * 8),
-                      (const double*)(b + P * 16), lr.shift[i],
-                      lr.bounds[i] ? (const long long*)(b + P * 24) : nullptr, p.res);
+        decode_result(p.ps->P, b, lr.bounds[i], lr.shift[i], p.res);
     }
     lr.queued = false;
     return RJ_OK;

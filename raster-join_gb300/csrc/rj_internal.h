@@ -138,7 +138,16 @@ struct rj_ctx {
 
     rj_timings tm{};
     cudaEvent_t ev[8]{};
-    int* d_err = nullptr;     // device status word of bounded waits
+    int* d_err = nullptr;     // device status word of rj_selftest_bounded_wait
+    // the current query's outputs (one scratch block, laid out as QueryOut says)
+    double* q_nonfinite = nullptr;
+    int* q_err = nullptr;            // status word: bounded waits, outline reads
+    unsigned* q_ctr = nullptr;       // zeroed work counters of its polygon passes
+    int q_ctr_used = 0;
+    void* pin = nullptr;             // pinned host copy of rj_execute's outputs
+    size_t pin_bytes = 0;
+    int live_plans = 0;              // prepared queries: their graphs hold scratch addresses
+    std::vector<rjh::DevBuf> retired;   // outgrown scratch those graphs may still use
     int sum_shift = 0;        // fixed-point scale 2^s of the current query's sums
     uint64_t row0 = 0, row1 = ~0ULL;   // rows of the current query (time index window)
     int server_running = 0;   // a serving loop owns the context
@@ -180,12 +189,7 @@ struct rj_plan {
     bool uses_tix = false;   // the captured row window came from the time index
     const void* ps = nullptr;
     uint64_t npts = 0;
-    // pinned host copies of the per-polygon outputs, written by the graph
-    unsigned long long* hc = nullptr;
-    unsigned long long* hq = nullptr;
-    double* hnf = nullptr;
-    long long* hb = nullptr;
-    int* derr = nullptr;
+    void* out = nullptr;     // pinned host copy of the outputs (QueryOut), written by the graph
 };
 
 struct rj_polyset {
@@ -220,6 +224,23 @@ inline bool query_tier(uint32_t flags, size_t npix, uint64_t rows) {
 
 int fail(rj_ctx* c, int code, const char* fmt, ...);
 
+// A query's outputs: one block, zeroed by one memset and read back by one
+// copy: count[P], fixed-point sum[P], non-finite sum[P], the status word, then
+// (error bounds only) bounds[4P].  Work counters of the polygon passes follow.
+constexpr int kQueryCounters = 8;
+struct QueryOut {
+    size_t sum, nonfinite, err, bounds, read, counters, bytes;   // byte offsets; `read`: bytes to copy back
+    QueryOut(size_t P, bool with_bounds) {
+        sum = P * 8;
+        nonfinite = P * 16;
+        err = P * 24;
+        bounds = err + 8;
+        counters = bounds + P * 32;
+        bytes = counters + kQueryCounters * 4;
+        read = with_bounds ? counters : bounds;
+    }
+};
+
 #define RJ_CUDA(call)                                                                         \
     do {                                                                                      \
         cudaError_t e_ = (call);                                                              \
@@ -251,15 +272,15 @@ int load_polyset(rj_ctx* ctx, PolySet& s, const float* xy, const int32_t* pindex
 void free_polyset(rj_ctx* ctx, PolySet& s);
 // rows [r0, r1) of the resident table a query can touch (all rows without a
 // time index on its time attribute)
+void decode_result(int P, const char* out, bool bounds, int shift, rj_result* res);
 void decode_result(int P, const unsigned long long* hc, const unsigned long long* hq, const double* hnf, int shift,
                    const long long* hb, rj_result* res);
 void free_batch_engine(rj_ctx* ctx);
 // One query's device work queued on ctx->stream (the readbacks some forms
-// need aside, no host synchronisation) with the context's scratch and error
-// word; the per-polygon outputs stay on the device for the caller to copy.
+// need aside, no host synchronisation) with the context's scratch; its output
+// block (QueryOut) stays on the device for the caller to copy.
 // ctx->sum_shift holds the query's fixed-point shift on return.
-int enqueue_query_untimed(rj_ctx* ctx, const rj_query* q, unsigned long long** oc, unsigned long long** os,
-                          double** onf, long long** ob);
+int enqueue_query_untimed(rj_ctx* ctx, const rj_query* q, char** out);
 void query_rows(const rj_ctx* ctx, const rj_query* q, uint64_t& r0, uint64_t& r1);
 int ensure_zones(rj_ctx* ctx);
 

@@ -161,13 +161,6 @@ struct PointArgs {
 };
 constexpr int kZoneShift = 10;               // zones of 1024 rows
 void launch_zone_boxes(const float2* xy, uint64_t n, float4* zones, int sms, cudaStream_t st);
-// per-tile transforms written by a kernel from its arguments (no host copy;
-// used while a query is captured into a graph)
-constexpr int kXfArgs = 16;
-struct XfArgs {
-    float4 v[kXfArgs];
-};
-void launch_write_xf(const XfArgs& a, int n, float4* dst, cudaStream_t st);
 // one CTA waits, bounded by limit_ns of wall time, on an mbarrier nothing
 // arrives on; sets bit 0 of *err when the wait runs out
 void launch_wait_selftest(int* err, uint64_t limit_ns, cudaStream_t st);
@@ -196,6 +189,14 @@ struct HybridArgs {
 void launch_col_absmax(const uint32_t* col, int typ, uint64_t n, unsigned* out_bits, int sms, cudaStream_t st);
 
 // polygon side
+// tile transforms passed as kernel arguments (up to kXfArgs per axis), which
+// the kernel also writes to dcol / drow for the later passes
+constexpr int kXfArgs = 16;
+struct XfArgs {
+    float4 v[kXfArgs];
+};
+void launch_transform_vertices_xf(const float2* verts, int V, const XfArgs& col, const XfArgs& row, int splitx, int T, int2* wv,
+                                  float2* wf, float4* dcol, float4* drow, int sms, cudaStream_t st);
 void launch_transform_vertices(const float2* verts, int V, const float4* colxf, const float4* rowxf,
                                int splitx, int T, int2* wv, float2* wf, int sms, cudaStream_t st);
 void launch_poly_info(int mode, const PolyPassArgs& a, int sms, cudaStream_t st);

@@ -20,23 +20,38 @@ namespace rj {
 thread_local int g_kernel_launches = 0;
 
 // ---------------------------------------------------------------------------
-__global__ void k_transform_vertices(const float2* __restrict__ verts, int V,
-                                     const float4* __restrict__ colxf,  // per tile column: (sx, tx, hx, -)
-                                     const float4* __restrict__ rowxf,  // per tile row:    (sy, ty, hy, -)
-                                     int splitx, int T,
-                                     int2* __restrict__ wv, float2* __restrict__ wf) {
+// tile column and row transforms: (sx, tx, hx, -) and (sy, ty, hy, -)
+template <class COL, class ROW>
+__device__ __forceinline__ void transform_vertices(const float2* __restrict__ verts, int V, COL&& col, ROW&& row, int splitx,
+                                                   int T, int2* __restrict__ wv, float2* __restrict__ wf) {
     size_t total = (size_t)T * V;
     for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < total; g += (size_t)gridDim.x * blockDim.x) {
         int t = (int)(g / V);
         int v = (int)(g - (size_t)t * V);
-        int cx = t % splitx, cy = t / splitx;
-        float4 cxf = __ldg(colxf + cx), ryf = __ldg(rowxf + cy);
+        const float4 cxf = col(t % splitx), ryf = row(t / splitx);
         float2 p = __ldg(verts + v);
         float wx = win_coord(p.x, cxf.x, cxf.y, cxf.z);
         float wy = win_coord(p.y, ryf.x, ryf.y, ryf.z);
         wv[g] = make_int2(snap_win(wx), snap_win(wy));
         if (wf) wf[g] = make_float2(wx, wy);
     }
+}
+
+__global__ void k_transform_vertices(const float2* verts, int V, const float4* __restrict__ colxf,
+                                     const float4* __restrict__ rowxf, int splitx, int T, int2* wv, float2* wf) {
+    transform_vertices(verts, V, [&](int c) { return __ldg(colxf + c); }, [&](int r) { return __ldg(rowxf + r); }, splitx, T,
+                       wv, wf);
+}
+
+// the transforms as arguments, also written where the later passes read them
+__global__ void k_transform_vertices_xf(const float2* verts, int V, __grid_constant__ const XfArgs col,
+                                        __grid_constant__ const XfArgs row, int splitx, int T, int2* wv, float2* wf,
+                                        float4* dcol, float4* drow) {
+    if (blockIdx.x == 0 && threadIdx.x < kXfArgs) {
+        if ((int)threadIdx.x < splitx) dcol[threadIdx.x] = col.v[threadIdx.x];
+        if ((int)threadIdx.x < T / splitx) drow[threadIdx.x] = row.v[threadIdx.x];
+    }
+    transform_vertices(verts, V, [&](int c) { return col.v[c]; }, [&](int r) { return row.v[r]; }, splitx, T, wv, wf);
 }
 
 // ---------------------------------------------------------------------------
@@ -634,6 +649,33 @@ __global__ void k_scan_sums(int* __restrict__ tile_sums, int ntiles, int* __rest
     if (threadIdx.x == blockDim.x - 1) *total_out = ex;
 }
 
+// Short arrays: one block, tile after tile.
+__global__ void __launch_bounds__(kScanThreads) k_scan_small(const int* in, int* out, int n) {
+    __shared__ int s_warp[32];
+    __shared__ int s_carry;
+    if (threadIdx.x == 0) s_carry = 0;
+    __syncthreads();
+    for (int base = 0; base < n; base += kScanTile) {
+        const int i0 = base + (int)threadIdx.x * kScanItems;
+        int v[kScanItems], local = 0;
+        #pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            v[k] = i0 + k < n ? in[i0 + k] : 0;
+            local += v[k];
+        }
+        int ex = s_carry + block_exclusive_scan(local, s_warp);
+        #pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            if (i0 + k < n) out[i0 + k] = ex;
+            ex += v[k];
+        }
+        __syncthreads();
+        if (threadIdx.x == blockDim.x - 1) s_carry = ex;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[n] = s_carry;
+}
+
 __global__ void k_scan_add(int* __restrict__ out, int n, const int* __restrict__ tile_sums) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < (size_t)n) out[i] += tile_sums[i / kScanTile];
@@ -718,6 +760,14 @@ void launch_transform_vertices(const float2* verts, int V, const float4* colxf, 
     ++g_kernel_launches;
 }
 
+void launch_transform_vertices_xf(const float2* verts, int V, const XfArgs& col, const XfArgs& row, int splitx, int T, int2* wv,
+                                  float2* wf, float4* dcol, float4* drow, int sms, cudaStream_t st) {
+    const size_t total = (size_t)T * V;
+    const int blocks = (int)std::max<size_t>(1, std::min<size_t>((total + 255) / 256, (size_t)sms * 8));
+    k_transform_vertices_xf<<<blocks, 256, 0, st>>>(verts, V, col, row, splitx, T, wv, wf, dcol, drow);
+    ++g_kernel_launches;
+}
+
 void launch_poly_info(int mode, const PolyPassArgs& a, int sms, cudaStream_t st) {
     int items = a.T * a.P;
     int blocks = std::min((items * 32 + 255) / 256, sms * 8);
@@ -769,6 +819,12 @@ int scan_tmp_ints(int n) {
 }
 
 bool launch_exclusive_scan(const int* in, int* out, int n, int* tmp, cudaStream_t st) {
+    // three launches cost about 7 us, one block about 1.2 us per tile of 4096
+    if (n <= 4 * kScanTile) {
+        k_scan_small<<<1, kScanThreads, 0, st>>>(in, out, n);
+        ++g_kernel_launches;
+        return true;
+    }
     int ntiles = (n + kScanTile - 1) / kScanTile;
     if (ntiles < 1) ntiles = 1;
     k_scan_tiles<<<ntiles, kScanThreads, 0, st>>>(in, out, n, tmp);

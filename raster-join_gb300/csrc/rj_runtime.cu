@@ -86,6 +86,10 @@ DevBuf& scratch_buf(rj_ctx* ctx, const char* key) {
 
 int scratch(rj_ctx* ctx, const char* key, size_t bytes, void** out) {
     DevBuf& b = scratch_buf(ctx, key);
+    if (ctx->live_plans && b.p && b.bytes < bytes) {   // a prepared query's graph may hold its address
+        ctx->retired.push_back(b);
+        b = DevBuf{};
+    }
     int rc = dev_alloc(ctx, b, bytes);
     if (rc) return rc;
     *out = b.p;
@@ -327,25 +331,28 @@ int transform_vertices(rj_ctx* ctx, const std::vector<float4>& colxf, const std:
     int rc;
     if ((rc = scratch_t(ctx, "colxf", colxf.size(), &dcol))) return rc;
     if ((rc = scratch_t(ctx, "rowxf", rowxf.size(), &drow))) return rc;
-    if (ctx->capturing) {
-        // a graph must not copy from host memory that is gone when it
-        // replays: the transforms travel as kernel arguments instead
-        if (colxf.size() > (size_t)kXfArgs || rowxf.size() > (size_t)kXfArgs)
-            return fail(ctx, RJ_E_UNSUPPORTED, "more than %d canvas tiles per axis: this query cannot be prepared", kXfArgs);
-        XfArgs ca{}, ra{};
-        for (size_t i = 0; i < colxf.size(); ++i) ca.v[i] = colxf[i];
-        for (size_t i = 0; i < rowxf.size(); ++i) ra.v[i] = rowxf[i];
-        launch_write_xf(ca, (int)colxf.size(), dcol, ctx->stream);
-        launch_write_xf(ra, (int)rowxf.size(), drow, ctx->stream);
+    // up to kXfArgs tiles per axis travel as kernel arguments (no copies; a
+    // graph must not copy from host memory that is gone when it replays)
+    const bool by_value = colxf.size() <= (size_t)kXfArgs && rowxf.size() <= (size_t)kXfArgs;
+    XfArgs ca{}, ra{};
+    if (by_value) {
+        std::copy(colxf.begin(), colxf.end(), ca.v);
+        std::copy(rowxf.begin(), rowxf.end(), ra.v);
     } else {
+        if (ctx->capturing)
+            return fail(ctx, RJ_E_UNSUPPORTED, "more than %d canvas tiles per axis: this query cannot be prepared", kXfArgs);
         RJ_CUDA(cudaMemcpyAsync(dcol, colxf.data(), colxf.size() * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
         RJ_CUDA(cudaMemcpyAsync(drow, rowxf.data(), rowxf.size() * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
     }
     if ((rc = scratch_t(ctx, "wv", (size_t)T * ctx->ps->V, wv))) return rc;
     *wf = nullptr;
     if (want_float && (rc = scratch_t(ctx, "wf", (size_t)T * ctx->ps->V, wf))) return rc;
-    launch_transform_vertices((const float2*)ctx->ps->d_verts.p, ctx->ps->V, dcol, drow, (int)colxf.size(), T, *wv,
-                              want_float ? *wf : nullptr, ctx->sms, ctx->stream);
+    if (by_value)
+        launch_transform_vertices_xf((const float2*)ctx->ps->d_verts.p, ctx->ps->V, ca, ra, (int)colxf.size(), T, *wv,
+                                     want_float ? *wf : nullptr, dcol, drow, ctx->sms, ctx->stream);
+    else
+        launch_transform_vertices((const float2*)ctx->ps->d_verts.p, ctx->ps->V, dcol, drow, (int)colxf.size(), T, *wv,
+                                  want_float ? *wf : nullptr, ctx->sms, ctx->stream);
     RJ_CUDA(cudaGetLastError());
     return RJ_OK;
 }
@@ -589,8 +596,8 @@ PointArgs make_point_args(rj_ctx* ctx, const DevFilter& f, unsigned long long* o
     pa.P = ctx->ps->P;
     pa.out_count = oc;
     pa.out_sum = os;
-    pa.out_nonfinite = (double*)scratch_buf(ctx, "out_nonfinite").p;
-    pa.err = ctx->d_err;
+    pa.out_nonfinite = ctx->q_nonfinite;
+    pa.err = ctx->q_err;
     pa.shape = ctx->point_shape;
     pa.wait_ns = ctx->wait_ns;
     // the zone check costs a dependent load per iteration: skip it when the
@@ -711,20 +718,18 @@ struct ExecState {
 // reuse: the bands of the pass just before (same polygons, tiles and band
 // layout) still stand; only the work counter is new.
 int poly_pass(rj_ctx* ctx, int mode, PolyPassArgs& a, const TierArgs* tier = nullptr, bool reuse = false) {
-    unsigned int* ctr;
     int rc;
     const int TP = a.T * a.P;
     int4* info_a;
     int2* info_b;
     int *nbands, *band_start, *tmp;
-    if ((rc = scratch_t(ctx, "work_ctr", 2, &ctr))) return rc;
     if ((rc = scratch_t(ctx, "pp_info_a", TP, &info_a))) return rc;
     if ((rc = scratch_t(ctx, "pp_info_b", TP, &info_b))) return rc;
     if ((rc = scratch_t(ctx, "pp_nbands", TP, &nbands))) return rc;
     if ((rc = scratch_t(ctx, "pp_band_start", (size_t)TP + 1, &band_start))) return rc;
     if ((rc = scratch_t(ctx, "pp_tmp", (size_t)scan_tmp_ints(TP), &tmp))) return rc;
-    if (!reuse) RJ_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned), ctx->stream));
-    a.work_ctr = ctr + (reuse ? 1 : 0);
+    if (ctx->q_ctr_used >= kQueryCounters) return fail(ctx, RJ_E_INVALID, "too many polygon passes in one query");
+    a.work_ctr = ctx->q_ctr + ctx->q_ctr_used++;
     a.info_a = info_a;
     a.info_b = info_b;
     a.nbands = nbands;
@@ -862,7 +867,7 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
         a.tier_pcnt = tr.pcnt;
         a.tier_bw = tr.bw;
         a.tier_bh = tr.bh;
-        a.err = ctx->d_err;
+        a.err = ctx->q_err;
         rc = poly_pass(ctx, MODE_BOUNDS, a);
         a.tier_code = nullptr;
         a.tier_pcnt = nullptr;
@@ -1390,13 +1395,12 @@ int label_blocks(rj_ctx* ctx, const DevFilter& f, const CanvasXf& cx, PolyPassAr
     const size_t nblk = (size_t)tr.bw * tr.bh;
     unsigned long long* cnt;   // multi blocks, covered pixel writes, labelled pixels
     if ((rc = scratch_t(ctx, "tier_full", nblk, &tr.full))) return rc;
-    if ((rc = scratch_t(ctx, "tier_mixed", nblk, &tr.mixed))) return rc;
+    if ((rc = scratch_t(ctx, "tier_cnt_mixed", 3 + (nblk + 1) / 2, &cnt))) return rc;   // zeroed together
     if ((rc = scratch_t(ctx, "tier_code", nblk, &tr.code))) return rc;
     if ((rc = scratch_t(ctx, "tier_plabel", nblk * 256, &tr.plabel))) return rc;
-    if ((rc = scratch_t(ctx, "tier_cnt", 3, &cnt))) return rc;
+    tr.mixed = reinterpret_cast<uint32_t*>(cnt + 3);
     RJ_CUDA(cudaMemsetAsync(tr.full, 0xFF, nblk * 4, ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(tr.mixed, 0, nblk * 4, ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(cnt, 0, 3 * 8, ctx->stream));
+    RJ_CUDA(cudaMemsetAsync(cnt, 0, 3 * 8 + nblk * 4, ctx->stream));
     if ((rc = poly_pass(ctx, MODE_TIER_CLASSIFY, a, &tr))) return rc;
     launch_tier_codes(tr, nblk, cnt, ctx->sms, ctx->stream);
     a.covered = cnt + 1;
@@ -1898,8 +1902,15 @@ void query_rows(const rj_ctx* ctx, const rj_query* q, uint64_t& r0, uint64_t& r1
         ctx->tix.rows(q->t_start, q->t_end, ctx->npts, r0, r1);
 }
 
-// Per-polygon device outputs -> rj_result: exact counts, sums decoded from
-// int64 fixed point (2^-shift) plus the fp64 sum of non-finite values, the
+// A query's output block, copied to the host -> rj_result.
+void decode_result(int P, const char* out, bool bounds, int shift, rj_result* res) {
+    const QueryOut o((size_t)P, bounds);
+    decode_result(P, (const unsigned long long*)out, (const unsigned long long*)(out + o.sum),
+                  (const double*)(out + o.nonfinite), shift, bounds ? (const long long*)(out + o.bounds) : nullptr, res);
+}
+
+// Per-polygon outputs -> rj_result: exact counts, sums decoded from int64
+// fixed point (2^-shift) plus the fp64 sum of non-finite values, the
 // reference's int32[3P] layout and the int32[4P] bounds.
 void decode_result(int P, const unsigned long long* hc, const unsigned long long* hq, const double* hnf, int shift,
                    const long long* hb, rj_result* res) {
@@ -1928,10 +1939,9 @@ void decode_result(int P, const unsigned long long* hc, const unsigned long long
 using namespace rjh;
 
 // The device work of one query, queued on the context's stream: cache
-// upkeep, the outputs zeroed, the join's kernels.  The per-polygon outputs
-// stay on the device (oc, os, onf, ob) for the caller to copy back.
-int enqueue_query(rj_ctx* ctx, const rj_query* q, Phase& ph, unsigned long long** poc, unsigned long long** pos,
-                  double** ponf, long long** pob, double* t_setup) {
+// upkeep, the outputs zeroed, the join's kernels.  The output block
+// (QueryOut) stays on the device for the caller to copy back.
+int enqueue_query(rj_ctx* ctx, const rj_query* q, Phase& ph, char** pout, double* t_setup) {
     int rc;
     const int P = ctx->ps->P;
     if (ctx->cache_owner != ctx->ps || ctx->cache_version != ctx->ps->version) {
@@ -1949,22 +1959,18 @@ int enqueue_query(rj_ctx* ctx, const rj_query* q, Phase& ph, unsigned long long*
     }
     g_kernel_launches = 0;
     ctx->edge_tests_dev = nullptr;
-    unsigned long long* oc;
-    unsigned long long* os;
-    double* onf;
-    long long* ob;
-    if ((rc = scratch_t(ctx, "out_count", P, &oc))) return rc;
-    if ((rc = scratch_t(ctx, "out_sum", P, &os))) return rc;
-    if ((rc = scratch_t(ctx, "out_nonfinite", P, &onf))) return rc;
-    if ((rc = scratch_t(ctx, "out_bounds", (size_t)4 * P, &ob))) return rc;
+    const bool bounds = q->function_type == RJ_RASTER_JOIN_BOUNDS;
+    const QueryOut o((size_t)P, bounds);
+    char* out;
+    if ((rc = scratch_t(ctx, "out", o.bytes, &out))) return rc;
+    ctx->q_nonfinite = (double*)(out + o.nonfinite);
+    ctx->q_err = (int*)(out + o.err);
+    ctx->q_ctr = (unsigned*)(out + o.counters);
+    ctx->q_ctr_used = 0;
     ph.mark(0);
-    RJ_CUDA(cudaMemsetAsync(oc, 0, P * sizeof(unsigned long long), ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(os, 0, P * sizeof(unsigned long long), ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(onf, 0, P * sizeof(double), ctx->stream));
+    RJ_CUDA(cudaMemsetAsync(out, 0, o.bytes, ctx->stream));
     ctx->sum_shift = 0;
-    RJ_CUDA(cudaMemsetAsync(ob, 0, (size_t)4 * P * sizeof(long long), ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-    ExecState es{oc, os, ob, &ph};
+    ExecState es{(unsigned long long*)out, (unsigned long long*)(out + o.sum), (long long*)(out + o.bounds), &ph};
     *t_setup = now_ms();
     switch (q->function_type) {
         case RJ_RASTER_JOIN: rc = exec_raster(ctx, q, es, false); break;
@@ -1972,20 +1978,70 @@ int enqueue_query(rj_ctx* ctx, const rj_query* q, Phase& ph, unsigned long long*
         case RJ_HYBRID_JOIN: rc = exec_hybrid(ctx, q, es); break;
         default: rc = exec_raster(ctx, q, es, true); break;
     }
-    if (rc) return rc;
-    *poc = oc;
-    *pos = os;
-    *ponf = onf;
-    *pob = ob;
-    return RJ_OK;
+    *pout = out;
+    return rc;
 }
 
 namespace rjh {
-int enqueue_query_untimed(rj_ctx* ctx, const rj_query* q, unsigned long long** oc, unsigned long long** os,
-                          double** onf, long long** ob) {
+void release_pin(rj_ctx* ctx);
+
+int enqueue_query_untimed(rj_ctx* ctx, const rj_query* q, char** out) {
     Phase ph(ctx, false);
     double t_setup = 0;
-    return enqueue_query(ctx, q, ph, oc, os, onf, ob, &t_setup);
+    return enqueue_query(ctx, q, ph, out, &t_setup);
+}
+
+// Pinned host memory of at least `bytes` for rj_execute's outputs.  Pinning
+// takes some 270 us, so the usual size is kept for the next context (at most
+// kPinKept buffers, freed with the last context of the process).
+constexpr size_t kPinSize = 64 * 1024, kPinKept = 16;
+std::mutex g_pin_mu;
+std::vector<void*> g_pin_free;
+int g_contexts = 0;
+
+int ensure_pin(rj_ctx* ctx, size_t bytes) {
+    if (ctx->pin_bytes >= bytes) return RJ_OK;
+    release_pin(ctx);
+    if (bytes <= kPinSize) {
+        bytes = kPinSize;
+        std::lock_guard<std::mutex> lock(g_pin_mu);
+        if (!g_pin_free.empty()) {
+            ctx->pin = g_pin_free.back();
+            g_pin_free.pop_back();
+            ctx->pin_bytes = bytes;
+            return RJ_OK;
+        }
+    }
+    if (cudaMallocHost(&ctx->pin, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->pin = nullptr;
+        return fail(ctx, RJ_E_OOM, "pinned memory for a query's outputs (%zu bytes)", bytes);
+    }
+    ctx->pin_bytes = bytes;
+    return RJ_OK;
+}
+
+// nothing in flight may still write it
+void release_pin(rj_ctx* ctx) {
+    if (!ctx->pin) return;
+    {
+        std::lock_guard<std::mutex> lock(g_pin_mu);
+        if (ctx->pin_bytes == kPinSize && g_pin_free.size() < kPinKept) {
+            g_pin_free.push_back(ctx->pin);
+            ctx->pin = nullptr;
+        }
+    }
+    if (ctx->pin) cudaFreeHost(ctx->pin);
+    ctx->pin = nullptr;
+    ctx->pin_bytes = 0;
+}
+
+void count_context(int d) {
+    std::lock_guard<std::mutex> lock(g_pin_mu);
+    g_contexts += d;
+    if (g_contexts > 0) return;
+    for (void* p : g_pin_free) cudaFreeHost(p);
+    g_pin_free.clear();
 }
 }  // namespace rjh
 
@@ -2039,7 +2095,8 @@ int rj_create(const rj_config* cfg, rj_ctx** out) {
         ctx->own_stream = true;
     }
     for (auto& ev : ctx->ev) cudaEventCreate(&ev);
-    if (cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess) {
+    count_context(1);
+    if (cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess || ensure_pin(ctx, 1)) {
         cudaGetLastError();
         rj_destroy(ctx);
         return RJ_E_OOM;
@@ -2068,6 +2125,9 @@ void rj_destroy(rj_ctx* ctx) {
     }
     free_polyset(ctx, ctx->own);
     for (auto& kv : ctx->scratch) dev_free(ctx, kv.second);
+    for (auto& b : ctx->retired) dev_free(ctx, b);
+    release_pin(ctx);
+    count_context(-1);
     for (auto& ev : ctx->ev)
         if (ev) cudaEventDestroy(ev);
     if (ctx->d_err) cudaFree(ctx->d_err);
@@ -2331,34 +2391,26 @@ int rj_execute(rj_ctx* ctx, const rj_query* q, rj_result* res) {
     int rc;
     const int P = ctx->ps->P;
     Phase ph(ctx, (q->flags & RJ_FLAG_PHASE_TIMING) != 0);
-    unsigned long long *oc, *os;
-    double* onf;
-    long long* ob;
+    const bool bounds = q->function_type == RJ_RASTER_JOIN_BOUNDS;
+    const QueryOut o((size_t)P, bounds);
+    char* out = nullptr;
     double t_setup = 0;
-    if ((rc = enqueue_query(ctx, q, ph, &oc, &os, &onf, &ob, &t_setup))) {
+    if ((rc = ensure_pin(ctx, o.read))) return rc;
+    if ((rc = enqueue_query(ctx, q, ph, &out, &t_setup))) {
         cudaStreamSynchronize(ctx->stream);
         return rc;
     }
-    std::vector<unsigned long long> hc(P), hq(P);
-    std::vector<double> hnf(P);
-    std::vector<long long> hb;
-    int derr = 0;
-    RJ_CUDA(cudaMemcpyAsync(hc.data(), oc, P * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
-    RJ_CUDA(cudaMemcpyAsync(hq.data(), os, P * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
-    RJ_CUDA(cudaMemcpyAsync(hnf.data(), onf, P * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    if (q->function_type == RJ_RASTER_JOIN_BOUNDS && res && res->bounds) {
-        hb.resize((size_t)4 * P);
-        RJ_CUDA(cudaMemcpyAsync(hb.data(), ob, (size_t)4 * P * sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream));
-    }
-    RJ_CUDA(cudaMemcpyAsync(&derr, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    const char* host = (const char*)ctx->pin;
+    RJ_CUDA(cudaMemcpyAsync(ctx->pin, out, o.read, cudaMemcpyDeviceToHost, ctx->stream));
     ph.mark(5);
     RJ_CUDA(cudaStreamSynchronize(ctx->stream));
     RJ_CUDA(cudaGetLastError());
+    const int derr = *(const int*)(host + o.err);
     if (derr & 4) return fail(ctx, RJ_E_INVALID, "error-bound outline read outside the tiered canvas's slots");
     if (derr) return fail(ctx, RJ_E_TIMEOUT, "a bounded device wait ran out (status 0x%x)", derr);
-    decode_result(P, hc.data(), hq.data(), hnf.data(), ctx->sum_shift, hb.empty() ? nullptr : hb.data(), res);
-    ctx->last_fixed.assign(hq.begin(), hq.end());
-    ctx->last_nonfinite = hnf;
+    decode_result(P, host, bounds, ctx->sum_shift, res);
+    ctx->last_fixed.assign((const long long*)(host + o.sum), (const long long*)(host + o.sum) + P);
+    ctx->last_nonfinite.assign((const double*)(host + o.nonfinite), (const double*)(host + o.nonfinite) + P);
     ctx->last_shift = ctx->sum_shift;
     // timings (GLHandler::printTimeStats fields)
     rj_timings& t = ctx->tm;
@@ -2422,17 +2474,13 @@ static void plan_free(rj_plan* p) {
     if (!p) return;
     if (p->exec) cudaGraphExecDestroy(p->exec);
     if (p->graph) cudaGraphDestroy(p->graph);
-    cudaFreeHost(p->hc);
-    cudaFreeHost(p->hq);
-    cudaFreeHost(p->hnf);
-    cudaFreeHost(p->hb);
-    cudaFreeHost(p->derr);
+    cudaFreeHost(p->out);
     delete p;
 }
 
-int rj_prepare(rj_ctx* ctx, const rj_query* q, rj_plan** out) {
-    if (!ctx || !q || !out) return RJ_E_INVALID;
-    *out = nullptr;
+int rj_prepare(rj_ctx* ctx, const rj_query* q, rj_plan** plan) {
+    if (!ctx || !q || !plan) return RJ_E_INVALID;
+    *plan = nullptr;
     std::lock_guard<std::recursive_mutex> lock(ctx->mu);
     if (ctx->streamed) return fail(ctx, RJ_E_UNSUPPORTED, "a host-streamed table cannot be prepared");
     if (ctx->server_running) return fail(ctx, RJ_E_BUSY, "a serving loop owns the context");
@@ -2453,11 +2501,8 @@ int rj_prepare(rj_ctx* ctx, const rj_query* q, rj_plan** out) {
     p->ps = ctx->ps;
     p->ps_version = ctx->ps->version;
     p->npts = ctx->npts;
-    if (cudaHostAlloc(&p->hc, P * sizeof(unsigned long long), 0) != cudaSuccess ||
-        cudaHostAlloc(&p->hq, P * sizeof(unsigned long long), 0) != cudaSuccess ||
-        cudaHostAlloc(&p->hnf, P * sizeof(double), 0) != cudaSuccess ||
-        cudaHostAlloc(&p->hb, (size_t)4 * P * sizeof(long long), 0) != cudaSuccess ||
-        cudaHostAlloc(&p->derr, sizeof(int), 0) != cudaSuccess) {
+    const QueryOut o((size_t)P, q->function_type == RJ_RASTER_JOIN_BOUNDS);
+    if (cudaHostAlloc(&p->out, o.read, 0) != cudaSuccess) {
         cudaGetLastError();
         plan_free(p);
         return fail(ctx, RJ_E_OOM, "pinned result buffers of the plan");
@@ -2465,9 +2510,7 @@ int rj_prepare(rj_ctx* ctx, const rj_query* q, rj_plan** out) {
     rj_query qc = *q;
     qc.flags &= ~RJ_FLAG_PHASE_TIMING;
     Phase ph(ctx, false);
-    unsigned long long *oc = nullptr, *os = nullptr;
-    double* onf = nullptr;
-    long long* ob = nullptr;
+    char* out = nullptr;   // the graph's output block
     double t_setup = 0;
     cudaError_t ce = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed);
     if (ce != cudaSuccess) {
@@ -2476,14 +2519,8 @@ int rj_prepare(rj_ctx* ctx, const rj_query* q, rj_plan** out) {
         return fail(ctx, RJ_E_CUDA, "cudaStreamBeginCapture: %s", cudaGetErrorString(ce));
     }
     ctx->capturing = true;
-    rc = enqueue_query(ctx, &qc, ph, &oc, &os, &onf, &ob, &t_setup);
-    if (!rc) {
-        cudaMemcpyAsync(p->hc, oc, P * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream);
-        cudaMemcpyAsync(p->hq, os, P * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream);
-        cudaMemcpyAsync(p->hnf, onf, P * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
-        cudaMemcpyAsync(p->hb, ob, (size_t)4 * P * sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream);
-        cudaMemcpyAsync(p->derr, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-    }
+    rc = enqueue_query(ctx, &qc, ph, &out, &t_setup);
+    if (!rc) cudaMemcpyAsync(p->out, out, o.read, cudaMemcpyDeviceToHost, ctx->stream);
     p->shift = ctx->sum_shift;
     ctx->capturing = false;
     cudaGraph_t g = nullptr;
@@ -2502,7 +2539,8 @@ int rj_prepare(rj_ctx* ctx, const rj_query* q, rj_plan** out) {
         plan_free(p);
         return fail(ctx, RJ_E_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(ce));
     }
-    *out = p;
+    ++ctx->live_plans;
+    *plan = p;
     return RJ_OK;
 }
 
@@ -2530,12 +2568,15 @@ int rj_execute_prepared(rj_plan* p, rj_result* res) {
     cudaSetDevice(ctx->device);
     RJ_CUDA(cudaGraphLaunch(p->exec, ctx->stream));
     RJ_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (*p->derr) return fail(ctx, RJ_E_TIMEOUT, "a bounded device wait ran out (status 0x%x)", *p->derr);
     const int P = p->P;
-    decode_result(P, p->hc, p->hq, p->hnf, p->shift, p->function_type == RJ_RASTER_JOIN_BOUNDS ? p->hb : nullptr,
-                  res);
-    ctx->last_fixed.assign(p->hq, p->hq + P);
-    ctx->last_nonfinite.assign(p->hnf, p->hnf + P);
+    const bool bounds = p->function_type == RJ_RASTER_JOIN_BOUNDS;
+    const QueryOut o((size_t)P, bounds);
+    const char* host = (const char*)p->out;
+    if (const int derr = *(const int*)(host + o.err))
+        return fail(ctx, RJ_E_TIMEOUT, "a bounded device wait ran out (status 0x%x)", derr);
+    decode_result(P, host, bounds, p->shift, res);
+    ctx->last_fixed.assign((const long long*)(host + o.sum), (const long long*)(host + o.sum) + P);
+    ctx->last_nonfinite.assign((const double*)(host + o.nonfinite), (const double*)(host + o.nonfinite) + P);
     ctx->last_shift = p->shift;
     rj_timings& t = ctx->tm;
     std::memset(&t, 0, sizeof t);
@@ -2551,9 +2592,14 @@ int rj_execute_prepared(rj_plan* p, rj_result* res) {
 void rj_plan_destroy(rj_plan* p) {
     if (!p) return;
     if (p->ctx) {
-        std::lock_guard<std::recursive_mutex> lock(p->ctx->mu);
-        cudaSetDevice(p->ctx->device);
+        rj_ctx* ctx = p->ctx;
+        std::lock_guard<std::recursive_mutex> lock(ctx->mu);
+        cudaSetDevice(ctx->device);
         plan_free(p);
+        if (--ctx->live_plans == 0) {
+            for (auto& b : ctx->retired) dev_free(ctx, b);
+            ctx->retired.clear();
+        }
         return;
     }
     plan_free(p);
