@@ -422,8 +422,9 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 2 : 3) k_poly_bands(PolyPa
                             P0 = pf[k];
                             P1 = pf[(k + 1 == n) ? 0 : k + 1];
                             const float ylo = (float)(jb + r), yhi = (float)(jb + r + 1);
-                            // x range of the edge inside the row, widened by more
-                            // than the fp32 error of the clip's own arithmetic
+                            // x range of the edge inside the row and a pixel more on
+                            // each side: on a nearly horizontal edge the clip's fp32
+                            // rounding of y moves its ends by up to a pixel
                             float xa, xb;
                             if (P0.y == P1.y) {
                                 xa = fminf(P0.x, P1.x);
@@ -435,9 +436,8 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 2 : 3) k_poly_bands(PolyPa
                                 xa = fminf(x_a, x_b);
                                 xb = fmaxf(x_a, x_b);
                             }
-                            const float slack = 0.05f + 2e-6f * (fabsf(P0.x) + fabsf(P1.x));
-                            i0 = max(xa - slack > 0.0f ? (int)floorf(xa - slack) : 0, 0);
-                            i1 = xb + slack < (float)a.resx ? (int)floorf(xb + slack) : a.resx - 1;
+                            i0 = max((int)floorf(xa) - 1, 0);
+                            i1 = min((int)floorf(xb) + 1, a.resx - 1);
                         }
                         // wide pairs: the whole warp, four pixels a lane
                         for (unsigned wide = __ballot_sync(FULL, i1 - i0 >= 16); wide; wide &= wide - 1u) {
