@@ -160,8 +160,7 @@ struct QPlan {
     size_t nblk = 0;             // blocks of the tiered canvas
     size_t est_slots = 0;        // upper bound on its mixed blocks
     int nslots = 0;
-    int* slot_buf = nullptr;
-    int* scan_tmp = nullptr;
+    int* slot_buf = nullptr;     // slots handed out
     size_t out_off = 0;          // first polygon of the query in the output block
     uint16_t* label = nullptr;
     uint32_t* cc = nullptr;
@@ -181,7 +180,7 @@ size_t canvas_bytes(const QPlan& p) {
     const bool agg = p.f.aggr != 0;
     if (p.tier) {
         const size_t base = 4 * al256(p.nblk * 4) + al256((p.nblk + 1) * 4) +
-                            al256((size_t)scan_tmp_ints((int)std::max<size_t>(p.nblk, 1)) * 4);
+                            al256(4);
         return base + (p.mode == BQ_TLABEL ? al256(p.est_slots * 256 * 2) : tier_canvas_bytes(p));
     }
     return p.mode == BQ_LABEL ? al256(p.npix * 2) : al256(p.npix * 4) + (agg ? al256(p.npix * 8) : 0);
@@ -455,10 +454,10 @@ int run_fused(Engine& e, std::vector<QPlan>& plans, uint32_t flags, BatchOut& bo
                 TierArgs& tr = p->tr;
                 tr.full = ar.take<uint32_t>(p->nblk);
                 tr.mixed = ar.take<uint32_t>(p->nblk);
-                p->slot_buf = ar.take<int>(p->nblk + 1);
-                tr.slot = p->slot_buf;
+                p->slot_buf = ar.take<int>(1);
+                tr.nslots = reinterpret_cast<uint32_t*>(p->slot_buf);
+                tr.cap = 0x7FFFFFFFu;   // the number is read back and checked against the bound
                 tr.code = ar.take<uint32_t>(p->nblk);
-                p->scan_tmp = ar.take<int>((size_t)scan_tmp_ints((int)std::max<size_t>(p->nblk, 1)));
                 tr.plabel = nullptr;
                 tr.bcnt = tr.pcnt = nullptr;
                 tr.bsum = tr.psum = nullptr;
@@ -472,7 +471,7 @@ int run_fused(Engine& e, std::vector<QPlan>& plans, uint32_t flags, BatchOut& bo
                         tr.psum = ar.take<long long>(p->est_slots * 256);
                     }
                 }
-                if (!tr.full || !tr.mixed || !p->slot_buf || !tr.code || !p->scan_tmp ||
+                if (!tr.full || !tr.mixed || !p->slot_buf || !tr.code ||
                     (p->mode == BQ_TLABEL ? !tr.plabel : (!tr.bcnt || !tr.pcnt || (p->f.aggr && (!tr.bsum || !tr.psum)))))
                     return fail(ctx, RJ_E_OOM, "batch arena too small for a tiered canvas");
             } else if (p->mode == BQ_LABEL) {
@@ -500,10 +499,9 @@ int run_fused(Engine& e, std::vector<QPlan>& plans, uint32_t flags, BatchOut& bo
             RJ_CUDA(cudaMemsetAsync(p->tr.mixed, 0, p->nblk * 4, st));
             if (!query_poly_pass(e, *p, MODE_TIER_CLASSIFY, ps, nullptr, nullptr, nullptr, &p->tr))
                 return fail(ctx, RJ_E_INVALID, "too many (tile, polygon) items");
-            if (!launch_exclusive_scan((const int*)p->tr.mixed, p->slot_buf, (int)p->nblk, p->scan_tmp, st))
-                return fail(ctx, RJ_E_INVALID, "tier scan failed");
-            launch_tier_codes(p->tr, p->nblk, tcnt + 3 * i, ctx->sms, st);
-            RJ_CUDA(cudaMemcpyAsync(&p->nslots, p->slot_buf + p->nblk, sizeof(int), cudaMemcpyDeviceToHost, st));
+            RJ_CUDA(cudaMemsetAsync(p->slot_buf, 0, sizeof(int), st));
+            launch_tier_codes(p->tr, p->nblk, tcnt + 3 * i, nullptr, ctx->sms, st);
+            RJ_CUDA(cudaMemcpyAsync(&p->nslots, p->slot_buf, sizeof(int), cudaMemcpyDeviceToHost, st));
         }
         if (any_tier) {
             RJ_CUDA(cudaStreamSynchronize(st));
@@ -921,6 +919,10 @@ int lanes_finish(Engine& e, LaneRun& lr) {
         if (p.status != RJ_OK) continue;
         const char* b = h + lr.off[i];
         if (const int derr = *(const int*)(b + QueryOut((size_t)p.ps->P, lr.bounds[i]).err)) {
+            if (derr == kErrSlots) {   // run again alone (rj_execute reads the number of slots back)
+                p.status = RJ_E_OOM;
+                continue;
+            }
             p.status = fail(e.ctx, RJ_E_TIMEOUT, "query %d: a bounded device wait ran out (status 0x%x)", p.idx, derr);
             continue;
         }

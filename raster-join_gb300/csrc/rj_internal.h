@@ -54,6 +54,9 @@ struct PolySet {
     double bbox[4] = {0, 0, 0, 0};
     float max_abs_coord = 0.f, max_edge_dx = 0.f, max_edge_dy = 0.f;
     double sum_dx = 0, sum_dy = 0;  // sums of |dx|, |dy| over all edges
+    // deepest vertex found inside another polygon of the set (distance to its
+    // outline; 0: none found by the bounded search of load_polyset)
+    double overlap_depth = 0;
     // one device allocation (d_block) holds the vertices, pindex and the
     // edge -> polygon map; d_verts, d_pindex and d_edge_poly point into it
     DevBuf d_block;
@@ -146,6 +149,7 @@ struct rj_ctx {
     int q_ctr_used = 0;
     void* pin = nullptr;             // pinned host copy of rj_execute's outputs
     size_t pin_bytes = 0;
+    bool exact_slots = false;        // tiered canvas: read the number of mixed blocks back
     int live_plans = 0;              // prepared queries: their graphs hold scratch addresses
     std::vector<rjh::DevBuf> retired;   // outgrown scratch those graphs may still use
     int sum_shift = 0;        // fixed-point scale 2^s of the current query's sums

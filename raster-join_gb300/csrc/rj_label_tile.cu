@@ -185,7 +185,7 @@ size_t label_tile_smem(int shape, int cell_words, int P, bool agg) {
 
 bool launch_label_tile(int shape, const LabelPointArgs& a, const LeanCols& lc_in, int sms, cudaStream_t st) {
     if (shape < 0 || shape >= kNumTileShapes || lc_in.ncol != 0 || a.ax.split != 1 || a.ay.split != 1) return false;
-    const bool agg = lc_in.aggr != 0, one = a.bs == 4 && !a.tr.slot;
+    const bool agg = lc_in.aggr != 0, one = a.bs == 4 && a.tr.own_place;
     LabelKernel k = agg ? (one ? tile_kernel<true, true>(shape) : tile_kernel<true, false>(shape))
                         : (one ? tile_kernel<false, true>(shape) : tile_kernel<false, false>(shape));
     LeanCols lc = lc_in;

@@ -20,7 +20,9 @@ struct TierArgs {
     int bw, bh;                  // blocks per tile row / per tile column
     uint32_t* full;              // [nblk] polygon covering the whole block, kTierEmpty, kTierMulti
     uint32_t* mixed;             // [nblk] 1: per-pixel block
-    const int* slot;             // [nblk] exclusive scan of mixed, or null: slot = block
+    bool own_place;              // the slot of a mixed block is the block itself
+    uint32_t* nslots;            // else: slots handed out so far (zeroed), at most cap
+    uint32_t cap;
     uint32_t* code;              // [nblk] lookup code (full polygon / empty / multi / mixed | slot)
     uint16_t* plabel;            // [nslots * 256] pixel labels of mixed blocks
     uint32_t* bcnt;              // [nblk] point counts of the blocks neither mixed nor empty (canvas form)
@@ -71,7 +73,10 @@ struct PolyPassArgs {
 
 size_t tier_smem_bytes();
 void launch_tier_pass(int mode, const PolyPassArgs& a, const TierArgs& tr, int sms, cudaStream_t st);
-void launch_tier_codes(const TierArgs& tr, size_t nblk, unsigned long long* multi, int sms, cudaStream_t st);
+void launch_tier_codes(const TierArgs& tr, size_t nblk, unsigned long long* multi, int* err, int sms, cudaStream_t st);
+// clears the mixed blocks' slots (and the block totals) of the arrays given
+void launch_tier_clear(const TierArgs& tr, size_t nblk, int sms, cudaStream_t st);
+constexpr int kErrSlots = 8;     // status bit: more mixed blocks than slots
 void launch_tier_nonempty(const TierArgs& tr, size_t nblk, unsigned long long* count, int sms, cudaStream_t st);
 
 struct GridArgs {

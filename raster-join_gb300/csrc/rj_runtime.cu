@@ -769,11 +769,39 @@ struct LabelPlan {
 // then the label form (disjoint coverage) or the canvas form.  Results equal
 // the flat canvas's; polygon-side work follows the perimeters.
 int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, const TierArgs& tr,
-                   size_t nblk, size_t spx, ExecState& es, bool* done);   // below
+                   size_t nblk, ExecState& es, bool* done);               // below
 struct LabelPlan;
 bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, ExecState& es,
                        LabelPlan& lp);                                    // below
 int run_label_points(rj_ctx* ctx, LabelPlan& lp, const TierArgs& tr, ExecState& es, bool* done);   // below
+
+// Whether the label form is known not to apply: some pixel centre lies in two
+// polygons, or, while that is unknown, a vertex lies so deep inside another
+// polygon that some pixel centre will (the canvas form gives the same results
+// in any case).
+bool known_overlap(const rj_ctx* ctx, const RasterPlan& rp, uint64_t ckey) {
+    const int o = ctx->ps->overlap_on(ckey);
+    if (o != -1) return o == 1;
+    const double* bb = ctx->ps->bbox;
+    const double px = std::max((bb[2] - bb[0]) / rp.actual_x, (bb[3] - bb[1]) / rp.actual_y);
+    return ctx->ps->overlap_depth > 4.0 * px;
+}
+
+// Upper bound on the mixed blocks of a tiered canvas.  An edge's part in one
+// tile touches at most |dx|/16 + |dy|/16 + 3 blocks; tile seams cut it into at
+// most |dx|/res + |dy|/res + 5 parts (a part within a pixel of a seam counts on
+// both sides).  The outline's blocks lie within two pixels of the edge in
+// bands of 16 rows widened by two: three block rows of |dx|/16 + 2.5 blocks a
+// band.  Blocks cut by a tile's edge are never full.
+constexpr size_t kSlotBytes = (size_t)512 << 20;   // bounds up to this much memory are taken unread
+size_t tier_slot_bound(const PolySet& s, const RasterPlan& rp, size_t nblk, bool outline) {
+    const double pw = (s.bbox[2] - s.bbox[0]) / rp.splitx / rp.resx, ph = (s.bbox[3] - s.bbox[1]) / rp.splity / rp.resy;
+    const double dx = s.sum_dx / pw, dy = s.sum_dy / ph;
+    const double parts = 5.0 * s.V + dx / rp.resx + dy / rp.resy;
+    const double edge = outline ? 3.0 * dx / 16 + 7.5 * dy / 16 + 20.0 * parts : dx / 16 + dy / 16 + 3.0 * parts;
+    const double rim = 2.0 * rp.splitx * rp.splity * ((rp.resx + 15) / 16 + (rp.resy + 15) / 16);
+    return (size_t)std::min((double)nblk, edge + rim + 64.0);
+}
 
 int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const DevFilter& f, ExecState& es,
                      PolyPassArgs& a, const CanvasXf& cx, uint64_t ckey, bool bounds) {
@@ -783,40 +811,42 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
     tr.bh = (rp.resy + 15) / 16;
     const size_t nblk = (size_t)a.T * tr.bw * tr.bh;
     if (nblk >= (size_t)1 << 24) return fail(ctx, RJ_E_UNSUPPORTED, "canvas too large for the tiered form");
-    int* slot;
-    int* tmp;
-    unsigned long long* cnt;   // multi blocks, covered pixel writes, labelled pixels
+    // multi blocks, covered pixel writes, labelled pixels, slots; then the
+    // mixed flags (zeroed together)
+    unsigned long long* cnt;
     if ((rc = scratch_t(ctx, "tier_full", nblk, &tr.full))) return rc;
-    if ((rc = scratch_t(ctx, "tier_mixed", nblk, &tr.mixed))) return rc;
-    if ((rc = scratch_t(ctx, "tier_slot", nblk + 1, &slot))) return rc;
+    if ((rc = scratch_t(ctx, "tier_cnt_mixed", 4 + (nblk + 1) / 2, &cnt))) return rc;
     if ((rc = scratch_t(ctx, "tier_code", nblk, &tr.code))) return rc;
-    if ((rc = scratch_t(ctx, "tier_tmp", (size_t)scan_tmp_ints((int)nblk), &tmp))) return rc;
-    if ((rc = scratch_t(ctx, "tier_cnt", 3, &cnt))) return rc;
-    tr.slot = slot;
+    tr.nslots = reinterpret_cast<uint32_t*>(cnt + 3);
+    tr.mixed = reinterpret_cast<uint32_t*>(cnt + 4);
     // error bounds: the blocks the outline pass reads are mixed too
     tr.outline = bounds ? 1 : 0;
     RJ_CUDA(cudaMemsetAsync(tr.full, 0xFF, nblk * 4, ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(tr.mixed, 0, nblk * 4, ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(cnt, 0, 3 * 8, ctx->stream));
+    RJ_CUDA(cudaMemsetAsync(cnt, 0, 4 * 8 + nblk * 4, ctx->stream));
     a.outline_rows = tr.outline;
     rc = poly_pass(ctx, MODE_TIER_CLASSIFY, a, &tr);
     a.outline_rows = 0;
     if (rc) return rc;
-    if (!launch_exclusive_scan((const int*)tr.mixed, slot, (int)nblk, tmp, ctx->stream))
-        return fail(ctx, RJ_E_INVALID, "tier scan failed");
-    launch_tier_codes(tr, nblk, cnt, ctx->sms, ctx->stream);
-    int nslots = 0;
     if ((rc = readback_guard(ctx, "the tiered canvas"))) return rc;
-    RJ_CUDA(cudaMemcpyAsync(&nslots, slot + nblk, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    RJ_CUDA(cudaStreamSynchronize(ctx->stream));
-    const size_t spx = (size_t)std::max(nslots, 1) * 256;
-    bool label = !bounds && !(q->flags & RJ_FLAG_FORCE_CANVAS) && ctx->ps->overlap_on(ckey) != 1 &&
+    // Slots of the mixed blocks: as many as the outlines can make when that is
+    // little memory (no wait for the device), else the exact number, read back.
+    bool label = !bounds && !(q->flags & RJ_FLAG_FORCE_CANVAS) && !known_overlap(ctx, rp, ckey) &&
                  ctx->ps->P <= kMaxLabelPolys;
+    const size_t bound = tier_slot_bound(*ctx->ps, rp, nblk, bounds);
+    const bool exact = ctx->exact_slots || bound * 256 * (f.aggr ? 12 : 4) > kSlotBytes;
+    tr.cap = exact ? 0x7FFFFFFFu : (uint32_t)bound;
+    launch_tier_codes(tr, nblk, cnt, ctx->q_err, ctx->sms, ctx->stream);
+    uint32_t nslots = (uint32_t)bound;
+    if (exact) {
+        RJ_CUDA(cudaMemcpyAsync(&nslots, tr.nslots, sizeof nslots, cudaMemcpyDeviceToHost, ctx->stream));
+        RJ_CUDA(cudaStreamSynchronize(ctx->stream));
+    }
+    const size_t spx = (size_t)std::max(nslots, 1u) * 256;
     if (label) {
         if ((rc = scratch_t(ctx, "tier_plabel", spx, &tr.plabel))) return rc;
-        RJ_CUDA(cudaMemsetAsync(tr.plabel, 0xFF, spx * 2, ctx->stream));
+        launch_tier_clear(tr, nblk, ctx->sms, ctx->stream);
         a.covered = cnt + 1;
-        if ((rc = poly_pass(ctx, MODE_TIER_LABEL, a, &tr))) return rc;
+        if ((rc = poly_pass(ctx, MODE_TIER_LABEL, a, &tr, true))) return rc;
         if (ctx->ps->overlap_on(ckey) == -1) {
             launch_tier_nonempty(tr, nblk, cnt + 2, ctx->sms, ctx->stream);
             unsigned long long hc[3] = {0, 0, 0};
@@ -840,18 +870,16 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
         return RJ_OK;
     }
     // canvas form: block sums + pixel canvases of the mixed blocks
+    tr.plabel = nullptr;
     if ((rc = scratch_t(ctx, "tier_bcnt", nblk, &tr.bcnt))) return rc;
     if ((rc = scratch_t(ctx, "tier_pcnt", spx, &tr.pcnt))) return rc;
-    RJ_CUDA(cudaMemsetAsync(tr.bcnt, 0, nblk * 4, ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(tr.pcnt, 0, spx * 4, ctx->stream));
     if (f.aggr) {
         if ((rc = scratch_t(ctx, "tier_bsum", nblk, &tr.bsum))) return rc;
         if ((rc = scratch_t(ctx, "tier_psum", spx, &tr.psum))) return rc;
-        RJ_CUDA(cudaMemsetAsync(tr.bsum, 0, nblk * 8, ctx->stream));
-        RJ_CUDA(cudaMemsetAsync(tr.psum, 0, spx * 8, ctx->stream));
     }
+    launch_tier_clear(tr, nblk, ctx->sms, ctx->stream);
     bool lean = false;
-    if ((rc = tier_lean_pass(ctx, f, rp, cx, tr, nblk, spx, es, &lean))) return rc;
+    if ((rc = tier_lean_pass(ctx, f, rp, cx, tr, nblk, es, &lean))) return rc;
     if (!lean && (rc = point_pass(ctx, f, es.out_count, es.out_sum, [&](const PointArgs& pa) {
                       launch_tier_splat_points(pa, cx, tr, ctx->sms, ctx->stream);
                   })))
@@ -860,7 +888,7 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
     a.canvas_c = nullptr;
     a.canvas_s = nullptr;
     a.label = nullptr;
-    if ((rc = poly_pass(ctx, MODE_TIER_REDUCE, a, &tr))) return rc;
+    if ((rc = poly_pass(ctx, MODE_TIER_REDUCE, a, &tr, !bounds))) return rc;   // (the outline's bands differ)
     if (bounds) {
         // the outline pass of the error bounds over the mixed blocks' counts
         a.tier_code = tr.code;
@@ -1390,6 +1418,7 @@ int label_blocks(rj_ctx* ctx, const DevFilter& f, const CanvasXf& cx, PolyPassAr
     int rc;
     *overlap = false;
     TierArgs tr{};
+    tr.own_place = true;
     tr.bw = (a.resx + 15) / 16;
     tr.bh = (a.resy + 15) / 16;
     const size_t nblk = (size_t)tr.bw * tr.bh;
@@ -1402,7 +1431,7 @@ int label_blocks(rj_ctx* ctx, const DevFilter& f, const CanvasXf& cx, PolyPassAr
     RJ_CUDA(cudaMemsetAsync(tr.full, 0xFF, nblk * 4, ctx->stream));
     RJ_CUDA(cudaMemsetAsync(cnt, 0, 3 * 8 + nblk * 4, ctx->stream));
     if ((rc = poly_pass(ctx, MODE_TIER_CLASSIFY, a, &tr))) return rc;
-    launch_tier_codes(tr, nblk, cnt, ctx->sms, ctx->stream);
+    launch_tier_codes(tr, nblk, cnt, ctx->q_err, ctx->sms, ctx->stream);
     a.covered = cnt + 1;
     if ((rc = poly_pass(ctx, MODE_TIER_LABEL, a, &tr, true))) return rc;
     if (ctx->ps->overlap_on(ckey) == -1) {
@@ -1433,7 +1462,7 @@ int label_blocks(rj_ctx* ctx, const DevFilter& f, const CanvasXf& cx, PolyPassAr
 // into the sums, which are cleared again after them.  *done = false: the pass does
 // not apply (the caller takes the generic pass).
 int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const CanvasXf& cx, const TierArgs& tr,
-                   size_t nblk, size_t spx, ExecState& es, bool* done) {
+                   size_t nblk, ExecState& es, bool* done) {
     *done = false;
     ctx->last_count_shape = ctx->last_count_bshift = -1;
     if (ctx->streamed || f.general || f.ncol > kLeanMaxCols) return RJ_OK;
@@ -1471,12 +1500,7 @@ int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const 
         return launch_tier_lean(cands[i], b, lc, ctx->sms, ctx->stream);
     });
     RJ_CUDA(cudaGetLastError());
-    if (timed_any) {
-        RJ_CUDA(cudaMemsetAsync(tr.bcnt, 0, nblk * 4, ctx->stream));
-        RJ_CUDA(cudaMemsetAsync(tr.pcnt, 0, spx * 4, ctx->stream));
-        if (tr.bsum) RJ_CUDA(cudaMemsetAsync(tr.bsum, 0, nblk * 8, ctx->stream));
-        if (tr.psum) RJ_CUDA(cudaMemsetAsync(tr.psum, 0, spx * 8, ctx->stream));
-    }
+    if (timed_any) launch_tier_clear(tr, nblk, ctx->sms, ctx->stream);
     if (pi < 0) return RJ_OK;
     ctx->passes = 1;
     ctx->copy_ms = 0;
@@ -1530,8 +1554,8 @@ int exec_raster(rj_ctx* ctx, const rj_query* q, ExecState& es, bool bounds) {
     const uint64_t ckey = canvas_key(rp.colxf, rp.rowxf, rp.resx, rp.resy);
     const uint64_t rows = std::min(ctx->row1, ctx->npts) - std::min(ctx->row0, ctx->npts);
     if (query_tier(q->flags, npix, rows)) return exec_raster_tier(ctx, q, rp, f, es, a, cx, ckey, bounds);
-    bool use_label = !bounds && !(q->flags & RJ_FLAG_FORCE_CANVAS) && ctx->ps->overlap_on(ckey) != 1 &&
-                     ctx->ps->P <= kMaxLabelPolys;
+    const bool use_label = !bounds && !(q->flags & RJ_FLAG_FORCE_CANVAS) && !known_overlap(ctx, rp, ckey) &&
+                           ctx->ps->P <= kMaxLabelPolys;
     if (use_label) {
         bool overlap = false;
         LabelPlan lp;
@@ -1768,6 +1792,40 @@ int exec_hybrid(rj_ctx* ctx, const rj_query* q, ExecState& es) {
     return RJ_OK;
 }
 
+// A bounded look for a vertex inside another polygon of the set: the distance
+// from the outline of the deepest found (first vertices of some polygons, at
+// most about 10 us of work), 0 when none is found.  It only steers the first
+// query on a canvas (known_overlap).
+double overlap_depth(const float* xy, const int32_t* pindex, int P, const std::vector<float4>& mbr) {
+    const int tries = std::min(P, std::max(4, 16384 / std::max(P, 1)));
+    int budget = 8192;   // edges looked at
+    double depth = 0;
+    for (int k = 0; k < tries && budget > 0 && P > 1; ++k) {
+        const int i = (int)((int64_t)k * P / tries);
+        if (pindex[i + 1] <= pindex[i]) continue;
+        const double x = xy[2 * pindex[i]], y = xy[2 * pindex[i] + 1];
+        for (int p = 0; p < P && budget > 0; ++p) {
+            const float4 m = mbr[p];
+            if (p == i || !(x > m.x && x < m.z && y > m.y && y < m.w)) continue;
+            const int v0 = pindex[p], n = pindex[p + 1] - v0;
+            budget -= n;
+            bool in = false;
+            double d2 = INFINITY;
+            for (int e = 0, f = n - 1; e < n; f = e++) {
+                const double ax = xy[2 * (v0 + f)], ay = xy[2 * (v0 + f) + 1];
+                const double ex = xy[2 * (v0 + e)] - ax, ey = xy[2 * (v0 + e) + 1] - ay;
+                const double l2 = ex * ex + ey * ey;
+                if ((ay > y) != (ay + ey > y) && x < ax + ex * (y - ay) / ey) in = !in;
+                const double t = l2 > 0 ? std::min(1.0, std::max(0.0, ((x - ax) * ex + (y - ay) * ey) / l2)) : 0.0;
+                const double px = ax + t * ex - x, py = ay + t * ey - y;
+                d2 = std::min(d2, px * px + py * py);
+            }
+            if (in) depth = std::max(depth, std::sqrt(d2));
+        }
+    }
+    return depth;
+}
+
 // Polygon collection -> PolySet (PolyHandler::addPolygonCollection
 // PolyHandler.cpp:49-80; bounds as readPolygons PolyHandler.cpp:178-186).
 int load_polyset(rj_ctx* ctx, PolySet& s, const float* xy, const int32_t* pindex, int32_t npolys,
@@ -1842,6 +1900,7 @@ int load_polyset(rj_ctx* ctx, PolySet& s, const float* xy, const int32_t* pindex
     }
     s.sum_dx = sdx;
     s.sum_dy = sdy;
+    s.overlap_depth = overlap_depth(xy, pindex, npolys, s.h_mbr);
     s.P = npolys;
     s.V = V;
     for (int i = 0; i < 4; ++i) s.bbox[i] = bb[i];
@@ -2406,6 +2465,13 @@ int rj_execute(rj_ctx* ctx, const rj_query* q, rj_result* res) {
     RJ_CUDA(cudaStreamSynchronize(ctx->stream));
     RJ_CUDA(cudaGetLastError());
     const int derr = *(const int*)(host + o.err);
+    if ((derr & kErrSlots) && !ctx->exact_slots) {
+        // (a bound on the mixed blocks was too low: once more with their number)
+        ctx->exact_slots = true;
+        rc = rj_execute(ctx, q, res);
+        ctx->exact_slots = false;
+        return rc;
+    }
     if (derr & 4) return fail(ctx, RJ_E_INVALID, "error-bound outline read outside the tiered canvas's slots");
     if (derr) return fail(ctx, RJ_E_TIMEOUT, "a bounded device wait ran out (status 0x%x)", derr);
     decode_result(P, host, bounds, ctx->sum_shift, res);

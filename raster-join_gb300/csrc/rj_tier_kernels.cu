@@ -61,6 +61,8 @@ struct TierWarp {
 static_assert(sizeof(TierWarp) % 16 == 0, "TierWarp keeps 16-byte alignment");
 constexpr size_t kTierSmem = (size_t)kTW * sizeof(TierWarp);
 
+__device__ __forceinline__ bool tier_mixed(uint32_t code) { return code >= kTierMixed && code < kTierMulti; }
+
 // bits [a, b) of a word, 0 <= a < b <= 32
 __device__ __forceinline__ uint32_t bitrange(int a, int b) {
     return (b >= 32 ? 0xFFFFFFFFu : ((1u << b) - 1u)) & ~((1u << a) - 1u);
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
             bool take = false;
             if (MODE == MODE_TIER_REDUCE) {
                 if ((Iw >> lane) & 1u) {
-                    if (__ldg(tr.mixed + b) != 0u) {
+                    if (tier_mixed(__ldg(tr.code + b))) {
                         take = true;
                     } else {
                         acc_c += __ldg(tr.bcnt + b);
@@ -262,7 +264,7 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
                     take = (Uw >> lane) & 1u;
                 }
             } else {
-                take = ((Uw >> lane) & 1u) && __ldg(tr.mixed + b) != 0u;
+                take = ((Uw >> lane) & 1u) && tier_mixed(__ldg(tr.code + b));
             }
             const uint32_t m = __ballot_sync(FULL, take);
             if (lane == k) Lw = m;
@@ -334,7 +336,7 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
                 const uint32_t m8 = (S.M[k * 8 + (pr >> 1)] >> ((pr & 1) * 16 + ph)) & 0xFFu;
                 if (!m8) continue;
                 const size_t b = blk0 + bc_lo + S.list[k];
-                const size_t q = (tr.slot ? (size_t)__ldg(tr.slot + b) : b) * 256 + (size_t)pr * 16 + ph;
+                const size_t q = (size_t)(__ldg(tr.code + b) & ~kTierMixed) * 256 + (size_t)pr * 16 + ph;
                 if (MODE == MODE_TIER_LABEL) {
                     uint16_t* dst = tr.plabel + q;
                     if (m8 == 0xFFu) {
@@ -382,28 +384,63 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
 
 // code[b]: kTierMixed | slot for mixed blocks, else the full polygon (or
 // empty / multi); counts the multi blocks (two polygons cover them whole).
-// Without slots (slot = block) it also clears the pixel labels of the mixed
-// blocks, a warp writing one block's 512 bytes at a time.
-__global__ void k_tier_codes(TierArgs tr, size_t nblk, unsigned long long* multi) {
+// Slots are handed out by one atomic per warp (their order does not matter; a
+// scan of the flags cost three launches and a second pass), or each block is
+// its own slot, whose pixel labels this then clears, a warp writing one
+// block's 512 bytes at a time.
+__global__ void k_tier_codes(TierArgs tr, size_t nblk, unsigned long long* multi, int* err) {
     unsigned long long c = 0;
     const int lane = threadIdx.x & 31;
     const uint4 none = make_uint4(~0u, ~0u, ~0u, ~0u);
     for (size_t b0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) - lane; b0 < nblk;
          b0 += (size_t)gridDim.x * blockDim.x) {
         const size_t b = b0 + lane;
-        bool mixed = false;
+        const bool mixed = b < nblk && tr.mixed[b] != 0u;
+        const unsigned m = __ballot_sync(0xffffffffu, mixed);
+        uint32_t slot = (uint32_t)b;
+        if (!tr.own_place && m) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(tr.nslots, (uint32_t)__popc(m));
+            slot = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+        }
         if (b < nblk) {
             const uint32_t f = tr.full[b];
-            mixed = tr.mixed[b] != 0u;
-            tr.code[b] = mixed ? kTierMixed | (tr.slot ? (uint32_t)tr.slot[b] : (uint32_t)b) : f;
+            uint32_t code = mixed ? kTierMixed | slot : f;
+            if (mixed && !tr.own_place && slot >= tr.cap) {   // (the host runs the query again with the exact number)
+                atomicOr(err, kErrSlots);
+                code = kTierEmpty;
+            }
+            tr.code[b] = code;
             c += (f == kTierMulti);
         }
-        if (tr.slot) continue;
-        for (unsigned m = __ballot_sync(0xffffffffu, mixed); m; m &= m - 1u)
-            reinterpret_cast<uint4*>(tr.plabel + (b0 + __ffs(m) - 1) * 256)[lane] = none;
+        if (tr.own_place)
+            for (unsigned w = m; w; w &= w - 1u) reinterpret_cast<uint4*>(tr.plabel + (b0 + __ffs(w) - 1) * 256)[lane] = none;
     }
     c = warp_sum_u64(c);
     if (lane == 0 && c) atomicAdd(multi, c);
+}
+
+__global__ void k_tier_clear(TierArgs tr, size_t nblk) {
+    const int lane = threadIdx.x & 31;
+    const uint4 none = make_uint4(~0u, ~0u, ~0u, ~0u), zero = make_uint4(0u, 0u, 0u, 0u);
+    for (size_t b0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) - lane; b0 < nblk;
+         b0 += (size_t)gridDim.x * blockDim.x) {
+        const size_t b = b0 + lane;
+        const uint32_t code = b < nblk ? __ldg(tr.code + b) : kTierEmpty;
+        if (b < nblk && tr.bcnt) tr.bcnt[b] = 0u;
+        if (b < nblk && tr.bsum) tr.bsum[b] = 0;
+        for (unsigned m = __ballot_sync(0xffffffffu, tier_mixed(code)); m; m &= m - 1u) {
+            const size_t at = (size_t)(__shfl_sync(0xffffffffu, code, __ffs(m) - 1) & ~kTierMixed) * 256;
+            if (tr.plabel) reinterpret_cast<uint4*>(tr.plabel + at)[lane] = none;
+            if (tr.pcnt) {
+                reinterpret_cast<uint4*>(tr.pcnt + at)[lane] = zero;
+                reinterpret_cast<uint4*>(tr.pcnt + at)[lane + 32] = zero;
+            }
+            if (tr.psum)
+                #pragma unroll
+                for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(tr.psum + at)[lane + 32 * i] = zero;
+        }
+    }
 }
 
 // labelled pixels of the mixed blocks (overlap check: equals the pixel writes
@@ -414,7 +451,7 @@ __global__ void k_tier_nonempty(TierArgs tr, size_t nblk, unsigned long long* co
     for (size_t b0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) - lane; b0 < nblk;
          b0 += (size_t)gridDim.x * blockDim.x) {
         const uint32_t code = b0 + lane < nblk ? __ldg(tr.code + b0 + lane) : kTierEmpty;
-        for (unsigned m = __ballot_sync(0xffffffffu, code >= kTierMixed && code < kTierMulti); m; m &= m - 1u) {
+        for (unsigned m = __ballot_sync(0xffffffffu, tier_mixed(code)); m; m &= m - 1u) {
             const uint32_t slot = __shfl_sync(0xffffffffu, code, __ffs(m) - 1) & ~kTierMixed;
             const uint4 v = reinterpret_cast<const uint4*>(tr.plabel + (size_t)slot * 256)[lane];
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -446,9 +483,15 @@ void launch_tier_pass(int mode, const PolyPassArgs& a, const TierArgs& tr, int s
     }
 }
 
-void launch_tier_codes(const TierArgs& tr, size_t nblk, unsigned long long* multi, int sms, cudaStream_t st) {
+void launch_tier_codes(const TierArgs& tr, size_t nblk, unsigned long long* multi, int* err, int sms, cudaStream_t st) {
     const int blocks = (int)std::min<size_t>((nblk + 255) / 256, (size_t)sms * 16);
-    k_tier_codes<<<std::max(blocks, 1), 256, 0, st>>>(tr, nblk, multi);
+    k_tier_codes<<<std::max(blocks, 1), 256, 0, st>>>(tr, nblk, multi, err);
+    ++g_kernel_launches;
+}
+
+void launch_tier_clear(const TierArgs& tr, size_t nblk, int sms, cudaStream_t st) {
+    const int blocks = (int)std::min<size_t>((nblk + 255) / 256, (size_t)sms * 16);
+    k_tier_clear<<<std::max(blocks, 1), 256, 0, st>>>(tr, nblk);
     ++g_kernel_launches;
 }
 
