@@ -209,7 +209,25 @@ __host__ __device__ __forceinline__ int32_t pix_of(int32_t X) {
 // top-left rule).  It then toggles every pixel i whose centre lies strictly
 // left of the exact intersection x; those are the pixels i < L with
 // L = ceil((x_int - 128)/256).  Returns L (may be <0 or >res; caller clamps).
+//
+// On the device the quotient is estimated in fp32 and corrected exactly: L is
+// right iff (L - 1) * den < num <= L * den.  |coordinates| <= 2^28 and the row
+// lies between the ends, so the estimate is off by at most a pixel or two and
+// the loops end after as many steps; the usual one does not enter them (two
+// 64-bit products instead of a 64-bit division of some 100 instructions).
 __host__ __device__ __forceinline__ int32_t cross_L(int32_t ax, int32_t ay, int32_t bx, int32_t by, int32_t cy) {
+#ifdef __CUDA_ARCH__
+    const int32_t dx = bx - ax, dy = by - ay, h = cy - ay;
+    int64_t num = (int64_t)(ax - kSub / 2) * dy + (int64_t)dx * h;
+    int64_t den = (int64_t)dy * kSub;
+    if (dy < 0) { num = -num; den = -den; }
+    const float x = fmaf((float)dx, __fdividef((float)h, (float)dy), (float)(ax - kSub / 2)) * (1.0f / kSub);
+    int32_t L = __float2int_ru(x);
+    int64_t r = num - (int64_t)L * den;   // in (-den, 0] when L is right
+    while (r > 0) { ++L; r -= den; }
+    while (r <= -den) { --L; r += den; }
+    return L;
+#else
     int64_t dy = (int64_t)by - ay;
     int64_t num = ((int64_t)ax - (kSub / 2)) * dy + ((int64_t)bx - ax) * ((int64_t)cy - ay);
     int64_t den = dy * kSub;
@@ -217,9 +235,8 @@ __host__ __device__ __forceinline__ int32_t cross_L(int32_t ax, int32_t ay, int3
     // ceil(num/den)
     int64_t q = floordiv64(num, den);
     if (q * den != num) ++q;
-    if (q > (int64_t)0x3fffffff) q = 0x3fffffff;
-    if (q < -(int64_t)0x3fffffff) q = -0x3fffffff;
     return (int32_t)q;
+#endif
 }
 __host__ __device__ __forceinline__ bool cross_row(int32_t ay, int32_t by, int32_t cy) {
     return (ay >= cy) != (by >= cy);
