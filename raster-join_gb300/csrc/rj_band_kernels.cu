@@ -16,10 +16,10 @@
 //     prefix with the sign of its rank's parity, which the lane finds by
 //     comparing with the row's others -- no sorting, no order between lanes;
 //   * outline: the (edge, row) pairs are spread the same way; a lane takes the
-//     few pixels of its pair (a wide pair is taken by the whole warp), reads
-//     their counts together and clips the edge only against pixels that hold
-//     points; whether a pixel centre lies inside is the parity of the row's
-//     crossings right of it.
+//     few pixels of its pair (a wide pair is taken by the whole warp) and reads
+//     their counts together; the pixels that hold points are packed into a
+//     queue and clipped 32 at a time; whether a pixel centre lies inside is the
+//     parity of the row's crossings right of it.
 #include <climits>
 
 #include "rj_bands.cuh"
@@ -185,25 +185,31 @@ struct BandWarp {
     int start[kBand + 1];          // first crossing of each row
     int cur[kBand];                // crossings of each row
 };
+// outline: pixels that hold points, waiting for their clip (vertex, column |
+// row << 16, count); fewer than 32 left over plus four of every lane
+struct OutlineQueue {
+    int k[160];
+    uint32_t at[160];
+    uint32_t val[160];
+};
 static_assert(sizeof(BandWarp) % 16 == 0, "BandWarp keeps 16-byte alignment");
 
 template <bool SPANS, bool OUTLINE, class C>
-__global__ void __launch_bounds__(kBW * 32, OUTLINE ? 2 : 3) k_poly_bands(PolyPassArgs a, const C* __restrict__ prefix) {
+__global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPassArgs a, const C* __restrict__ prefix) {
     __shared__ BandWarp s_band[kBW];
+    __shared__ OutlineQueue s_queue[OUTLINE ? kBW : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned FULL = 0xffffffffu;
     const int TP = a.T * a.P;
-    const int total = a.band_start[TP];
     BandWarp& S = s_band[warp];
+    BandItems work(a.band_start, TP, a.work_ctr, gridDim.x * kBW, lane);
 
     for (;;) {
-        int item = 0;
-        if (lane == 0) item = (int)atomicAdd(a.work_ctr, 1u);
-        item = __shfl_sync(FULL, item, 0);
-        if (item >= total) break;
-        const int tp = warp_find_owner(a.band_start, TP, item, lane);
+        const int item = work.take(a.band_start, TP, a.work_ctr, lane);
+        if (item < 0) break;
+        const int tp = work.tp;
         const int t = tp / a.P, p = tp - t * a.P;
-        const int band = item - a.band_start[tp];
+        const int band = item - work.tp_first;
         const int4 ia = a.info_a[tp];
         const int2 ib = a.info_b[tp];
         const int i_lo = ia.x, i_hi = ia.y, j_lo = ib.x, j_hi = ib.y;
@@ -218,25 +224,12 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 2 : 3) k_poly_bands(PolyPa
         // edges within a pixel of the band's rows
         const int64_t band_lo = (int64_t)jb * kSub - kSub;
         const int64_t band_hi = (int64_t)(je + 1) * kSub + kSub;
-        int nb = 0;
-        for (int k0 = 0; k0 < n; k0 += 32) {
-            const int k = k0 + lane;
-            bool take = false;
-            int4 e = make_int4(0, 0, 0, 0);
-            if (k < n) {
-                const int2 A = pv[k];
-                const int2 B = pv[(k + 1 == n) ? 0 : k + 1];
-                take = (max(A.y, B.y) >= band_lo) && (min(A.y, B.y) <= band_hi);
-                e = make_int4(A.x, A.y, B.x, B.y);
-            }
-            const unsigned m = __ballot_sync(FULL, take);
-            const int pos = nb + __popc(m & ((1u << lane) - 1u));
-            if (take && pos < kBEdges) {
+        const int nb = stage_edges(pv, n, band_lo, band_hi, lane, [&](int pos, int k, const int4& e) {
+            if (pos < kBEdges) {
                 S.edge[pos] = e;
                 if (OUTLINE) S.eidx[pos] = k;
             }
-            nb += __popc(m);
-        }
+        });
         const bool overflow = nb > kBEdges;
         const int ne = overflow ? n : nb;
         auto edge_at = [&](int e) -> int4 {
@@ -371,37 +364,49 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 2 : 3) k_poly_bands(PolyPa
                         for (int u = 0; u < 4; ++u) v[u] = i + u <= last ? (uint32_t)(w[u + 1] - w[u]) : 0u;
                     }
                 };
-                auto visit = [&](const float2& P0, const float2& P1, int i, int r, uint32_t val) {
-                    const int j = jb + r;
-                    if (a.line_filter) {
-                        // varying interpolation along the line (projection of
-                        // the pixel centre), kept within 0.5 px: line-bound.frag:221
-                        const float cxp = (float)i + 0.5f, cyp = (float)j + 0.5f;
-                        const float dx = __fsub_rn(P1.x, P0.x), dy = __fsub_rn(P1.y, P0.y);
-                        const float l2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-                        if (!(l2 > 0.0f)) return;
-                        const float tt = __fdiv_rn(__fadd_rn(__fmul_rn(__fsub_rn(cxp, P0.x), dx),
-                                                             __fmul_rn(__fsub_rn(cyp, P0.y), dy)), l2);
-                        const float qx = __fadd_rn(P0.x, __fmul_rn(tt, dx));
-                        const float qy = __fadd_rn(P0.y, __fmul_rn(tt, dy));
-                        if (fabsf(__fsub_rn(qx, cxp)) >= 0.5f || fabsf(__fsub_rn(qy, cyp)) >= 0.5f) return;
+                OutlineQueue& Q = s_queue[OUTLINE ? warp : 0];
+                int qn = 0;
+                // the clip of the last 32 (or fewer) queued pixels
+                auto drain = [&]() {
+                    const int first = max(qn - 32, 0), x = first + lane;
+                    if (x < qn) {
+                        const int k = Q.k[x], i = (int)(Q.at[x] & 0xFFFFu), r = (int)(Q.at[x] >> 16), j = jb + r;
+                        const uint32_t val = Q.val[x];
+                        const float2 P0 = pf[k], P1 = pf[(k + 1 == n) ? 0 : k + 1];
+                        bool ok = true;
+                        if (a.line_filter) {
+                            // varying interpolation along the line (projection of
+                            // the pixel centre), kept within 0.5 px: line-bound.frag:221
+                            const float cxp = (float)i + 0.5f, cyp = (float)j + 0.5f;
+                            const float dx = __fsub_rn(P1.x, P0.x), dy = __fsub_rn(P1.y, P0.y);
+                            const float l2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+                            ok = l2 > 0.0f;
+                            const float tt = __fdiv_rn(__fadd_rn(__fmul_rn(__fsub_rn(cxp, P0.x), dx),
+                                                                 __fmul_rn(__fsub_rn(cyp, P0.y), dy)), l2);
+                            const float qx = __fadd_rn(P0.x, __fmul_rn(tt, dx));
+                            const float qy = __fadd_rn(P0.y, __fmul_rn(tt, dy));
+                            if (fabsf(__fsub_rn(qx, cxp)) >= 0.5f || fabsf(__fsub_rn(qy, cyp)) >= 0.5f) ok = false;
+                        }
+                        float frac;
+                        if (ok && compute_fraction(P0.x, P0.y, P1.x, P1.y, (float)i, (float)j, (float)(i + 1), (float)(j + 1),
+                                                   frac)) {
+                            // inside test of the pixel centre: the coverage rule (an
+                            // odd number of the row's crossings right of i)
+                            bool inside = false;
+                            if (r >= cl && r <= ch) {
+                                if (slow) inside = inside_slow(i, r);
+                                else
+                                    for (int c = S.start[r] - base, e = c + S.cur[r]; c < e; ++c)
+                                        inside ^= (int)(S.cross[c] & 0xFFFFu) > i;
+                            }
+                            if (frac > 0.5f) frac = __fsub_rn(1.0f, frac);
+                            const int add = (int)ceilf(__fmul_rn(frac, (float)val));
+                            if (inside) { b_fp += add; b_fp1 += val; }
+                            else        { b_fn += add; b_fn1 += val; }
+                        }
                     }
-                    float frac;
-                    if (!compute_fraction(P0.x, P0.y, P1.x, P1.y, (float)i, (float)j, (float)(i + 1), (float)(j + 1), frac))
-                        return;
-                    // inside test of the pixel centre: the coverage rule (an odd
-                    // number of the row's crossings right of i)
-                    bool inside = false;
-                    if (r >= cl && r <= ch) {
-                        if (slow) inside = inside_slow(i, r);
-                        else
-                            for (int k = S.start[r] - base, e = k + S.cur[r]; k < e; ++k)
-                                inside ^= (int)(S.cross[k] & 0xFFFFu) > i;
-                    }
-                    if (frac > 0.5f) frac = __fsub_rn(1.0f, frac);
-                    const int add = (int)ceilf(__fmul_rn(frac, (float)val));
-                    if (inside) { b_fp += add; b_fp1 += val; }
-                    else        { b_fn += add; b_fn1 += val; }
+                    qn = first;
+                    __syncwarp();
                 };
                 // (edge, row) pairs whose rectangles can touch: rows j with
                 // j <= the edge's top and j + 1 >= its bottom
@@ -417,10 +422,8 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 2 : 3) k_poly_bands(PolyPa
                     [](int k, int lo) { return __shfl_sync(0xffffffffu, k, lo); },
                     [&](bool live, int k, int r) {
                         int i0 = 0, i1 = -1;
-                        float2 P0 = make_float2(0.f, 0.f), P1 = P0;
                         if (live) {
-                            P0 = pf[k];
-                            P1 = pf[(k + 1 == n) ? 0 : k + 1];
+                            const float2 P0 = pf[k], P1 = pf[(k + 1 == n) ? 0 : k + 1];
                             const float ylo = (float)(jb + r), yhi = (float)(jb + r + 1);
                             // x range of the edge inside the row and a pixel more on
                             // each side: on a nearly horizontal edge the clip's fp32
@@ -439,29 +442,49 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 2 : 3) k_poly_bands(PolyPa
                             i0 = max((int)floorf(xa) - 1, 0);
                             i1 = min((int)floorf(xb) + 1, a.resx - 1);
                         }
-                        // wide pairs: the whole warp, four pixels a lane
-                        for (unsigned wide = __ballot_sync(FULL, i1 - i0 >= 16); wide; wide &= wide - 1u) {
-                            const int src = __ffs(wide) - 1;
-                            const int wk = __shfl_sync(FULL, k, src), wr = __shfl_sync(FULL, r, src);
-                            const int w0 = __shfl_sync(FULL, i0, src), w1 = __shfl_sync(FULL, i1, src);
-                            const float2 Q0 = pf[wk], Q1 = pf[(wk + 1 == n) ? 0 : wk + 1];
-                            for (int i = w0 + lane * 4; i <= w1; i += 128) {
-                                uint32_t v[4];
-                                counts(i, w1, wr, v);
-                                #pragma unroll 1
-                                for (int u = 0; u < 4; ++u)
-                                    if (v[u]) visit(Q0, Q1, i + u, wr, v[u]);
+                        // rounds of four pixels a lane: wide pairs one after the
+                        // other, by the whole warp, then every lane its own (one
+                        // place for the reads, the queue and the clip: inlined
+                        // twice over, the code outgrew the instruction cache)
+                        unsigned wide = __ballot_sync(FULL, i1 - i0 >= 16);
+                        if ((wide >> lane) & 1u) i1 = -1 - i1;   // (kept for the others to read)
+                        int wi = 0;
+                        for (;;) {
+                            int rk = k, rr = r, ri = i0, re = i1;
+                            if (wide) {
+                                const int src = __ffs(wide) - 1;
+                                rk = __shfl_sync(FULL, k, src);
+                                rr = __shfl_sync(FULL, r, src);
+                                re = -1 - __shfl_sync(FULL, i1, src);
+                                ri = __shfl_sync(FULL, i0, src) + wi + lane * 4;
+                                wi += 128;
+                                if (ri - lane * 4 + 128 > re) {
+                                    wide &= wide - 1u;
+                                    wi = 0;
+                                }
+                            } else {
+                                if (!__any_sync(FULL, i0 <= i1)) break;
+                                i0 += 4;
                             }
+                            uint32_t v[4] = {0u, 0u, 0u, 0u};
+                            if (ri <= re) counts(ri, re, rr, v);
+                            #pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const unsigned m = __ballot_sync(FULL, v[u] != 0u);
+                                if (v[u]) {
+                                    const int x = qn + __popc(m & ((1u << lane) - 1u));
+                                    Q.k[x] = rk;
+                                    Q.at[x] = (uint32_t)(ri + u) | ((uint32_t)rr << 16);
+                                    Q.val[x] = v[u];
+                                }
+                                qn += __popc(m);
+                            }
+                            __syncwarp();
+                            #pragma unroll 1
+                            while (qn >= 32) drain();
                         }
-                        if (i1 - i0 < 16)
-                            for (int i = i0; i <= i1; i += 4) {
-                                uint32_t v[4];
-                                counts(i, i1, r, v);
-                                #pragma unroll 1
-                                for (int u = 0; u < 4; ++u)
-                                    if (v[u]) visit(P0, P1, i + u, r, v[u]);
-                            }
                     });
+                if (qn > 0) drain();
             }
             __syncwarp();
             ra = rb;

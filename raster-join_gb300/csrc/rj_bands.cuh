@@ -17,6 +17,68 @@ __device__ __forceinline__ void edge_rows(int32_t ay, int32_t by, int jb, int& r
     r1 = (int)(a1 > kBand - 1 ? kBand - 1 : a1);
 }
 
+// Work items (tile, polygon, band) of a persistent warp: taken a few at a time
+// from the counter, the next ones asked for before these are worked on, the
+// owner looked up when it changes.  A pass over few items is latency from end
+// to end, so every dependent load saved counts.
+struct BandItems {
+    int next, first, last, chunk, total;
+    int tp, tp_first, tp_last;      // owner of the current item, its items [tp_first, tp_last)
+    __device__ __forceinline__ BandItems(const int* band_start, int TP, unsigned* ctr, int nwarps, int lane) {
+        total = band_start[TP];
+        chunk = min(max(total / (nwarps * 4), 1), 4);
+        next = lane == 0 ? (int)atomicAdd(ctr, (unsigned)chunk) : 0;
+        first = last = 0;
+        tp = -1;
+        tp_first = tp_last = 0;
+    }
+    // the next item, or -1 (the whole warp calls this)
+    __device__ __forceinline__ int take(const int* band_start, int TP, unsigned* ctr, int lane) {
+        if (first >= last) {
+            first = __shfl_sync(0xffffffffu, next, 0);
+            if (first >= total) return -1;
+            last = min(first + chunk, total);
+            if (lane == 0) next = (int)atomicAdd(ctr, (unsigned)chunk);
+        }
+        const int item = first++;
+        if (tp < 0 || item >= tp_last) {
+            tp = warp_find_owner(band_start, TP, item, lane);
+            tp_first = __ldg(band_start + tp);
+            tp_last = __ldg(band_start + tp + 1);
+        }
+        return item;
+    }
+};
+
+// Edges of the ring pv[0, n) that meet the fixed-point rows [lo, hi], staged in
+// order (f(position, vertex, edge) for each that is taken); returns how many
+// there are.  Four rounds of vertices are loaded before the first is used.
+template <class F>
+__device__ __forceinline__ int stage_edges(const int2* __restrict__ pv, int n, int64_t lo, int64_t hi, int lane, F&& f) {
+    int nb = 0;
+    for (int k0 = 0; k0 < n; k0 += 128) {
+        int2 A[4], B[4];
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k = k0 + u * 32 + lane;
+            A[u] = B[u] = make_int2(0, 0);
+            if (k < n) {
+                A[u] = pv[k];
+                B[u] = pv[(k + 1 == n) ? 0 : k + 1];
+            }
+        }
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k = k0 + u * 32 + lane;
+            const bool take = k < n && max(A[u].y, B[u].y) >= lo && min(A[u].y, B[u].y) <= hi;
+            const unsigned m = __ballot_sync(0xffffffffu, take);
+            if (take) f(nb + __popc(m & ((1u << lane) - 1u)), k, make_int4(A[u].x, A[u].y, B[u].x, B[u].y));
+            nb += __popc(m);
+        }
+    }
+    return nb;
+}
+
 // f(q, r) for every row r of the ranges that range(e, q, r0, cnt) gives the
 // items e < ne (rows r0 .. r0 + cnt - 1, payload q), spread over the lanes: an
 // edge of 16 rows gives 16 lanes work instead of one lane 16 rounds.  Every

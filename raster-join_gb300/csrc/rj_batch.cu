@@ -179,8 +179,7 @@ size_t tier_canvas_bytes(const QPlan& p) {
 size_t canvas_bytes(const QPlan& p) {
     const bool agg = p.f.aggr != 0;
     if (p.tier) {
-        const size_t base = 4 * al256(p.nblk * 4) + al256((p.nblk + 1) * 4) +
-                            al256(4);
+        const size_t base = al256(p.nblk * 8) + 2 * al256(p.nblk * 4) + al256(4);
         return base + (p.mode == BQ_TLABEL ? al256(p.est_slots * 256 * 2) : tier_canvas_bytes(p));
     }
     return p.mode == BQ_LABEL ? al256(p.npix * 2) : al256(p.npix * 4) + (agg ? al256(p.npix * 8) : 0);
@@ -452,7 +451,7 @@ int run_fused(Engine& e, std::vector<QPlan>& plans, uint32_t flags, BatchOut& bo
             p->cs = nullptr;
             if (p->tier && p->mode != BQ_SKIP) {
                 TierArgs& tr = p->tr;
-                tr.full = ar.take<uint32_t>(p->nblk);
+                tr.full = ar.take<unsigned long long>(p->nblk);
                 tr.mixed = ar.take<uint32_t>(p->nblk);
                 p->slot_buf = ar.take<int>(1);
                 tr.nslots = reinterpret_cast<uint32_t*>(p->slot_buf);
@@ -495,7 +494,7 @@ int run_fused(Engine& e, std::vector<QPlan>& plans, uint32_t flags, BatchOut& bo
             QPlan* p = wave[i];
             if (!p->tier || p->mode == BQ_SKIP) continue;
             any_tier = true;
-            RJ_CUDA(cudaMemsetAsync(p->tr.full, 0xFF, p->nblk * 4, st));
+            RJ_CUDA(cudaMemsetAsync(p->tr.full, 0, p->nblk * 8, st));
             RJ_CUDA(cudaMemsetAsync(p->tr.mixed, 0, p->nblk * 4, st));
             if (!query_poly_pass(e, *p, MODE_TIER_CLASSIFY, ps, nullptr, nullptr, nullptr, &p->tr))
                 return fail(ctx, RJ_E_INVALID, "too many (tile, polygon) items");

@@ -18,7 +18,9 @@ constexpr uint32_t kTierMulti = 0xFFFFFFFEu;   // two or more polygons cover it 
 constexpr uint32_t kTierMixed = 0x80000000u;   // | slot: per-pixel data in the slot
 struct TierArgs {
     int bw, bh;                  // blocks per tile row / per tile column
-    uint32_t* full;              // [nblk] polygon covering the whole block, kTierEmpty, kTierMulti
+    // [nblk] polygons covering the whole block: their number << 32 + the sum of
+    // their ids (zeroed; one add without a result per polygon)
+    unsigned long long* full;
     uint32_t* mixed;             // [nblk] 1: per-pixel block
     bool own_place;              // the slot of a mixed block is the block itself
     uint32_t* nslots;            // else: slots handed out so far (zeroed), at most cap

@@ -153,18 +153,16 @@ k_poly_label(PolyPassArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned FULL = 0xffffffffu;
     const int TP = a.T * a.P;
-    const int total = a.band_start[TP];
+    BandItems work(a.band_start, TP, a.work_ctr, gridDim.x * kPolyWarps, lane);
     int4* my_edge = s_poly + (size_t)warp * kBandCap;
     int* my_cross = reinterpret_cast<int*>(s_poly + (size_t)kPolyWarps * kBandCap) + (size_t)warp * kCrossCap;
 
     for (;;) {
-        int item = 0;
-        if (lane == 0) item = (int)atomicAdd(a.work_ctr, 1u);
-        item = __shfl_sync(FULL, item, 0);
-        if (item >= total) break;
-        const int tp = warp_find_owner(a.band_start, TP, item, lane);
+        const int item = work.take(a.band_start, TP, a.work_ctr, lane);
+        if (item < 0) break;
+        const int tp = work.tp;
         const int t = tp / a.P, p = tp - t * a.P;
-        const int band = item - a.band_start[tp];
+        const int band = item - work.tp_first;
         const int4 ia = a.info_a[tp];
         const int2 ib = a.info_b[tp];
         const int i_lo = ia.x, i_hi = ia.y, j_lo = ib.x, j_hi = ib.y;
@@ -179,23 +177,9 @@ k_poly_label(PolyPassArgs a) {
         // fixed-point y window of the band (one pixel of margin each side)
         const int64_t band_lo = (int64_t)jb * kSub - kSub;
         const int64_t band_hi = (int64_t)(je + 1) * kSub + kSub;
-        int nb = 0;
-        for (int k0 = 0; k0 < n; k0 += 32) {
-            int k = k0 + lane;
-            bool take = false;
-            int4 e = make_int4(0, 0, 0, 0);
-            if (k < n) {
-                int2 A = pv[k];
-                int2 B = pv[(k + 1 == n) ? 0 : k + 1];
-                int lo = min(A.y, B.y), hi = max(A.y, B.y);
-                take = (hi >= band_lo) && (lo <= band_hi);
-                e = make_int4(A.x, A.y, B.x, B.y);
-            }
-            unsigned m = __ballot_sync(FULL, take);
-            int pos = nb + __popc(m & ((1u << lane) - 1u));
-            if (take && pos < kBandCap) my_edge[pos] = e;
-            nb += __popc(m);
-        }
+        const int nb = stage_edges(pv, n, band_lo, band_hi, lane, [&](int pos, int, const int4& e) {
+            if (pos < kBandCap) my_edge[pos] = e;
+        });
         const bool overflow = nb > kBandCap;
         __syncwarp();
 

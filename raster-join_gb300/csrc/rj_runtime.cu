@@ -812,17 +812,16 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
     const size_t nblk = (size_t)a.T * tr.bw * tr.bh;
     if (nblk >= (size_t)1 << 24) return fail(ctx, RJ_E_UNSUPPORTED, "canvas too large for the tiered form");
     // multi blocks, covered pixel writes, labelled pixels, slots; then the
-    // mixed flags (zeroed together)
+    // blocks' covering polygons and mixed flags (zeroed together)
     unsigned long long* cnt;
-    if ((rc = scratch_t(ctx, "tier_full", nblk, &tr.full))) return rc;
-    if ((rc = scratch_t(ctx, "tier_cnt_mixed", 4 + (nblk + 1) / 2, &cnt))) return rc;
+    if ((rc = scratch_t(ctx, "tier_blocks", 4 + nblk + (nblk + 1) / 2, &cnt))) return rc;
     if ((rc = scratch_t(ctx, "tier_code", nblk, &tr.code))) return rc;
     tr.nslots = reinterpret_cast<uint32_t*>(cnt + 3);
-    tr.mixed = reinterpret_cast<uint32_t*>(cnt + 4);
+    tr.full = cnt + 4;
+    tr.mixed = reinterpret_cast<uint32_t*>(tr.full + nblk);
     // error bounds: the blocks the outline pass reads are mixed too
     tr.outline = bounds ? 1 : 0;
-    RJ_CUDA(cudaMemsetAsync(tr.full, 0xFF, nblk * 4, ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(cnt, 0, 4 * 8 + nblk * 4, ctx->stream));
+    RJ_CUDA(cudaMemsetAsync(cnt, 0, 4 * 8 + nblk * 12, ctx->stream));
     a.outline_rows = tr.outline;
     rc = poly_pass(ctx, MODE_TIER_CLASSIFY, a, &tr);
     a.outline_rows = 0;
@@ -1423,13 +1422,12 @@ int label_blocks(rj_ctx* ctx, const DevFilter& f, const CanvasXf& cx, PolyPassAr
     tr.bh = (a.resy + 15) / 16;
     const size_t nblk = (size_t)tr.bw * tr.bh;
     unsigned long long* cnt;   // multi blocks, covered pixel writes, labelled pixels
-    if ((rc = scratch_t(ctx, "tier_full", nblk, &tr.full))) return rc;
-    if ((rc = scratch_t(ctx, "tier_cnt_mixed", 3 + (nblk + 1) / 2, &cnt))) return rc;   // zeroed together
+    if ((rc = scratch_t(ctx, "tier_blocks", 4 + nblk + (nblk + 1) / 2, &cnt))) return rc;   // zeroed together
     if ((rc = scratch_t(ctx, "tier_code", nblk, &tr.code))) return rc;
     if ((rc = scratch_t(ctx, "tier_plabel", nblk * 256, &tr.plabel))) return rc;
-    tr.mixed = reinterpret_cast<uint32_t*>(cnt + 3);
-    RJ_CUDA(cudaMemsetAsync(tr.full, 0xFF, nblk * 4, ctx->stream));
-    RJ_CUDA(cudaMemsetAsync(cnt, 0, 3 * 8 + nblk * 4, ctx->stream));
+    tr.full = cnt + 4;
+    tr.mixed = reinterpret_cast<uint32_t*>(tr.full + nblk);
+    RJ_CUDA(cudaMemsetAsync(cnt, 0, 4 * 8 + nblk * 12, ctx->stream));
     if ((rc = poly_pass(ctx, MODE_TIER_CLASSIFY, a, &tr))) return rc;
     launch_tier_codes(tr, nblk, cnt, ctx->q_err, ctx->sms, ctx->stream);
     a.covered = cnt + 1;

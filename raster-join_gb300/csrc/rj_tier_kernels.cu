@@ -28,9 +28,8 @@
 //     pixel, which holds for the whole block row unless the block is flagged.
 //     Over the 16 rows: I = blocks covered throughout (full for the polygon),
 //     U = blocks the polygon covers somewhere.
-//   * the blocks whose pixels matter (labels: U and mixed; reduce: U and not
-//     full, or full and mixed -- a mixed block's points are in its pixel slot
-//     only) are listed, up to 64 at a time; sweep 2 toggles per-pixel bits of
+//   * the blocks whose pixels matter (U and mixed; a mixed block's points are
+//     in its pixel slot only) are listed, up to 64 at a time; sweep 2 toggles per-pixel bits of
 //     the listed blocks only, and their 16-bit row masks follow from the
 //     block's first-pixel coverage and a 16-bit prefix XOR;
 //   * the listed blocks' pixel slots are then read or written by the whole
@@ -45,7 +44,7 @@ namespace {
 
 constexpr int kTW = 8;            // warps per block
 constexpr int kTBand = kBand;     // rows per work item: one block row
-constexpr int kTEdgeCap = 256;    // staged edges per warp
+constexpr int kTEdgeCap = 112;    // staged edges per warp (more: read from global memory)
 constexpr int kTBW = 16;          // block-bitmap words per row: 512 block columns = 8192 pixels
 constexpr int kTList = 64;        // blocks whose pixels one round visits
 
@@ -55,6 +54,7 @@ struct TierWarp {
     uint32_t X[kTBand * kTBW];          // block toggles, then coverage at each block's first pixel
     uint32_t C[kTBand * kTBW];          // blocks with a crossing inside (pixel offsets 1..15)
     uint32_t M[kTList * kTBand / 2];    // listed blocks: pixel toggles, then row masks (two rows a word)
+    uint32_t slot[kTList];              // listed blocks' slots
     uint16_t list[kTList];              // listed block columns (relative to bc_lo)
     uint8_t map[kTBW * 32];             // block column -> list index, 0xFF when not listed
 };
@@ -78,13 +78,13 @@ __device__ __forceinline__ uint32_t prefix_xor(uint32_t x) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs tr) {
+__global__ void __launch_bounds__(kTW * 32, 4) k_tier_pass(PolyPassArgs a, TierArgs tr) {
     extern __shared__ int4 s_tier[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned FULL = 0xffffffffu;
     const int TP = a.T * a.P;
-    const int total = a.band_start[TP];
     TierWarp& S = reinterpret_cast<TierWarp*>(s_tier)[warp];
+    BandItems work(a.band_start, TP, a.work_ctr, gridDim.x * kTW, lane);
     for (int w = lane; w < kTBand * kTBW; w += 32) {
         S.X[w] = 0u;
         S.C[w] = 0u;
@@ -93,13 +93,11 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
     __syncwarp();
     const int hw = lane & 15, half = lane >> 4;   // sweep 1: row 2k + half, block word hw
     for (;;) {
-        int item = 0;
-        if (lane == 0) item = (int)atomicAdd(a.work_ctr, 1u);
-        item = __shfl_sync(FULL, item, 0);
-        if (item >= total) break;
-        const int tp = warp_find_owner(a.band_start, TP, item, lane);
+        const int item = work.take(a.band_start, TP, a.work_ctr, lane);
+        if (item < 0) break;
+        const int tp = work.tp;
         const int t = tp / a.P, p = tp - t * a.P;
-        const int band = item - a.band_start[tp];
+        const int band = item - work.tp_first;
         const int4 ia = a.info_a[tp];
         const int2 ib = a.info_b[tp];
         const int i_lo = ia.x, i_hi = ia.y, j_lo = ib.x, j_hi = ib.y;
@@ -116,23 +114,9 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
         // stage the edges that can cross a row centre of the band
         const int64_t band_lo = (int64_t)jb * kSub - kSub;
         const int64_t band_hi = (int64_t)(jb + kTBand) * kSub + kSub;
-        int nb = 0;
-        for (int k0 = 0; k0 < n; k0 += 32) {
-            const int k = k0 + lane;
-            bool take = false;
-            int4 e = make_int4(0, 0, 0, 0);
-            if (k < n) {
-                const int2 A = pv[k];
-                const int2 B = pv[(k + 1 == n) ? 0 : k + 1];
-                const int lo = min(A.y, B.y), hi = max(A.y, B.y);
-                take = (hi >= band_lo) && (lo <= band_hi);
-                e = make_int4(A.x, A.y, B.x, B.y);
-            }
-            const unsigned m = __ballot_sync(FULL, take);
-            const int pos = nb + __popc(m & ((1u << lane) - 1u));
-            if (take && pos < kTEdgeCap) S.edge[pos] = e;
-            nb += __popc(m);
-        }
+        const int nb = stage_edges(pv, n, band_lo, band_hi, lane, [&](int pos, int, const int4& e) {
+            if (pos < kTEdgeCap) S.edge[pos] = e;
+        });
         const bool overflow = nb > kTEdgeCap;
         const int ne = overflow ? n : nb;
         __syncwarp();
@@ -230,7 +214,7 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
                 if (!((Uw >> lane) & 1u)) continue;
                 const size_t b = blk0 + bc_lo + rel;
                 if ((Iw >> lane) & 1u) {
-                    if (atomicCAS(tr.full + b, kTierEmpty, (uint32_t)p) != kTierEmpty) atomicExch(tr.full + b, kTierMulti);
+                    atomicAdd(tr.full + b, (1ull << 32) + (unsigned long long)p);
                 } else {
                     tr.mixed[b] = 1u;
                 }
@@ -242,32 +226,38 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
 
         unsigned long long acc_c = 0;
         long long acc_s = 0;
-        // listed blocks: reduce -- covered and not full, or full and mixed
-        // (a mixed block's points are in its pixel slot only; the other full
-        // blocks take their block totals); labels -- covered and mixed
+        // listed blocks: covered and mixed (a block covered but not full is
+        // mixed; reduce: the full blocks that are not mixed give their totals)
         uint32_t Lw = 0u;   // lane k < nbw: listed blocks of word k
-        for (int k = 0; k < nbw; ++k) {
-            const uint32_t Iw = __shfl_sync(FULL, I, k), Uw = __shfl_sync(FULL, U, k);
-            if (!Uw) continue;
-            const int rel = k * 32 + lane;
-            const size_t b = blk0 + bc_lo + rel;
-            bool take = false;
-            if (MODE == MODE_TIER_REDUCE) {
-                if ((Iw >> lane) & 1u) {
-                    if (tier_mixed(__ldg(tr.code + b))) {
-                        take = true;
-                    } else {
-                        acc_c += __ldg(tr.bcnt + b);
-                        if (tr.bsum) acc_s += __ldg(tr.bsum + b);
-                    }
-                } else {
-                    take = (Uw >> lane) & 1u;
-                }
-            } else {
-                take = ((Uw >> lane) & 1u) && tier_mixed(__ldg(tr.code + b));
+        // (the words' block codes are loaded four words at a time)
+        for (int k0 = 0; k0 < nbw; k0 += 4) {
+            uint32_t code[4], cb[4];
+            long long sb[4];
+            #pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t Uw = k0 + u < nbw ? __shfl_sync(FULL, U, k0 + u) : 0u;
+                code[u] = (Uw >> lane) & 1u ? __ldg(tr.code + blk0 + bc_lo + (k0 + u) * 32 + lane) : kTierEmpty;
             }
-            const uint32_t m = __ballot_sync(FULL, take);
-            if (lane == k) Lw = m;
+            if (MODE == MODE_TIER_REDUCE) {
+                #pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    // a covered block that is not mixed is full: its total
+                    const bool whole = code[u] != kTierEmpty && !tier_mixed(code[u]);
+                    const size_t b = blk0 + bc_lo + (k0 + u) * 32 + lane;
+                    cb[u] = whole ? __ldg(tr.bcnt + b) : 0u;
+                    sb[u] = whole && tr.bsum ? __ldg(tr.bsum + b) : 0;
+                }
+                #pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    acc_c += cb[u];
+                    acc_s += sb[u];
+                }
+            }
+            #pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t m = __ballot_sync(FULL, tier_mixed(code[u]));
+                if (lane == k0 + u) Lw = m;
+            }
         }
         // list positions: exclusive prefix of the words' counts
         const int cnt = lane < nbw ? __popc(Lw) : 0;
@@ -292,6 +282,7 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
                     if (g >= start) {
                         S.map[lane * 32 + bit] = (uint8_t)(g - start);
                         S.list[g - start] = (uint16_t)(lane * 32 + bit);
+                        S.slot[g - start] = __ldg(tr.code + blk0 + bc_lo + lane * 32 + bit) & ~kTierMixed;
                     }
                     ++g;
                 }
@@ -335,8 +326,7 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
             for (int k = 0; k < nk; ++k) {
                 const uint32_t m8 = (S.M[k * 8 + (pr >> 1)] >> ((pr & 1) * 16 + ph)) & 0xFFu;
                 if (!m8) continue;
-                const size_t b = blk0 + bc_lo + S.list[k];
-                const size_t q = (size_t)(__ldg(tr.code + b) & ~kTierMixed) * 256 + (size_t)pr * 16 + ph;
+                const size_t q = (size_t)S.slot[k] * 256 + (size_t)pr * 16 + ph;
                 if (MODE == MODE_TIER_LABEL) {
                     uint16_t* dst = tr.plabel + q;
                     if (m8 == 0xFFu) {
@@ -384,34 +374,50 @@ __global__ void __launch_bounds__(kTW * 32) k_tier_pass(PolyPassArgs a, TierArgs
 
 // code[b]: kTierMixed | slot for mixed blocks, else the full polygon (or
 // empty / multi); counts the multi blocks (two polygons cover them whole).
-// Slots are handed out by one atomic per warp (their order does not matter; a
-// scan of the flags cost three launches and a second pass), or each block is
+// Slots are handed out by one atomic per 256 blocks (their order does not
+// matter; one per warp took 150 us for 6.2M blocks, this 35), or each block is
 // its own slot, whose pixel labels this then clears, a warp writing one
 // block's 512 bytes at a time.
-__global__ void k_tier_codes(TierArgs tr, size_t nblk, unsigned long long* multi, int* err) {
+constexpr int kCodeThreads = 256;
+__global__ void __launch_bounds__(kCodeThreads) k_tier_codes(TierArgs tr, size_t nblk, unsigned long long* multi, int* err) {
+    __shared__ uint32_t s_warp[kCodeThreads / 32];
+    __shared__ uint32_t s_base;
     unsigned long long c = 0;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint4 none = make_uint4(~0u, ~0u, ~0u, ~0u);
-    for (size_t b0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) - lane; b0 < nblk;
-         b0 += (size_t)gridDim.x * blockDim.x) {
-        const size_t b = b0 + lane;
+    // (block-uniform trip count)
+    for (size_t first = (size_t)blockIdx.x * kCodeThreads; first < nblk; first += (size_t)gridDim.x * kCodeThreads) {
+        const size_t b = first + threadIdx.x, b0 = b - lane;
         const bool mixed = b < nblk && tr.mixed[b] != 0u;
         const unsigned m = __ballot_sync(0xffffffffu, mixed);
         uint32_t slot = (uint32_t)b;
-        if (!tr.own_place && m) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(tr.nslots, (uint32_t)__popc(m));
-            slot = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+        if (!tr.own_place) {
+            if (lane == 0) s_warp[warp] = (uint32_t)__popc(m);
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                uint32_t n = 0;
+                #pragma unroll
+                for (int w = 0; w < kCodeThreads / 32; ++w) {
+                    const uint32_t k = s_warp[w];
+                    s_warp[w] = n;
+                    n += k;
+                }
+                s_base = n ? atomicAdd(tr.nslots, n) : 0u;
+            }
+            __syncthreads();
+            slot = s_base + s_warp[warp] + __popc(m & ((1u << lane) - 1u));
+            __syncthreads();
         }
         if (b < nblk) {
-            const uint32_t f = tr.full[b];
-            uint32_t code = mixed ? kTierMixed | slot : f;
+            const unsigned long long f = tr.full[b];
+            const uint32_t n = (uint32_t)(f >> 32);
+            uint32_t code = mixed ? kTierMixed | slot : n == 0 ? kTierEmpty : n == 1 ? (uint32_t)f : kTierMulti;
             if (mixed && !tr.own_place && slot >= tr.cap) {   // (the host runs the query again with the exact number)
                 atomicOr(err, kErrSlots);
                 code = kTierEmpty;
             }
             tr.code[b] = code;
-            c += (f == kTierMulti);
+            c += n > 1;
         }
         if (tr.own_place)
             for (unsigned w = m; w; w &= w - 1u) reinterpret_cast<uint4*>(tr.plabel + (b0 + __ffs(w) - 1) * 256)[lane] = none;
@@ -485,7 +491,7 @@ void launch_tier_pass(int mode, const PolyPassArgs& a, const TierArgs& tr, int s
 
 void launch_tier_codes(const TierArgs& tr, size_t nblk, unsigned long long* multi, int* err, int sms, cudaStream_t st) {
     const int blocks = (int)std::min<size_t>((nblk + 255) / 256, (size_t)sms * 16);
-    k_tier_codes<<<std::max(blocks, 1), 256, 0, st>>>(tr, nblk, multi, err);
+    k_tier_codes<<<std::max(blocks, 1), kCodeThreads, 0, st>>>(tr, nblk, multi, err);
     ++g_kernel_launches;
 }
 
