@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPa
     const unsigned FULL = 0xffffffffu;
     const int TP = a.T * a.P;
     BandWarp& S = s_band[warp];
-    BandItems work(a.band_start, TP, a.work_ctr, gridDim.x * kBW, lane);
+    BandItems work(a.band_start, TP, a.work_ctr, kBW, warp, lane);
 
     for (;;) {
         const int item = work.take(a.band_start, TP, a.work_ctr, lane);

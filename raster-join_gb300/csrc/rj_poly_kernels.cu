@@ -153,7 +153,7 @@ k_poly_label(PolyPassArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned FULL = 0xffffffffu;
     const int TP = a.T * a.P;
-    BandItems work(a.band_start, TP, a.work_ctr, gridDim.x * kPolyWarps, lane);
+    BandItems work(a.band_start, TP, a.work_ctr, kPolyWarps, warp, lane);
     int4* my_edge = s_poly + (size_t)warp * kBandCap;
     int* my_cross = reinterpret_cast<int*>(s_poly + (size_t)kPolyWarps * kBandCap) + (size_t)warp * kCrossCap;
 

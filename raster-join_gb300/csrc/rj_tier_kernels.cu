@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kTW * 32, 4) k_tier_pass(PolyPassArgs a, TierA
     const unsigned FULL = 0xffffffffu;
     const int TP = a.T * a.P;
     TierWarp& S = reinterpret_cast<TierWarp*>(s_tier)[warp];
-    BandItems work(a.band_start, TP, a.work_ctr, gridDim.x * kTW, lane);
+    BandItems work(a.band_start, TP, a.work_ctr, kTW, warp, lane);
     for (int w = lane; w < kTBand * kTBW; w += 32) {
         S.X[w] = 0u;
         S.C[w] = 0u;
