@@ -9,53 +9,38 @@
 // shared memory (the label map in L2 only for blocks whose pixels differ).
 // A labelled pixel is inside exactly one polygon and away from every
 // outline: the point goes to that polygon's histogram (plain shared-memory
-// atomics, count and two-word fixed-point sum).  A
-// pixel marked border (within the fp32 error radius of an outline, isBorder
-// hybrid.glsl:174-185) sends the point to the exact test through the
-// classified grid: such points are appended to a block-wide queue with one
-// atomic per warp (ballot + prefix, no divergent per-lane appends) and run
-// in full blocks, one point per thread, when the queue holds a block's worth.
-#include "rj_lean.cuh"
+// atomics, count and two-word fixed-point sum).  A pixel marked border (within
+// the fp32 error radius of an outline, isBorder hybrid.glsl:174-185) sends the
+// point to the exact test through the classified grid.
+//
+// Warps work alone.  The points that pass the filters (without filters: those
+// whose block does not decide) are packed into the warp's queue and looked up
+// 32 at a time; a batch only issues its label load, the next batch's turn uses
+// it, and border points go on into a second queue that is tested 32 at a time.
+//
+// Measured (100M points, filters on four columns and avg, 24 B each, 260 cells):
+// hybrid 512 us and index 508, 4.7 TB/s; 672 and 690 with block-wide queues,
+// whose barriers came every iteration, and a label read each point waited for.
+// Without filters 580 us.  What bounds it is the issue rate together with the
+// latency that 32 warps of 64 registers can hide; three blocks of 512 threads
+// per SM spill and take 850 us.
+#include "rj_label_core.cuh"
 #include "rj_point_core.cuh"
 
 namespace rj {
 
 namespace {
 
-// Hist-like adapter for exact_probe: adds to the block's histogram copy.
+// Hist-like adapter for exact_probe: adds to the warp's histogram copy.
 template <bool AGG>
 struct LeanHist {
-    uint32_t* cnt;
-    uint32_t* lo;
-    uint32_t* hi;
+    uint32_t* hist;
+    uint32_t P;
     const LeanCols* lc;
-    __device__ __forceinline__ void add(int p, float v) const {
-        atomicAdd(cnt + p, 1u);
-        if (AGG) {
-            if (isfinite(v)) {
-                const unsigned long long q = (unsigned long long)fixed_value(v, lc->scale);
-                const uint32_t qlo = (uint32_t)q;
-                const uint32_t old = atomicAdd(lo + p, qlo);
-                atomicAdd(hi + p, (uint32_t)(q >> 32) + ((old + qlo < old) ? 1u : 0u));
-            } else {
-                atomicAdd(lc->nonfinite + p, (double)v);
-            }
-        }
-    }
+    __device__ __forceinline__ void add(int p, float v) const { label_add<AGG>(hist, P, *lc, (uint32_t)p, v); }
 };
 
-template <int NCOL>
-__device__ __forceinline__ bool hyb_pass(const LeanCols& lc, const uint32_t (&v)[NCOL > 0 ? NCOL : 1]) {
-    bool ok = true;
-    #pragma unroll
-    for (int c = 0; c < NCOL; ++c) {
-        const uint32_t key = v[c] ^ ((uint32_t)((int32_t)v[c] >> 31) & lc.fm[c]);
-        ok &= (key - lc.lo[c]) <= lc.span[c];
-    }
-    return ok;
-}
-
-// kind of a point: 0 none, 1 labelled (label in *lab), 2 border (exact test).
+// Where a point lies: 0 nowhere, 1 pixel (px, py), 2 the exact test decides.
 //
 // Hybrid canvas (mode 0): a labelled pixel lies in one polygon with no edge
 // within the border radius (at least one pixel) of it, so every location
@@ -66,201 +51,196 @@ __device__ __forceinline__ bool hyb_pass(const LeanCols& lc, const uint32_t (&v)
 // the exact rasterize decides, so the canvas bounds (half-open [-1, 1),
 // hybrid.glsl:187-200) and NaN are handled exactly as before.
 // Classified grid (mode 1): the cell of the exact test itself (index.glsl:
-// 382-385, fp32 division, int() truncation), as the ExactMapper computes it.
-__device__ __forceinline__ int hyb_classify(const HybLeanArgs& a, const uint16_t* sc, float x, float y, uint32_t& lab) {
-    int px, py, resx;
+// 382-385, fp32 division, int() truncation).  A product with the reciprocal
+// gives the same cell unless it comes within its error of an integer; there,
+// and near the grid's rim, the division decides.
+__device__ __forceinline__ int hyb_pixel(const HybLeanArgs& a, float x, float y, int& px, int& py) {
     if (a.mode == 0) {
-        resx = a.h.resx;
         const float fx = fmaf(x, a.fast.x, a.fast.y), fy = fmaf(y, a.fast.z, a.fast.w);
         if (fx >= 2.0f && fx < (float)(a.h.resx - 2) && fy >= 2.0f && fy < (float)(a.h.resy - 2)) {
             px = (int)fx;
             py = (int)fy;
-        } else {
-            if (!hyb_rasterize(a.h, x, y, px, py)) return 0;
-            if (px >= a.h.resx || py >= a.h.resy) return 2;
+            return 1;
         }
-    } else {
-        resx = a.ix.res;
-        const float gx = __fdiv_rn(__fsub_rn(x, a.ix.lbx), a.ix.csx);
-        const float gy = __fdiv_rn(__fsub_rn(y, a.ix.lby), a.ix.csy);
-        if (!(gx > -1.0f && gx < (float)a.ix.res && gy > -1.0f && gy < (float)a.ix.res)) return 0;
-        px = (int)gx;
-        py = (int)gy;
+        if (!hyb_rasterize(a.h, x, y, px, py)) return 0;
+        return px >= a.h.resx || py >= a.h.resy ? 2 : 1;
     }
-    uint32_t c = sc[(py >> a.bs) * a.nbx + (px >> a.bs)];
-    if (c == kCodeMixed) c = __ldg(a.label + (size_t)py * resx + px);
-    if (c == kBorderLabel) return 2;
-    lab = c;
-    return c < (uint32_t)a.P ? 1 : 0;
+    const float dx = __fsub_rn(x, a.ix.lbx), dy = __fsub_rn(y, a.ix.lby);
+    float gx = dx * a.fast.x, gy = dy * a.fast.z;
+    const bool sure = fabsf(gx - floorf(gx) - 0.5f) < a.fast.y && fabsf(gy - floorf(gy) - 0.5f) < a.fast.y &&
+                      gx >= 1.0f && gx < (float)(a.ix.res - 1) && gy >= 1.0f && gy < (float)(a.ix.res - 1);
+    if (!sure) {
+        gx = __fdiv_rn(dx, a.ix.csx);
+        gy = __fdiv_rn(dy, a.ix.csy);
+        if (!(gx > -1.0f && gx < (float)a.ix.res && gy > -1.0f && gy < (float)a.ix.res)) return 0;
+    }
+    px = (int)gx;
+    py = (int)gy;
+    return 1;
 }
+
+constexpr int kExactQueue = 64;         // border points of a warp: fewer than 32 left over plus a batch's
+
+template <int NV>
+__host__ __device__ constexpr int hyb_queue() { return 32 + 64 * NV; }   // left over + one iteration's points
 
 }  // namespace
 
-// A classified point: a labelled one into the histogram, a border one into
-// the block's queue (one reservation per warp: ballot + prefix; every lane of
-// the warp calls this).
-template <bool AGG>
-__device__ __forceinline__ void hyb_take(const LeanHist<AGG>& hist, int* qn, float* qx, float* qy, float* qv,
-                                         int lane, int kind, uint32_t lab, float x, float y, float val) {
-    if (kind == 1) hist.add((int)lab, val);
-    const unsigned m = __ballot_sync(0xffffffffu, kind == 2);
-    if (m) {
-        int at = 0;
-        if (lane == 0) at = atomicAdd(qn, __popc(m));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (kind == 2) {
-            const int s = at + __popc(m & ((1u << lane) - 1u));
-            qx[s] = x;
-            qy[s] = y;
-            qv[s] = val;
-        }
-    }
-}
-
-// COMPACT: the points that pass the filters are first packed per warp into
-// shared memory (ballot + prefix), then classified and counted 32 at a time,
-// so that the pixel, label and histogram work runs on full warps even when
-// the filters drop most points.
-template <int BLOCK, int NV, int NCOL, bool AGG, bool COMPACT>
-__device__ __forceinline__ void hybrid_lean_body(const HybLeanArgs& a, const LeanCols& lc) {
+template <int BLOCK, int NV, int MINB, int NI, int NF, bool AGG>
+__global__ void __launch_bounds__(BLOCK, MINB) k_hybrid_lean(HybLeanArgs a, LeanCols lc) {
     extern __shared__ uint32_t s_words[];
     constexpr int HW = AGG ? 3 : 1;
-    constexpr int QCAP = BLOCK * (1 + 2 * NV);        // < BLOCK left over + every point of one iteration
-    constexpr int WCAP = 32 * 2 * NV;                 // one warp's points of one iteration
-    uint32_t* s_code = s_words;
-    uint32_t* s_hist = s_code + a.code_words;          // lc.copies x HW x P
-    float* qx = reinterpret_cast<float*>(s_hist + lc.copies * HW * a.P);
-    float* qy = qx + QCAP;
-    float* qv = qy + QCAP;
-    int* qn = reinterpret_cast<int*>(qv + QCAP);
-    // per-warp staging of the points that pass the filters (COMPACT)
-    float* wx = reinterpret_cast<float*>(qn + 4) + (threadIdx.x >> 5) * WCAP * (AGG ? 3 : 2);
-    float* wy = wx + WCAP;
-    float* wv = wy + WCAP;
+    constexpr int NCOL = NI + NF;
+    constexpr int NA = NCOL > 0 ? NCOL : 1;
+    constexpr int QC = hyb_queue<NV>();
+    constexpr int W = BLOCK / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2* q = reinterpret_cast<float2*>(s_words) + warp * QC;
+    float2* eq = reinterpret_cast<float2*>(s_words) + W * QC + warp * kExactQueue;
+    uint32_t* s_vals = s_words + 2 * W * (QC + kExactQueue);
+    uint32_t* qv = s_vals + warp * QC;                                  // AGG: their values (raw)
+    uint32_t* ev = s_vals + W * QC + warp * kExactQueue;
+    uint32_t* s_code = s_vals + (AGG ? W * (QC + kExactQueue) : 0);
+    uint32_t* s_hist = s_code + a.code_words;                           // lc.copies x HW x P
     {
         const uint32_t* g = reinterpret_cast<const uint32_t*>(a.codes);
         for (int i = threadIdx.x; i < a.code_words; i += BLOCK) s_code[i] = __ldg(g + i);
         for (int i = threadIdx.x; i < lc.copies * HW * a.P; i += BLOCK) s_hist[i] = 0u;
-        if (threadIdx.x == 0) *qn = 0;
     }
     __syncthreads();
     const uint16_t* sc = reinterpret_cast<const uint16_t*>(s_code);
-    uint32_t* h_cnt = s_hist + ((threadIdx.x >> 5) & (lc.copies - 1)) * HW * a.P;
-    const LeanHist<AGG> hist{h_cnt, h_cnt + a.P, h_cnt + 2 * a.P, &lc};
-    const int lane = threadIdx.x & 31;
+    const uint32_t P = (uint32_t)a.P;
+    const int resx = a.mode == 0 ? a.h.resx : a.ix.res;
+    uint32_t* hist = s_hist + (warp & (lc.copies - 1)) * HW * a.P;
+    const LeanHist<AGG> exact{hist, P, &lc};
+    int qn = 0, en = 0;                 // queued points, queued border points (warp-uniform)
+    bool tail = false, pending = false;
+    // the batch in flight: its labels
+    uint32_t lab = kEmptyLabel, raw1 = 0u;
+    float2 at1 = make_float2(0.f, 0.f);
+
+    // counts the batch in flight and sends off the last 32 (or fewer) queued points
+    auto drain = [&]() {
+        if (lab < P) label_add<AGG>(hist, P, lc, lab, AGG ? agg_value(lc.aggr_typ, raw1) : 0.f);
+        const unsigned m = __ballot_sync(0xffffffffu, lab == kBorderLabel);
+        if (lab == kBorderLabel) {
+            const int s = en + __popc(m & ((1u << lane) - 1u));
+            eq[s] = at1;
+            if (AGG) ev[s] = raw1;
+        }
+        en += __popc(m);
+        __syncwarp();
+        while (en >= (tail ? 1 : 32)) {
+            const int i = max(en - 32, 0) + lane;
+            if (i < en) exact_probe(a.ix, eq[i].x, eq[i].y, AGG ? agg_value(lc.aggr_typ, ev[i]) : 0.f, exact);
+            en = max(en - 32, 0);
+            __syncwarp();
+        }
+        pending = qn > 0;
+        lab = kEmptyLabel;
+        const int first = max(qn - 32, 0);
+        if (first + lane < qn) {
+            at1 = q[first + lane];
+            if (AGG) raw1 = qv[first + lane];
+            int px, py;
+            const int kind = hyb_pixel(a, at1.x, at1.y, px, py);
+            if (kind == 1) {
+                lab = NCOL > 0 ? sc[(py >> a.bs) * a.nbx + (px >> a.bs)] : kCodeMixed;
+                if (lab == kCodeMixed) lab = __ldg(a.label + (size_t)py * resx + px);
+            } else if (kind == 2) {
+                lab = kBorderLabel;
+            }
+        }
+        qn = first;
+        __syncwarp();
+    };
 
     const uint64_t npairs = a.n >> 1;
     constexpr uint64_t kPerIter = (uint64_t)BLOCK * NV;
-    const uint64_t warp_ofs = (uint64_t)(threadIdx.x >> 5) * 32 * NV;
-    const uint64_t lane_ofs = warp_ofs + lane;
-    // block-uniform trip count (the queue drain below has block barriers)
-    for (uint64_t base = (uint64_t)blockIdx.x * kPerIter; base < npairs; base += (uint64_t)gridDim.x * kPerIter) {
-        bool skip = false;
-        if (a.zones) {
-            const uint64_t r0 = a.zrow0 + 2 * (base + warp_ofs);
-            const uint64_t r1 = a.zrow0 + min(2 * (base + warp_ofs + 32 * NV), a.n) - 1;
-            bool meets = false;
-            if (r0 <= r1 && (uint64_t)lane <= (r1 >> kZoneShift) - (r0 >> kZoneShift)) {
-                const float4 b = __ldg(a.zones + (r0 >> kZoneShift) + lane);
-                meets = !(b.z < a.qbox.x || b.x > a.qbox.z || b.w < a.qbox.y || b.y > a.qbox.w);
+    for (uint64_t base = (uint64_t)blockIdx.x * kPerIter + (uint64_t)warp * 32 * NV; !tail;
+         base += (uint64_t)gridDim.x * kPerIter) {
+        if (base >= npairs) {
+            tail = true;
+            // the last point of an odd-sized table
+            if ((a.n & 1) && blockIdx.x == 0 && warp == 0) {
+                const uint64_t i = a.n - 1;
+                bool ok = true;
+                if (lane == 0) {
+                    uint32_t v[NA], raw = 0u;
+                    #pragma unroll
+                    for (int c = 0; c < NCOL; ++c) v[c] = __ldg(reinterpret_cast<const uint32_t*>(lc.col[c]) + i);
+                    ok = cols_pass<NI, NF>(lc, v);
+                    q[qn] = __ldg(reinterpret_cast<const float2*>(a.xy) + i);
+                    if (AGG) {
+                        if (lc.aggr_ci < 0) raw = __ldg(reinterpret_cast<const uint32_t*>(lc.aggr_col) + i);
+                        #pragma unroll
+                        for (int c = 0; c < NCOL; ++c)
+                            if (c == lc.aggr_ci) raw = v[c];
+                        qv[qn] = raw;
+                    }
+                }
+                qn += __shfl_sync(0xffffffffu, ok ? 1 : 0, 0);
+                __syncwarp();
             }
-            skip = !__any_sync(0xffffffffu, meets);
-        }
-        if (!skip) {
+        } else if (tl_zone<NV>(a, base)) {
             float4 p[NV];
-            uint2 cv[NCOL > 0 ? NCOL : 1][NV];
+            uint2 cv[NA][NV];
             uint2 av[NV];
             #pragma unroll
             for (int k = 0; k < NV; ++k) {
-                const uint64_t i = base + lane_ofs + (uint64_t)k * 32;
+                const uint64_t i = base + lane + (uint64_t)k * 32;
                 const bool live = i < npairs;
                 p[k] = live ? __ldcs(a.xy + i) : make_float4(NAN, NAN, NAN, NAN);
                 #pragma unroll
                 for (int c = 0; c < NCOL; ++c) cv[c][k] = live ? __ldcs(lc.col[c] + i) : make_uint2(0u, 0u);
                 if (AGG) av[k] = (live && lc.aggr_ci < 0) ? __ldcs(lc.aggr_col + i) : make_uint2(0u, 0u);
             }
-            int nst = 0;                               // staged points of this warp (COMPACT)
+            auto value = [&](int j) -> uint32_t {
+                uint32_t raw = (j & 1) ? av[j >> 1].y : av[j >> 1].x;
+                #pragma unroll
+                for (int c = 0; c < NCOL; ++c)
+                    if (c == lc.aggr_ci) raw = (j & 1) ? cv[c][j >> 1].y : cv[c][j >> 1].x;
+                return raw;
+            };
+            uint32_t push = 0u;   // points to queue
             #pragma unroll
             for (int j = 0; j < 2 * NV; ++j) {
-                const int k = j >> 1;
-                const bool hi = (j & 1) != 0;
-                uint32_t v[NCOL > 0 ? NCOL : 1];
-                #pragma unroll
-                for (int c = 0; c < NCOL; ++c) v[c] = hi ? cv[c][k].y : cv[c][k].x;
-                const float x = hi ? p[k].z : p[k].x;
-                const float y = hi ? p[k].w : p[k].y;
-                float val = 0.f;
-                if (AGG) {
-                    uint32_t raw = hi ? av[k].y : av[k].x;
+                if (NCOL > 0) {
+                    uint32_t v[NA];
                     #pragma unroll
-                    for (int cc = 0; cc < NCOL; ++cc)
-                        if (cc == lc.aggr_ci) raw = v[cc];
-                    val = agg_value(lc.aggr_typ, raw);
-                }
-                if (COMPACT) {
-                    const bool ok = hyb_pass<NCOL>(lc, v);
-                    const unsigned m = __ballot_sync(0xffffffffu, ok);
-                    if (ok) {
-                        const int s = nst + __popc(m & ((1u << lane) - 1u));
-                        wx[s] = x;
-                        wy[s] = y;
-                        if (AGG) wv[s] = val;
-                    }
-                    nst += __popc(m);
+                    for (int c = 0; c < NCOL; ++c) v[c] = (j & 1) ? cv[c][j >> 1].y : cv[c][j >> 1].x;
+                    const bool ok = cols_pass<NI, NF>(lc, v) && base + lane + (uint64_t)(j >> 1) * 32 < npairs;
+                    push |= ok ? 1u << j : 0u;
                 } else {
-                    uint32_t lab = 0;
-                    const int kind = hyb_pass<NCOL>(lc, v) ? hyb_classify(a, sc, x, y, lab) : 0;
-                    hyb_take<AGG>(hist, qn, qx, qy, qv, lane, kind, lab, x, y, val);
+                    int px, py;
+                    const int kind = hyb_pixel(a, (j & 1) ? p[j >> 1].z : p[j >> 1].x, (j & 1) ? p[j >> 1].w : p[j >> 1].y,
+                                               px, py);
+                    uint32_t l = kind == 2 ? kBorderLabel : kEmptyLabel;
+                    if (kind == 1) l = sc[(py >> a.bs) * a.nbx + (px >> a.bs)];
+                    if (l < P) label_add<AGG>(hist, P, lc, l, AGG ? agg_value(lc.aggr_typ, value(j)) : 0.f);
+                    push |= l == kCodeMixed || l == kBorderLabel ? 1u << j : 0u;
                 }
             }
-            if (COMPACT) {
-                __syncwarp();
-                for (int kb = 0; kb < nst; kb += 32) {
-                    const int k = kb + lane;
-                    const bool live = k < nst;
-                    const float x = live ? wx[k] : 0.f, y = live ? wy[k] : 0.f;
-                    const float val = (AGG && live) ? wv[k] : 0.f;
-                    uint32_t lab = 0;
-                    const int kind = live ? hyb_classify(a, sc, x, y, lab) : 0;
-                    hyb_take<AGG>(hist, qn, qx, qy, qv, lane, kind, lab, x, y, val);
-                }
-                __syncwarp();
-            }
-        }
-        // drain full blocks of queued points, one point per thread
-        __syncthreads();
-        while (*qn >= BLOCK) {
-            const int s = *qn - BLOCK + (int)threadIdx.x;
-            exact_probe(a.ix, qx[s], qy[s], qv[s], hist);
-            __syncthreads();
-            if (threadIdx.x == 0) *qn -= BLOCK;
-            __syncthreads();
-        }
-    }
-    // the last point of an odd-sized table
-    if ((a.n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
-        const uint64_t i = a.n - 1;
-        const float2 q = __ldg(reinterpret_cast<const float2*>(a.xy) + i);
-        uint32_t v[NCOL > 0 ? NCOL : 1];
-        #pragma unroll
-        for (int c = 0; c < NCOL; ++c) v[c] = __ldg(reinterpret_cast<const uint32_t*>(lc.col[c]) + i);
-        float val = 0.f;
-        if (AGG) {
-            uint32_t raw = lc.aggr_ci < 0 ? __ldg(reinterpret_cast<const uint32_t*>(lc.aggr_col) + i) : 0u;
+            // queue positions: one prefix sum over the lanes
+            int incl = __popc(push);
+            const int own = incl;
             #pragma unroll
-            for (int cc = 0; cc < NCOL; ++cc)
-                if (cc == lc.aggr_ci) raw = v[cc];
-            val = agg_value(lc.aggr_typ, raw);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            int at = qn + incl - own;
+            #pragma unroll
+            for (int j = 0; j < 2 * NV; ++j)
+                if ((push >> j) & 1u) {
+                    q[at] = (j & 1) ? make_float2(p[j >> 1].z, p[j >> 1].w) : make_float2(p[j >> 1].x, p[j >> 1].y);
+                    if (AGG) qv[at] = value(j);
+                    ++at;
+                }
+            qn += __shfl_sync(0xffffffffu, incl, 31);
+            __syncwarp();
         }
-        uint32_t lab = 0;
-        const int kind = hyb_pass<NCOL>(lc, v) ? hyb_classify(a, sc, q.x, q.y, lab) : 0;
-        if (kind == 1) hist.add((int)lab, val);
-        if (kind == 2) exact_probe(a.ix, q.x, q.y, val, hist);
-    }
-    __syncthreads();
-    {
-        const int cnt = *qn;
-        if ((int)threadIdx.x < cnt) exact_probe(a.ix, qx[threadIdx.x], qy[threadIdx.x], qv[threadIdx.x], hist);
+        while (qn >= 32 || (tail && (qn > 0 || pending))) drain();
     }
     __syncthreads();
     for (int b = threadIdx.x; b < a.P; b += BLOCK) {
@@ -279,24 +259,15 @@ __device__ __forceinline__ void hybrid_lean_body(const HybLeanArgs& a, const Lea
     }
 }
 
-template <int BLOCK, int NV, int NCOL, bool AGG, bool COMPACT>
-__global__ void __launch_bounds__(BLOCK) k_hybrid_lean(HybLeanArgs a, LeanCols lc) {
-    hybrid_lean_body<BLOCK, NV, NCOL, AGG, COMPACT>(a, lc);
-}
-
-// The same pass with a register budget of two blocks per SM (64 registers at
-// 512 threads): no spills, fewer resident warps.  The tuner decides.
-template <int BLOCK, int NV, int NCOL, bool AGG, bool COMPACT>
-__global__ void __launch_bounds__(BLOCK, 2) k_hybrid_lean_r2(HybLeanArgs a, LeanCols lc) {
-    hybrid_lean_body<BLOCK, NV, NCOL, AGG, COMPACT>(a, lc);
-}
-
-// Block codes from a label map: one warp per block.
+// Block codes from a label map: one warp per block, eight pixels a load where
+// rows and blocks allow (a 16 x 16 block is one load per lane).  On 4096 x 4096
+// pixels 37 us with two-byte loads, 14 us now.
 __global__ void k_block_codes(const uint16_t* __restrict__ label, int resx, int resy, int bs, int nbx, int nby,
                               uint16_t* __restrict__ codes) {
     const int lane = threadIdx.x & 31;
     const int B = 1 << bs;
     const int nb = nbx * nby;
+    const bool wide = (resx & 7) == 0 && bs >= 3;
     for (int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); b < nb;
          b += (int)((gridDim.x * blockDim.x) >> 5)) {
         const int bx = b % nbx, by = b / nbx;
@@ -304,9 +275,19 @@ __global__ void k_block_codes(const uint16_t* __restrict__ label, int resx, int 
         const int w = min(x0 + B, resx) - x0, h = min(y0 + B, resy) - y0;
         const uint16_t first = __ldg(label + (size_t)y0 * resx + x0);
         bool same = true;
-        for (int i = lane; i < w * h; i += 32) {
-            const int yy = y0 + i / w, xx = x0 + i % w;
-            same &= (__ldg(label + (size_t)yy * resx + xx) == first);
+        if (wide) {
+            const uint32_t both = first * 0x10001u;
+            const int w8 = w >> 3;
+            for (int i = lane; i < w8 * h; i += 32) {
+                const int yy = w == B ? i >> (bs - 3) : i / w8;
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(label + (size_t)(y0 + yy) * resx + x0) + (i - yy * w8));
+                same &= v.x == both && v.y == both && v.z == both && v.w == both;
+            }
+        } else {
+            for (int i = lane; i < w * h; i += 32) {
+                const int yy = y0 + i / w, xx = x0 + i % w;
+                same &= (__ldg(label + (size_t)yy * resx + xx) == first);
+            }
         }
         same = __all_sync(0xffffffffu, same);
         if (lane == 0) codes[b] = same ? first : kCodeMixed;
@@ -342,50 +323,50 @@ namespace {
 using HybKernel = void (*)(HybLeanArgs, LeanCols);
 
 struct HybShape {
-    int block;
-    int nv;
-    bool compact;
+    int block, nv, minb;
 };
-// 3 and 6: the register budget of two blocks per SM
-constexpr HybShape kHybShapes[] = {{512, 2, false}, {1024, 2, false}, {256, 4, false}, {512, 2, false},
-                                   {512, 2, true},  {256, 4, true},   {512, 2, true},  {1024, 2, true},
-                                   {512, 1, true}};
+constexpr HybShape kHybShapes[] = {{512, 2, 2}, {1024, 2, 1}};
 constexpr int kNumHybShapes = (int)(sizeof(kHybShapes) / sizeof(kHybShapes[0]));
 
-template <int NCOL, bool AGG>
-HybKernel pick_hyb(int shape) {
+template <int NI, int NF, bool AGG>
+HybKernel hyb_kernel(int shape) {
     switch (shape) {
-        case 0: return k_hybrid_lean<512, 2, NCOL, AGG, false>;
-        case 1: return k_hybrid_lean<1024, 2, NCOL, AGG, false>;
-        case 2: return k_hybrid_lean<256, 4, NCOL, AGG, false>;
-        case 3: return k_hybrid_lean_r2<512, 2, NCOL, AGG, false>;
-        case 4: return k_hybrid_lean<512, 2, NCOL, AGG, true>;
-        case 5: return k_hybrid_lean<256, 4, NCOL, AGG, true>;
-        case 6: return k_hybrid_lean_r2<512, 2, NCOL, AGG, true>;
-        case 7: return k_hybrid_lean<1024, 2, NCOL, AGG, true>;
-        default: return k_hybrid_lean<512, 1, NCOL, AGG, true>;
+        case 0: return k_hybrid_lean<512, 2, 2, NI, NF, AGG>;
+        case 1: return k_hybrid_lean<1024, 2, 1, NI, NF, AGG>;
+        default: return nullptr;
     }
 }
 
 template <bool AGG>
-HybKernel pick_hyb_ncol(int ncol, int shape) {
-    switch (ncol) {
-        case 0: return pick_hyb<0, AGG>(shape);
-        case 1: return pick_hyb<1, AGG>(shape);
-        case 2: return pick_hyb<2, AGG>(shape);
-        case 3: return pick_hyb<3, AGG>(shape);
-        case 4: return pick_hyb<4, AGG>(shape);
+HybKernel hyb_kernel_cols(int shape, int ni, int nf) {
+    switch (ni * 5 + nf) {
+        case 0: return hyb_kernel<0, 0, AGG>(shape);
+        case 1: return hyb_kernel<0, 1, AGG>(shape);
+        case 2: return hyb_kernel<0, 2, AGG>(shape);
+        case 3: return hyb_kernel<0, 3, AGG>(shape);
+        case 4: return hyb_kernel<0, 4, AGG>(shape);
+        case 5: return hyb_kernel<1, 0, AGG>(shape);
+        case 6: return hyb_kernel<1, 1, AGG>(shape);
+        case 7: return hyb_kernel<1, 2, AGG>(shape);
+        case 8: return hyb_kernel<1, 3, AGG>(shape);
+        case 10: return hyb_kernel<2, 0, AGG>(shape);
+        case 11: return hyb_kernel<2, 1, AGG>(shape);
+        case 12: return hyb_kernel<2, 2, AGG>(shape);
+        case 15: return hyb_kernel<3, 0, AGG>(shape);
+        case 16: return hyb_kernel<3, 1, AGG>(shape);
+        case 20: return hyb_kernel<4, 0, AGG>(shape);
         default: return nullptr;
     }
 }
 
 int g_hyb_optin = -1;
 
+// histogram copies: a power of two up to the warps of the block, within 32 KB
 int hyb_copies(int shape, int P, bool agg) {
     const int warps = kHybShapes[shape].block / 32;
     int copies = 1;
     const size_t per = (size_t)P * (agg ? 3 : 1) * 4;
-    while (copies * 2 <= warps && per * copies * 2 <= 48 * 1024) copies *= 2;
+    while (copies * 2 <= warps && per * copies * 2 <= 32 * 1024) copies *= 2;
     return copies;
 }
 
@@ -396,15 +377,15 @@ int hybrid_lean_shapes() { return kNumHybShapes; }
 size_t hybrid_lean_smem(int shape, int code_words, int P, bool agg) {
     if (shape < 0 || shape >= kNumHybShapes) return 0;
     const HybShape& s = kHybShapes[shape];
-    const size_t qcap = (size_t)s.block * (1 + 2 * s.nv);
-    const size_t stage = s.compact ? (size_t)s.block * 2 * s.nv * (agg ? 3 : 2) * 4 : 0;   // per-warp staging
-    return (size_t)code_words * 4 + (size_t)hyb_copies(shape, P, agg) * P * (agg ? 3 : 1) * 4 + qcap * 12 + 16 + stage;
+    const size_t queues = (size_t)(s.block / 32) * (32 + 64 * s.nv + kExactQueue) * (agg ? 12 : 8);
+    return queues + (size_t)code_words * 4 + (size_t)hyb_copies(shape, P, agg) * P * (agg ? 3 : 1) * 4;
 }
 
 bool launch_hybrid_lean(int shape, const HybLeanArgs& a, const LeanCols& lc_in, int sms, cudaStream_t st) {
     if (shape < 0 || shape >= kNumHybShapes || lc_in.ncol < 0 || lc_in.ncol > 4) return false;
     const bool agg = lc_in.aggr != 0;
-    HybKernel k = agg ? pick_hyb_ncol<true>(lc_in.ncol, shape) : pick_hyb_ncol<false>(lc_in.ncol, shape);
+    const int ni = lc_in.nint, nf = lc_in.ncol - lc_in.nint;
+    HybKernel k = agg ? hyb_kernel_cols<true>(shape, ni, nf) : hyb_kernel_cols<false>(shape, ni, nf);
     if (!k) return false;
     if (g_hyb_optin < 0) {
         int dev = 0;

@@ -263,7 +263,8 @@ struct HybLeanArgs {
     // the canvas less a 2-pixel rim (near the rim: the exact rasterize)
     // mode 1: the classified grid's cells (index join); label holds per cell
     // the one polygon a FULL cell lies in, kBorderLabel for cells with a
-    // candidate list, kEmptyLabel for empty cells
+    // candidate list, kEmptyLabel for empty cells; fast = (1 / cell width, how
+    // far from a cell's middle the product with it is sure, 1 / height, -)
     int mode;
     float4 fast;
 };

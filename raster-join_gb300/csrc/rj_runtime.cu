@@ -1073,7 +1073,10 @@ int hybrid_lean_pass(rj_ctx* ctx, const DevFilter& f, int mode, const HybXf& h, 
     a.ix = ix;
     a.mode = mode;
     const int resx = mode == 0 ? h.resx : ix.res, resy = mode == 0 ? h.resy : ix.res;
-    if (mode == 0) {
+    if (mode == 1) {
+        // (cells per unit; how far from a cell's middle its product is sure)
+        a.fast = make_float4(1.0f / ix.csx, 0.5f - (float)resx * 2.4e-7f, 1.0f / ix.csy, 0.0f);
+    } else {
         // pixel coordinate = (u + 1) / 2 * res with u = (v - o) / d
         const double ax = (double)h.resx / (2.0 * h.dx), ay = (double)h.resy / (2.0 * h.dy);
         a.fast = make_float4((float)ax, (float)(0.5 * h.resx - ax * h.ox), (float)ay, (float)(0.5 * h.resy - ay * h.oy));
@@ -1099,7 +1102,7 @@ int hybrid_lean_pass(rj_ctx* ctx, const DevFilter& f, int mode, const HybXf& h, 
             }
     if (cands.empty()) return RJ_OK;
     char key[200];
-    std::snprintf(key, sizeof key, "hyb:%d:%d:%d:%d:%d:%d:%d:%d:%d", mode, lc.ncol, lc.aggr, lc.aggr_ci >= 0,
+    std::snprintf(key, sizeof key, "hybq:%d:%d:%d:%d:%d:%d:%d:%d:%d", mode, lc.ncol, lc.aggr, lc.aggr_ci >= 0,
                   tune_bucket((double)P), tune_bucket((double)resx * resy), tune_bucket((double)a.n), ctx->count_shape,
                   ctx->count_bshift);
     int tuned_i = -1;
