@@ -109,7 +109,7 @@ struct ClsArgs {
     // level 2: explicit (polygon, fine cell) pairs refined from EDGE coarse pairs
     int2* plist;
     int* plist_n;
-    int level;                   // 1 or 2
+    int level;                   // 1, 2, or 3: pairs of level 1 with the results of level 2 (scale 1)
     int scale;                   // fine cells per coarse cell along an axis
     float lbx, lby, csx, csy;    // fine grid lower-left / cell size (fp32, as the points use)
     int res;                     // fine grid resolution

@@ -346,18 +346,18 @@ __device__ __forceinline__ int pair_poly(const ClsArgs& a, int k) {
     return lo;
 }
 
-// rectangle of fine cells [gx, gx+n) x [gy, gy+n) of the fine grid
+// rectangle of fine cells [gx, gx+n) x [gy, gy+n) of the fine grid.  The edges
+// of a pair are counted by one kernel and written by another: every rounding is
+// spelled out, so that both see the same rectangle.
 __device__ __forceinline__ CellRect cells_rect(const ClsArgs& a, int gx, int gy, int n) {
-    float x0 = a.lbx + (float)gx * a.csx, x1 = a.lbx + (float)(gx + n) * a.csx;
-    float y0 = a.lby + (float)gy * a.csy, y1 = a.lby + (float)(gy + n) * a.csy;
     // cell 0 also receives points with (p - lb)/cs in (-1, 0): int() truncates
-    if (gx == 0) x0 = a.lbx - a.csx;
-    if (gy == 0) y0 = a.lby - a.csy;
+    const float x0 = __fmaf_rn(gx == 0 ? -1.0f : (float)gx, a.csx, a.lbx), x1 = __fmaf_rn((float)(gx + n), a.csx, a.lbx);
+    const float y0 = __fmaf_rn(gy == 0 ? -1.0f : (float)gy, a.csy, a.lby), y1 = __fmaf_rn((float)(gy + n), a.csy, a.lby);
     CellRect r;
-    r.cx = 0.5f * (x0 + x1);
-    r.cy = 0.5f * (y0 + y1);
-    r.hw = 0.5f * (x1 - x0) + a.margin;
-    r.hh = 0.5f * (y1 - y0) + a.margin;
+    r.cx = __fmul_rn(0.5f, __fadd_rn(x0, x1));
+    r.cy = __fmul_rn(0.5f, __fadd_rn(y0, y1));
+    r.hw = __fadd_rn(__fmul_rn(0.5f, __fsub_rn(x1, x0)), a.margin);
+    r.hh = __fadd_rn(__fmul_rn(0.5f, __fsub_rn(y1, y0)), a.margin);
     return r;
 }
 
@@ -384,8 +384,8 @@ __device__ __forceinline__ bool seg_meets_box(float ax, float ay, float bx, floa
 
 // per edge of the pair: bit0 meets R, bit1 kept (may toggle), bit2 straddle-only
 __device__ __forceinline__ int edge_class(const CellRect& r, float2 vi, float2 vj) {
-    const float ax = vi.x - r.cx, ay = vi.y - r.cy;
-    const float bx = vj.x - r.cx, by = vj.y - r.cy;
+    const float ax = __fsub_rn(vi.x, r.cx), ay = __fsub_rn(vi.y, r.cy);
+    const float bx = __fsub_rn(vj.x, r.cx), by = __fsub_rn(vj.y, r.cy);
     int c = seg_meets_box(ax, ay, bx, by, r.hw, r.hh) ? 1 : 0;
     const bool band = !(fmaxf(ay, by) < -r.hh || fminf(ay, by) > r.hh) && !(fmaxf(ax, bx) < -r.hw);
     if (band) {
@@ -395,64 +395,182 @@ __device__ __forceinline__ int edge_class(const CellRect& r, float2 vi, float2 v
     return c;
 }
 
+// The polygon's edges, 32 at a time in order, as f(end, start, live) by
+// the whole warp; groups with no edge in the rectangle's rows, which neither
+// meet it nor toggle anything, are passed over.  An outline is local, so few
+// groups are left, and the loads of four are in flight at a time.
+template <class F>
+__device__ __forceinline__ void for_near_edges(const float2* __restrict__ v, int nv, const CellRect& r, int lane, F&& f) {
+    for (int e0 = 0; e0 < nv; e0 += 128) {
+        float2 vi[4], vj[4];
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int e = e0 + 32 * u + lane;
+            const bool live = e < nv;
+            vi[u] = live ? __ldg(v + e) : make_float2(0.f, 0.f);
+            vj[u] = live ? __ldg(v + (e == 0 ? nv - 1 : e - 1)) : make_float2(0.f, 0.f);
+        }
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const bool live = e0 + 32 * u + lane < nv;
+            const float ay = __fsub_rn(vi[u].y, r.cy), by = __fsub_rn(vj[u].y, r.cy);
+            if (__any_sync(0xffffffffu, live && !(fmaxf(ay, by) < -r.hh || fminf(ay, by) > r.hh)))
+                f(vi[u], vj[u], live);
+        }
+    }
+}
+
+// What the edges say about one (cell, polygon) pair.
+struct PairEdges {
+    int meets = 0, nr = 0, nf = 0;
+    bool inside = false;
+};
+
+__device__ __forceinline__ PairEdges pair_edges_warp(const float2* __restrict__ v, int nv, const CellRect& r, int lane) {
+    const unsigned FULL = 0xffffffffu;
+    PairEdges t;
+    for_near_edges(v, nv, r, lane, [&](float2 vi, float2 vj, bool live) {
+        int c = 0;
+        bool tog = false;
+        if (live) {
+            c = edge_class(r, vi, vj);
+            tog = edge_toggles(vi.x, vi.y, vj.x, vj.y, r.cx, r.cy);
+        }
+        t.meets |= __any_sync(FULL, c & 1);
+        t.nr += __popc(__ballot_sync(FULL, (c & 6) == 6));
+        t.nf += __popc(__ballot_sync(FULL, (c & 6) == 2));
+        t.inside ^= (__popc(__ballot_sync(FULL, tog)) & 1) != 0;
+    });
+    return t;
+}
+
+// Level 1, a pair per lane: neighbouring pairs mostly share their polygon, so
+// each of its edges is one broadcast load and a few comparisons for 32 cells.
+// Edges left of the cell's rectangle say nothing, edges right of it only
+// whether they straddle its middle; the others are marked, and the lanes then
+// work off their own marks together.  With a warp per pair (the edges over the
+// lanes) a pair is one load latency after another, whatever its edges are:
+// 65,000 cells of 260 polygons with 100 vertices, 120,000 pairs, took 89 us
+// and 19 more for level 2; 38 us now for both.  Polygons of more than kLaneEdges vertices are still walked by
+// the warp, pair by pair: a lane alone would be at it for too long.
+constexpr int kLaneEdges = 512;
+
+__global__ void __launch_bounds__(128, 6) k_cls_pairs(ClsArgs a) {
+    const int lane = threadIdx.x & 31;
+    const unsigned FULL = 0xffffffffu;
+    for (int k0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) & ~31u); k0 < a.npairs; k0 += (int)(gridDim.x * blockDim.x)) {
+        const int k = k0 + lane;
+        const bool valid = k < a.npairs;
+        int p = -1, gx = 0, gy = 0;
+        const int n = a.scale;
+        if (valid) {
+            p = pair_poly(a, k);
+            const int4 r = __ldg(a.prange + p);
+            const int w = r.y - r.x, l = k - __ldg(a.pair_off + p);
+            gx = (r.x + l % w) * n;
+            gy = (r.z + l / w) * n;
+        }
+        const CellRect r = cells_rect(a, gx, gy, n);
+        PairEdges res;
+        for (unsigned todo = __ballot_sync(FULL, valid); todo;) {
+            const int pl = __shfl_sync(FULL, p, __ffs(todo) - 1);
+            const bool mine = p == pl;
+            const unsigned group = __ballot_sync(FULL, mine);
+            todo &= ~group;
+            const int v0 = __ldg(a.pindex + pl), nv = __ldg(a.pindex + pl + 1) - v0;
+            const float2* v = a.verts + v0;
+            if (nv <= kLaneEdges) {
+                float2 vj = nv ? __ldg(v + nv - 1) : make_float2(0.f, 0.f);
+                for (int e0 = 0; e0 < nv; e0 += 32) {
+                    unsigned marks = 0u;
+                    #pragma unroll 1
+                    for (int e1 = 0; e1 < 32 && e0 + e1 < nv; e1 += 8) {
+                        float2 vi[8];
+                        #pragma unroll
+                        for (int u = 0; u < 8; ++u) vi[u] = __ldg(v + min(e0 + e1 + u, nv - 1));
+                        #pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const float ax = __fsub_rn(vi[u].x, r.cx), ay = __fsub_rn(vi[u].y, r.cy);
+                            const float bx = __fsub_rn(vj.x, r.cx), by = __fsub_rn(vj.y, r.cy);
+                            if (mine && e0 + e1 + u < nv && !(fmaxf(ay, by) < -r.hh || fminf(ay, by) > r.hh) &&
+                                !(ax < -r.hw && bx < -r.hw)) {
+                                if (ax > r.hw && bx > r.hw) {
+                                    ++res.nr;
+                                    res.inside ^= (vi[u].y > r.cy) != (vj.y > r.cy);
+                                } else {
+                                    marks |= 1u << (e1 + u);
+                                }
+                            }
+                            vj = vi[u];
+                        }
+                    }
+                    while (__any_sync(FULL, marks != 0u)) {
+                        if (marks) {
+                            const int e = e0 + __ffs(marks) - 1;
+                            marks &= marks - 1;
+                            const float2 vi = __ldg(v + e), vp = __ldg(v + (e == 0 ? nv - 1 : e - 1));
+                            const int c = edge_class(r, vi, vp);
+                            res.meets |= c & 1;
+                            res.nr += (c & 6) == 6;
+                            res.nf += (c & 6) == 2;
+                            res.inside ^= edge_toggles(vi.x, vi.y, vp.x, vp.y, r.cx, r.cy);
+                        }
+                    }
+                }
+            } else {
+                for (unsigned g = group; g; g &= g - 1) {
+                    const int who = __ffs(g) - 1;
+                    const CellRect rr{__shfl_sync(FULL, r.cx, who), __shfl_sync(FULL, r.cy, who),
+                                      __shfl_sync(FULL, r.hw, who), __shfl_sync(FULL, r.hh, who)};
+                    const PairEdges t = pair_edges_warp(v, nv, rr, lane);
+                    if (lane == who) res = t;
+                }
+            }
+        }
+        const int kind = res.meets ? 0 : (res.inside ? -1 : -2);
+        const int cell = gy * a.res + gx;
+        if (a.level == 3) {   // one fine cell per coarse cell: this is level 2 as well
+            if (valid) {
+                a.info[k] = (kind == 0) ? make_int4(p, res.nr, res.nf, cell) : make_int4(p, kind, 0, cell);
+                a.ecount[k] = (kind == 0) ? res.nr + res.nf : 0;
+                if (kind != -2) atomicAdd(a.cell_kept + cell, 1);
+            }
+            continue;
+        }
+        if (valid) a.info[k] = make_int4(p, kind, 0, cell);
+        // the fine cells of full and of edge pairs, pair by pair
+        for (unsigned m = __ballot_sync(FULL, valid && kind == -1); m; m &= m - 1) {
+            const int x = __shfl_sync(FULL, gx, __ffs(m) - 1), y = __shfl_sync(FULL, gy, __ffs(m) - 1);
+            for (int s = lane; s < n * n; s += 32) atomicAdd(a.cell_kept + (y + s / n) * a.res + x + s % n, 1);
+        }
+        unsigned m = __ballot_sync(FULL, valid && kind == 0);
+        int base = 0;
+        if (m && lane == 0) base = atomicAdd(a.plist_n, __popc(m) * n * n);
+        base = __shfl_sync(FULL, base, 0);
+        for (; m; m &= m - 1) {
+            const int who = __ffs(m) - 1;
+            const int q = __shfl_sync(FULL, p, who), x = __shfl_sync(FULL, gx, who), y = __shfl_sync(FULL, gy, who);
+            for (int s = lane; s < n * n; s += 32) a.plist[base + s] = make_int2(q, (y + s / n) * a.res + x + s % n);
+            base += n * n;
+        }
+    }
+}
+
+// Level 2, a pair per warp (the list mixes polygons).
 __global__ void k_cls_classify(ClsArgs a) {
     const int lane = threadIdx.x & 31;
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    const unsigned FULL = 0xffffffffu;
-    const int npairs = a.level == 1 ? a.npairs : *a.plist_n;
+    const int npairs = *a.plist_n;
     for (int k = wid; k < npairs; k += nw) {
-        int p, gx, gy, n;
-        if (a.level == 1) {
-            p = pair_poly(a, k);
-            const int4 r = __ldg(a.prange + p);
-            const int w = r.y - r.x, l = k - __ldg(a.pair_off + p);
-            gx = (r.x + l % w) * a.scale;
-            gy = (r.z + l / w) * a.scale;
-            n = a.scale;
-        } else {
-            const int2 q = a.plist[k];
-            p = q.x;
-            gx = q.y % a.res;
-            gy = q.y / a.res;
-            n = 1;
-        }
+        const int2 q = a.plist[k];
+        const int p = q.x, cell = q.y;
         const int v0 = __ldg(a.pindex + p), nv = __ldg(a.pindex + p + 1) - v0;
-        const CellRect r = cells_rect(a, gx, gy, n);
-        int meets = 0, nr = 0, nf = 0;
-        bool inside = false;
-        for (int e0 = 0; e0 < nv; e0 += 32) {
-            int e = e0 + lane;
-            int c = 0;
-            bool tog = false;
-            if (e < nv) {
-                float2 vi = __ldg(a.verts + v0 + e);
-                float2 vj = __ldg(a.verts + v0 + (e == 0 ? nv - 1 : e - 1));
-                c = edge_class(r, vi, vj);
-                tog = edge_toggles(vi.x, vi.y, vj.x, vj.y, r.cx, r.cy);
-            }
-            meets += __popc(__ballot_sync(FULL, c & 1));
-            nr += __popc(__ballot_sync(FULL, (c & 6) == 6));
-            nf += __popc(__ballot_sync(FULL, (c & 6) == 2));
-            inside ^= (__popc(__ballot_sync(FULL, tog)) & 1) != 0;
-        }
-        const int kind = meets ? 0 : (inside ? -1 : -2);
-        if (a.level == 1) {
-            if (lane == 0) a.info[k] = make_int4(p, kind, 0, gy * a.res + gx);
-            if (kind == -1) {
-                for (int s = lane; s < n * n; s += 32)
-                    atomicAdd(a.cell_kept + (gy + s / n) * a.res + gx + s % n, 1);
-            } else if (kind == 0) {
-                int base = 0;
-                if (lane == 0) base = atomicAdd(a.plist_n, n * n);
-                base = __shfl_sync(FULL, base, 0);
-                for (int s = lane; s < n * n; s += 32)
-                    a.plist[base + s] = make_int2(p, (gy + s / n) * a.res + gx + s % n);
-            }
-        } else if (lane == 0) {
-            const int cell = gy * a.res + gx;
-            a.info[k] = (kind == 0) ? make_int4(p, nr, nf, cell) : make_int4(p, kind, 0, cell);
-            a.ecount[k] = (kind == 0) ? nr + nf : 0;
+        const PairEdges t = pair_edges_warp(a.verts + v0, nv, cells_rect(a, cell % a.res, cell / a.res, 1), lane);
+        const int kind = t.meets ? 0 : (t.inside ? -1 : -2);
+        if (lane == 0) {
+            a.info[k] = (kind == 0) ? make_int4(p, t.nr, t.nf, cell) : make_int4(p, kind, 0, cell);
+            a.ecount[k] = (kind == 0) ? t.nr + t.nf : 0;
             if (kind != -2) atomicAdd(a.cell_kept + cell, 1);
         }
     }
@@ -461,7 +579,7 @@ __global__ void k_cls_classify(ClsArgs a) {
 // Kept pairs into the cell-major list (order inside a cell is immaterial).
 // Level 1: FULL coarse pairs expand to their fine cells.  Level 2: kept pairs.
 __global__ void k_cls_emit(ClsArgs a) {
-    const int npairs = a.level == 1 ? a.npairs : *a.plist_n;
+    const int npairs = a.level == 2 ? *a.plist_n : a.npairs;
     const int nn = a.scale * a.scale;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < npairs; k += gridDim.x * blockDim.x) {
         int4 in = a.info[k];
@@ -490,7 +608,7 @@ __global__ void k_cls_fill_edges(ClsArgs a) {
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     const unsigned FULL = 0xffffffffu;
-    const int npairs = *a.plist_n;
+    const int npairs = a.level == 2 ? *a.plist_n : a.npairs;
     for (int k = wid; k < npairs; k += nw) {
         if (a.ecount[k] == 0) continue;
         const int4 in = a.info[k];
@@ -499,15 +617,8 @@ __global__ void k_cls_fill_edges(ClsArgs a) {
         const CellRect r = cells_rect(a, cell % a.res, cell / a.res, 1);
         float4* out = a.edges + a.eoff[k];
         int wr = 0, wf = nr;
-        for (int e0 = 0; e0 < nv; e0 += 32) {
-            int e = e0 + lane;
-            int c = 0;
-            float2 vi = make_float2(0.f, 0.f), vj = vi;
-            if (e < nv) {
-                vi = __ldg(a.verts + v0 + e);
-                vj = __ldg(a.verts + v0 + (e == 0 ? nv - 1 : e - 1));
-                c = edge_class(r, vi, vj);
-            }
+        for_near_edges(a.verts + v0, nv, r, lane, [&](float2 vi, float2 vj, bool live) {
+            const int c = live ? edge_class(r, vi, vj) : 0;
             const bool is_r = (c & 6) == 6, is_f = (c & 6) == 2;
             const unsigned mr = __ballot_sync(FULL, is_r), mf = __ballot_sync(FULL, is_f);
             const unsigned below = (1u << lane) - 1u;
@@ -515,7 +626,7 @@ __global__ void k_cls_fill_edges(ClsArgs a) {
             if (is_f) out[wf + __popc(mf & below)] = make_float4(vi.x, vi.y, vj.x, vj.y);
             wr += __popc(mr);
             wf += __popc(mf);
-        }
+        });
     }
 }
 
@@ -848,10 +959,12 @@ bool launch_exclusive_scan(const int* in, int* out, int n, int* tmp, cudaStream_
 
 void launch_cls_classify(const ClsArgs& c, int sms, cudaStream_t st) {
     // level 2 reads its pair count on the device; c.npairs is then an upper bound
-    int blocks = (int)std::min<long long>(((long long)c.npairs * 32 + 255) / 256, (long long)sms * 32);
-    if (blocks < 1) blocks = 1;
+    const bool lanes = c.level != 2;
+    const long long want = lanes ? ((long long)c.npairs + 127) / 128 : ((long long)c.npairs * 32 + 255) / 256;
+    const int blocks = (int)std::max(1LL, std::min(want, (long long)sms * 32));
     ++g_kernel_launches;
-    k_cls_classify<<<blocks, 256, 0, st>>>(c);
+    if (lanes) k_cls_pairs<<<blocks, 128, 0, st>>>(c);
+    else k_cls_classify<<<blocks, 256, 0, st>>>(c);
 }
 void launch_cls_emit(const ClsArgs& c, int sms, cudaStream_t st) {
     int blocks = std::min((c.npairs + 255) / 256, sms * 16);

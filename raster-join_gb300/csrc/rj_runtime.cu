@@ -517,10 +517,11 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
         c1.level = 1;
         c1.npairs = npairs1;
         c1.info = info1;
-        if (npairs1 > 0) launch_cls_classify(c1, ctx->sms, ctx->stream);
+        if (npairs1 > 0 && scale > 1) launch_cls_classify(c1, ctx->sms, ctx->stream);
         // level 2: fine cells of the coarse EDGE pairs.  Its pair count stays on
         // the device; buffers are sized for the upper bound (every coarse pair
-        // refined) so no host round trip is needed before the scans.
+        // refined) so no host round trip is needed before the scans.  With one
+        // fine cell per coarse cell both levels are one pass.
         const int npairs2 = (int)max_fine;
         int4* info2;
         int *ecount, *eoff;
@@ -531,7 +532,7 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
         if ((rc = scratch_t(ctx, "cls_tmp", (size_t)ntmp, &tmp))) return rc;
         RJ_CUDA(cudaMemsetAsync(ecount, 0, sizeof(int) * (size_t)std::max(npairs2, 1), ctx->stream));
         ClsArgs c2 = c;
-        c2.level = 2;
+        c2.level = scale > 1 ? 2 : 3;
         c2.npairs = npairs2;
         c2.info = info2;
         c2.ecount = ecount;
@@ -554,7 +555,7 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
         c2.edges = edges;
         uint32_t* code;
         if ((rc = scratch_t(ctx, "cls_code", ncells, &code))) return rc;
-        if (npairs1 > 0) launch_cls_emit(c1, ctx->sms, ctx->stream);
+        if (npairs1 > 0 && scale > 1) launch_cls_emit(c1, ctx->sms, ctx->stream);
         if (npairs2 > 0) {
             launch_cls_emit(c2, ctx->sms, ctx->stream);
             launch_cls_fill_edges(c2, ctx->sms, ctx->stream);
