@@ -23,7 +23,7 @@ SOURCES = ["rj_runtime.cu", "rj_point_kernels.cu", "rj_point_exact.cu", "rj_poly
            "rj_batch.cu", "rj_batch_kernels.cu", "rj_batch_direct.cu", "rj_tier_kernels.cu",
            "rj_hybrid_lean.cu", "rj_splat_kernels.cu",
            "rj_tier_lean.cu", "rj_label_count.cu", "rj_label_sum.cu",
-           "rj_label_tile.cu", "rj_band_kernels.cu"]
+           "rj_label_tile.cu", "rj_band_kernels.cu", "rj_splat_bins.cu"]
 HEADERS = ["rj_device.cuh", "rj_launch.h", "rj_internal.h", "rj_point_map.cuh", "rj_point_core.cuh",
            "rj_batch_common.cuh", "rj_lean.cuh", "rj_label_core.cuh", "rj_bands.cuh",
            os.path.join("..", "..", "include", "rj.h")]

@@ -343,6 +343,11 @@ int splat_lean_shapes();
 // when the canvas does not fit
 size_t splat_lean_smem(int shape, size_t npix, bool agg);
 bool launch_splat_lean(int shape, const SplatLeanArgs& a, const LeanCols& lc, int sms, cudaStream_t st);
+// the same counts through bins of the canvas (rj_splat_bins.cu); `scratch`:
+// splat_bins_bytes for the table's rows
+bool splat_bins_fit(int resx, int resy, int sms, bool agg);
+size_t splat_bins_bytes(int resx, int resy, int sms, uint64_t n);
+bool launch_splat_bins(const SplatLeanArgs& a, const LeanCols& lc, void* scratch, int sms, cudaStream_t st);
 
 // point side
 // smem_hist: histogram capacity decision done by the launcher.

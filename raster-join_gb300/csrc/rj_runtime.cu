@@ -61,6 +61,14 @@ int dev_alloc(rj_ctx* ctx, DevBuf& b, size_t bytes) {
         return fail(ctx, RJ_E_OOM, "device memory budget exceeded: need %zu more bytes, %zu of %lld in use",
                     bytes, (size_t)ctx->used.load(), (long long)ctx->budget);
     cudaError_t e = cudaMalloc(&b.p, bytes);
+    if (e != cudaSuccess && !ctx->capturing) {   // what a query can do without gives way
+        cudaGetLastError();
+        const auto spare = ctx->scratch.find("splat_bins");
+        if (spare != ctx->scratch.end() && spare->second.p && &spare->second != &b) {
+            dev_free(ctx, spare->second);
+            e = cudaMalloc(&b.p, bytes);
+        }
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         b.p = nullptr;
@@ -1164,6 +1172,12 @@ int hybrid_lean_pass(rj_ctx* ctx, const DevFilter& f, int mode, const HybXf& h, 
     return RJ_OK;
 }
 
+constexpr int kSplatBins = 6;                    // shape index of the pass through bins
+// ... which is tried from this many points: its floor is the pass over the whole
+// canvas and three launches (30M points onto 4000 x 4000 pixels: 213 us against
+// 187 for atomics in L2; 100M: 531 against 587)
+constexpr uint64_t kBinMinPoints = 1ull << 26;
+
 // Lean point pass onto the point canvas (rj_splat_kernels.cu): one canvas
 // tile, a resident table, interval-form filters on at most four columns,
 // count or sum.  The shape (canvas copies in shared memory, or atomics
@@ -1201,6 +1215,23 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
             const size_t sm = splat_lean_smem(sh, npix, agg);
             if (sm > 0 && sm <= 200 * 1024) cands.push_back(sh);
         }
+    // the pass through bins (rj_splat_bins.cu): its scratch is optional, so it is
+    // left alone under a memory budget and inside a capture
+    void* bin_scratch = nullptr;
+    const bool force_bins = ctx->count_shape == kSplatBins;
+    if ((force_bins || (ctx->count_shape < 0 && a.n >= kBinMinPoints)) && ctx->budget <= 0 && !ctx->capturing &&
+        ctx->scratch_ns.empty() && splat_bins_fit(rp.resx, rp.resy, ctx->sms, agg) &&
+        scratch(ctx, "splat_bins", splat_bins_bytes(rp.resx, rp.resy, ctx->sms, a.n), &bin_scratch) != RJ_OK)
+        bin_scratch = nullptr;
+    if (force_bins && bin_scratch) {
+        ctx->passes = 1;
+        ctx->copy_ms = 0;
+        if (!launch_splat_bins(a, lc, bin_scratch, ctx->sms, ctx->stream)) return RJ_OK;
+        RJ_CUDA(cudaGetLastError());
+        ctx->last_count_shape = kSplatBins;
+        *done = true;
+        return RJ_OK;
+    }
     if (cands.empty()) return RJ_OK;
     char key[200];
     std::snprintf(key, sizeof key, "splat:%d:%d:%d:%d:%d:%d", lc.ncol, lc.aggr, lc.aggr_ci >= 0,
@@ -1218,6 +1249,25 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
         b.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 27);
         return launch_splat_lean(cands[i], b, lc, ctx->sms, ctx->stream);
     });
+    // that shape or the bins, again per query class
+    int bins = 0;
+    if (pi >= 0 && bin_scratch) {
+        std::snprintf(key, sizeof key, "bins:%d:%d:%d", lc.ncol, tune_bucket((double)npix), tune_bucket((double)a.n));
+        SplatLeanArgs w = a;
+        w.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 16);
+        if (!tuned_get(ctx, key, &bins)) {   // the first launch loads the kernels
+            timed_any = true;
+            launch_splat_bins(w, lc, bin_scratch, ctx->sms, ctx->stream);
+            cudaStreamSynchronize(ctx->stream);
+        }
+        bins = tune_pick(ctx, key, 2, [&](size_t i) {
+            timed_any = true;
+            SplatLeanArgs b = a;
+            b.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 27);
+            return i ? launch_splat_bins(b, lc, bin_scratch, ctx->sms, ctx->stream)
+                     : launch_splat_lean(cands[(size_t)pi], b, lc, ctx->sms, ctx->stream);
+        });
+    }
     RJ_CUDA(cudaGetLastError());
     if (timed_any) {
         RJ_CUDA(cudaMemsetAsync(canvas_c, 0, npix * sizeof(uint32_t), ctx->stream));
@@ -1226,9 +1276,11 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
     if (pi < 0) return RJ_OK;
     ctx->passes = 1;
     ctx->copy_ms = 0;
-    if (!launch_splat_lean(cands[(size_t)pi], a, lc, ctx->sms, ctx->stream)) return RJ_OK;
+    if (bins == 1 ? !launch_splat_bins(a, lc, bin_scratch, ctx->sms, ctx->stream)
+                  : !launch_splat_lean(cands[(size_t)pi], a, lc, ctx->sms, ctx->stream))
+        return RJ_OK;
     RJ_CUDA(cudaGetLastError());
-    ctx->last_count_shape = cands[(size_t)pi];
+    ctx->last_count_shape = bins == 1 ? kSplatBins : cands[(size_t)pi];
     *done = true;
     return RJ_OK;
 }
