@@ -254,6 +254,8 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPa
             }
         }
         __syncwarp();
+        unsigned pairs = 0;   // of crossings in one row
+        int most = 0;         // crossings of a row
         {
             // differences -> counts -> first crossing of each row
             int c = lane < kBand ? S.start[lane] : 0;
@@ -263,6 +265,8 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPa
                 if (lane >= o) c += v;
             }
             int x = lane < kBand ? c : 0;
+            most = __reduce_max_sync(FULL, x);
+            pairs = __reduce_add_sync(FULL, (unsigned)min(x, 4096) * (unsigned)min(x, 4096));
             #pragma unroll
             for (int o = 1; o < kBand; o <<= 1) {
                 const int v = __shfl_up_sync(FULL, x, o);
@@ -277,6 +281,20 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPa
         unsigned long long acc_c = 0, acc_s = 0;
         long long b_fn = 0, b_fp = 0, b_fn1 = 0, b_fp1 = 0;
         const int nrows = je - jb + 1;
+        // Rows with few crossings rank each against the others.  Where that is
+        // dearer, a row is a bitmap instead, one bit per column, a crossing
+        // flipping its bit: the parity of the bits left of it is its rank's, and
+        // as a ring crosses a row an even number of times, one running parity
+        // serves all rows of a group.  About 6 instructions per pair against 25
+        // per word and 60 per edge and group of rows, each for 32 at a time.  On
+        // ten rings of up to 2,000 vertices, 1192 x 1137 pixels, 83 us; 784 with
+        // ranks and a test of every pixel in rows of more than 512 crossings.
+        // (Not in the outline pass: the code for both made it spill, 2,000 stars
+        // and 200M points at 1 m took 19.2 ms instead of 15.7.)
+        const int width = i_lo <= i_hi ? (i_hi - i_lo + 2 + 31) >> 5 : 0;   // words of a row
+        const int fit = width > 0 ? kBCross / width : 0;                    // rows of a group
+        const bool bits = !OUTLINE && fit > 0 && (most > kBCross || pairs > 4u * (unsigned)(nrows * width) +
+                                                                    10u * (unsigned)((nrows + fit - 1) / fit * ne));
         // inside test over every edge (a row with more crossings than are held)
         auto inside_slow = [&](int i, int r) {
             const int32_t cy = (jb + r) * kSub + kSub / 2;
@@ -294,12 +312,53 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPa
 
         for (int ra = 0; ra < nrows;) {
             int rb = ra + 1;
-            while (rb < nrows && S.start[rb + 1] - S.start[ra] <= kBCross) ++rb;
+            if (bits) rb = min(ra + fit, nrows);
+            else
+                while (rb < nrows && S.start[rb + 1] - S.start[ra] <= kBCross) ++rb;
             const int base = S.start[ra], m = S.start[rb] - base;
-            const bool slow = m > kBCross;   // then one row
+            const bool slow = !bits && m > kBCross;   // then one row
             if (lane < kBand) S.cur[lane] = 0;
+            if (bits)
+                for (int w = lane; w < (rb - ra) * width; w += 32) S.cross[w] = 0u;
             __syncwarp();
-            if (m > 0 && !slow) {
+            if (m > 0 && bits) {
+                for_edge_rows(ne, jb, lane, edge_at, [&](const int4& q, int r) {
+                    const int32_t cy = (jb + r) * kSub + kSub / 2;
+                    if (r < max(ra, cl) || r >= rb || r > ch || !cross_row(q.y, q.w, cy)) return;
+                    const int b = min(max(cross_L(q.x, q.y, q.z, q.w, cy), i_lo), i_hi + 1) - i_lo;
+                    atomicXor(&S.cross[(r - ra) * width + (b >> 5)], 1u << (b & 31));
+                });
+                __syncwarp();
+                unsigned carry = 0u;
+                for (int w0 = 0; w0 < (rb - ra) * width; w0 += 32) {
+                    const int w = w0 + lane;
+                    unsigned t = w < (rb - ra) * width ? S.cross[w] : 0u;
+                    const unsigned odd = __ballot_sync(FULL, __popc(t) & 1);
+                    unsigned before = (__popc(odd & ((1u << lane) - 1u)) ^ carry) & 1u;
+                    carry ^= __popc(odd) & 1u;
+                    const int r = ra + w / width, x0 = i_lo + (w % width) * 32;
+                    while (__any_sync(FULL, t != 0u)) {
+                        C c[4];
+                        unsigned long long cs[4];
+                        bool plus[4];
+                        #pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int L = t ? x0 + __ffs(t) - 1 : 0;   // (nothing is left of column 0)
+                            plus[u] = before != 0u;
+                            before ^= t ? 1u : 0u;
+                            t &= t - 1;
+                            c[u] = prefix_at(r, L);
+                            cs[u] = a.canvas_s && L > 0
+                                        ? (unsigned long long)__ldg(a.canvas_s + row0 + (size_t)r * a.resx + L - 1) : 0ull;
+                        }
+                        #pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            acc_c += plus[u] ? (unsigned long long)c[u] : 0ull - c[u];
+                            acc_s += plus[u] ? cs[u] : 0ull - cs[u];
+                        }
+                    }
+                }
+            } else if (m > 0 && !slow) {
                 for_edge_rows(ne, jb, lane, edge_at, [&](const int4& q, int r) {
                     const int32_t cy = (jb + r) * kSub + kSub / 2;
                     if (r < max(ra, cl) || r >= rb || r > ch || !cross_row(q.y, q.w, cy)) return;
@@ -308,7 +367,7 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPa
                 });
             }
             __syncwarp();
-            if (SPANS && m > 0 && i_lo <= i_hi) {
+            if (SPANS && !bits && m > 0 && i_lo <= i_hi) {
                 if (!slow) {
                     for (int x = lane; x < m; x += 32) {
                         const uint32_t mine = S.cross[x];

@@ -84,3 +84,44 @@ def test_band_passes_match_oracle(handler, shape, fbo, cell):
         handler.flags = 0
         handler.max_fbo_size = 8192
     assert b[:2 * len(polys)].any()
+
+
+@pytest.mark.parametrize("nv", [130, 700, 2500])
+@pytest.mark.parametrize("fbo", [8192, 311])
+def test_jagged_outlines_match_oracle(handler, nv, fbo):
+    """Rings that cross a row up to thousands of times (rows kept as bitmaps),
+    beside plain ones in the same bands: counts, sums and error bounds."""
+    rng = np.random.default_rng(nv)
+    polys = []
+    for k in range(6):
+        ang = np.sort(rng.uniform(0, 2 * np.pi, nv if k % 3 else 9))
+        rad = rng.uniform(5, 330, len(ang))
+        polys.append(np.c_[500 + 90 * k + rad * np.cos(ang), 500 + 40 * (k % 2) + rad * np.sin(ang)].astype(np.float32))
+    verts = np.concatenate(polys)
+    pidx = np.r_[0, np.cumsum([len(p) for p in polys])].astype(np.int32)
+    xy = rng.uniform(100, 1400, (200_001, 2)).astype(np.float32)
+    val = rng.uniform(-50, 90, len(xy)).astype(np.float32)
+    dh = rj.DataHandler()
+    dh.add_column(1, rj.Location, xy)
+    dh.add_column(2, rj.Float, val)
+    dh.setPolygons(verts, pidx)
+    dh.setAggregation(rj.Avg, 2)
+    handler.setDataHandler(dh)
+    handler.setCellSize(1.0)
+    handler.max_fbo_size = fbo
+    handler.flags = rj.FLAG_FORCE_CANVAS | rj.FLAG_FLAT_CANVAS
+    f = oracle.Columns({2: (oracle.Float, val)}).filt([], aggr_attrib=2)
+    try:
+        got = handler.execute(rj.RasterJoinFn)
+        want = oracle.raster_join(xy, verts, pidx, 1.0, f=f, max_res=fbo)
+        np.testing.assert_array_equal(got.count, want[0])
+        np.testing.assert_allclose(got.sum, want[1], rtol=1e-6, atol=1e-9 * max(1.0, float(np.abs(want[1]).max())))
+        dh.setAggregation(rj.Count, -1)
+        handler.setDataHandler(dh)
+        bnd = handler.execute(rj.RasterJoinBoundFn)
+        want = oracle.raster_join(xy, verts, pidx, 1.0, max_res=fbo, bounds=True)
+        np.testing.assert_array_equal(bnd.count, want[0])
+        np.testing.assert_array_equal(bnd.bounds, want[2])
+    finally:
+        handler.flags = 0
+        handler.max_fbo_size = 8192
