@@ -966,6 +966,7 @@ int label_map(rj_ctx* ctx, PolyPassArgs& a, const char* key, size_t npix, const 
 // the polygon count, canvas size and table size in octave buckets.  Scans
 // below kTuneMinPoints take the default shape without timing anything.
 constexpr uint64_t kTuneMinPoints = 1ull << 22;
+constexpr uint64_t kTuneWarm = 1ull << 16, kTuneMost = 1ull << 27;   // points of the untimed and the timed launch
 constexpr int kMaxShapes = 11;   // shape indices rj_set_tuning takes (a pass without that shape runs its generic form)
 inline int tune_bucket(double v) { return (int)std::floor(std::log2(std::max(v, 1.0))); }
 
@@ -1021,9 +1022,11 @@ void tuned_put(const rj_ctx* ctx, const std::string& key, int v) {
 }
 
 // The autotuner of the lean passes: the candidate kept for `key`, else each
-// candidate timed once by `timed(i)` (CUDA events on the context's stream;
-// returns false when it cannot run), the fastest kept.  Returns the index,
-// or -1 when none ran.
+// candidate timed once by `timed(i, points)` (CUDA events on the context's
+// stream; returns false when it cannot run), the fastest kept.  A short launch
+// comes first, untimed: with the loading of its kernel in the time, a candidate
+// twice as fast could lose (1B points over tiles at 1 m: 2.9 ms one process,
+// 2.5 the next).  Returns the index, or -1 when none ran.
 template <class Timed>
 int tune_pick(rj_ctx* ctx, const std::string& key, size_t ncand, Timed&& timed) {
     if (ncand == 1) return 0;
@@ -1035,8 +1038,9 @@ int tune_pick(rj_ctx* ctx, const std::string& key, size_t ncand, Timed&& timed) 
     float best = 1e30f;
     int besti = -1;
     for (size_t i = 0; i < ncand; ++i) {
+        if (!timed(i, kTuneWarm)) continue;   // loads the kernel, which takes longer than many a scan
         cudaEventRecord(e0, ctx->stream);
-        if (!timed(i)) continue;
+        if (!timed(i, kTuneMost)) continue;
         cudaEventRecord(e1, ctx->stream);
         cudaEventSynchronize(e1);
         float ms = 0.f;
@@ -1150,13 +1154,10 @@ int hybrid_lean_pass(rj_ctx* ctx, const DevFilter& f, int mode, const HybXf& h, 
     LeanCols tl = lc;
     tl.out_sum = tsum;
     tl.nonfinite = tnf;
-    const int pi = small && !have ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i) {
+    const int pi = small && !have ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i, uint64_t most) {
         HybLeanArgs b = args_for(cands[i].second);
         b.out_count = tout;
-        HybLeanArgs w = b;
-        w.n = std::min<uint64_t>(b.n & ~1ULL, 1ULL << 16);   // first launch of a shape loads it
-        if (!launch_hybrid_lean(cands[i].first, w, tl, ctx->sms, ctx->stream)) return false;
-        b.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 27);
+        b.n = std::min<uint64_t>(a.n & ~1ULL, most);
         return launch_hybrid_lean(cands[i].first, b, tl, ctx->sms, ctx->stream);
     });
     RJ_CUDA(cudaGetLastError());
@@ -1240,30 +1241,20 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
     const bool have = tuned_get(ctx, key, &tuned_i);
     const bool small = a.n < kTuneMinPoints;
     bool timed_any = false;
-    const int pi = small && !have ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i) {
+    const int pi = small && !have ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i, uint64_t most) {
         timed_any = true;
-        SplatLeanArgs w = a;
-        w.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 16);   // first launch of a shape loads it
-        if (!launch_splat_lean(cands[i], w, lc, ctx->sms, ctx->stream)) return false;
         SplatLeanArgs b = a;
-        b.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 27);
+        b.n = std::min<uint64_t>(a.n & ~1ULL, most);
         return launch_splat_lean(cands[i], b, lc, ctx->sms, ctx->stream);
     });
     // that shape or the bins, again per query class
     int bins = 0;
     if (pi >= 0 && bin_scratch) {
         std::snprintf(key, sizeof key, "bins:%d:%d:%d", lc.ncol, tune_bucket((double)npix), tune_bucket((double)a.n));
-        SplatLeanArgs w = a;
-        w.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 16);
-        if (!tuned_get(ctx, key, &bins)) {   // the first launch loads the kernels
-            timed_any = true;
-            launch_splat_bins(w, lc, bin_scratch, ctx->sms, ctx->stream);
-            cudaStreamSynchronize(ctx->stream);
-        }
-        bins = tune_pick(ctx, key, 2, [&](size_t i) {
+        bins = tune_pick(ctx, key, 2, [&](size_t i, uint64_t most) {
             timed_any = true;
             SplatLeanArgs b = a;
-            b.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 27);
+            b.n = std::min<uint64_t>(a.n & ~1ULL, most);
             return i ? launch_splat_bins(b, lc, bin_scratch, ctx->sms, ctx->stream)
                      : launch_splat_lean(cands[(size_t)pi], b, lc, ctx->sms, ctx->stream);
         });
@@ -1439,13 +1430,10 @@ int run_label_points(rj_ctx* ctx, LabelPlan& lp, const TierArgs& tr, ExecState& 
         LeanCols tl = lp.lc;
         tl.out_sum = tsum;
         tl.nonfinite = tnf;
-        const int pi = tune_pick(ctx, lp.key, cands.size(), [&](size_t i) {
+        const int pi = tune_pick(ctx, lp.key, cands.size(), [&](size_t i, uint64_t most) {
             LabelPointArgs b = lp.sides[(size_t)cands[i].second].a;
-            const uint64_t n = b.n;
             b.out_count = tout;
-            b.n = std::min<uint64_t>(n & ~1ULL, 1ULL << 16);   // first launch of a shape loads it
-            if (!launch(cands[i].first, b, tl)) return false;
-            b.n = std::min<uint64_t>(n & ~1ULL, 1ULL << 28);
+            b.n = std::min<uint64_t>(b.n & ~1ULL, most);
             return launch(cands[i].first, b, tl);
         });
         RJ_CUDA(cudaGetLastError());
@@ -1544,13 +1532,10 @@ int tier_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, const 
     const bool have = tuned_get(ctx, key, &tuned_i);
     const bool small = a.n < kTuneMinPoints;
     bool timed_any = false;
-    const int pi = small && !have ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i) {
+    const int pi = small && !have ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i, uint64_t most) {
         timed_any = true;
         TierLeanArgs b = a;
-        TierLeanArgs w = a;
-        w.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 16);   // first launch of a shape loads it
-        if (!launch_tier_lean(cands[i], w, lc, ctx->sms, ctx->stream)) return false;
-        b.n = std::min<uint64_t>(a.n & ~1ULL, 1ULL << 27);
+        b.n = std::min<uint64_t>(a.n & ~1ULL, most);
         return launch_tier_lean(cands[i], b, lc, ctx->sms, ctx->stream);
     });
     RJ_CUDA(cudaGetLastError());
