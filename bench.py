@@ -689,7 +689,7 @@ def run_headline(args, rj, torch, local, world):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": profiled_traffic("raster_count", n),
-                     "kernel": "k_label_count (shape %d, block codes 2^%d px)" % shape, "kernel_ms": mean_pt,
+                     "kernel": "k_label_tile (shape %d, block codes 2^%d px)" % shape, "kernel_ms": mean_pt,
                      "algorithmic_bytes_per_launch": n * HEADLINE_BYTES_PER_POINT, "peak_kind": peak_kind},
         "clocks": clocks,
         "checks": {"full_table_vs_canvas_path": canvas_equal,

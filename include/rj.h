@@ -303,7 +303,9 @@ RJ_API int rj_column_absmax(const rj_ctx *ctx, int32_t attrib_id, double *out);
  *                            sets that overlap on it, the error-bounds
  *                            join); RJ_TUNE_COUNT_SHAPE indexes them there
  *                            too (canvas copies in shared memory, or
- *                            atomics into the canvas in global memory)
+ *                            atomics into the canvas in global memory); the
+ *                            index after them is the count through bins of
+ *                            the canvas
  *   RJ_TUNE_HYBRID_SHAPES    (read only) number of shapes of the lean pass
  *                            of the hybrid and index joins; RJ_TUNE_COUNT_SHAPE
  *                            indexes them there

