@@ -106,6 +106,7 @@ struct ClsArgs {
     const int* pair_off;         // [P+1] first coarse pair of each polygon
     const int4* prange;          // [P] coarse candidate cells [stx, enx) x [sty, eny)
     int npairs;                  // pairs of the level being classified
+    float edges_per_pair;        // mean number of edges of a pair's polygon
     // level 2: explicit (polygon, fine cell) pairs refined from EDGE coarse pairs
     int2* plist;
     int* plist_n;

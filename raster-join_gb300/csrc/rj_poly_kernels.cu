@@ -444,7 +444,7 @@ __device__ __forceinline__ PairEdges pair_edges_warp(const float2* __restrict__ 
     return t;
 }
 
-// Level 1, a pair per lane: neighbouring pairs mostly share their polygon, so
+// Levels 1 and 3, a pair per lane: neighbouring pairs mostly share their polygon, so
 // each of its edges is one broadcast load and a few comparisons for 32 cells.
 // Edges left of the cell's rectangle say nothing, edges right of it only
 // whether they straddle its middle; the others are marked, and the lanes then
@@ -556,19 +556,42 @@ __global__ void __launch_bounds__(128, 6) k_cls_pairs(ClsArgs a) {
     }
 }
 
-// Level 2, a pair per warp (the list mixes polygons).
+// A pair per warp: level 2, whose list mixes polygons, and the other levels when
+// there are too few pairs to give every warp 32 (launch_cls_classify).
 __global__ void k_cls_classify(ClsArgs a) {
     const int lane = threadIdx.x & 31;
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    const int npairs = *a.plist_n;
+    const int npairs = a.level == 2 ? *a.plist_n : a.npairs;
+    const int n = a.level == 1 ? a.scale : 1;
     for (int k = wid; k < npairs; k += nw) {
-        const int2 q = a.plist[k];
-        const int p = q.x, cell = q.y;
-        const int v0 = __ldg(a.pindex + p), nv = __ldg(a.pindex + p + 1) - v0;
-        const PairEdges t = pair_edges_warp(a.verts + v0, nv, cells_rect(a, cell % a.res, cell / a.res, 1), lane);
+        int p, gx, gy;
+        if (a.level == 2) {
+            const int2 q = a.plist[k];
+            p = q.x;
+            gx = q.y % a.res;
+            gy = q.y / a.res;
+        } else {
+            p = pair_poly(a, k);
+            const int4 r = __ldg(a.prange + p);
+            const int w = r.y - r.x, l = k - __ldg(a.pair_off + p);
+            gx = (r.x + l % w) * n;
+            gy = (r.z + l / w) * n;
+        }
+        const int v0 = __ldg(a.pindex + p), nv = __ldg(a.pindex + p + 1) - v0, cell = gy * a.res + gx;
+        const PairEdges t = pair_edges_warp(a.verts + v0, nv, cells_rect(a, gx, gy, n), lane);
         const int kind = t.meets ? 0 : (t.inside ? -1 : -2);
-        if (lane == 0) {
+        if (a.level == 1) {
+            if (lane == 0) a.info[k] = make_int4(p, kind, 0, cell);
+            int base = 0;
+            if (kind == 0 && lane == 0) base = atomicAdd(a.plist_n, n * n);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            for (int s = lane; s < n * n; s += 32) {
+                const int c = (gy + s / n) * a.res + gx + s % n;
+                if (kind == -1) atomicAdd(a.cell_kept + c, 1);
+                else if (kind == 0) a.plist[base + s] = make_int2(p, c);
+            }
+        } else if (lane == 0) {
             a.info[k] = (kind == 0) ? make_int4(p, t.nr, t.nf, cell) : make_int4(p, kind, 0, cell);
             a.ecount[k] = (kind == 0) ? t.nr + t.nf : 0;
             if (kind != -2) atomicAdd(a.cell_kept + cell, 1);
@@ -959,7 +982,12 @@ bool launch_exclusive_scan(const int* in, int* out, int n, int* tmp, cudaStream_
 
 void launch_cls_classify(const ClsArgs& c, int sms, cudaStream_t st) {
     // level 2 reads its pair count on the device; c.npairs is then an upper bound
-    const bool lanes = c.level != 2;
+    // A pair per lane takes about 0.38 us per edge and round of 32 pairs per warp,
+    // a pair per warp 2 us and 0.007 per edge (120,000 pairs of 100 edges: 38 us
+    // against 89; 20,000 pairs of jagged rings of 260: 400 against 180).
+    const double slots = sms * 24.0, edges = c.edges_per_pair;
+    const bool lanes = c.level != 2 && c.npairs / slots * (2.0 + 0.007 * edges) >
+                                           std::max(1.0, c.npairs / (32.0 * slots)) * 0.38 * edges;
     const long long want = lanes ? ((long long)c.npairs + 127) / 128 : ((long long)c.npairs * 32 + 255) / 256;
     const int blocks = (int)std::max(1LL, std::min(want, (long long)sms * 32));
     ++g_kernel_launches;

@@ -461,6 +461,7 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
         std::vector<int> off(P + 1);
         std::vector<int4> rng(P);
         long long total = 0;
+        double edge_sum = 0;
         for (int p = 0; p < P; ++p) {
             off[p] = (int)total;
             const float4 m = ctx->ps->h_mbr[p];
@@ -479,6 +480,7 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
             }
             rng[p] = make_int4(stx, enx, sty, eny);
             total += (long long)(enx - stx) * (eny - sty);
+            edge_sum += (double)(enx - stx) * (eny - sty) * (ctx->ps->h_pindex[p + 1] - ctx->ps->h_pindex[p]);
         }
         off[P] = (int)total;
         const long long max_fine = total * scale * scale;
@@ -509,6 +511,7 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
         c.plist = plist;
         c.plist_n = plist_n;
         c.scale = scale;
+        c.edges_per_pair = total > 0 ? (float)(edge_sum / (double)total) : 0.0f;
         c.lbx = lbx; c.lby = lby; c.csx = csx; c.csy = csy;
         c.res = G;
         const double U = std::ldexp(1.0, -24);

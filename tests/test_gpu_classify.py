@@ -1,5 +1,5 @@
-"""The classified grid of the exact tests, built a pair per lane up to 512
-vertices of a polygon and a pair per warp above: outlines on both sides of that
+"""The classified grid of the exact tests, built a pair of cell and polygon per
+warp or per lane (polygons of more than 512 vertices by the warp): outlines on both sides of that
 limit, side by side in one set so that warps hold pairs of several polygons,
 coarse and fine grids; index and hybrid counts equal the oracle's, on points
 crowded along the outlines."""
@@ -11,25 +11,29 @@ import rasterjoin as rj
 
 pytestmark = pytest.mark.gpu
 
+# many edges per pair: a warp per pair; few: a lane per pair, but for the rings
+# of more than 512
 SIZES = [3, 4, 7, 8, 9, 100, 511, 512, 513, 640, 1200, 5, 31, 33, 2000, 3]
+SMALL = [3, 4, 7, 8, 9, 100, 32, 64, 513, 65, 512, 5, 31, 33, 3, 3]
 
 
-def _set(overlap):
+def _set(overlap, sizes=SIZES):
     rng = np.random.default_rng(17)
     polys = []
-    for i, n in enumerate(SIZES):
+    for i, n in enumerate(sizes):
         cx, cy = 500.0 + 1000.0 * (i % 4), 500.0 + 1000.0 * (i // 4)
         ang = np.sort(rng.uniform(0, 2 * np.pi, n)) if n > 4 else 2 * np.pi * (np.arange(n) + 0.3) / n
         rad = rng.uniform(150.0, 460.0, n) * (1.6 if overlap else 1.0)
         polys.append(np.c_[cx + rad * np.cos(ang), cy + rad * np.sin(ang)])
     v = np.concatenate(polys).astype(np.float32)
-    return v, np.r_[0, np.cumsum(SIZES)].astype(np.int32)
+    return v, np.r_[0, np.cumsum(sizes)].astype(np.int32)
 
 
 @pytest.mark.parametrize("overlap", [False, True])
-@pytest.mark.parametrize("res", [1, 5, 64, 300])
-def test_joins_match_oracle(handler, overlap, res):
-    verts, pidx = _set(overlap)
+@pytest.mark.parametrize("res", [1, 5, 64, 300, 500])
+@pytest.mark.parametrize("sizes", [SIZES, SMALL])
+def test_joins_match_oracle(handler, overlap, res, sizes):
+    verts, pidx = _set(overlap, sizes)
     rng = np.random.default_rng(18)
     on = verts[rng.integers(0, len(verts), 100_000)] + rng.normal(0, 2.0, (100_000, 2))
     xy = np.r_[rng.uniform(-300, 4300, (150_001, 2)), on].astype(np.float32)
