@@ -444,15 +444,16 @@ __device__ __forceinline__ PairEdges pair_edges_warp(const float2* __restrict__ 
     return t;
 }
 
-// Levels 1 and 3, a pair per lane: neighbouring pairs mostly share their polygon, so
-// each of its edges is one broadcast load and a few comparisons for 32 cells.
+// Levels 1 and 3, a pair per lane: neighbouring pairs mostly share their polygon,
+// so each of its edges is one broadcast load and a few comparisons for 32 cells.
 // Edges left of the cell's rectangle say nothing, edges right of it only
 // whether they straddle its middle; the others are marked, and the lanes then
 // work off their own marks together.  With a warp per pair (the edges over the
 // lanes) a pair is one load latency after another, whatever its edges are:
-// 65,000 cells of 260 polygons with 100 vertices, 120,000 pairs, took 89 us
-// and 19 more for level 2; 38 us now for both.  Polygons of more than kLaneEdges vertices are still walked by
-// the warp, pair by pair: a lane alone would be at it for too long.
+// 65,000 cells of 260 polygons with 100 vertices, 120,000 pairs, took 89 us and
+// 19 more for level 2; 38 us now for both.  Polygons of more than kLaneEdges
+// vertices are still walked by the warp, pair by pair: a lane alone would be at
+// it for too long.
 constexpr int kLaneEdges = 512;
 
 __global__ void __launch_bounds__(128, 6) k_cls_pairs(ClsArgs a) {

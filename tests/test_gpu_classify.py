@@ -1,8 +1,8 @@
 """The classified grid of the exact tests, built a pair of cell and polygon per
-warp or per lane (polygons of more than 512 vertices by the warp): outlines on both sides of that
-limit, side by side in one set so that warps hold pairs of several polygons,
-coarse and fine grids; index and hybrid counts equal the oracle's, on points
-crowded along the outlines."""
+warp or per lane (polygons of more than 512 vertices by the warp): outlines on
+both sides of that limit, side by side in one set so that warps hold pairs of
+several polygons, coarse and fine grids; index and hybrid counts equal the
+oracle's, on points crowded along the outlines."""
 import numpy as np
 import pytest
 
