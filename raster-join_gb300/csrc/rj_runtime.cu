@@ -1114,7 +1114,7 @@ int hybrid_lean_pass(rj_ctx* ctx, const DevFilter& f, int mode, const HybXf& h, 
         for (int sh = 0; sh < hybrid_lean_shapes(); ++sh)
             if (ctx->count_shape < 0 || ctx->count_shape == sh) {
                 const size_t sm = hybrid_lean_smem(sh, (int)code_words(bs), P, lc.aggr != 0);
-                if (sm > 0 && sm <= 200 * 1024) cands.push_back({sh, bs});
+                if (sm > 0 && sm <= 220 * 1024) cands.push_back({sh, bs});   // (the warps' queues take 43 or 86 KB)
             }
     if (cands.empty()) return RJ_OK;
     char key[200];
