@@ -344,6 +344,9 @@ RJ_API int rj_get_tuning(const rj_ctx *ctx, int32_t knob, int32_t *value);
  * still describes the rows (a reload drops it); else rj_execute_prepared
  * returns RJ_E_INVALID.  The
  * zone map is not used by a plan (a reloaded table needs none).
+ * Other queries in between do not disturb it: a cached grid or scratch its
+ * graph reads is kept for it until rj_plan_destroy when another query needs
+ * a larger one or rebuilds the grid.
  * Queries whose execution reads a value back to the host before it can go
  * on cannot be captured (tiered canvases, an index or hybrid join that
  * rebuilds its grid each call): rj_prepare returns RJ_E_UNSUPPORTED, as it

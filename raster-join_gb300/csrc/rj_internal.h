@@ -18,6 +18,7 @@ namespace rjh {
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    std::vector<uint64_t> plans;   // prepared queries whose graphs hold its address (scratch only)
 };
 
 struct Column {
@@ -150,8 +151,8 @@ struct rj_ctx {
     void* pin = nullptr;             // pinned host copy of rj_execute's outputs
     size_t pin_bytes = 0;
     bool exact_slots = false;        // tiered canvas: read the number of mixed blocks back
-    int live_plans = 0;              // prepared queries: their graphs hold scratch addresses
-    std::vector<rjh::DevBuf> retired;   // outgrown scratch those graphs may still use
+    uint64_t plan_ids = 0;           // number of the last prepared query
+    std::vector<rjh::DevBuf> retired;   // scratch that queries no longer use but the graphs of prepared ones do
     int sum_shift = 0;        // fixed-point scale 2^s of the current query's sums
     uint64_t row0 = 0, row1 = ~0ULL;   // rows of the current query (time index window)
     int server_running = 0;   // a serving loop owns the context
@@ -184,6 +185,7 @@ struct rj_plan {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t stream = nullptr;
+    uint64_t id = 0;         // among the context's prepared queries
     int P = 0;
     int function_type = 0;
     int shift = 0;

@@ -84,22 +84,40 @@ void dev_free(rj_ctx* ctx, DevBuf& b) {
         cudaFree(b.p);
         ctx->used -= b.bytes;
     }
-    b.p = nullptr;
-    b.bytes = 0;
+    b = DevBuf{};
 }
 
 DevBuf& scratch_buf(rj_ctx* ctx, const char* key) {
     return ctx->scratch_ns.empty() ? ctx->scratch[key] : ctx->scratch[std::string(key) + ctx->scratch_ns];
 }
 
+// A buffer about to be replaced or written anew: when a prepared query's graph
+// holds its address, the graph keeps it (until drop_plan) and the key starts
+// over with a new one.
+void leave_to_plans(rj_ctx* ctx, DevBuf& b) {
+    if (b.plans.empty()) return;
+    ctx->retired.push_back(std::move(b));
+    b = DevBuf{};
+}
+
+// The buffers that only plan `id` still used are given back.
+void drop_plan(rj_ctx* ctx, uint64_t id) {
+    const auto forget = [id](DevBuf& b) { b.plans.erase(std::remove(b.plans.begin(), b.plans.end(), id), b.plans.end()); };
+    for (auto& kv : ctx->scratch) forget(kv.second);
+    for (size_t i = 0; i < ctx->retired.size();) {
+        forget(ctx->retired[i]);
+        if (!ctx->retired[i].plans.empty()) { ++i; continue; }
+        dev_free(ctx, ctx->retired[i]);
+        ctx->retired.erase(ctx->retired.begin() + (long)i);
+    }
+}
+
 int scratch(rj_ctx* ctx, const char* key, size_t bytes, void** out) {
     DevBuf& b = scratch_buf(ctx, key);
-    if (ctx->live_plans && b.p && b.bytes < bytes) {   // a prepared query's graph may hold its address
-        ctx->retired.push_back(b);
-        b = DevBuf{};
-    }
+    if (b.bytes < bytes) leave_to_plans(ctx, b);
     int rc = dev_alloc(ctx, b, bytes);
     if (rc) return rc;
+    if (ctx->capturing && (b.plans.empty() || b.plans.back() != ctx->plan_ids)) b.plans.push_back(ctx->plan_ids);
     *out = b.p;
     return RJ_OK;
 }
@@ -377,6 +395,9 @@ int build_grid(rj_ctx* ctx, int res, int clamp, IndexArgs& ia, bool with_pair_ce
     const size_t ncells = (size_t)res * res;
     if (!(g.valid && g.res == res && g.clamp == clamp && (g.pair_cell || !with_pair_cell))) {
         int *cnt, *cursor, *tmp;
+        // (a graph over the cached grid only reads it)
+        g.valid = false;
+        for (const char* key : {"grid_start", "grid_entries"}) leave_to_plans(ctx, scratch_buf(ctx, key));
         if ((rc = scratch_t(ctx, "grid_cnt", ncells, &cnt))) return rc;
         if ((rc = scratch_t(ctx, "grid_start", ncells + 1, &cell_start))) return rc;
         if ((rc = scratch_t(ctx, "grid_tmp", (size_t)scan_tmp_ints((int)ncells), &tmp))) return rc;
@@ -454,6 +475,7 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
     int* start2;
     int4* entries2;
     float4* edges;
+    uint32_t* code;
     if (!(xc.valid && xc.res == G && xc.user_res == user_res)) {
         // candidate ranges on the query grid, in fp32 as the reference computes them
         const float rcsx = (float)(dx / user_res), rcsy = (float)(dy / user_res);
@@ -489,6 +511,9 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
         int *doff, *cell_kept, *cursor, *tmp, *plist_n;
         int4 *drng, *info1;
         int2* plist;
+        // (a graph over the cached grid only reads it)
+        xc.valid = false;
+        for (const char* key : {"cls_start", "cls_entries", "cls_edges", "cls_code"}) leave_to_plans(ctx, scratch_buf(ctx, key));
         if ((rc = scratch_t(ctx, "cls_off", (size_t)P + 1, &doff))) return rc;
         if ((rc = scratch_t(ctx, "cls_rng", (size_t)P, &drng))) return rc;
         if ((rc = scratch_t(ctx, "cls_info1", (size_t)std::max(npairs1, 1), &info1))) return rc;
@@ -564,7 +589,6 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
         if ((rc = scratch_t(ctx, "cls_edges", (size_t)std::max(totals[1], 1), &edges))) return rc;
         c1.entries = c2.entries = entries2;
         c2.edges = edges;
-        uint32_t* code;
         if ((rc = scratch_t(ctx, "cls_code", ncells, &code))) return rc;
         if (npairs1 > 0 && scale > 1) launch_cls_emit(c1, ctx->sms, ctx->stream);
         if (npairs2 > 0) {
@@ -582,8 +606,9 @@ int build_exact(rj_ctx* ctx, int user_res, ExactIndex& ix, int max_scale = 1024)
         if ((rc = scratch_t(ctx, "cls_start", ncells + 1, &start2))) return rc;
         if ((rc = scratch_t(ctx, "cls_entries", std::max<size_t>(xc.nentries, 1), &entries2))) return rc;
         if ((rc = scratch_t(ctx, "cls_edges", std::max<size_t>(xc.nedges, 1), &edges))) return rc;
+        if ((rc = scratch_t(ctx, "cls_code", ncells, &code))) return rc;
     }
-    ix.code = (const uint32_t*)scratch_buf(ctx, "cls_code").p;
+    ix.code = code;
     ix.cell_start = start2;
     ix.entries = entries2;
     ix.edges = edges;
@@ -2599,6 +2624,7 @@ int rj_prepare(rj_ctx* ctx, const rj_query* q, rj_plan** plan) {
     const int P = ctx->ps->P;
     rj_plan* p = new rj_plan();
     p->ctx = ctx;
+    p->id = ++ctx->plan_ids;
     p->stream = ctx->stream;
     p->P = P;
     p->function_type = q->function_type;
@@ -2636,6 +2662,7 @@ int rj_prepare(rj_ctx* ctx, const rj_query* q, rj_plan** plan) {
     if (rc || ce != cudaSuccess || !g) {
         cudaGetLastError();
         if (g) cudaGraphDestroy(g);
+        drop_plan(ctx, p->id);
         plan_free(p);
         if (rc) return rc;
         return fail(ctx, RJ_E_UNSUPPORTED, "the query's work could not be captured: %s", cudaGetErrorString(ce));
@@ -2644,10 +2671,10 @@ int rj_prepare(rj_ctx* ctx, const rj_query* q, rj_plan** plan) {
     ce = cudaGraphInstantiate(&p->exec, g, 0);
     if (ce != cudaSuccess) {
         cudaGetLastError();
+        drop_plan(ctx, p->id);
         plan_free(p);
         return fail(ctx, RJ_E_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(ce));
     }
-    ++ctx->live_plans;
     *plan = p;
     return RJ_OK;
 }
@@ -2703,11 +2730,9 @@ void rj_plan_destroy(rj_plan* p) {
         rj_ctx* ctx = p->ctx;
         std::lock_guard<std::recursive_mutex> lock(ctx->mu);
         cudaSetDevice(ctx->device);
+        const uint64_t id = p->id;
         plan_free(p);
-        if (--ctx->live_plans == 0) {
-            for (auto& b : ctx->retired) dev_free(ctx, b);
-            ctx->retired.clear();
-        }
+        drop_plan(ctx, id);
         return;
     }
     plan_free(p);
