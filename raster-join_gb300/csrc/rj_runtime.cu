@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <algorithm>
+#include <initializer_list>
 #include <map>
 #include <string>
 #include <thread>
@@ -840,8 +841,21 @@ size_t tier_slot_bound(const PolySet& s, const RasterPlan& rp, size_t nblk, bool
     return (size_t)std::min((double)nblk, edge + rim + 64.0);
 }
 
-int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const DevFilter& f, ExecState& es,
-                     PolyPassArgs& a, const CanvasXf& cx, uint64_t ckey, bool bounds) {
+// Whether the memory budget holds buffers of these sizes under these keys.
+bool budget_holds(rj_ctx* ctx, std::initializer_list<std::pair<const char*, size_t>> want) {
+    if (ctx->budget <= 0) return true;
+    size_t total = ctx->used;
+    for (const auto& w : want) {
+        const DevBuf& b = scratch_buf(ctx, w.first);
+        const size_t bytes = (w.second + 255) & ~size_t(255);
+        if (bytes > b.bytes) total += bytes - (b.plans.empty() ? b.bytes : 0);
+    }
+    return (int64_t)total <= ctx->budget;
+}
+
+// `exact`: the number of mixed blocks is read back (set when it was).
+int tier_attempt(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const DevFilter& f, ExecState& es, PolyPassArgs& a,
+                 const CanvasXf& cx, uint64_t ckey, bool bounds, bool& exact) {
     int rc;
     TierArgs tr{};
     tr.bw = (rp.resx + 15) / 16;
@@ -865,11 +879,18 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
     if (rc) return rc;
     if ((rc = readback_guard(ctx, "the tiered canvas"))) return rc;
     // Slots of the mixed blocks: as many as the outlines can make when that is
-    // little memory (no wait for the device), else the exact number, read back.
+    // little memory and the budget holds it (no wait for the device), else the
+    // exact number, read back.
     bool label = !bounds && !(q->flags & RJ_FLAG_FORCE_CANVAS) && !known_overlap(ctx, rp, ckey) &&
                  ctx->ps->P <= kMaxLabelPolys;
     const size_t bound = tier_slot_bound(*ctx->ps, rp, nblk, bounds);
-    const bool exact = ctx->exact_slots || bound * 256 * (f.aggr ? 12 : 4) > kSlotBytes;
+    const bool canvas = !label || ctx->ps->overlap_on(ckey) != 0;   // taken, or possible
+    exact = exact || bound * 256 * (f.aggr ? 12 : 4) > kSlotBytes ||
+            !budget_holds(ctx, {{"tier_plabel", label ? bound * 512 : 0},
+                                {"tier_bcnt", canvas ? nblk * 4 : 0},
+                                {"tier_pcnt", canvas ? bound * 1024 : 0},
+                                {"tier_bsum", canvas && f.aggr ? nblk * 8 : 0},
+                                {"tier_psum", canvas && f.aggr ? bound * 2048 : 0}});
     tr.cap = exact ? 0x7FFFFFFFu : (uint32_t)bound;
     launch_tier_codes(tr, nblk, cnt, ctx->q_err, ctx->sms, ctx->stream);
     uint32_t nslots = (uint32_t)bound;
@@ -939,6 +960,22 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
     }
     es.ph->mark(4);
     return RJ_OK;
+}
+
+int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const DevFilter& f, ExecState& es,
+                     PolyPassArgs& a, const CanvasXf& cx, uint64_t ckey, bool bounds) {
+    bool exact = ctx->exact_slots;
+    const int rc = tier_attempt(ctx, q, rp, f, es, a, cx, ckey, bounds, exact);
+    if (rc != RJ_E_OOM || exact) return rc;
+    // no room for as many slots as there can be (nothing was counted yet): once
+    // more with as many as there are
+    for (const char* key : {"tier_plabel", "tier_pcnt", "tier_psum"}) {
+        DevBuf& b = scratch_buf(ctx, key);
+        if (b.plans.empty()) dev_free(ctx, b);
+    }
+    ctx->err.clear();
+    exact = true;
+    return tier_attempt(ctx, q, rp, f, es, a, cx, ckey, bounds, exact);
 }
 
 // Polygon pass over a point canvas (MODE_REDUCE, MODE_BOUNDS): its rows become
