@@ -309,6 +309,11 @@ RJ_API int rj_column_absmax(const rj_ctx *ctx, int32_t attrib_id, double *out);
  *   RJ_TUNE_HYBRID_SHAPES    (read only) number of shapes of the lean pass
  *                            of the hybrid and index joins; RJ_TUNE_COUNT_SHAPE
  *                            indexes them there
+ *   RJ_TUNE_TIER_SLOTS       tiered canvases: pixel slots taken for the blocks
+ *                            on outlines without reading their number back.
+ *                            -1 = as many as the outlines can make, else at
+ *                            most this many; a query that needs more runs
+ *                            again with the exact number
  *   RJ_TUNE_WAIT_LIMIT       microseconds a bounded device wait of the
  *                            bulk-copy pipeline (RJ_TUNE_POINT_SHAPE 2) may
  *                            take before it gives up and the call returns
@@ -326,6 +331,7 @@ RJ_API int rj_column_absmax(const rj_ctx *ctx, int32_t attrib_id, double *out);
 #define RJ_TUNE_WAIT_LIMIT         6
 #define RJ_TUNE_SPLAT_SHAPES       7
 #define RJ_TUNE_HYBRID_SHAPES      8
+#define RJ_TUNE_TIER_SLOTS         9
 RJ_API int rj_set_tuning(rj_ctx *ctx, int32_t knob, int32_t value);
 RJ_API int rj_get_tuning(const rj_ctx *ctx, int32_t knob, int32_t *value);
 

@@ -160,6 +160,7 @@ struct rj_ctx {
     int point_shape = -1;
     int count_shape = -1, count_bshift = -1;
     int hybrid_exact_scale = 1;
+    int tier_slots = -1;             // most slots a tiered canvas takes unread, -1 = by the outlines
     uint64_t wait_ns = rj::kWaitLimitNs;   // bound of the pipeline's device waits
     int last_count_shape = -1, last_count_bshift = -1;
     // exact partial sums of the last query (rj_get_sum_partials)

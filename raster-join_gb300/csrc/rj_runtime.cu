@@ -883,7 +883,8 @@ int tier_attempt(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const Dev
     // exact number, read back.
     bool label = !bounds && !(q->flags & RJ_FLAG_FORCE_CANVAS) && !known_overlap(ctx, rp, ckey) &&
                  ctx->ps->P <= kMaxLabelPolys;
-    const size_t bound = tier_slot_bound(*ctx->ps, rp, nblk, bounds);
+    size_t bound = tier_slot_bound(*ctx->ps, rp, nblk, bounds);
+    if (ctx->tier_slots >= 0) bound = std::min(bound, (size_t)ctx->tier_slots);
     const bool canvas = !label || ctx->ps->overlap_on(ckey) != 0;   // taken, or possible
     exact = exact || bound * 256 * (f.aggr ? 12 : 4) > kSlotBytes ||
             !budget_holds(ctx, {{"tier_plabel", label ? bound * 512 : 0},
@@ -906,9 +907,11 @@ int tier_attempt(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const Dev
         if ((rc = poly_pass(ctx, MODE_TIER_LABEL, a, &tr, true))) return rc;
         if (ctx->ps->overlap_on(ckey) == -1) {
             launch_tier_nonempty(tr, nblk, cnt + 2, ctx->sms, ctx->stream);
-            unsigned long long hc[3] = {0, 0, 0};
+            unsigned long long hc[4] = {0, 0, 0, 0};
             RJ_CUDA(cudaMemcpyAsync(hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, ctx->stream));
             RJ_CUDA(cudaStreamSynchronize(ctx->stream));
+            // (blocks without a slot are in neither count: no verdict without them)
+            if ((uint32_t)hc[3] > tr.cap) return fail(ctx, RJ_E_OOM, "more blocks on outlines than slots");
             ctx->ps->overlap[ckey] = (hc[0] != 0 || hc[1] != hc[2]) ? 1 : 0;
         }
         label = ctx->ps->overlap_on(ckey) == 0;
@@ -967,8 +970,9 @@ int exec_raster_tier(rj_ctx* ctx, const rj_query* q, const RasterPlan& rp, const
     bool exact = ctx->exact_slots;
     const int rc = tier_attempt(ctx, q, rp, f, es, a, cx, ckey, bounds, exact);
     if (rc != RJ_E_OOM || exact) return rc;
-    // no room for as many slots as there can be (nothing was counted yet): once
-    // more with as many as there are
+    // no room for as many slots as there can be, or too few of them for the
+    // overlap check (nothing was counted yet): once more with as many as there are
+    RJ_CUDA(cudaMemsetAsync(ctx->q_err, 0, sizeof(int), ctx->stream));
     for (const char* key : {"tier_plabel", "tier_pcnt", "tier_psum"}) {
         DevBuf& b = scratch_buf(ctx, key);
         if (b.plans.empty()) dev_free(ctx, b);
@@ -2814,6 +2818,10 @@ int rj_set_tuning(rj_ctx* ctx, int32_t knob, int32_t value) {
             if (value < 1) return fail(ctx, RJ_E_INVALID, "wait limit %d us: at least 1", value);
             ctx->wait_ns = (uint64_t)value * 1000ull;
             return RJ_OK;
+        case RJ_TUNE_TIER_SLOTS:
+            if (value < -1) return fail(ctx, RJ_E_INVALID, "tier slots %d: -1 or more", value);
+            ctx->tier_slots = value;
+            return RJ_OK;
         case RJ_TUNE_HYBRID_EXACT_SCALE:
             if (value != 1 && value != 2 && value != 4)
                 return fail(ctx, RJ_E_INVALID, "hybrid exact scale %d: 1, 2 or 4", value);
@@ -2836,6 +2844,7 @@ int rj_get_tuning(const rj_ctx* ctx, int32_t knob, int32_t* value) {
         case RJ_TUNE_LEAN_SHAPES: *value = label_shapes(); return RJ_OK;
         case RJ_TUNE_SPLAT_SHAPES: *value = splat_lean_shapes(); return RJ_OK;
         case RJ_TUNE_HYBRID_SHAPES: *value = hybrid_lean_shapes(); return RJ_OK;
+        case RJ_TUNE_TIER_SLOTS: *value = ctx->tier_slots; return RJ_OK;
         case RJ_TUNE_WAIT_LIMIT: *value = (int32_t)std::min<uint64_t>(ctx->wait_ns / 1000ull, 0x7FFFFFFFull); return RJ_OK;
         default: return RJ_E_INVALID;
     }
