@@ -918,7 +918,7 @@ int lanes_finish(Engine& e, LaneRun& lr) {
         if (p.status != RJ_OK) continue;
         const char* b = h + lr.off[i];
         if (const int derr = *(const int*)(b + QueryOut((size_t)p.ps->P, lr.bounds[i]).err)) {
-            if (derr == kErrSlots) {   // run again alone (rj_execute reads the number of slots back)
+            if (derr & kErrSlots) {   // run again alone (rj_execute reads the number of slots back)
                 p.status = RJ_E_OOM;
                 continue;
             }

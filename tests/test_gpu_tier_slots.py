@@ -58,3 +58,32 @@ def test_short_of_slots(built, slots, overlap):
             h.setTuning(rj.TUNE_TIER_SLOTS, -2)
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("slots", [0, 1])
+@pytest.mark.parametrize("overlap", [False, True])
+def test_batch_short_of_slots(built, slots, overlap):
+    """Batched queries run again alone, error bounds too (whose outline pass
+    reads blocks that have no slot)."""
+    verts, pidx, xy = _set(overlap)
+    want = oracle.raster_join(xy, verts, pidx, 1.0, max_res=1500, bounds=True)
+    h = rj.GLHandler()
+    try:
+        dh = rj.DataHandler()
+        dh.add_column(1, rj.Location, xy)
+        dh.setPolygons(verts, pidx)
+        h.setDataHandler(dh)
+        h.setCellSize(1.0)
+        h.max_fbo_size = 1500
+        h.flags = rj.FLAG_TIERED_CANVAS
+        h.setTuning(rj.TUNE_TIER_SLOTS, slots)
+        fns = [rj.RasterJoinBoundFn, rj.RasterJoinFn, rj.RasterJoinBoundFn, rj.RasterJoinFn]
+        h.upload()
+        got, status, _ = h.execute_batch([h.make_query(fn) for fn in fns], [None] * len(fns))
+        assert not np.any(status)
+        for fn, g in zip(fns, got):
+            np.testing.assert_array_equal(g.count, want[0])
+            if fn == rj.RasterJoinBoundFn:
+                np.testing.assert_array_equal(g.bounds, want[2])
+    finally:
+        h.close()
