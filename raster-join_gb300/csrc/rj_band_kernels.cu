@@ -183,11 +183,17 @@ __device__ bool compute_fraction(float x0, float y0, float x1, float y1,
 constexpr int kBW = 8;             // warps per block
 constexpr int kBEdges = 128;       // staged edges per warp
 constexpr int kBCross = 512;       // crossings held per warp (rows of the band taken in groups that fit)
+// Bits of a column beside the four of a band's row.  A hybrid canvas can be far
+// wider than a raster tile's 8192 pixels; from 31 * 2^22 columns on its border
+// radius, at least columns * 2^-22, is refused.
+constexpr int kColBits = 28;
+constexpr uint32_t kColMask = (1u << kColBits) - 1u;
+static_assert(kBand <= 1 << (32 - kColBits), "a band's rows fit beside the column");
 
 struct BandWarp {
     int4 edge[kBEdges];
     int eidx[kBEdges];
-    uint32_t cross[kBCross];       // crossing column, clamped to the polygon's columns, | row << 16
+    uint32_t cross[kBCross];       // crossing column, clamped to the polygon's columns, | row << kColBits
     int start[kBand + 1];          // first crossing of each row
     int cur[kBand];                // crossings of each row
 };
@@ -369,7 +375,7 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPa
                     const int32_t cy = (jb + r) * kSub + kSub / 2;
                     if (r < max(ra, cl) || r >= rb || r > ch || !cross_row(q.y, q.w, cy)) return;
                     const int L = max(min(max(cross_L(q.x, q.y, q.z, q.w, cy), i_lo), i_hi + 1), 0);
-                    S.cross[S.start[r] - base + atomicAdd(&S.cur[r], 1)] = (uint32_t)L | ((uint32_t)r << 16);
+                    S.cross[S.start[r] - base + atomicAdd(&S.cur[r], 1)] = (uint32_t)L | ((uint32_t)r << kColBits);
                 });
             }
             __syncwarp();
@@ -377,7 +383,7 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPa
                 if (!slow) {
                     for (int x = lane; x < m; x += 32) {
                         const uint32_t mine = S.cross[x];
-                        const int r = (int)(mine >> 16), L = (int)(mine & 0xFFFFu);
+                        const int r = (int)(mine >> kColBits), L = (int)(mine & kColMask);
                         const int f = S.start[r] - base, e = f + S.cur[r];
                         bool odd = false;
                         for (int k = f; k < e; ++k) {
@@ -462,7 +468,7 @@ __global__ void __launch_bounds__(kBW * 32, OUTLINE ? 3 : 4) k_poly_bands(PolyPa
                                 if (slow) inside = inside_slow(i, r);
                                 else
                                     for (int c = S.start[r] - base, e = c + S.cur[r]; c < e; ++c)
-                                        inside ^= (int)(S.cross[c] & 0xFFFFu) > i;
+                                        inside ^= (int)(S.cross[c] & kColMask) > i;
                             }
                             if (frac > 0.5f) frac = __fsub_rn(1.0f, frac);
                             const int add = (int)ceilf(__fmul_rn(frac, (float)val));
