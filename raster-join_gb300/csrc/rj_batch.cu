@@ -1325,7 +1325,7 @@ int rj_cluster_points(rj_ctx* ctx, int32_t attrib, int32_t nbuckets, int32_t cel
         const size_t esz = col.type == RJ_LOCATION ? 8 : 4;
         const size_t bytes = esz * ((n + 3) & ~3ULL) + 256;
         if (ctx->budget > 0 && (int64_t)(ctx->used + bytes) > ctx->budget) ce = cudaErrorMemoryAllocation;
-        else ce = cudaMalloc(&fresh[c], bytes);
+        else ce = dev_malloc(ctx, &fresh[c], bytes);
         if (ce != cudaSuccess) {
             cudaGetLastError();
             for (void* p : fresh)

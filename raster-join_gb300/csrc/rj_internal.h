@@ -230,6 +230,7 @@ inline bool query_tier(uint32_t flags, size_t npix, uint64_t rows) {
 }
 
 int fail(rj_ctx* c, int code, const char* fmt, ...);
+cudaError_t dev_malloc(rj_ctx* ctx, void** p, size_t bytes);
 
 // A query's outputs: one block, zeroed by one memset and read back by one
 // copy: count[P], fixed-point sum[P], non-finite sum[P], the status word, then

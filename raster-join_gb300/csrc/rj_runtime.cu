@@ -48,6 +48,17 @@ int readback_guard(rj_ctx* ctx, const char* what) {
     return RJ_OK;
 }
 
+// cudaMalloc; when there is no room, what a query can do without gives way.
+cudaError_t dev_malloc(rj_ctx* ctx, void** p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess || ctx->capturing) return e;
+    const auto spare = ctx->scratch.find("splat_bins");
+    if (spare == ctx->scratch.end() || !spare->second.p) return e;
+    cudaGetLastError();
+    dev_free(ctx, spare->second);
+    return cudaMalloc(p, bytes);
+}
+
 int dev_alloc(rj_ctx* ctx, DevBuf& b, size_t bytes) {
     if (b.p && b.bytes >= bytes) return RJ_OK;
     if (b.p) {
@@ -61,15 +72,7 @@ int dev_alloc(rj_ctx* ctx, DevBuf& b, size_t bytes) {
     if (ctx->budget > 0 && (int64_t)(ctx->used + bytes) > ctx->budget)
         return fail(ctx, RJ_E_OOM, "device memory budget exceeded: need %zu more bytes, %zu of %lld in use",
                     bytes, (size_t)ctx->used.load(), (long long)ctx->budget);
-    cudaError_t e = cudaMalloc(&b.p, bytes);
-    if (e != cudaSuccess && !ctx->capturing) {   // what a query can do without gives way
-        cudaGetLastError();
-        const auto spare = ctx->scratch.find("splat_bins");
-        if (spare != ctx->scratch.end() && spare->second.p && &spare->second != &b) {
-            dev_free(ctx, spare->second);
-            e = cudaMalloc(&b.p, bytes);
-        }
-    }
+    const cudaError_t e = dev_malloc(ctx, &b.p, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         b.p = nullptr;
@@ -1286,14 +1289,18 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
             if (sm > 0 && sm <= 200 * 1024) cands.push_back(sh);
         }
     // the pass through bins (rj_splat_bins.cu): its scratch is optional, so it is
-    // left alone under a memory budget and inside a capture
+    // left alone under a memory budget and inside a capture, and only held for
+    // a query class whose kept choice it is
     void* bin_scratch = nullptr;
-    const bool force_bins = ctx->count_shape == kSplatBins;
-    if ((force_bins || (ctx->count_shape < 0 && a.n >= kBinMinPoints)) && ctx->budget <= 0 && !ctx->capturing &&
-        ctx->scratch_ns.empty() && splat_bins_fit(rp.resx, rp.resy, ctx->sms, agg) &&
-        scratch(ctx, "splat_bins", splat_bins_bytes(rp.resx, rp.resy, ctx->sms, a.n), &bin_scratch) != RJ_OK)
+    const auto take_bins = [&] {
+        if (scratch(ctx, "splat_bins", splat_bins_bytes(rp.resx, rp.resy, ctx->sms, a.n), &bin_scratch) == RJ_OK) return true;
+        ctx->err.clear();
         bin_scratch = nullptr;
-    if (force_bins && bin_scratch) {
+        return false;
+    };
+    const bool may_bin = ctx->budget <= 0 && !ctx->capturing && ctx->scratch_ns.empty() &&
+                         splat_bins_fit(rp.resx, rp.resy, ctx->sms, agg);
+    if (ctx->count_shape == kSplatBins && may_bin && take_bins()) {
         ctx->passes = 1;
         ctx->copy_ms = 0;
         if (!launch_splat_bins(a, lc, bin_scratch, ctx->sms, ctx->stream)) return RJ_OK;
@@ -1318,15 +1325,19 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
     });
     // that shape or the bins, again per query class
     int bins = 0;
-    if (pi >= 0 && bin_scratch) {
+    if (pi >= 0 && ctx->count_shape < 0 && a.n >= kBinMinPoints && may_bin) {
         std::snprintf(key, sizeof key, "bins:%d:%d:%d", lc.ncol, tune_bucket((double)npix), tune_bucket((double)a.n));
-        bins = tune_pick(ctx, key, 2, [&](size_t i, uint64_t most) {
-            timed_any = true;
-            SplatLeanArgs b = a;
-            b.n = std::min<uint64_t>(a.n & ~1ULL, most);
-            return i ? launch_splat_bins(b, lc, bin_scratch, ctx->sms, ctx->stream)
-                     : launch_splat_lean(cands[(size_t)pi], b, lc, ctx->sms, ctx->stream);
-        });
+        const bool settled = tuned_get(ctx, key, &bins);
+        if (!settled || bins == 1) bins = 0, take_bins();
+        if (bin_scratch)
+            bins = tune_pick(ctx, key, 2, [&](size_t i, uint64_t most) {
+                timed_any = true;
+                SplatLeanArgs b = a;
+                b.n = std::min<uint64_t>(a.n & ~1ULL, most);
+                return i ? launch_splat_bins(b, lc, bin_scratch, ctx->sms, ctx->stream)
+                         : launch_splat_lean(cands[(size_t)pi], b, lc, ctx->sms, ctx->stream);
+            });
+        if (bin_scratch && bins != 1) dev_free(ctx, scratch_buf(ctx, "splat_bins"));
     }
     RJ_CUDA(cudaGetLastError());
     if (timed_any) {
@@ -2439,7 +2450,7 @@ static int load_points_impl(rj_ctx* ctx, const rj_column* cols, int32_t ncols, u
                 ctx->cols.clear();
                 return fail(ctx, RJ_E_OOM, "point table exceeds the device memory budget");
             }
-            cudaError_t e = cudaMalloc(&c.d, bytes);
+            cudaError_t e = dev_malloc(ctx, &c.d, bytes);
             if (e != cudaSuccess) {
                 cudaGetLastError();
                 for (Column& o : ctx->cols) if (o.owned) cudaFree(o.d);
