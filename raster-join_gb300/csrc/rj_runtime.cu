@@ -1079,6 +1079,13 @@ bool lean_cols_of(const PointArgs& pa, unsigned long long* out_sum, LeanCols& lc
 
 // Autotuned choices per device and query class, shared by every context of
 // the process: a choice depends on the GPU and the class, not on the context.
+// The choice is an index into the class's candidates, which follow from exact
+// sizes where the rest of a key only holds octaves: the key names them too.
+uint64_t cands_key(const std::vector<std::pair<int, int>>& cands) {
+    uint64_t h = 1469598103934665603ULL;   // FNV-1a
+    for (const auto& c : cands) h = (h ^ (uint64_t)(c.first * 256 + c.second)) * 1099511628211ULL;
+    return h;
+}
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tuned;
 bool tuned_get(const rj_ctx* ctx, const std::string& key, int* v) {
@@ -1187,9 +1194,9 @@ int hybrid_lean_pass(rj_ctx* ctx, const DevFilter& f, int mode, const HybXf& h, 
             }
     if (cands.empty()) return RJ_OK;
     char key[200];
-    std::snprintf(key, sizeof key, "hybq:%d:%d:%d:%d:%d:%d:%d:%d:%d", mode, lc.ncol, lc.aggr, lc.aggr_ci >= 0,
+    std::snprintf(key, sizeof key, "hybq:%d:%d:%d:%d:%d:%d:%d:%d:%d:%llx", mode, lc.ncol, lc.aggr, lc.aggr_ci >= 0,
                   tune_bucket((double)P), tune_bucket((double)resx * resy), tune_bucket((double)a.n), ctx->count_shape,
-                  ctx->count_bshift);
+                  ctx->count_bshift, (unsigned long long)cands_key(cands));
     int tuned_i = -1;
     const bool have = tuned_get(ctx, key, &tuned_i);
     const bool small = a.n < kTuneMinPoints;
@@ -1311,8 +1318,10 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
     }
     if (cands.empty()) return RJ_OK;
     char key[200];
-    std::snprintf(key, sizeof key, "splat:%d:%d:%d:%d:%d:%d", lc.ncol, lc.aggr, lc.aggr_ci >= 0,
-                  tune_bucket((double)npix), tune_bucket((double)a.n), ctx->count_shape);
+    std::vector<std::pair<int, int>> named;
+    for (int sh : cands) named.push_back({sh, 0});
+    std::snprintf(key, sizeof key, "splat:%d:%d:%d:%d:%d:%d:%llx", lc.ncol, lc.aggr, lc.aggr_ci >= 0,
+                  tune_bucket((double)npix), tune_bucket((double)a.n), ctx->count_shape, (unsigned long long)cands_key(named));
     int tuned_i = -1;
     const bool have = tuned_get(ctx, key, &tuned_i);
     const bool small = a.n < kTuneMinPoints;
@@ -1468,9 +1477,11 @@ bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, co
                 lp.cands.push_back({sh, (int)k});
     if (lp.cands.empty()) return false;
     lp.small = a.n < kTuneMinPoints;
-    std::snprintf(lp.key, sizeof lp.key, "label:%d:%d:%d:%d:%d:%d:%d:%d:%d", lp.lc.ncol, lp.lc.aggr, lp.lc.aggr_ci >= 0,
+    std::vector<std::pair<int, int>> named;   // (shape, side in pixels for blocks, else finer or coarser)
+    for (const auto& c : lp.cands) named.push_back({c.first, lp.tile ? lp.sides[(size_t)c.second].shift : c.second});
+    std::snprintf(lp.key, sizeof lp.key, "label:%d:%d:%d:%d:%d:%d:%d:%d:%d:%llx", lp.lc.ncol, lp.lc.aggr, lp.lc.aggr_ci >= 0,
                   rp.splitx * rp.splity > 1, tune_bucket((double)a.P), tune_bucket(npx), tune_bucket((double)a.n),
-                  ctx->count_shape, ctx->count_bshift);
+                  ctx->count_shape, ctx->count_bshift, (unsigned long long)cands_key(named));
     lp.have = tuned_get(ctx, lp.key, &lp.tuned);
     return true;
 }
