@@ -296,6 +296,7 @@ struct TileAxis {
     int split, res;              // tiles, pixels of a tile
     float s, H;                  // scale, 256 * half resolution
     float lb, inv_td;            // canvas edge, 1 / tile extent (for the tile guess)
+    int edge;                    // a point at least this many pixels inside a tile lies in no other
 };
 struct LabelPointArgs {
     const float4* xy;            // location column as point pairs, 16-byte aligned

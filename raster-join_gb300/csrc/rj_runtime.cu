@@ -1371,7 +1371,15 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
 bool tile_axis(const std::vector<float4>& xf, const float4* dxf, int res, float lb, TileAxis& x) {
     for (const float4& t : xf)
         if (t.x != xf[0].x || t.z != xf[0].z) return false;
-    x = TileAxis{dxf, (int)xf.size(), res, xf[0].x, xf[0].z * (float)kSub, lb, (float)(1.0 / (double)xf[0].w)};
+    // Two tiles place a point apart by the roundings of their offsets: of the
+    // origin and of the product, each 2^-24 of the offset.  Below a pixel (a
+    // canvas within some 4 million pixels of the origin) points a pixel inside a
+    // tile are in that one alone.
+    double t = 0;
+    for (const float4& f : xf) t = std::max(t, std::fabs((double)f.y));
+    const double apart = 4.0 * (double)xf[0].z * t * std::ldexp(1.0, -24) + 0.01;
+    const int edge = (int)std::min(std::max(std::ceil(apart), 1.0), 65536.0);
+    x = TileAxis{dxf, (int)xf.size(), res, xf[0].x, xf[0].z * (float)kSub, lb, (float)(1.0 / (double)xf[0].w), edge};
     return true;
 }
 

@@ -7,9 +7,9 @@
 // (rj_lean.cuh), no warp grouping.
 //
 // Tiles: per axis the tile is guessed with one multiplication; when the
-// pixel in the guessed tile lies at least one pixel inside it, no other tile's
-// window can hold the point and that is the only hit.  Otherwise (within a
-// pixel of a seam, or a guess off by one) the guessed tile and both
+// pixel in the guessed tile lies far enough inside it (TileAxis::edge, one pixel
+// unless the canvas is far from the origin), no other tile's window can hold the
+// point and that is the only hit.  Otherwise (near a seam, or a guess off by one) the guessed tile and both
 // neighbours are tried exactly, as the generic mapping does: near a seam a
 // point can fall in two tiles' windows and counts in both (every tile is
 // rendered with all points, RasterJoin.cpp:224-231).

@@ -1,0 +1,49 @@
+"""Tiled canvases so far from the origin (in pixels) that fp32 moves a point by
+whole pixels: neighbouring tiles disagree on where it lies by more than a pixel.
+Points around the seams and the rim, every form, against the oracle."""
+import numpy as np
+import pytest
+
+import oracle
+import rasterjoin as rj
+from rasterjoin import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(handler, lo, ext, fbo, seams):
+    verts, pidx = synth.voronoi_polygons(40, seed=5, box=ext, verts_per_poly=30, jitter=5.0)
+    verts = (verts.astype(np.float64) + lo).astype(np.float32)
+    bb = np.r_[verts.min(0), verts.max(0)].astype(np.float64)
+    rng = np.random.default_rng(fbo)
+    xy = rng.uniform(bb[:2] - 30, bb[2:] + 30, (150_001, 2))
+    split = int(np.ceil(np.ceil(ext) / fbo))
+    for k in range(2):
+        i = slice(k * 50_000, (k + 1) * 50_000)
+        at = rng.integers(0, split + 1, 50_000) if seams else rng.choice([0, split], 50_000)
+        xy[i, k] = bb[k] + at * (bb[2 + k] - bb[k]) / split + rng.uniform(-14, 14, 50_000)
+    xy = xy.astype(np.float32)
+    dh = rj.DataHandler()
+    dh.add_column(1, rj.Location, xy)
+    dh.setPolygons(verts, pidx)
+    handler.setDataHandler(dh)
+    handler.setCellSize(1.0)
+    handler.max_fbo_size = fbo
+    want = oracle.raster_join(xy, verts, pidx, 1.0, max_res=fbo, bounds=True)
+    assert want[0].sum() > 50_000
+    try:
+        for fn, flag in ((rj.RasterJoinFn, 0), (rj.RasterJoinFn, rj.FLAG_FORCE_CANVAS), (rj.RasterJoinBoundFn, 0)):
+            handler.flags = rj.FLAG_TIERED_CANVAS | flag
+            got = handler.execute(fn)
+            assert handler.getTuning(rj.TUNE_COUNT_SHAPE) >= 0      # a lean pass ran
+            np.testing.assert_array_equal(got.count, want[0])
+        np.testing.assert_array_equal(got.bounds, want[2])
+    finally:
+        handler.flags = 0
+        handler.max_fbo_size = 8192
+
+
+@pytest.mark.parametrize("lo,ext,fbo", [((9565671.0, 9565671.0), 8850.0, 943), ((500000.0, 4100000.0), 6000.0, 1700),
+                                        ((-10160196.0, 4100000.0), 8718.0, 1679), ((36316732.0, -36316732.0), 5064.0, 876)])
+def test_seams(handler, lo, ext, fbo):
+    _run(handler, np.asarray(lo), ext, fbo, True)
