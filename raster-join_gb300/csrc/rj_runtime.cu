@@ -1416,29 +1416,31 @@ bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, co
         double e = 0;
         for (const float4& t : xf)
             e = std::max(e, (double)t.z * (6.0 * std::fabs((double)t.x) * std::max(std::fabs(lo), std::fabs(hi)) + 16.0));
-        e = e * std::ldexp(1.0, -23) + 1.0 / 256.0;
-        return e < 0.5 ? e : 1e30;
+        return e * std::ldexp(1.0, -23) + 1.0 / 256.0;
     };
-    lp.errx = err_of(rp.colxf, bb[0], bb[2]);
-    lp.erry = err_of(rp.rowxf, bb[1], bb[3]);
+    const double ex = err_of(rp.colxf, bb[0], bb[2]), ey = err_of(rp.rowxf, bb[1], bb[3]);
+    lp.errx = ex < 0.5 ? ex : 1e30;
+    lp.erry = ey < 0.5 ? ey : 1e30;
     // Cell sides: about 64k or 16k cells (128 KB or 32 KB of codes), at least
     // 4 pixels.  Small scans take the coarse map, whose load they feel.
     const double px = (bb[2] - bb[0]) / ((double)rp.resx * rp.splitx), py = (bb[3] - bb[1]) / ((double)rp.resy * rp.splity);
     const double npx = (double)rp.resx * rp.splitx * rp.resy * rp.splity;
-    // cells of one axis: `side` pixels each, covering [lo, hi] and two pixels
-    // beyond; index = round(v * ca + o) with an integer offset o
-    auto axis = [](double lo, double hi, double pixel, double side, float* ca, float* cc, int* n, double* o) {
+    // cells of one axis: `side` pixels each, covering [lo, hi] and beyond it what
+    // the pixels' error can bring onto the canvas, and two pixels; index =
+    // round(v * ca + o) with an integer offset o
+    auto axis = [](double lo, double hi, double pixel, double err, double side, float* ca, float* cc, int* n, double* o) {
+        const double beyond = (2.0 + err) * pixel;
         *ca = (float)(1.0 / (side * pixel));
-        *o = std::ceil(-0.5 - (lo - 2.0 * pixel) * (double)*ca);
-        const double m = std::floor((hi + 2.0 * pixel) * (double)*ca + *o + 0.5) + 1.0;
+        *o = std::ceil(-0.5 - (lo - beyond) * (double)*ca);
+        const double m = std::floor((hi + beyond) * (double)*ca + *o + 0.5) + 1.0;
         *cc = (float)(12582912.0 + *o);   // an integer below 2^24: exact
         *n = (int)std::min(m, 1e6);
         return std::fabs(*o) + m < (double)(1 << 21);
     };
     auto add_side = [&](double side, int shift) {
         LabelPlan::Side d{a, 0, 0, shift};
-        if (!axis(bb[0], bb[2], px, side, &d.a.cax, &d.a.ccx, &d.a.cnx, &d.ox) ||
-            !axis(bb[1], bb[3], py, side, &d.a.cay, &d.a.ccy, &d.a.cny, &d.oy))
+        if (!axis(bb[0], bb[2], px, ex, side, &d.a.cax, &d.a.ccx, &d.a.cnx, &d.ox) ||
+            !axis(bb[1], bb[3], py, ey, side, &d.a.cay, &d.a.ccy, &d.a.cny, &d.oy))
             return;
         const long long cells = (long long)(d.a.cnx + 1) * (d.a.cny + 1);
         if (cells > 100 * 1024) return;

@@ -11,8 +11,8 @@ from rasterjoin import synth
 pytestmark = pytest.mark.gpu
 
 
-def _run(handler, lo, ext, fbo, seams):
-    verts, pidx = synth.voronoi_polygons(40, seed=5, box=ext, verts_per_poly=30, jitter=5.0)
+def _run(handler, lo, ext, fbo, polygons):
+    verts, pidx = polygons
     verts = (verts.astype(np.float64) + lo).astype(np.float32)
     bb = np.r_[verts.min(0), verts.max(0)].astype(np.float64)
     rng = np.random.default_rng(fbo)
@@ -20,8 +20,7 @@ def _run(handler, lo, ext, fbo, seams):
     split = int(np.ceil(np.ceil(ext) / fbo))
     for k in range(2):
         i = slice(k * 50_000, (k + 1) * 50_000)
-        at = rng.integers(0, split + 1, 50_000) if seams else rng.choice([0, split], 50_000)
-        xy[i, k] = bb[k] + at * (bb[2 + k] - bb[k]) / split + rng.uniform(-14, 14, 50_000)
+        xy[i, k] = bb[k] + rng.integers(0, split + 1, 50_000) * (bb[2 + k] - bb[k]) / split + rng.uniform(-14, 14, 50_000)
     xy = xy.astype(np.float32)
     dh = rj.DataHandler()
     dh.add_column(1, rj.Location, xy)
@@ -46,4 +45,14 @@ def _run(handler, lo, ext, fbo, seams):
 @pytest.mark.parametrize("lo,ext,fbo", [((9565671.0, 9565671.0), 8850.0, 943), ((500000.0, 4100000.0), 6000.0, 1700),
                                         ((-10160196.0, 4100000.0), 8718.0, 1679), ((36316732.0, -36316732.0), 5064.0, 876)])
 def test_seams(handler, lo, ext, fbo):
-    _run(handler, np.asarray(lo), ext, fbo, True)
+    _run(handler, np.asarray(lo), ext, fbo, synth.voronoi_polygons(40, seed=5, box=ext, verts_per_poly=30, jitter=5.0))
+
+
+@pytest.mark.parametrize("lo,ext,fbo", [(38799352.0, 6547.0, 1176), (54720284.0, 6241.0, 2055), (50627588.0, 7458.0, 784),
+                                        (60792624.0, 4212.0, 685), (53300116.0, 4468.0, 752), (40853684.0, 8358.0, 1197)])
+def test_rim(handler, lo, ext, fbo):
+    """Points four metres (pixels) off the canvas that fp32 puts on it, in
+    extents where the coarse cells end right there; strips up to the rim."""
+    x = np.linspace(0.0, ext, 9)
+    strips = np.concatenate([[(a, 0), (b, 0), (b, ext), (a, ext)] for a, b in zip(x[:-1], x[1:])])
+    _run(handler, np.asarray((lo, lo)), ext, fbo, (strips, 4 * np.arange(9, dtype=np.int32)))
