@@ -1497,8 +1497,8 @@ bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, co
 }
 
 // Builds the cell codes from the canvas's block codes and runs the planned
-// pass.  *done = false: it could not be launched (the caller takes the generic
-// pass).
+// pass.  *done = false: it could not be launched, or there is no memory for the
+// codes (the caller takes the generic pass).
 int run_label_points(rj_ctx* ctx, LabelPlan& lp, const TierArgs& tr, ExecState& es, bool* done) {
     *done = false;
     const auto& cands = lp.cands;
@@ -1514,7 +1514,10 @@ int run_label_points(rj_ctx* ctx, LabelPlan& lp, const TierArgs& tr, ExecState& 
         LabelPlan::Side& d = lp.sides[k];
         d.a.tr = tr;
         uint16_t* cells;
-        if ((rc = scratch_t(ctx, k == 0 ? "label_cells0" : "label_cells1", (size_t)d.a.cell_words * 2, &cells))) return rc;
+        if ((rc = scratch_t(ctx, k == 0 ? "label_cells0" : "label_cells1", (size_t)d.a.cell_words * 2, &cells))) {
+            if (rc == RJ_E_OOM) ctx->err.clear();
+            return rc == RJ_E_OOM ? RJ_OK : rc;
+        }
         if (lp.tile) launch_label_blocks(tr, d.a.bs, d.a.cnx, d.a.cny, d.a.P, cells, ctx->sms, ctx->stream);
         else launch_label_cells(d.a, (float)d.ox, (float)d.oy, (float)lp.errx, (float)lp.erry, cells, ctx->sms, ctx->stream);
         d.a.cells = cells;
@@ -1554,11 +1557,20 @@ int run_label_points(rj_ctx* ctx, LabelPlan& lp, const TierArgs& tr, ExecState& 
     return RJ_OK;
 }
 
-// Label form of a one-tile canvas, for the lean pass: block codes, and the
-// pixel labels of the mixed blocks alone, each at its own place (slot = block:
-// no scan, no readback, no map to clear).  *overlap = true: some pixel centre
-// lies in two polygons (the caller takes the canvas path); else *done tells
-// whether the point pass ran.
+// Gives back the memory of the label form's blocks, but what a plan's graph holds.
+void drop_label_blocks(rj_ctx* ctx) {
+    if (ctx->capturing) return;
+    for (const char* key : {"tier_blocks", "tier_code", "tier_plabel", "label_cells0", "label_cells1"}) {
+        DevBuf& b = scratch_buf(ctx, key);
+        if (b.plans.empty()) dev_free(ctx, b);
+    }
+}
+
+// Label form of a one-tile canvas: block codes, and the pixel labels of the
+// mixed blocks alone, each at its own place (slot = block: no scan, no
+// readback, no map to clear), then the point pass.  *overlap = true: some pixel
+// centre lies in two polygons and nothing was counted (the caller takes the
+// canvas path).
 int label_blocks(rj_ctx* ctx, const DevFilter& f, const CanvasXf& cx, PolyPassArgs& a, uint64_t ckey, LabelPlan& lp,
                  ExecState& es, bool* overlap) {
     int rc;
@@ -1701,9 +1713,19 @@ int exec_raster(rj_ctx* ctx, const rj_query* q, ExecState& es, bool bounds) {
     if (use_label) {
         bool overlap = false;
         LabelPlan lp;
-        if (T == 1 && plan_label_points(ctx, f, rp, cx, es, lp)) {
-            if ((rc = label_blocks(ctx, f, cx, a, ckey, lp, es, &overlap))) return rc;
-        } else {
+        bool blocks = T == 1 && plan_label_points(ctx, f, rp, cx, es, lp);
+        if (blocks) {
+            rc = label_blocks(ctx, f, cx, a, ckey, lp, es, &overlap);
+            if (rc == RJ_E_OOM) {   // the flat map takes 3 % less (nothing was counted yet)
+                drop_label_blocks(ctx);
+                ctx->err.clear();
+                ctx->last_count_shape = ctx->last_count_bshift = -1;
+                blocks = false;
+            } else if (rc) {
+                return rc;
+            }
+        }
+        if (!blocks) {
             uint16_t* label;
             int ov = 0;
             if ((rc = label_map(ctx, a, "label", npix, nullptr, 0, ckey, &label, &ov))) return rc;
@@ -1720,6 +1742,7 @@ int exec_raster(rj_ctx* ctx, const rj_query* q, ExecState& es, bool bounds) {
             es.ph->mark(4);
             return RJ_OK;
         }
+        if (ctx->budget > 0) drop_label_blocks(ctx);   // no label form on this canvas from now on
     }
     es.ph->mark(2);
     // canvas path: point pass (additive splat) then polygon pass

@@ -77,3 +77,36 @@ def test_budget_between_exact_and_bound(built, overlap, batch):
     finally:
         free.close()
         tight.close()
+
+
+@pytest.mark.parametrize("overlap,mb", [(False, 124), (True, 368)])
+def test_one_tile_budget_of_the_flat_map(built, overlap, mb):
+    """A budget that holds a flat label map of 8000 x 8000 pixels (128 MB; with
+    the counts of overlapping polygons 384), but not the blocks, which take 3 %
+    more: the query and a plan of it run, equal to those without a budget."""
+    rng = np.random.default_rng(5)
+    polys = [np.array([[x, y], [x + w, y], [x + w, y + w], [x, y + w]]) for x in range(0, 8000, 1000) for y in range(0, 8000, 1000)
+             for w in ((1000, 700) if overlap and (x + y) % 3000 == 0 else (1000,))]
+    verts = np.concatenate(polys).astype(np.float32)
+    pidx = 4 * np.arange(len(polys) + 1, dtype=np.int32)
+    xy = rng.uniform(-10, 8010, (5001, 2)).astype(np.float32)
+    got = []
+    for budget in (0, mb):
+        h = rj.GLHandler(gpu_mem_mb=budget)
+        try:
+            dh = rj.DataHandler()
+            dh.add_column(1, rj.Location, xy)
+            dh.setPolygons(verts, pidx)
+            h.setDataHandler(dh)
+            h.setCellSize(1.0)
+            h.flags = rj.FLAG_FLAT_CANVAS
+            got.append(h.execute(rj.RasterJoinFn))
+            got.append(h.execute(rj.RasterJoinFn))
+            plan = h.prepare(rj.RasterJoinFn)
+            got.append(plan.execute())
+            plan.close()
+        finally:
+            h.close()
+    assert got[0].count.sum() > 4900
+    for g in got[1:]:
+        np.testing.assert_array_equal(g.count, got[0].count)
