@@ -113,7 +113,7 @@ __device__ __forceinline__ void map_points4(const BatchQuery* __restrict__ Q, co
 
 template <class K>
 inline int blocks_per_sm_k(K kernel, int block, size_t smem) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(reinterpret_cast<const void*>(kernel), smem);
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) != cudaSuccess) {
         cudaGetLastError();

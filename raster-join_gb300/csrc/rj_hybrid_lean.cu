@@ -396,7 +396,7 @@ bool launch_hybrid_lean(int shape, const HybLeanArgs& a, const LeanCols& lc_in, 
     lc.copies = hyb_copies(shape, a.P, agg);
     const size_t smem = hybrid_lean_smem(shape, a.code_words, a.P, agg);
     if (smem > (size_t)g_hyb_optin) return false;
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (allow_smem(reinterpret_cast<const void*>(k), smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

@@ -114,7 +114,7 @@ bool launch_label_kernel(LabelKernel k, int block, int nv, size_t smem, const La
         cudaDeviceGetAttribute(&g_label_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     }
     if (smem > (size_t)g_label_optin) return false;
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (allow_smem(reinterpret_cast<const void*>(k), smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

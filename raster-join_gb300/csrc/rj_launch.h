@@ -39,6 +39,10 @@ struct TierArgs {
 
 // Kernels launched by this thread since the last reset (reported per call).
 extern thread_local int g_kernel_launches;
+// Dynamic shared memory a kernel may be launched with.  The limit belongs to the
+// kernel, not to the launch, so it is only ever raised: lowered for one query,
+// it would refuse the launch that another thread is about to make.
+cudaError_t allow_smem(const void* kernel, size_t bytes);
 
 struct PolyPassArgs {
     const int2* wv;              // [T][V] fixed-point window coordinates

@@ -535,8 +535,7 @@ template <class M, bool AGG, bool SMEM, int NG, int BLOCK>
 static void launch_plain_t(const PointArgs& pa, const M& mp, int sms, cudaStream_t st) {
     constexpr int QCAP = BLOCK * (1 + 4 * NG);
     size_t smem = (SMEM ? hist_bytes(pa.P, AGG) : 0) + queue_bytes(M::kDefer, QCAP);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_points<M, AGG, SMEM, NG, BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(reinterpret_cast<const void*>(k_points<M, AGG, SMEM, NG, BLOCK>), smem);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_points<M, AGG, SMEM, NG, BLOCK>, BLOCK, smem);
     if (per_sm < 1) per_sm = 1;
@@ -580,8 +579,7 @@ static bool launch_pipe_t(const PointArgs& pa, const M& mp, int sms, cudaStream_
     if (fixed + 2 * stage_bytes > avail) return false;
     const int stages = (int)std::min<size_t>(4, (avail - fixed) / stage_bytes);
     const size_t smem = fixed + (size_t)stages * stage_bytes;
-    if (cudaFuncSetAttribute(k_points_pipe<M, AGG, SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess) {
+    if (allow_smem(reinterpret_cast<const void*>(k_points_pipe<M, AGG, SMEM>), smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

@@ -11,6 +11,8 @@
 //    (HybridJoin.cpp:197-268) as a conservative supercover + dilation.
 #include <climits>
 #include <cstdio>
+#include <map>
+#include <mutex>
 
 #include "rj_bands.cuh"
 #include "rj_launch.h"
@@ -18,6 +20,21 @@
 namespace rj {
 
 thread_local int g_kernel_launches = 0;
+
+cudaError_t allow_smem(const void* kernel, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> allowed;   // (device, kernel)
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& now = allowed[{dev, kernel}];
+    if (bytes <= now) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) now = bytes;
+    return e;
+}
 
 // ---------------------------------------------------------------------------
 // tile column and row transforms: (sx, tx, hx, -) and (sy, ty, hy, -)
@@ -916,7 +933,7 @@ void launch_poly_info(int mode, const PolyPassArgs& a, int sms, cudaStream_t st)
 
 void launch_poly_label(const PolyPassArgs& a, int sms, cudaStream_t st) {
     ++g_kernel_launches;
-    cudaFuncSetAttribute(k_poly_label, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPolySmem);
+    allow_smem(reinterpret_cast<const void*>(k_poly_label), kPolySmem);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_poly_label, kPolyWarps * 32, kPolySmem);
     k_poly_label<<<sms * std::max(per_sm, 1), kPolyWarps * 32, kPolySmem, st>>>(a);

@@ -303,8 +303,8 @@ size_t splat_bins_bytes(int resx, int resy, int sms, uint64_t n) {
 bool launch_splat_bins(const SplatLeanArgs& a_in, const LeanCols& lc_in, void* scratch, int sms, cudaStream_t st) {
     if (lc_in.ncol < 0 || lc_in.ncol > 4) return false;
     const BinKernel points = bin_kernel(lc_in.ncol);
-    if (cudaFuncSetAttribute(points, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPointSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(k_bin_counts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmem) != cudaSuccess) {
+    if (allow_smem(reinterpret_cast<const void*>(points), kPointSmem) != cudaSuccess ||
+        allow_smem(reinterpret_cast<const void*>(k_bin_counts), kCountSmem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

@@ -237,8 +237,7 @@ bool launch_splat_lean(int shape, const SplatLeanArgs& a, const LeanCols& lc_in,
         if (!lc.copies) return false;
         smem = (size_t)lc.copies * npix * (agg ? 3 : 1) * 4;
         if (smem > (size_t)g_splat_optin) return false;
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        if (allow_smem(reinterpret_cast<const void*>(k), smem) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }

@@ -483,7 +483,7 @@ void launch_tier_pass(int mode, const PolyPassArgs& a, const TierArgs& tr, int s
     ++g_kernel_launches;
     auto go = [&](auto kernel) {
         // every instance needs the opt-in (the three kernels share one pointer type)
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTierSmem);
+        allow_smem(reinterpret_cast<const void*>(kernel), kTierSmem);
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTW * 32, kTierSmem);
         kernel<<<sms * std::max(per_sm, 1), kTW * 32, kTierSmem, st>>>(a, tr);
