@@ -289,6 +289,7 @@ RJ_API int rj_column_absmax(const rj_ctx *ctx, int32_t attrib_id, double *out);
  *                            class on the table itself, the fastest is
  *                            kept), else a shape index
  *                            0..rj_get_tuning(RJ_TUNE_COUNT_SHAPES)-1
+ *                            (larger ones up to 10 are taken, and autotuned)
  *   RJ_TUNE_COUNT_BLOCK_SHIFT code map of that pass: -1 = autotuned, else
  *                            log2 of the block or cell side in pixels (4..8)
  *   RJ_TUNE_HYBRID_EXACT_SCALE classified grid of the hybrid join's exact

@@ -1039,7 +1039,10 @@ int label_map(rj_ctx* ctx, PolyPassArgs& a, const char* key, size_t npix, const 
 // below kTuneMinPoints take the default shape without timing anything.
 constexpr uint64_t kTuneMinPoints = 1ull << 22;
 constexpr uint64_t kTuneWarm = 1ull << 16, kTuneMost = 1ull << 27;   // points of the untimed and the timed launch
-constexpr int kMaxShapes = 11;   // shape indices rj_set_tuning takes (a pass without that shape runs its generic form)
+// Shape indices rj_set_tuning takes: those of the label pass when it had most.
+// Past its shapes the label pass chooses by itself, the others run their
+// generic form.
+constexpr int kMaxShapes = 11;
 inline int tune_bucket(double v) { return (int)std::floor(std::log2(std::max(v, 1.0))); }
 
 // Filters and aggregate of a query in the lean passes' form (interval
@@ -1481,9 +1484,12 @@ bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, co
     auto smem = [&](int sh, const LabelPointArgs& g) {
         return lp.tile ? label_tile_smem(sh, g.cell_words, a.P, lp.agg) : label_points_smem(sh, g.cell_words, a.P, lp.agg);
     };
+    // (an index past the shapes, as saved when there were more, does not force one)
+    const int nshapes = lp.tile ? label_tile_shapes() : label_shapes();
+    const int force = ctx->count_shape < nshapes ? ctx->count_shape : -1;
     for (size_t k = 0; k < lp.sides.size(); ++k)
-        for (int sh = 0; sh < (lp.tile ? label_tile_shapes() : label_shapes()); ++sh)
-            if ((ctx->count_shape < 0 || ctx->count_shape == sh) && smem(sh, lp.sides[k].a) <= 224 * 1024)
+        for (int sh = 0; sh < nshapes; ++sh)
+            if ((force < 0 || force == sh) && smem(sh, lp.sides[k].a) <= 224 * 1024)
                 lp.cands.push_back({sh, (int)k});
     if (lp.cands.empty()) return false;
     lp.small = a.n < kTuneMinPoints;
@@ -1491,7 +1497,7 @@ bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, co
     for (const auto& c : lp.cands) named.push_back({c.first, lp.tile ? lp.sides[(size_t)c.second].shift : c.second});
     std::snprintf(lp.key, sizeof lp.key, "label:%d:%d:%d:%d:%d:%d:%d:%d:%d:%llx", lp.lc.ncol, lp.lc.aggr, lp.lc.aggr_ci >= 0,
                   rp.splitx * rp.splity > 1, tune_bucket((double)a.P), tune_bucket(npx), tune_bucket((double)a.n),
-                  ctx->count_shape, ctx->count_bshift, (unsigned long long)cands_key(named));
+                  force, ctx->count_bshift, (unsigned long long)cands_key(named));
     lp.have = tuned_get(ctx, lp.key, &lp.tuned);
     return true;
 }

@@ -32,3 +32,31 @@ def test_forced_side(handler, res, shift, lean):
         handler.flags = 0
     np.testing.assert_array_equal(got.count, oracle.raster_join(xy, verts, pidx, ext / (res - 0.5))[0])
     assert ran == (shift if lean else -1)
+
+
+@pytest.mark.parametrize("cell,filters", [(100.0, False), (100.0, True), (5.0, False)])
+def test_shape_indices_past_the_shapes(handler, cell, filters):
+    """Indices that older libraries had shapes for still give a lean pass; others
+    are refused."""
+    verts, pidx = synth.voronoi_polygons(40, seed=5, verts_per_poly=30)
+    pts = synth.points(100_001, seed=82, columns=True)
+    dh = rj.DataHandler()
+    dh.add_column(1, rj.Location, pts["xy"])
+    dh.add_column(4, rj.Int, pts["f1"])
+    dh.setPolygons(verts, pidx)
+    if filters:
+        dh.setQueryConstraints([(4, rj.GTE, 2)])
+    handler.setDataHandler(dh)
+    handler.setCellSize(cell)
+    try:
+        want = handler.execute(rj.RasterJoinFn).count
+        for shape in range(11):
+            handler.setTuning(rj.TUNE_COUNT_SHAPE, shape)
+            np.testing.assert_array_equal(handler.execute(rj.RasterJoinFn).count, want)
+            ran = handler.getTuning(rj.TUNE_COUNT_SHAPE)
+            assert ran == shape if shape < 3 else ran >= 0
+        for shape in (-2, 11):
+            with pytest.raises(rj.RJError):
+                handler.setTuning(rj.TUNE_COUNT_SHAPE, shape)
+    finally:
+        handler.setTuning(rj.TUNE_COUNT_SHAPE, -1)
