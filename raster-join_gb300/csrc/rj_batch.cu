@@ -649,10 +649,7 @@ int run_fused(Engine& e, std::vector<QPlan>& plans, uint32_t flags, BatchOut& bo
             {
                 // canvas extent plus two pixels: a location outside it maps to
                 // no pixel of any tile (window range test and snapping)
-                const double mx = 2.0 * (p->ps->bbox[2] - p->ps->bbox[0]) / p->rp.actual_x + 1e-3;
-                const double my = 2.0 * (p->ps->bbox[3] - p->ps->bbox[1]) / p->rp.actual_y + 1e-3;
-                d.box = make_float4((float)(p->ps->bbox[0] - mx), (float)(p->ps->bbox[1] - my),
-                                    (float)(p->ps->bbox[2] + mx), (float)(p->ps->bbox[3] + my));
+                d.box = raster_reach(p->ps->bbox, p->rp);
                 // zone checks only when the query's reach misses part of the table
                 const float4 tb = ctx->table_box;
                 const bool covers = d.box.x <= tb.x && d.box.y <= tb.y && d.box.z >= tb.z && d.box.w >= tb.w;

@@ -271,6 +271,7 @@ struct RasterPlan {
     int resx = 1, resy = 1;
     std::vector<float4> colxf, rowxf;
 };
+float4 raster_reach(const double* bb, const RasterPlan& rp);
 int plan_raster_bbox(rj_ctx* ctx, const double* bbox, const rj_query* q, RasterPlan& rp);
 // identity of a canvas geometry (tiles, resolution, per-tile transforms)
 uint64_t canvas_key(const std::vector<float4>& colxf, const std::vector<float4>& rowxf, int resx, int resy);

@@ -197,6 +197,25 @@ int plan_raster_bbox(rj_ctx* ctx, const double* bbox, const rj_query* q, RasterP
     return RJ_OK;
 }
 
+// fp32 error in pixels of a window coordinate of one axis: each of its four
+// operations rounds once, s and t are rounded too, three roundings more for a
+// cell's edges (plan_label_points); and the snap's half step.
+double pixel_error(const std::vector<float4>& xf, double lo, double hi) {
+    double e = 0;
+    for (const float4& t : xf)
+        e = std::max(e, (double)t.z * (6.0 * std::fabs((double)t.x) * std::max(std::fabs(lo), std::fabs(hi)) + 16.0));
+    return e * std::ldexp(1.0, -23) + 1.0 / 256.0;
+}
+
+// The canvas, two pixels more and the pixels' error: locations outside reach no
+// pixel of any tile.
+float4 raster_reach(const double* bb, const RasterPlan& rp) {
+    const double mx = (2.0 + pixel_error(rp.colxf, bb[0], bb[2])) * (bb[2] - bb[0]) / rp.actual_x + 1e-3;
+    const double my = (2.0 + pixel_error(rp.rowxf, bb[1], bb[3])) * (bb[3] - bb[1]) / rp.actual_y + 1e-3;
+    return make_float4(std::nextafterf((float)(bb[0] - mx), -INFINITY), std::nextafterf((float)(bb[1] - my), -INFINITY),
+                       std::nextafterf((float)(bb[2] + mx), INFINITY), std::nextafterf((float)(bb[3] + my), INFINITY));
+}
+
 int plan_raster(rj_ctx* ctx, const rj_query* q, RasterPlan& rp) { return plan_raster_bbox(ctx, ctx->ps->bbox, q, rp); }
 
 uint64_t canvas_key(const std::vector<float4>& colxf, const std::vector<float4>& rowxf, int resx, int resy) {
@@ -1411,17 +1430,8 @@ bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, co
     a.zrow0 = pa.row0;
     a.qbox = pa.qbox;
     const double* bb = ctx->ps->bbox;
-    // fp32 error in pixels of the exact window coordinate (each of its four
-    // operations rounds once; s and t are rounded too) and of the cell edges'
-    // (three roundings more), plus the snap's half step; beyond half a pixel
-    // no cell is taken as uniform
-    auto err_of = [](const std::vector<float4>& xf, double lo, double hi) {
-        double e = 0;
-        for (const float4& t : xf)
-            e = std::max(e, (double)t.z * (6.0 * std::fabs((double)t.x) * std::max(std::fabs(lo), std::fabs(hi)) + 16.0));
-        return e * std::ldexp(1.0, -23) + 1.0 / 256.0;
-    };
-    const double ex = err_of(rp.colxf, bb[0], bb[2]), ey = err_of(rp.rowxf, bb[1], bb[3]);
+    // beyond half a pixel of fp32 error no cell is taken as uniform
+    const double ex = pixel_error(rp.colxf, bb[0], bb[2]), ey = pixel_error(rp.rowxf, bb[1], bb[3]);
     lp.errx = ex < 0.5 ? ex : 1e30;
     lp.erry = ey < 0.5 ? ey : 1e30;
     // Cell sides: about 64k or 16k cells (128 KB or 32 KB of codes), at least
@@ -1682,12 +1692,7 @@ int exec_raster(rj_ctx* ctx, const rj_query* q, ExecState& es, bool bounds) {
     const int T = rp.splitx * rp.splity;
     const size_t tile_px = (size_t)rp.resx * rp.resy;
     const size_t npix = tile_px * T;
-    {
-        // canvas plus two pixels: locations outside reach no pixel of any tile
-        const double* bb = ctx->ps->bbox;
-        const double mx = 2.0 * (bb[2] - bb[0]) / rp.actual_x + 1e-3, my = 2.0 * (bb[3] - bb[1]) / rp.actual_y + 1e-3;
-        ctx->qbox = make_float4((float)(bb[0] - mx), (float)(bb[1] - my), (float)(bb[2] + mx), (float)(bb[3] + my));
-    }
+    ctx->qbox = raster_reach(ctx->ps->bbox, rp);
 
     es.ph->mark(1);
     int2* wv;

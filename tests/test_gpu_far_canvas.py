@@ -56,3 +56,36 @@ def test_rim(handler, lo, ext, fbo):
     x = np.linspace(0.0, ext, 9)
     strips = np.concatenate([[(a, 0), (b, 0), (b, ext), (a, ext)] for a, b in zip(x[:-1], x[1:])])
     _run(handler, np.asarray((lo, lo)), ext, fbo, (strips, 4 * np.arange(9, dtype=np.int32)))
+
+
+@pytest.mark.parametrize("lo,ext,cell,fbo", [(37861176.0, 3417.0, 0.9, 1675), (39100696.0, 5340.0, 0.6, 1045),
+                                             (41181008.0, 4921.0, 0.7, 915)])
+def test_rim_rows_are_not_skipped(handler, lo, ext, cell, fbo):
+    """Whole zones of rows four metres off the canvas that fp32 puts on it, alone
+    and in a fused batch."""
+    x = np.linspace(0.0, ext, 9)
+    strips = np.concatenate([[(a, 0), (b, 0), (b, ext), (a, ext)] for a, b in zip(x[:-1], x[1:])])
+    verts = (strips + lo).astype(np.float32)
+    pidx = 4 * np.arange(9, dtype=np.int32)
+    rng = np.random.default_rng(fbo)
+    y = rng.uniform(lo, lo + ext, 50_000)
+    xy = np.r_[np.c_[np.full(20_000, lo - 4.0), y[:20_000]], np.c_[np.full(20_000, lo + ext + 4.0), y[20_000:40_000]],
+               np.c_[rng.uniform(lo, lo + ext, 10_000), y[40_000:]]].astype(np.float32)
+    dh = rj.DataHandler()
+    dh.add_column(1, rj.Location, xy)
+    dh.setPolygons(verts, pidx)
+    handler.setDataHandler(dh)
+    handler.setCellSize(cell)
+    handler.max_fbo_size = fbo
+    want = oracle.raster_join(xy, verts, pidx, cell, max_res=fbo)[0]
+    assert want.sum() > 15_000
+    try:
+        for flag in (0, rj.FLAG_FLAT_CANVAS, rj.FLAG_FORCE_CANVAS, rj.FLAG_TIERED_CANVAS):
+            handler.flags = flag
+            np.testing.assert_array_equal(handler.execute(rj.RasterJoinFn).count, want)
+        got = handler.execute_batch([handler.make_query(rj.RasterJoinFn)] * 2, [None] * 2, flags=rj.BATCH_FUSE_ALL)[0]
+        for g in got:
+            np.testing.assert_array_equal(g.count, want)
+    finally:
+        handler.flags = 0
+        handler.max_fbo_size = 8192
