@@ -1,6 +1,8 @@
 // rj_bands.cuh -- (edge, row) pairs of a band of pixel rows spread over a
 // warp's lanes (the polygon-side passes over outlines).
 #pragma once
+#include <climits>
+
 #include "rj_device.cuh"
 
 namespace rj {
@@ -58,12 +60,15 @@ struct BandItems {
 };
 
 // Edges of the ring pv[0, n) that meet the fixed-point rows [lo, hi], staged in
-// order (f(position, vertex, edge) for each that is taken); returns how many
-// there are.  Four rounds of vertices are loaded before the first is used.
+// order from vertex k0 on (f(position, vertex, edge) for each that is taken);
+// returns how many there are.  Four rounds of vertices are loaded before the
+// first is used; the last rounds are those after which there is no room for
+// another four, and k0 is left behind them.
 template <class F>
-__device__ __forceinline__ int stage_edges(const int2* __restrict__ pv, int n, int64_t lo, int64_t hi, int lane, F&& f) {
+__device__ __forceinline__ int stage_edges(const int2* __restrict__ pv, int n, int64_t lo, int64_t hi, int lane, int& k0,
+                                           int room, F&& f) {
     int nb = 0;
-    for (int k0 = 0; k0 < n; k0 += 128) {
+    for (; k0 < n && nb <= room - 128; k0 += 128) {
         int2 A[4], B[4];
         #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -84,6 +89,12 @@ __device__ __forceinline__ int stage_edges(const int2* __restrict__ pv, int n, i
         }
     }
     return nb;
+}
+
+template <class F>
+__device__ __forceinline__ int stage_edges(const int2* __restrict__ pv, int n, int64_t lo, int64_t hi, int lane, F&& f) {
+    int k0 = 0;
+    return stage_edges(pv, n, lo, hi, lane, k0, INT_MAX, f);
 }
 
 // f(q, r) for every row r of the ranges that range(e, q, r0, cnt) gives the

@@ -50,7 +50,14 @@ namespace {
 
 constexpr int kTW = 8;            // warps per block
 constexpr int kTBand = kBand;     // rows per work item: one block row
-constexpr int kTEdgeCap = 112;    // staged edges per warp (more: read from global memory)
+// Staged edges per warp.  Where a band has more, up to four times as many are
+// staged as vertex numbers and read from global memory; where it has more than
+// that, every sweep stages them anew, so many at a time.  (Going through all of
+// the polygon's edges instead, four rings of 160,000 vertices on 20,000 x 20,000
+// pixels, counts: 26.6 ms from 113 edges on, 13.6 from 257 on; now 8.1.  Shared
+// memory for 256 edges leaves three blocks per SM instead of four.)
+constexpr int kTEdgeCap = 112;
+constexpr int kTIndexCap = kTEdgeCap * (int)(sizeof(int4) / sizeof(int));
 constexpr int kTBW = 16;          // block-bitmap words per row: 512 block columns = 8192 pixels
 constexpr int kTList = 64;        // blocks whose pixels one round visits
 
@@ -81,6 +88,15 @@ __device__ __forceinline__ uint32_t prefix_xor(uint32_t x) {
     x ^= x << 8;
     x ^= x << 16;
     return x;
+}
+
+// The numbers of the edges' vertices, staged from k0 on; returns how many there
+// are and the vertex reached.  (A call, as few bands come here: inlined for
+// every sweep it cost 1B points at 1 m 6 to 10 us of 2513, so 2 to 6.)
+__device__ __noinline__ int2 stage_numbers(const int2* __restrict__ pv, int n, int64_t lo, int64_t hi, int k0, int room, int* index) {
+    const int m = stage_edges(pv, n, lo, hi, (int)(threadIdx.x & 31u), k0, room, [&](int pos, int k, const int4&) { index[pos] = k; });
+    __syncwarp();
+    return make_int2(m, k0);
 }
 
 template <int MODE>
@@ -120,17 +136,32 @@ __global__ void __launch_bounds__(kTW * 32, 4) k_tier_pass(PolyPassArgs a, TierA
         // stage the edges that can cross a row centre of the band
         const int64_t band_lo = (int64_t)jb * kSub - kSub;
         const int64_t band_hi = (int64_t)(jb + kTBand) * kSub + kSub;
+        int* index = reinterpret_cast<int*>(S.edge);
         const int nb = stage_edges(pv, n, band_lo, band_hi, lane, [&](int pos, int, const int4& e) {
             if (pos < kTEdgeCap) S.edge[pos] = e;
         });
-        const bool overflow = nb > kTEdgeCap;
-        const int ne = overflow ? n : nb;
+        const bool numbers = nb > kTEdgeCap, pieces = nb > kTIndexCap;
         __syncwarp();
+        if (numbers && !pieces) stage_numbers(pv, n, band_lo, band_hi, 0, INT_MAX, index);
         auto edge_at = [&](int e) -> int4 {
-            if (!overflow) return S.edge[e];
-            const int2 A = pv[e];
-            const int2 B = pv[(e + 1 == n) ? 0 : e + 1];
+            if (!numbers) return S.edge[e];
+            const int k = index[e];
+            const int2 A = pv[k];
+            const int2 B = pv[(k + 1 == n) ? 0 : k + 1];
             return make_int4(A.x, A.y, B.x, B.y);
+        };
+        // f(number of staged edges) until the band's edges are through
+        auto for_staged = [&](auto&& f) {
+            for (int k = pieces ? 0 : n, m = nb;;) {
+                if (pieces) {
+                    const int2 s = stage_numbers(pv, n, band_lo, band_hi, k, kTIndexCap, index);
+                    m = s.x;
+                    k = s.y;
+                }
+                f(m);
+                __syncwarp();
+                if (k >= n) break;
+            }
         };
         if (MODE == MODE_TIER_CLASSIFY && tr.outline) {
             // blocks within two pixels of an edge near this band (rows
@@ -138,33 +169,34 @@ __global__ void __launch_bounds__(kTW * 32, 4) k_tier_pass(PolyPassArgs a, TierA
             // reads per-pixel counts up to a pixel beside each edge, rows one
             // beyond the polygon's included
             const float ylo = (float)(jb - 2), yhi = (float)(jb + kTBand + 2);
-            for (int e = lane; e < ne; e += 32) {
-                const int4 q = edge_at(e);
-                const float ax = q.x * (1.0f / kSub), ay = q.y * (1.0f / kSub);
-                const float bx = q.z * (1.0f / kSub), by = q.w * (1.0f / kSub);
-                const float y0 = fmaxf(fminf(ay, by), ylo), y1 = fminf(fmaxf(ay, by), yhi);
-                if (!(y0 <= y1)) continue;
-                float x0, x1;
-                if (ay == by) {
-                    x0 = fminf(ax, bx);
-                    x1 = fmaxf(ax, bx);
-                } else {
-                    const float ta = fminf(fmaxf((y0 - ay) / (by - ay), 0.0f), 1.0f);
-                    const float tb = fminf(fmaxf((y1 - ay) / (by - ay), 0.0f), 1.0f);
-                    const float xa = ax + (bx - ax) * ta, xb = ax + (bx - ax) * tb;
-                    x0 = fminf(xa, xb);
-                    x1 = fmaxf(xa, xb);
+            for_staged([&](int ne) {
+                for (int e = lane; e < ne; e += 32) {
+                    const int4 q = edge_at(e);
+                    const float ax = q.x * (1.0f / kSub), ay = q.y * (1.0f / kSub);
+                    const float bx = q.z * (1.0f / kSub), by = q.w * (1.0f / kSub);
+                    const float y0 = fmaxf(fminf(ay, by), ylo), y1 = fminf(fmaxf(ay, by), yhi);
+                    if (!(y0 <= y1)) continue;
+                    float x0, x1;
+                    if (ay == by) {
+                        x0 = fminf(ax, bx);
+                        x1 = fmaxf(ax, bx);
+                    } else {
+                        const float ta = fminf(fmaxf((y0 - ay) / (by - ay), 0.0f), 1.0f);
+                        const float tb = fminf(fmaxf((y1 - ay) / (by - ay), 0.0f), 1.0f);
+                        const float xa = ax + (bx - ax) * ta, xb = ax + (bx - ax) * tb;
+                        x0 = fminf(xa, xb);
+                        x1 = fmaxf(xa, xb);
+                    }
+                    const int c0 = max((int)floorf(x0) - 2, 0), c1 = min((int)floorf(x1) + 2, a.resx - 1);
+                    const int r0 = max((int)floorf(y0) - 2, 0), r1 = min((int)floorf(y1) + 2, a.resy - 1);
+                    if (c0 > c1 || r0 > r1) continue;
+                    const size_t tile0 = (size_t)t * tr.bw * tr.bh;
+                    for (int br2 = r0 >> 4; br2 <= (r1 >> 4); ++br2)
+                        for (int bc = c0 >> 4; bc <= (c1 >> 4); ++bc) tr.mixed[tile0 + (size_t)br2 * tr.bw + bc] = 1u;
                 }
-                const int c0 = max((int)floorf(x0) - 2, 0), c1 = min((int)floorf(x1) + 2, a.resx - 1);
-                const int r0 = max((int)floorf(y0) - 2, 0), r1 = min((int)floorf(y1) + 2, a.resy - 1);
-                if (c0 > c1 || r0 > r1) continue;
-                const size_t tile0 = (size_t)t * tr.bw * tr.bh;
-                for (int br2 = r0 >> 4; br2 <= (r1 >> 4); ++br2)
-                    for (int bc = c0 >> 4; bc <= (c1 >> 4); ++bc) tr.mixed[tile0 + (size_t)br2 * tr.bw + bc] = 1u;
-            }
+            });
         }
 
-        __syncwarp();                                   // staged edges read; the next item restages them
         if (nbc <= 0) continue;                         // outline rows only
 
         // rows of the band inside the polygon's crossing rows and the canvas
@@ -173,19 +205,20 @@ __global__ void __launch_bounds__(kTW * 32, 4) k_tier_pass(PolyPassArgs a, TierA
         if (!live) continue;
 
         // sweep 1: block toggles and inside-crossing flags per live row
-        for_edge_rows(ne, jb, lane, edge_at, [&](const int4& q, int r) {
-            const int32_t cy = (jb + r) * kSub + kSub / 2;
-            if (!((live >> r) & 1u) || !cross_row(q.y, q.w, cy)) return;
-            const int L = max(cross_L(q.x, q.y, q.z, q.w, cy), i_lo);
-            if (L > i_hi) return;
-            const int rb = ((L + 15) >> 4) - bc_lo;
-            if (rb < nbc) atomicXor(&S.X[r * kTBW + (rb >> 5)], 1u << (rb & 31));
-            if (L & 15) {
-                const int cb = (L >> 4) - bc_lo;
-                atomicOr(&S.C[r * kTBW + (cb >> 5)], 1u << (cb & 31));
-            }
+        for_staged([&](int ne) {
+            for_edge_rows(ne, jb, lane, edge_at, [&](const int4& q, int r) {
+                const int32_t cy = (jb + r) * kSub + kSub / 2;
+                if (!((live >> r) & 1u) || !cross_row(q.y, q.w, cy)) return;
+                const int L = max(cross_L(q.x, q.y, q.z, q.w, cy), i_lo);
+                if (L > i_hi) return;
+                const int rb = ((L + 15) >> 4) - bc_lo;
+                if (rb < nbc) atomicXor(&S.X[r * kTBW + (rb >> 5)], 1u << (rb & 31));
+                if (L & 15) {
+                    const int cb = (L >> 4) - bc_lo;
+                    atomicOr(&S.C[r * kTBW + (cb >> 5)], 1u << (cb & 31));
+                }
+            });
         });
-        __syncwarp();
         // block columns [fb, lb] lie wholly inside [i_lo, i_hi]; word hw's valid blocks
         const int fb = ((i_lo + 15) >> 4) - bc_lo, lb = ((i_hi + 1) >> 4) - 1 - bc_lo;
         const int wa = max(fb - hw * 32, 0), wb = min(lb - hw * 32 + 1, 32);
@@ -296,15 +329,16 @@ __global__ void __launch_bounds__(kTW * 32, 4) k_tier_pass(PolyPassArgs a, TierA
             __syncwarp();
             // sweep 2: pixel toggles of the listed blocks (crossings inside a
             // block only; one at a block's first pixel is in X already)
-            for_edge_rows(ne, jb, lane, edge_at, [&](const int4& q, int r) {
-                const int32_t cy = (jb + r) * kSub + kSub / 2;
-                if (!((live >> r) & 1u) || !cross_row(q.y, q.w, cy)) return;
-                const int L = max(cross_L(q.x, q.y, q.z, q.w, cy), i_lo);
-                if (L > i_hi || !(L & 15)) return;
-                const int k = S.map[(L >> 4) - bc_lo];
-                if (k != 0xFF) atomicXor(&S.M[k * 8 + (r >> 1)], (1u << (L & 15)) << ((r & 1) * 16));
+            for_staged([&](int ne) {
+                for_edge_rows(ne, jb, lane, edge_at, [&](const int4& q, int r) {
+                    const int32_t cy = (jb + r) * kSub + kSub / 2;
+                    if (!((live >> r) & 1u) || !cross_row(q.y, q.w, cy)) return;
+                    const int L = max(cross_L(q.x, q.y, q.z, q.w, cy), i_lo);
+                    if (L > i_hi || !(L & 15)) return;
+                    const int k = S.map[(L >> 4) - bc_lo];
+                    if (k != 0xFF) atomicXor(&S.M[k * 8 + (r >> 1)], (1u << (L & 15)) << ((r & 1) * 16));
+                });
             });
-            __syncwarp();
             // row masks: coverage at the block's first pixel, then the block's
             // own crossings, clipped to [i_lo, i_hi]
             for (int w = lane; w < nk * 8; w += 32) {
