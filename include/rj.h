@@ -285,7 +285,7 @@ RJ_API int rj_column_absmax(const rj_ctx *ctx, int32_t attrib_id, double *out);
  *                            pipeline, 3 = 4 points x 512 threads
  *   RJ_TUNE_COUNT_SHAPE      lean raster label pass (polygons that do not
  *                            overlap, a resident table): -1 = autotuned (each
- *                            shape is timed once per context and query
+ *                            shape is timed once per process and query
  *                            class on the table itself, the fastest is
  *                            kept), else a shape index
  *                            0..rj_get_tuning(RJ_TUNE_COUNT_SHAPES)-1
@@ -294,11 +294,12 @@ RJ_API int rj_column_absmax(const rj_ctx *ctx, int32_t attrib_id, double *out);
  *                            log2 of the block or cell side in pixels (4..8)
  *   RJ_TUNE_HYBRID_EXACT_SCALE classified grid of the hybrid join's exact
  *                            tests: the query grid refined 1, 2 or 4 times
- *   RJ_TUNE_COUNT_SHAPES     (read only) number of plain count-pass shapes
- *   RJ_TUNE_LEAN_SHAPES      (read only) number of shapes of the same pass
- *                            with filters (interval form, <= 4 columns) or
- *                            a summed aggregate; RJ_TUNE_COUNT_SHAPE indexes
- *                            the shapes of the form the query takes
+ *   RJ_TUNE_COUNT_SHAPES     (read only) number of shapes of that pass over
+ *                            one tile without filters (count or sum)
+ *   RJ_TUNE_LEAN_SHAPES      (read only) number of its shapes with filters
+ *                            (interval form, <= 4 columns) or over several
+ *                            tiles; RJ_TUNE_COUNT_SHAPE indexes the shapes of
+ *                            the form the query takes
  *   RJ_TUNE_SPLAT_SHAPES     (read only) number of shapes of the lean pass
  *                            onto a point canvas (one canvas tile: polygon
  *                            sets that overlap on it, the error-bounds

@@ -10,7 +10,7 @@
 // k_poly_bands: one warp per (tile, polygon, band of 16 rows).
 //   * the band's edges are staged in shared memory;
 //   * the (edge, row) crossings of the whole band are spread over the lanes
-//     (one exact division each) and kept in lists, one per row;
+//     (one exact crossing each) and kept in lists, one per row;
 //   * spans: the sorted crossings c0 <= c1 <= ... of a row bound the spans
 //     [c0, c1), [c2, c3), ...; a crossing's contribution to the sum is its
 //     prefix with the sign of its rank's parity, which the lane finds by

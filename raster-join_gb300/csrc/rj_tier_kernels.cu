@@ -20,7 +20,7 @@
 // to the blocks the polygon's outline passes through (plus one entry per full
 // block), not to the pixels of its area:
 //   * the band's (edge, row) crossing pairs are spread over the lanes, one
-//     exact division each;
+//     exact crossing each;
 //   * sweep 1 -- every crossing of a live row toggles one bit of a per-row
 //     block bitmap (at the first block whose first pixel lies at or right of
 //     it) and, when it falls strictly inside a block, flags that block; a
