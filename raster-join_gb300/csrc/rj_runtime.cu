@@ -1215,12 +1215,13 @@ int hybrid_lean_pass(rj_ctx* ctx, const DevFilter& f, int mode, const HybXf& h, 
             }
     if (cands.empty()) return RJ_OK;
     char key[200];
-    std::snprintf(key, sizeof key, "hybq:%d:%d:%d:%d:%d:%d:%d:%d:%d:%llx", mode, lc.ncol, lc.aggr, lc.aggr_ci >= 0,
-                  tune_bucket((double)P), tune_bucket((double)resx * resy), tune_bucket((double)a.n), ctx->count_shape,
-                  ctx->count_bshift, (unsigned long long)cands_key(cands));
+    const bool small = a.n < kTuneMinPoints;   // (no choice is kept for such a class: no key)
+    if (!small)
+        std::snprintf(key, sizeof key, "hybq:%d:%d:%d:%d:%d:%d:%d:%d:%d:%llx", mode, lc.ncol, lc.aggr, lc.aggr_ci >= 0,
+                      tune_bucket((double)P), tune_bucket((double)resx * resy), tune_bucket((double)a.n), ctx->count_shape,
+                      ctx->count_bshift, (unsigned long long)cands_key(cands));
     int tuned_i = -1;
-    const bool have = tuned_get(ctx, key, &tuned_i);
-    const bool small = a.n < kTuneMinPoints;
+    const bool have = !small && tuned_get(ctx, key, &tuned_i);
     const bool known = cands.size() == 1 || have || small;
     int rc;
     std::map<int, uint16_t*> codes;
@@ -1254,7 +1255,7 @@ int hybrid_lean_pass(rj_ctx* ctx, const DevFilter& f, int mode, const HybXf& h, 
     LeanCols tl = lc;
     tl.out_sum = tsum;
     tl.nonfinite = tnf;
-    const int pi = small && !have ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i, uint64_t most) {
+    const int pi = small ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i, uint64_t most) {
         HybLeanArgs b = args_for(cands[i].second);
         b.out_count = tout;
         b.n = std::min<uint64_t>(a.n & ~1ULL, most);
@@ -1339,15 +1340,15 @@ int splat_lean_pass(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, uint3
     }
     if (cands.empty()) return RJ_OK;
     char key[200];
-    std::vector<std::pair<int, int>> named;
-    for (int sh : cands) named.push_back({sh, 0});
-    std::snprintf(key, sizeof key, "splat:%d:%d:%d:%d:%d:%d:%llx", lc.ncol, lc.aggr, lc.aggr_ci >= 0,
-                  tune_bucket((double)npix), tune_bucket((double)a.n), ctx->count_shape, (unsigned long long)cands_key(named));
-    int tuned_i = -1;
-    const bool have = tuned_get(ctx, key, &tuned_i);
-    const bool small = a.n < kTuneMinPoints;
+    const bool small = a.n < kTuneMinPoints;   // (no key, as above)
+    if (!small) {
+        std::vector<std::pair<int, int>> named;
+        for (int sh : cands) named.push_back({sh, 0});
+        std::snprintf(key, sizeof key, "splat:%d:%d:%d:%d:%d:%d:%llx", lc.ncol, lc.aggr, lc.aggr_ci >= 0,
+                      tune_bucket((double)npix), tune_bucket((double)a.n), ctx->count_shape, (unsigned long long)cands_key(named));
+    }
     bool timed_any = false;
-    const int pi = small && !have ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i, uint64_t most) {
+    const int pi = small ? 0 : tune_pick(ctx, key, cands.size(), [&](size_t i, uint64_t most) {
         timed_any = true;
         SplatLeanArgs b = a;
         b.n = std::min<uint64_t>(a.n & ~1ULL, most);
@@ -1502,6 +1503,7 @@ bool plan_label_points(rj_ctx* ctx, const DevFilter& f, const RasterPlan& rp, co
                 lp.cands.push_back({sh, (int)k});
     if (lp.cands.empty()) return false;
     lp.small = a.n < kTuneMinPoints;
+    if (lp.small) return true;   // (no key, as above)
     std::vector<std::pair<int, int>> named;   // (shape, side in pixels for blocks, else finer or coarser)
     for (const auto& c : lp.cands) named.push_back({c.first, lp.tile ? lp.sides[(size_t)c.second].shift : c.second});
     std::snprintf(lp.key, sizeof lp.key, "label:%d:%d:%d:%d:%d:%d:%d:%d:%d:%llx", lp.lc.ncol, lp.lc.aggr, lp.lc.aggr_ci >= 0,
