@@ -1622,10 +1622,12 @@ int label_blocks(rj_ctx* ctx, const DevFilter& f, const CanvasXf& cx, PolyPassAr
     }
     bool lean = false;
     if ((rc = run_label_points(ctx, lp, tr, es, &lean))) return rc;
-    if (!lean)
+    if (!lean) {
+        es.ph->mark(2);   // (run_label_points may have come to nothing before its own)
         rc = point_pass(ctx, f, es.out_count, es.out_sum, [&](const PointArgs& pa) {
             launch_tier_label_points(pa, cx, tr, ctx->sms, ctx->stream);
         });
+    }
     return rc;
 }
 

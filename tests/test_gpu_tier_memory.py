@@ -110,3 +110,40 @@ def test_one_tile_budget_of_the_flat_map(built, overlap, mb):
     assert got[0].count.sum() > 4900
     for g in got[1:]:
         np.testing.assert_array_equal(g.count, got[0].count)
+
+
+def test_phase_times_without_room_for_the_block_codes(built):
+    """Tables that leave room for the blocks of 4000 x 4000 pixels, for these
+    without the 125 KB of their codes, or for the flat label map only: the same
+    counts, and the phases are timed, call after call."""
+    polys = [np.array([[x, y], [x + 500, y], [x + 500, y + 500], [x, y + 500]]) for x in range(0, 4000, 500)
+             for y in range(0, 4000, 500)]
+    verts = np.concatenate(polys).astype(np.float32)
+    pidx = 4 * np.arange(len(polys) + 1, dtype=np.int32)
+    rows = range(1_030_000, 1_180_000, 12_288)   # 96 KB each
+    xy = np.random.default_rng(5).uniform(1, 3999, (rows[-1], 2)).astype(np.float32)
+    lean = []
+    for n in rows:
+        got = []
+        for budget in (0, 40):
+            h = rj.GLHandler(gpu_mem_mb=budget)
+            try:
+                dh = rj.DataHandler()
+                dh.add_column(1, rj.Location, xy[:n])
+                dh.setPolygons(verts, pidx)
+                h.setDataHandler(dh)
+                h.setCellSize(1.0)
+                h.flags = rj.FLAG_FLAT_CANVAS | rj.FLAG_PHASE_TIMING
+                h.setTuning(rj.TUNE_COUNT_BLOCK_SHIFT, 4)
+                for _ in range(3):
+                    got.append(h.execute(rj.RasterJoinFn))
+                    t = h.timings()
+                    assert t["poly_render_ms"] > 0 and t["pt_render_ms"] > 0
+                if budget:
+                    lean.append(h.getTuning(rj.TUNE_COUNT_SHAPE) >= 0)
+            finally:
+                h.close()
+        assert got[0].count.sum() >= n
+        for g in got[1:]:
+            np.testing.assert_array_equal(g.count, got[0].count)
+    assert lean[0] and not lean[-1]
